@@ -1,5 +1,7 @@
-// batch.cu -- cyc_batch_fit: many fits sharing one dataset, advanced
-// coordinate by coordinate in one persistent kernel (lr, pr, clr, cpr).
+// batch.cu -- cyc_batch_fit: many fits sharing one dataset in one persistent
+// launch: one fit to a cluster (ccd.cu; lr, pr, clr, cpr), or, where the fits
+// outnumber what the device holds that way (see run_batch), eight fits to a
+// group advanced together coordinate by coordinate (k_batch below; lr, pr).
 //
 // The reference runs such fits (CV folds x prior grid, bootstrap replicates)
 // as independent CyclicCoordinateDescent clones on CPU threads
@@ -7,11 +9,10 @@
 // runs the serial coordinate loop of findMode
 // (src/cyclops/CyclicCoordinateDescent.cpp:1008-1021).
 //
-// Layout and schedule (B200):
-//  * fits are packed G to a group; a group is one thread-block cluster of C
-//    CTAs; the cluster's CTAs split the rows into C contiguous ranges
-//    (aligned to strata for clr/cpr), so the per-row state a CTA touches is
-//    its own and only the per-fit (gradient, Hessian) partials cross CTAs,
+// Layout and schedule of k_batch (B200):
+//  * fits are packed G = 8 to a group; a group is one thread-block cluster of
+//    C CTAs; the cluster's CTAs split the rows into C contiguous ranges, so
+//    the per-row state a CTA touches is its own and only the per-fit (gradient, Hessian) partials cross CTAs,
 //    through distributed shared memory, once per coordinate;
 //  * per-(row, fit) state is the linear predictor only, stored
 //    xb[group][row][G] so the G fits of one row share one 32-byte sector
@@ -38,7 +39,8 @@
 #include <vector>
 
 #include "engine.cuh"
-#include "solver_common.cuh"
+#include "ccd.cuh"
+#include "row_terms.cuh"
 #include "variance_search.h"
 
 namespace cg = cooperative_groups;
@@ -53,7 +55,7 @@ constexpr int kMaxC = 8;          // CTAs per cluster (portable limit)
 constexpr int kAsyncBytes = 32768;
 
 struct BatchArgs {
-    int model, K, J, S, C;
+    int model, K, J, C;
     const int* fmt;
     const long long* col_ptr;
     const long long* val_ptr;
@@ -62,18 +64,12 @@ struct BatchArgs {
     const int* split;             // J x (C+1): first entry of rank r's rows, relative to the column
     const int* rpart;             // C+1 row boundaries
     const double* y;
-    const int* strat;             // K (grouped)
-    const int* strat_ptr;         // S+1 (grouped)
     const int* fixb;              // J
     const unsigned char* lane_fix; // [groups][J]: fits (bit f) holding column j at its value in this
                                   // launch (the inactive columns of the KKT swindle), or null
     const int* ptype;             // J
     void* xb;                     // [groups][K][G] T
-    int xb_smem;                  // one-fit groups: a CTA keeps its rows' linear predictors in shared
-                                  // memory when they fit (the capacity in rows), 0 = global memory
     const void* w;                // [groups][K][G] T
-    double* denom;                // grouped: [groups][S][G]
-    const double* nw;             // grouped: [groups][S][G]
     const double* xjy;            // [F][J]
     double* beta;                 // [F][J]
     double* hdelta;               // [F][J]
@@ -99,30 +95,6 @@ struct BatchArgs {
     unsigned long long* counters; // [3 + groups]: grad fit-entries, update fit-entries, steps, then
                                   // per group the bytes of row ids / values it streamed
 };
-
-template <class T>
-struct Kahan {
-    T s = 0, c = 0;
-    __device__ __forceinline__ void add(T v) {
-        const T yv = v - c;
-        const T t = s + yv;
-        c = (t - s) - yv;
-        s = t;
-    }
-    __device__ __forceinline__ double value() const { return (double)s - (double)c; }
-};
-
-template <>
-struct Kahan<double> {
-    double s = 0;
-    __device__ __forceinline__ void add(double v) { s += v; }
-    __device__ __forceinline__ double value() const { return s; }
-};
-
-__device__ __forceinline__ float fexp(float x) { return __expf(x); }
-__device__ __forceinline__ double fexp(double x) { return exp(x); }
-__device__ __forceinline__ float flog(float x) { return __logf(x); }
-__device__ __forceinline__ double flog(double x) { return log(x); }
 
 // sum (a, b) over the CTA's slots that share this thread's fit lane; result
 // for lane f lands in out[f] (threads < G then read it)
@@ -155,8 +127,7 @@ __device__ __forceinline__ T row_weight(const T* wg, const signed char* fold, in
 }
 
 template <class T, int MODEL, int G, int WM>
-__device__ __forceinline__ double objective_partial(const BatchArgs& A, int grp, int r0, int r1, int s0, int s1,
-                                                    const T* xbg, const T* wg, int fitfold, int fl, bool use_ll) {
+__device__ __forceinline__ double objective_partial(const BatchArgs& A, int grp, int r0, int r1, const T* xbg, const T* wg, int fitfold, int fl, bool use_ll) {
     Kahan<double> acc;
     const int slot = threadIdx.x / G, nslots = kBT / G;
     for (int k = r0 + slot; k < r1; k += nslots) {
@@ -173,58 +144,8 @@ __device__ __forceinline__ double objective_partial(const BatchArgs& A, int grp,
             acc.add(c);
         }
     }
-    if (use_ll && (MODEL == CYC_CLR || MODEL == CYC_CPR)) {
-        const double* dg = A.denom + (size_t)grp * A.S * G;
-        const double* ng = A.nw + (size_t)grp * A.S * G;
-        for (int s = s0 + slot; s < s1; s += nslots) acc.add(-ng[(size_t)s * G + fl] * log(dg[(size_t)s * G + fl]));
-    }
     return acc.value();
 }
-
-// per-row contribution to (gradient, Hessian) of an independent-rows model
-// (Logistic / PoissonRegression::incrementGradientAndHessian,
-// ModelSpecifics.h:540-568, 1508-1543); the logistic probability is formed as
-// 1 / (1 + exp(-xb)), which equals exb / (1 + exb) without overflowing
-// the row's mean under the model: the logistic probability, or exp(xb)
-template <class T, int MODEL>
-__device__ __forceinline__ T row_mean(T v) {
-    if (MODEL == CYC_LR) return T(1) / (T(1) + fexp(-v));
-    return fexp(v);
-}
-
-// (gradient, Hessian) terms of one entry from its row's mean
-template <class T, int MODEL>
-__device__ __forceinline__ void mean_terms(T m, T x, T wt, bool ind, T& gi, T& hi) {
-    if (MODEL == CYC_LR) {
-        const T g1 = m * x;
-        gi = wt * g1;
-        hi = wt * (ind ? g1 * (T(1) - g1) : x * x * m * (T(1) - m));
-    } else {
-        const T n1 = m * x;
-        gi = wt * n1;
-        hi = wt * (ind ? n1 : n1 * x);
-    }
-}
-
-template <class T, int MODEL>
-__device__ __forceinline__ void row_terms(T v, T x, T wt, bool ind, T& gi, T& hi) {
-    mean_terms<T, MODEL>(row_mean<T, MODEL>(v), x, wt, ind, gi, hi);
-}
-
-// (callers skip rows of weight zero: their terms are exactly zero, and the
-// exp() they would cost is the FP64 pipe's largest load)
-template <class T, int MODEL>
-__device__ __forceinline__ void row_gh(T v, T x, T wt, bool ind, Kahan<T>& ag, Kahan<T>& ah) {
-    T gi, hi;
-    row_terms<T, MODEL>(v, x, wt, ind, gi, hi);
-    ag.add(gi);
-    ah.add(hi);
-}
-
-// xb + delta * x as one fused multiply-add, the same wherever a batch
-// replays an update (the owning CTA and every CTA's copy of a shared row)
-__device__ __forceinline__ float upd_fma(float d, float x, float v) { return __fmaf_rn(d, x, v); }
-__device__ __forceinline__ double upd_fma(double d, double x, double v) { return __fma_rn(d, x, v); }
 
 // N consecutive values of one row of the [K][G] layout (16-byte aligned
 // when N * sizeof(T) is a multiple of 16)
@@ -682,30 +603,17 @@ __device__ __forceinline__ void cache_update(const BatchCache<T, G>& bc, T* xbg,
     }
 }
 
-// Items of one coordinate a thread keeps in registers between the gradient
-// and the update: columns with at most kRegItems * (kBT / G) entries in this
-// CTA's rows take this path (one load round trip, no reload for the update);
-// longer ones stream through twice.
-constexpr int kRegItems = 8;
 // coordinates staged in shared memory at a time
 constexpr int kChunk = 128;
 // row ids of short columns staged per chunk (dynamic shared memory)
 constexpr int kStage = 4096;
 
-// Columns processed together: consecutive short columns whose rows are
-// pairwise disjoint (planned on the host, ConflictFreeRuns) form a run of at
-// most kRunMax columns.  For independent-rows models the gradient of a column
-// depends only on the linear predictor of its own rows, so the columns of a
-// run see exactly the state the serial coordinate loop would show them, and
-// their updates touch disjoint rows: the run gives the serial CCD result while
-// paying for one load round trip and one cluster barrier.  Warp w of every
-// CTA takes column w of the run.
+// Columns processed together: consecutive short columns form a batch of at
+// most kRunMax; warp w of every CTA takes column w of the batch, and the batch
+// pays for one load round trip and one cluster barrier.
 constexpr int kRunMax = kBT / 32;
-// entries per slot of a run column (a warp has 32/G slots)
-constexpr int kRunItems = 8;
-// With G = 8 fits per group (independent-rows models) a batch may share rows
-// between its columns: at most kDirtyMax such rows, replayed serially (see
-// k_batch).  Columns of at most kBatchCap entries in every CTA's rows join.
+// A batch may share rows between its columns: at most kDirtyMax such rows,
+// replayed serially (see k_batch).  Columns of at most kBatchCap entries in every CTA's rows join.
 constexpr int kDirtyMax = 32;
 constexpr int kBatchCap = 256;
 
@@ -722,14 +630,6 @@ struct BatchShape {
 // levels of the serial replay a batch may have (each costs a step chain)
 constexpr int kLevelMax = kRunMax;
 
-// 8-fit groups of independent-rows models take the thread-per-row paths
-template <int MODEL, int G>
-constexpr bool row_stream() { return G == 8 && MODEL != CYC_CLR && MODEL != CYC_CPR; }
-
-// bytes after the staged row ids: staged values, or the cp.async row slots
-template <class T, int MODEL, int G>
-constexpr size_t staged_value_bytes() { return row_stream<MODEL, G>() ? (size_t)kAsyncBytes : kStage * sizeof(T); }
-
 template <class T, int MODEL, int G, int WM>
 __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
     cg::cluster_group cluster = cg::this_cluster();
@@ -737,25 +637,14 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
     const int rank = (int)cluster.block_rank();
     const int grp = blockIdx.x / C;
     const int r0 = A.rpart[rank], r1 = A.rpart[rank + 1];
-    const bool grouped = (MODEL == CYC_CLR || MODEL == CYC_CPR);
-    // independent rows, 8 fits per group: columns stream thread per row (all
-    // fits of a row by vector loads) and short columns go in batches
-    constexpr bool kRowStream = row_stream<MODEL, G>();
+    // columns stream thread per row (all fits of a row by vector loads) and
+    // short columns go in batches
     using LayW = RowLayout<T, G, false>;   // a warp per column (batches)
     using LayB = RowLayout<T, G, true>;    // the CTA per column (single columns)
-    // strata of my rows (partition boundaries are stratum starts); none if my range is empty
-    const int s0 = (grouped && r0 < r1) ? A.strat[r0] : 0;
-    const int s1 = (grouped && r0 < r1) ? (r1 >= A.K ? A.S : A.strat[r1]) : 0;
     T* xbg = (T*)A.xb + (size_t)grp * A.K * G;
     const T* wg = (WM == 0) ? (const T*)A.w + (size_t)grp * A.K * G : nullptr;
-    double* dg = grouped ? A.denom + (size_t)grp * A.S * G : nullptr;
-    const double* ng = grouped ? A.nw + (size_t)grp * A.S * G : nullptr;
     const int fl = threadIdx.x % G;
-    const int slot = threadIdx.x / G;
-    constexpr int NS = kBT / G;
-    constexpr int WS = 32 / G;                // slots per warp
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wslot = lane / G;
     const int fg = grp * G;                   // first fit of the group
     const int fitfold = (WM == 1) ? A.fitfold[fg + fl] : 0;
 
@@ -765,7 +654,6 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
     __shared__ double2 s_scr[kBT / 32][G];
     __shared__ double2 s_red[G];
     __shared__ double s_obj[2][kMaxC][G];
-    __shared__ double s_delta[G];
     __shared__ double s_dr[kRunMax][G];
     __shared__ double s_last[G];
     __shared__ int s_done[G];
@@ -799,31 +687,18 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
     double (*c_hd)[G] = reinterpret_cast<double (*)[G]>(dyn_smem + kChunk * G * sizeof(double));
     double (*c_xjy)[G] = reinterpret_cast<double (*)[G]>(dyn_smem + 2 * kChunk * G * sizeof(double));
     int* s_sidx = reinterpret_cast<int*>(dyn_smem + 3 * kChunk * G * sizeof(double));
-    // staged values of short sparse columns (per-lane paths), or, for 8-fit
-    // groups of independent-rows models, each thread's cp.async row slots
-    T* s_sx = reinterpret_cast<T*>(dyn_smem + 3 * kChunk * G * sizeof(double) + kStage * sizeof(int));
-    T* s_abuf = s_sx + (size_t)threadIdx.x * LayB::D * LayB::FPT;
-    // the batch cache (8-fit groups of independent-rows models) shares those bytes
-    const BatchCache<T, kRowStream ? G : 8> bcache(s_sx);
+    // each thread's cp.async row slots; the batch cache shares those bytes
+    T* s_slots = reinterpret_cast<T*>(dyn_smem + 3 * kChunk * G * sizeof(double) + kStage * sizeof(int));
+    T* s_abuf = s_slots + (size_t)threadIdx.x * LayB::D * LayB::FPT;
+    const BatchCache<T, G> bcache(s_slots);
     // shared rows of the open batch: as pushed by their owners (by parity; the
     // replay then moves this CTA's copy of the current parity in place), their
     // model means at the batch's start and now, and their weights
-    T* s_dirty = reinterpret_cast<T*>(reinterpret_cast<unsigned char*>(s_sx) + staged_value_bytes<T, MODEL, G>());
+    T* s_dirty = reinterpret_cast<T*>(reinterpret_cast<unsigned char*>(s_slots) + kAsyncBytes);
     T (*s_dst)[kDirtyMax][G] = reinterpret_cast<T (*)[kDirtyMax][G]>(s_dirty);
     T (*s_m0)[G] = reinterpret_cast<T (*)[G]>(s_dirty + 2 * kDirtyMax * G);
     T (*s_mc)[G] = reinterpret_cast<T (*)[G]>(s_dirty + 3 * kDirtyMax * G);
     T (*s_dw)[G] = reinterpret_cast<T (*)[G]>(s_dirty + 4 * kDirtyMax * G);
-    // one-fit groups whose rows fit: the CTA's linear predictors live in
-    // shared memory for the launch (every access to them is of the CTA's own
-    // rows), loaded here and written back at the end; xbg then addresses
-    // them by absolute row
-    T* const xb_global = xbg;
-    T* const s_xb = s_dirty + 5 * kDirtyMax * G;
-    const bool xb_local = (G == 1) && A.xb_smem > 0 && (r1 - r0) <= A.xb_smem;
-    if (xb_local) {
-        for (int i = threadIdx.x; i < r1 - r0; i += kBT) s_xb[i] = xb_global[r0 + i];
-        xbg = s_xb - r0;                 // rows r0 .. r1 - 1 only
-    }
 
     const bool use_ll = (A.conv == CYC_CONV_MITTAL || A.conv == CYC_CONV_LANGE);
     if (threadIdx.x < G) {
@@ -845,7 +720,7 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
     // initial objective (findMode :949-953)
     int opar = 0;
     {
-        const double p = objective_partial<T, MODEL, G, WM>(A, grp, r0, r1, s0, s1, xbg, wg, fitfold, fl, use_ll);
+        const double p = objective_partial<T, MODEL, G, WM>(A, grp, r0, r1, xbg, wg, fitfold, fl, use_ll);
         block_reduce_lanes<G>(p, 0.0, s_red, s_scr);
         if (threadIdx.x < G)
             for (int r = 0; r < C; ++r) *cluster.map_shared_rank(&s_obj[opar][rank][threadIdx.x], r) = s_red[threadIdx.x].x;
@@ -854,7 +729,7 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
             const int f = fg + threadIdx.x;
             double o = 0.0;
             for (int r = 0; r < C; ++r) o += s_obj[opar][r][threadIdx.x];
-            if (use_ll && (MODEL == CYC_PR || MODEL == CYC_CPR)) o += A.llfixed[f];
+            if (use_ll && MODEL == CYC_PR) o += A.llfixed[f];
             if (A.conv == CYC_CONV_LANGE) {
                 const double* bf = A.beta + (size_t)f * A.J;
                 for (int j = 0; j < A.J; ++j) o += log_density(A.ptype[j], A.variance[f], bf[j]);
@@ -864,7 +739,6 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
         opar ^= 1;
     }
     __syncthreads();
-    bool done_l = s_done[fl] != 0;   // this thread's fit lane has converged
     unsigned done_m = 0;             // all converged fits of the group (bit f)
     for (int f = 0; f < G; ++f) done_m |= (s_done[f] ? 1u : 0u) << f;
     const double var_l = A.variance[fg + fl];
@@ -945,7 +819,7 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
                 // a column every running fit holds fixed (an active-set
                 // pass) is not staged: it is skipped, or read in place
                 const bool held = A.lane_fix && ((~(unsigned)c_lfix[qq] & ~done_m & ((1u << G) - 1u)) == 0);
-                if (!grouped && !c_fix[qq] && !held && !dn && n > 0 && n <= kRegItems * NS && off + n <= kStage) {
+                if (!c_fix[qq] && !held && !dn && n > 0 && n <= kBatchCap && off + n <= kStage) {
                     c_off[qq] = off;
                     c_sq[ns] = qq;
                     c_soff[ns] = off;
@@ -971,7 +845,6 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
                 const int qq = c_sq[lo];
                 const long long e = c_e0[qq] + (t - c_soff[lo]);
                 s_sidx[t] = __ldg(A.idx + c_cp[qq] + e);
-                if constexpr (!kRowStream) s_sx[t] = (c_fmt[qq] == CYC_SPARSE) ? (T)__ldg(A.val + c_vp[qq] + e) : T(1);
             }
         }
         __syncthreads();
@@ -986,7 +859,6 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
                 for (int w = 0; w < L; ++w) moving |= ~(unsigned)c_lfix[q + w];
                 if ((moving & ~done_m & ((1u << G) - 1u)) == 0) { q += L; continue; }
             }
-            if constexpr (kRowStream) {
             if (L > 1) {
                 // ---- a batch of L short columns (planned: plan_runs); warp w takes column q + w
                 const int nd = c_nd[q], dr0 = c_dr0[q];
@@ -1205,253 +1077,6 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
                 par ^= 1;
                 ++q;
             }
-            } else {
-              if (L > 1) {
-                  // ---- a run of L conflict-free short columns: warp w takes column q + w
-                  const int qq = q + warp;
-                  int kk[kRunItems];
-                  T vv[kRunItems], xx[kRunItems];
-                  bool ind = true;
-                  if (warp < L) {
-                      const int fmt = c_fmt[qq];
-                      ind = (fmt == CYC_INDICATOR || fmt == CYC_INTERCEPT);
-                      const int e0 = c_e0[qq], n = c_e1[qq] - e0, so = c_off[qq];
-                      const int* cidx = A.idx + c_cp[qq];
-                      const double* cval = A.val + c_vp[qq];
-                      #pragma unroll
-                      for (int r = 0; r < kRunItems; ++r) {
-                          const int e = wslot + r * WS;
-                          const bool ok = e < n && !done_l;
-                          kk[r] = !ok ? -1 : (so >= 0 ? s_sidx[so + e] : __ldg(cidx + e0 + e));
-                          xx[r] = (!ok || ind) ? T(1) : (so >= 0 ? s_sx[so + e] : (T)__ldg(cval + e0 + e));
-                      }
-                      T ww[kRunItems];
-                      #pragma unroll
-                      for (int r = 0; r < kRunItems; ++r) {
-                          vv[r] = kk[r] >= 0 ? xbg[(size_t)kk[r] * G + fl] : T(0);
-                          ww[r] = kk[r] >= 0 ? row_weight<T, WM>(wg, A.fold, fitfold, kk[r], G, fl) : T(0);
-                      }
-                      Kahan<T> ag, ah;
-                      #pragma unroll
-                      for (int r = 0; r < kRunItems; ++r)
-                          if (kk[r] >= 0 && ww[r] != T(0)) row_gh<T, MODEL>(vv[r], xx[r], ww[r], ind, ag, ah);
-                      double g = ag.value(), h = ah.value();
-                      for (int o = G; o < 32; o <<= 1) {
-                          g += __shfl_xor_sync(0xffffffffu, g, o);
-                          h += __shfl_xor_sync(0xffffffffu, h, o);
-                      }
-                      if (lane < G)
-                          for (int r = 0; r < C; ++r)
-                              *cluster.map_shared_rank(&s_part[par][rank][warp][lane], r) = make_double2(g, h);
-                  }
-                  if (C > 1) cluster.sync(); else __syncthreads();
-                  double dl = 0.0;
-                  if (warp < L) {
-                      if (lane < G) {
-                          double g = 0.0, h = 0.0;
-                          for (int r = 0; r < C; ++r) {
-                              const double2 pp = s_part[par][r][warp][lane];
-                              g += pp.x;
-                              h += pp.y;
-                          }
-                          g -= c_xjy[qq][lane];                     // :1181-1183
-                          if (!s_done[lane] && !((c_lfix[qq] >> lane) & 1u)) {
-                              if (h < 0.0) { g = 0.0; h = 0.0; }    // ccdUpdateBeta :1407-1410
-                              const double b = c_beta[qq][lane];
-                              double hd = c_hd[qq][lane];
-                              dl = prior_delta(c_pt[qq], var_l, b, g, h);
-                              dl = apply_bounds(&hd, dl);
-                              c_hd[qq][lane] = hd;
-                              if (dl != 0.0) c_beta[qq][lane] = b + dl;
-                          }
-                          s_dr[warp][lane] = dl;
-                      }
-                      dl = __shfl_sync(0xffffffffu, dl, fl);
-                      if (dl != 0.0) {
-                          const T d = (T)dl;
-                          #pragma unroll
-                          for (int r = 0; r < kRunItems; ++r)
-                              if (kk[r] >= 0) xbg[(size_t)kk[r] * G + fl] = vv[r] + d * xx[r];
-                      }
-                  }
-                  __syncthreads();
-                  if (threadIdx.x == 0) count_run(q, L);
-                  par ^= 1;
-                  q += L;
-                  continue;
-              }
-              // ---- a single column
-              const int fmt = c_fmt[q];
-              const bool dense = (fmt == CYC_DENSE || fmt == CYC_INTERCEPT);
-              const bool ind = (fmt == CYC_INDICATOR || fmt == CYC_INTERCEPT);
-              const int* cidx = A.idx + c_cp[q];
-              const double* cval = A.val + c_vp[q];
-              const int e0 = c_e0[q], e1 = c_e1[q];
-              const bool regpath = !grouped && (e1 - e0) <= kRegItems * NS;
-              Kahan<T> ag, ah;
-              int kk[kRegItems];
-              T vv[kRegItems], xx[kRegItems];
-              if (regpath) {
-                  const int so = c_off[q];
-                  #pragma unroll
-                  for (int r = 0; r < kRegItems; ++r) {
-                      const int e = slot + r * NS;                 // relative to e0
-                      const bool ok = e < e1 - e0 && !done_l;
-                      kk[r] = !ok ? -1 : (so >= 0 ? s_sidx[so + e] : (dense ? e0 + e : __ldg(cidx + e0 + e)));
-                      xx[r] = (!ok || ind) ? T(1) : (so >= 0 ? s_sx[so + e] : (T)__ldg(cval + e0 + e));
-                  }
-                  T ww[kRegItems];
-                  #pragma unroll
-                  for (int r = 0; r < kRegItems; ++r) {
-                      vv[r] = kk[r] >= 0 ? xbg[(size_t)kk[r] * G + fl] : T(0);
-                      ww[r] = kk[r] >= 0 ? row_weight<T, WM>(wg, A.fold, fitfold, kk[r], G, fl) : T(0);
-                  }
-                  #pragma unroll
-                  for (int r = 0; r < kRegItems; ++r)
-                      if (kk[r] >= 0 && ww[r] != T(0)) row_gh<T, MODEL>(vv[r], xx[r], ww[r], ind, ag, ah);
-              } else if (!grouped) {
-                  if (!done_l) {
-                      // long column: batches of kRegItems entries per thread, loads first
-                      for (int base = e0 + slot; base < e1; base += kRegItems * NS) {
-                          int k2[kRegItems];
-                          T x2[kRegItems], v2[kRegItems], w2[kRegItems];
-                          #pragma unroll
-                          for (int r = 0; r < kRegItems; ++r) {
-                              const int e = base + r * NS;
-                              k2[r] = (e < e1) ? (dense ? e : __ldg(cidx + e)) : -1;
-                              x2[r] = (e < e1 && !ind) ? (T)__ldg(cval + e) : T(1);
-                          }
-                          #pragma unroll
-                          for (int r = 0; r < kRegItems; ++r) {
-                              v2[r] = k2[r] >= 0 ? xbg[(size_t)k2[r] * G + fl] : T(0);
-                              w2[r] = k2[r] >= 0 ? row_weight<T, WM>(wg, A.fold, fitfold, k2[r], G, fl) : T(0);
-                          }
-                          #pragma unroll
-                          for (int r = 0; r < kRegItems; ++r)
-                              if (k2[r] >= 0 && w2[r] != T(0)) row_gh<T, MODEL>(v2[r], x2[r], w2[r], ind, ag, ah);
-                      }
-                  }
-              } else {
-                  for (int e = e0 + slot; e < e1; e += NS) {
-                      const int k = dense ? e : __ldg(cidx + e);
-                      const int s = A.strat[k];
-                      if (e > e0) {
-                          const int kp = dense ? e - 1 : __ldg(cidx + e - 1);
-                          if (A.strat[kp] == s) continue;
-                      }
-                      T n1 = 0, n2 = 0;
-                      int qe = e;
-                      int kq = k;
-                      do {                                  // the run of stratum s in this column
-                          const T x = ind ? T(1) : (T)__ldg(cval + qe);
-                          const T ex = fexp(xbg[(size_t)kq * G + fl]);
-                          n1 += ex * x;
-                          if (!ind) n2 += ex * x * x;
-                          ++qe;
-                          if (qe >= e1) break;
-                          kq = dense ? qe : __ldg(cidx + qe);
-                      } while (A.strat[kq] == s);
-                      const double d = dg[(size_t)s * G + fl];
-                      const double nwv = ng[(size_t)s * G + fl];
-                      const double t = (double)n1 / d;        // ConditionalLogisticRegression::incrementGradientAndHessian
-                      const double gg = nwv * t;
-                      ag.add((T)gg);
-                      ah.add((T)(ind ? gg * (1.0 - t) : nwv * ((double)n2 / d - t * t)));
-                  }
-              }
-              block_reduce_lanes<G>(ag.value(), ah.value(), s_red, s_scr);
-              if (threadIdx.x < G)
-                  for (int r = 0; r < C; ++r) *cluster.map_shared_rank(&s_part[par][rank][0][threadIdx.x], r) = s_red[threadIdx.x];
-              if (C > 1) cluster.sync(); else __syncthreads();
-              // ---- coordinate step, identical in every CTA of the cluster
-              if (threadIdx.x < G) {
-                  double g = 0.0, h = 0.0;
-                  for (int r = 0; r < C; ++r) {
-                      const double2 pp = s_part[par][r][0][threadIdx.x];
-                      g += pp.x;
-                      h += pp.y;
-                  }
-                  g -= c_xjy[q][threadIdx.x];                    // :1181-1183
-                  double delta = 0.0;
-                  if (!s_done[threadIdx.x] && !((c_lfix[q] >> threadIdx.x) & 1u)) {
-                      if (h < 0.0) { g = 0.0; h = 0.0; }          // ccdUpdateBeta :1407-1410
-                      const double b = c_beta[q][threadIdx.x];
-                      double hd = c_hd[q][threadIdx.x];
-                      delta = prior_delta(c_pt[q], var_l, b, g, h);
-                      delta = apply_bounds(&hd, delta);
-                      c_hd[q][threadIdx.x] = hd;
-                      if (delta != 0.0) c_beta[q][threadIdx.x] = b + delta;
-                  }
-                  s_delta[threadIdx.x] = delta;
-              }
-              __syncthreads();
-              const double dl = s_delta[fl];
-              if (threadIdx.x == 0) {
-                  // as count_run, over this CTA's entries of the column
-                  int act = 0, upd = 0;
-                  for (int f = 0; f < G; ++f) { act += !s_done[f]; upd += (s_delta[f] != 0.0); }
-                  const long long nnc = e1 - e0;
-                  n_grad += (unsigned long long)(act * nnc);
-                  n_upd += (unsigned long long)(upd * nnc);
-                  if (rank == 0) n_steps += act;
-                  // the column streamed by this group: row ids (not for dense) and
-                  // values (sparse, dense), once for the gradient, again for an update
-                  const long long cb = nnc * ((dense ? 0 : 4) + (ind ? 0 : 8));
-                  n_idx += (unsigned long long)(cb * (1 + (upd ? 1 : 0)));
-              }
-              // ---- updateXBeta for my rows
-              if (dl != 0.0) {
-                  const T d = (T)dl;
-                  if (regpath) {
-                      #pragma unroll
-                      for (int r = 0; r < kRegItems; ++r)
-                          if (kk[r] >= 0) xbg[(size_t)kk[r] * G + fl] = vv[r] + d * xx[r];
-                  } else if (!grouped) {
-                      for (int base = e0 + slot; base < e1; base += kRegItems * NS) {
-                          int k2[kRegItems];
-                          T x2[kRegItems], v2[kRegItems];
-                          #pragma unroll
-                          for (int r = 0; r < kRegItems; ++r) {
-                              const int e = base + r * NS;
-                              k2[r] = (e < e1) ? (dense ? e : __ldg(cidx + e)) : -1;
-                              x2[r] = (e < e1 && !ind) ? (T)__ldg(cval + e) : T(1);
-                          }
-                          #pragma unroll
-                          for (int r = 0; r < kRegItems; ++r) v2[r] = k2[r] >= 0 ? xbg[(size_t)k2[r] * G + fl] : T(0);
-                          #pragma unroll
-                          for (int r = 0; r < kRegItems; ++r)
-                              if (k2[r] >= 0) xbg[(size_t)k2[r] * G + fl] = v2[r] + d * x2[r];
-                      }
-                  } else {
-                      for (int e = e0 + slot; e < e1; e += NS) {
-                          const int k = dense ? e : __ldg(cidx + e);
-                          const int s = A.strat[k];
-                          if (e > e0) {
-                              const int kp = dense ? e - 1 : __ldg(cidx + e - 1);
-                              if (A.strat[kp] == s) continue;
-                          }
-                          double acc = dg[(size_t)s * G + fl];
-                          int qe = e;
-                          int kq = k;
-                          do {
-                              const T x = ind ? T(1) : (T)__ldg(cval + qe);
-                              T* pp = xbg + (size_t)kq * G + fl;
-                              const T old = *pp;
-                              const T nv = old + d * x;
-                              *pp = nv;
-                              acc += (double)fexp(nv) - (double)fexp(old);
-                              ++qe;
-                              if (qe >= e1) break;
-                              kq = dense ? qe : __ldg(cidx + qe);
-                          } while (A.strat[kq] == s);
-                          dg[(size_t)s * G + fl] = acc;
-                      }
-                  }
-              }
-              __syncthreads();
-              par ^= 1;
-              ++q;
-            }
         }
         // chunk done: rank 0 writes the group's beta and trust regions back
         if (rank == 0)
@@ -1464,7 +1089,7 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
         __syncthreads();
       }
         // ---- convergence test (performCheckConvergence)
-        const double p = objective_partial<T, MODEL, G, WM>(A, grp, r0, r1, s0, s1, xbg, wg, fitfold, fl, use_ll);
+        const double p = objective_partial<T, MODEL, G, WM>(A, grp, r0, r1, xbg, wg, fitfold, fl, use_ll);
         block_reduce_lanes<G>(p, 0.0, s_red, s_scr);
         if (threadIdx.x < G)
             for (int r = 0; r < C; ++r) *cluster.map_shared_rank(&s_obj[opar][rank][threadIdx.x], r) = s_red[threadIdx.x].x;
@@ -1473,7 +1098,7 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
             const int f = fg + threadIdx.x;
             double o = 0.0;
             for (int r = 0; r < C; ++r) o += s_obj[opar][r][threadIdx.x];
-            if (use_ll && (MODEL == CYC_PR || MODEL == CYC_CPR)) o += A.llfixed[f];
+            if (use_ll && MODEL == CYC_PR) o += A.llfixed[f];
             if (A.conv == CYC_CONV_LANGE) {
                 const double* bf = A.beta + (size_t)f * A.J;
                 for (int j = 0; j < A.J; ++j) o += log_density(A.ptype[j], A.variance[f], bf[j]);
@@ -1502,14 +1127,9 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
             s_all_done = all;
         }
         __syncthreads();
-        done_l = s_done[fl] != 0;
         done_m = 0;
         for (int f = 0; f < G; ++f) done_m |= (s_done[f] ? 1u : 0u) << f;
         if (s_all_done) break;
-    }
-    if (xb_local) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < r1 - r0; i += kBT) xb_global[r0 + i] = s_xb[i];
     }
     if (C > 1) cluster.sync();   // no CTA leaves while others may still read its shared memory
     if (rank == 0 && threadIdx.x < G) {
@@ -1527,25 +1147,6 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
 }
 
 // ---- set-up kernels ----------------------------------------------------------
-
-// first entry of column j whose row is >= rpart[r]
-__global__ void k_splits(int J, int C, const int* fmt, const long long* col_ptr, const int* idx,
-                         const int* rpart, int* split) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= J * (C + 1)) return;
-    const int j = t / (C + 1), r = t % (C + 1);
-    const int f = fmt[j];
-    if (f == CYC_DENSE || f == CYC_INTERCEPT) { split[t] = rpart[r]; return; }
-    const int* c = idx + col_ptr[j];
-    int lo = 0, hi = (int)(col_ptr[j + 1] - col_ptr[j]);
-    const int key = rpart[r];
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (c[mid] < key) lo = mid + 1;
-        else hi = mid;
-    }
-    split[t] = lo;
-}
 
 // one fit's weights (K doubles, or all ones) into the [group][K][G] layout
 template <class T>
@@ -1825,11 +1426,11 @@ __global__ void k_batch_llfixed(int K, int G, int F, const double* c, const T* w
 // its batch it shares a row with, so columns of one level touch disjoint
 // rows.  Each shared row gets a slot, and every entry on a shared row is
 // listed with (slot, column within the batch, position in the column).
-// dmax = 0 gives the conflict-free runs used with one fit per group.
-// `batch_rows` > 0 also closes a batch before its entries in any one CTA's
-// rows would exceed that many (the batch cache holds them all).
-static RunPlan plan_runs(const Dataset& ds, const std::vector<int>& rpart, const std::vector<int>& fixb, int cap,
-                         bool allow, int dmax, int batch_rows = 0, int lvl_max = kLevelMax) {
+// Batches are planned without regard to the batch cache: those whose entries
+// fit it in every CTA take the cached path, the rest stream.
+static RunPlan plan_runs(const Dataset& ds, const std::vector<int>& rpart, const std::vector<int>& fixb,
+                         const BatchShape& shape) {
+    const int cap = shape.cap, dmax = shape.dmax, lvl_max = shape.lvl;
     const int J = ds.J, K = ds.K, C = (int)rpart.size() - 1;
     RunPlan P;
     P.len.assign(J, 1);
@@ -1846,9 +1447,7 @@ static RunPlan plan_runs(const Dataset& ds, const std::vector<int>& rpart, const
     std::vector<Ent> ents;
     std::vector<int> shared;            // row ids in order of their slots
     int run_id = -1, start = -1, len = 0;
-    std::vector<int> bsum(C, 0);        // the open batch's entries per CTA
     auto close = [&] {
-        std::fill(bsum.begin(), bsum.end(), 0);
         if (start < 0) return;
         P.len[start] = len;
         P.dr0[start] = (int)P.drow.size();
@@ -1872,7 +1471,7 @@ static RunPlan plan_runs(const Dataset& ds, const std::vector<int>& rpart, const
     for (int j = 0; j < J; ++j) {
         if (j % kChunk == 0) close();
         const int f = ds.fmt[j];
-        bool small = allow && (f == CYC_SPARSE || f == CYC_INDICATOR) && !fixb[j];
+        bool small = (f == CYC_SPARSE || f == CYC_INDICATOR) && !fixb[j];
         const int* rows = ds.h_idx.data() + ds.col_ptr[j];
         const int n = (int)(ds.col_ptr[j + 1] - ds.col_ptr[j]);
         if (small) {
@@ -1896,14 +1495,10 @@ static RunPlan plan_runs(const Dataset& ds, const std::vector<int>& rpart, const
                     fresh += rs[rows[e]].dslot < 0;
                     level = std::max(level, rs[rows[e]].rlvl + 1);
                 }
-        bool full = false;
-        if (batch_rows > 0)
-            for (int r = 0; r < C; ++r) full |= bsum[r] + cnt[r] > batch_rows;
-        if (start >= 0 && (len == kRunMax || (int)shared.size() + fresh > dmax || level > lvl_max || full)) {
+        if (start >= 0 && (len == kRunMax || (int)shared.size() + fresh > dmax || level > lvl_max)) {
             close();
             level = 1;
         }
-        for (int r = 0; r < C; ++r) bsum[r] += cnt[r];
         if (start < 0) {
             start = j;
             ++run_id;
@@ -1940,8 +1535,8 @@ static void launch_batch(const BatchArgs& a, int ngroups, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ngroups * a.C);
     cfg.blockDim = dim3(kBT);
-    const size_t dyn = 3 * kChunk * G * sizeof(double) + kStage * sizeof(int) + staged_value_bytes<T, MODEL, G>() +
-                       5 * kDirtyMax * G * sizeof(T) + (G == 1 ? (size_t)a.xb_smem * sizeof(T) : 0);
+    const size_t dyn = 3 * kChunk * G * sizeof(double) + kStage * sizeof(int) + (size_t)kAsyncBytes +
+                       5 * kDirtyMax * G * sizeof(T);
     CYC_CHECK_CUDA(cudaFuncSetAttribute(k_batch<T, MODEL, G, WM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     cfg.dynamicSmemBytes = dyn;
     cfg.stream = stream;
@@ -1962,9 +1557,7 @@ static void launch_model(const BatchArgs& a, int ngroups, cudaStream_t stream) {
     switch (a.model) {
     case CYC_LR: cv ? launch_batch<T, CYC_LR, G, 1>(a, ngroups, stream) : launch_batch<T, CYC_LR, G, 0>(a, ngroups, stream); break;
     case CYC_PR: cv ? launch_batch<T, CYC_PR, G, 1>(a, ngroups, stream) : launch_batch<T, CYC_PR, G, 0>(a, ngroups, stream); break;
-    case CYC_CLR: cv ? launch_batch<T, CYC_CLR, G, 1>(a, ngroups, stream) : launch_batch<T, CYC_CLR, G, 0>(a, ngroups, stream); break;
-    case CYC_CPR: cv ? launch_batch<T, CYC_CPR, G, 1>(a, ngroups, stream) : launch_batch<T, CYC_CPR, G, 0>(a, ngroups, stream); break;
-    default: throw Error{CYC_ERR_UNSUPPORTED, "batched fits support lr, pr, clr, cpr"};
+    default: throw Error{CYC_ERR_UNSUPPORTED, "grouped batches support lr and pr"};
     }
 }
 
@@ -1994,25 +1587,27 @@ struct BatchRunner {
     DevBuf<double> d_denom, d_nw, d_xjy, d_beta, d_hdelta, d_var, d_llfixed, d_obj, d_stage, d_fixedc;
     DevBuf<unsigned long long> d_counters;
     DevBuf<unsigned char> d_lfix;
+    // one-fit groups (ccd.cu): threads a CTA, the column lists and the moving steps per column
+    int threads = 0;
+    DevBuf<int> d_cols, d_ncols, d_out;
+    DevBuf<unsigned> d_upd;
+    std::vector<std::vector<int>> lists;     // one for all fits, or one a fit (active-set passes)
+    std::vector<int> all_cols;               // the columns not fixed
+    bool unit_weights = false;               // no fit has weights or a fold
 
     BatchRunner(Dataset& d, cudaStream_t s, int F_, int G_, int C_ = 0, BatchShape sh = BatchShape{})
         : ds(d), stream(s), F(F_), G(G_), shape(sh) {
         ngroups = (F + G - 1) / G;
         Fp = ngroups * G;
         const int K = ds.K;
-        C = C_ > 0 ? std::min(kMaxC, C_) : default_cluster(K);
-        // row partition, aligned to strata for grouped models
-        rpart.assign(C + 1, K);
-        for (int r = 0; r < C; ++r) {
-            int b = (int)((long long)K * r / C);
-            if (model_grouped(ds.model)) {
-                auto it = std::lower_bound(ds.strat_ptr.begin(), ds.strat_ptr.end(), b);
-                b = (it == ds.strat_ptr.end()) ? K : *it;
-            }
-            rpart[r] = b;
+        if (G == 1) {
+            const CcdShape sh1 = ccd_shape(ds, F);
+            C = sh1.C;
+            threads = sh1.threads;
+        } else {
+            C = C_ > 0 ? std::min(kMaxC, C_) : default_cluster(K);
         }
-        rpart[C] = K;
-        for (int r = 1; r <= C; ++r) rpart[r] = std::max(rpart[r], rpart[r - 1]);
+        rpart = ccd_rows(ds, C);     // aligned to strata for grouped models
     }
 
     // weights come either from per-fit host vectors (`specs`) or, for a CV
@@ -2020,7 +1615,7 @@ struct BatchRunner {
     const int* d_fold = nullptr;
     DevBuf<int> d_fitfold;
 
-    DevBuf<signed char> d_fold8;
+    DevBuf<signed char> d_fold8, d_entry_fold;
 
     int n_folds = 0;
 
@@ -2041,9 +1636,7 @@ struct BatchRunner {
         d_rpart.alloc(C + 1);
         CYC_CHECK_CUDA(cudaMemcpyAsync(d_rpart.get(), rpart.data(), (C + 1) * sizeof(int), cudaMemcpyHostToDevice, stream));
         d_split.alloc((size_t)J * (C + 1));
-        launch(k_splits, (J * (C + 1) + 255) / 256, 256, 0, stream, J, C, ds.d_fmt.get(), ds.d_col_ptr.get(), ds.d_idx.get(),
-                                                                  d_rpart.get(), d_split.get());
-        CYC_CHECK_LAUNCH();
+        ccd_splits(ds, C, d_rpart.get(), d_split.get(), stream);
         std::vector<int> fixb(J, 0), pt(J, prior.prior_type), act(Fp, 0);
         if (ds.has_offset) fixb[0] = 1;
         for (int j : fixed_cols) fixb[j] = 1;
@@ -2052,27 +1645,32 @@ struct BatchRunner {
         std::vector<double> var(Fp, 1.0);
         for (int f = 0; f < F; ++f) var[f] = specs[f].variance;
         d_fixb.alloc(J); d_ptype.alloc(J); d_active.alloc(Fp); d_var.alloc(Fp);
-        {
+        if (G == 1) {
+            lists.assign(1, {});
+            for (int j = 0; j < J; ++j)
+                if (!fixb[j]) lists[0].push_back(j);
+            all_cols = lists[0];
+            unit_weights = !d_fold && std::all_of(specs, specs + F, [](const cyc_fit_spec& sp) { return !sp.weights; });
+            upload_lists();
+            d_upd.alloc((size_t)Fp * J);
+            CYC_CHECK_CUDA(cudaMemsetAsync(d_upd.get(), 0, (size_t)Fp * J * sizeof(unsigned), stream));
+            if (model_grouped(ds.model)) ds.ensure_entry_strata();
+            if (d_fold) {
+                d_entry_fold.alloc(std::max<long long>(1, ds.nnz_idx));
+                ccd_entry_folds(ds, d_fold8.get(), d_entry_fold.get(), stream);
+            }
+        } else {
             const RunPlan* plan = nullptr;
-            const bool rows8 = (G == 8) && model_independent(ds.model);
-            // batches are planned without regard to the cache: those whose
-            // entries fit it in every CTA take the cached path, the rest stream
-            const int brows = 0;
-            const int cap = rows8 ? shape.cap : (32 / G) * kRunItems;
-            const int dmax = rows8 ? shape.dmax : 0;
-            const int lvl = rows8 ? shape.lvl : kLevelMax;
             for (auto& pl : ds.run_plans)
-                if (pl.C == C && pl.G == G && pl.batch_rows == brows && pl.cap == cap && pl.dmax == dmax &&
-                    pl.max_levels == lvl && pl.fixed == fixed_cols)
+                if (pl.C == C && pl.cap == shape.cap && pl.dmax == shape.dmax && pl.max_levels == shape.lvl &&
+                    pl.fixed == fixed_cols)
                     plan = &pl;
             if (!plan) {
-                RunPlan pl = plan_runs(ds, rpart, fixb, cap, model_independent(ds.model), dmax, brows, lvl);
+                RunPlan pl = plan_runs(ds, rpart, fixb, shape);
                 pl.C = C;
-                pl.G = G;
-                pl.batch_rows = brows;
-                pl.cap = cap;
-                pl.dmax = dmax;
-                pl.max_levels = lvl;
+                pl.cap = shape.cap;
+                pl.dmax = shape.dmax;
+                pl.max_levels = shape.lvl;
                 pl.fixed = fixed_cols;
                 ds.run_plans.push_back(std::move(pl));
                 plan = &ds.run_plans.back();
@@ -2178,23 +1776,49 @@ struct BatchRunner {
         CYC_CHECK_CUDA(cudaMemsetAsync(d_counters.get(), 0, (3 + ngroups) * sizeof(unsigned long long), stream));
     }
 
-    void run(const cyc_control& ctl, double tol, float* ms) {
+    // the columns each fit steps through (one-fit groups)
+    void upload_lists() {
+        const int J = ds.J;
+        std::vector<int> c(lists.size() * (size_t)J, 0), n(lists.size());
+        for (size_t i = 0; i < lists.size(); ++i) {
+            std::copy(lists[i].begin(), lists[i].end(), c.begin() + i * (size_t)J);
+            n[i] = (int)lists[i].size();
+        }
+        d_cols.alloc(c.size());
+        d_ncols.alloc(n.size());
+        CYC_CHECK_CUDA(cudaMemcpyAsync(d_cols.get(), c.data(), c.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
+        CYC_CHECK_CUDA(cudaMemcpyAsync(d_ncols.get(), n.data(), n.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
+        CYC_CHECK_CUDA(cudaStreamSynchronize(stream));   // the host arrays go away
+    }
+
+    void launch_one_fit(const cyc_control& ctl, double tol) {
+        CcdArgs a{};
+        a.model = ds.model; a.K = ds.K; a.J = ds.J; a.S = ds.S; a.F = F; a.C = C; a.threads = threads;
+        a.weights = d_fold ? 1 : (unit_weights ? 0 : 2);
+        a.fmt = ds.d_fmt.get(); a.col_ptr = ds.d_col_ptr.get(); a.val_ptr = ds.d_val_ptr.get();
+        a.idx = ds.d_idx.get(); a.val = ds.d_val.get(); a.entry_strat = ds.d_entry_strat.get();
+        a.split = d_split.get(); a.rpart = d_rpart.get(); a.y = ds.d_y.get(); a.strat = ds.d_strat.get();
+        a.cols = d_cols.get(); a.ncols = d_ncols.get();
+        a.cols_stride = lists.size() > 1 ? ds.J : 0; a.ncols_stride = lists.size() > 1 ? 1 : 0;
+        a.ptype = d_ptype.get(); a.xb = d_xb.get(); a.w = d_w.get();
+        a.fold = d_fold ? d_fold8.get() : nullptr; a.fitfold = d_fold ? d_fitfold.get() : nullptr;
+        a.entry_fold = d_entry_fold.get();
+        a.denom = d_denom.get(); a.nw = d_nw.get(); a.xjy = d_xjy.get(); a.beta = d_beta.get();
+        a.hdelta = d_hdelta.get(); a.variance = d_var.get(); a.llfixed = d_llfixed.get(); a.active = d_active.get();
+        a.col_updates = d_upd.get();
+        a.conv = ctl.convergence_type; a.tol = tol; a.max_iter = ctl.max_iterations;
+        a.out_iter = d_iter.get(); a.out_flag = d_flag.get();
+        launch_ccd<T>(a, rpart, stream);
+    }
+
+    void launch_eight_fit(const cyc_control& ctl, double tol) {
         BatchArgs a{};
-        a.model = ds.model; a.K = ds.K; a.J = ds.J; a.S = ds.S; a.C = C;
+        a.model = ds.model; a.K = ds.K; a.J = ds.J; a.C = C;
         a.fmt = ds.d_fmt.get(); a.col_ptr = ds.d_col_ptr.get(); a.val_ptr = ds.d_val_ptr.get();
         a.idx = ds.d_idx.get(); a.val = ds.d_val.get(); a.split = d_split.get(); a.rpart = d_rpart.get();
-        a.y = ds.d_y.get(); a.strat = ds.d_strat.get(); a.strat_ptr = ds.d_strat_ptr.get();
+        a.y = ds.d_y.get();
         a.fixb = d_fixb.get(); a.lane_fix = d_lfix.get(); a.ptype = d_ptype.get(); a.xb = d_xb.get(); a.w = d_w.get();
-        // one-fit groups keep a CTA's linear predictors in shared memory when
-        // its rows fit in 128 KB (CYC_BATCH_XB_SMEM=0 keeps them in global memory)
-        a.xb_smem = 0;
-        const char* xs = std::getenv("CYC_BATCH_XB_SMEM");
-        if (G == 1 && !(xs && std::atoi(xs) == 0)) {
-            int rows = 0;
-            for (int r = 0; r < C; ++r) rows = std::max(rows, rpart[r + 1] - rpart[r]);
-            if ((size_t)rows * sizeof(T) <= (size_t)128 * 1024) a.xb_smem = rows;
-        }
-        a.denom = d_denom.get(); a.nw = d_nw.get(); a.xjy = d_xjy.get(); a.beta = d_beta.get();
+        a.xjy = d_xjy.get(); a.beta = d_beta.get();
         a.hdelta = d_hdelta.get(); a.variance = d_var.get(); a.llfixed = d_llfixed.get(); a.active = d_active.get();
         a.fold = d_fold ? d_fold8.get() : nullptr;
         a.fitfold = d_fold ? d_fitfold.get() : nullptr;
@@ -2208,12 +1832,16 @@ struct BatchRunner {
         a.de_x = d_dex.get();
         a.conv = ctl.convergence_type; a.tol = tol; a.max_iter = ctl.max_iterations;
         a.out_iter = d_iter.get(); a.out_flag = d_flag.get(); a.out_obj = d_obj.get(); a.counters = d_counters.get();
+        launch_model<T, 8>(a, ngroups, stream);
+    }
+
+    void run(const cyc_control& ctl, double tol, float* ms) {
         cudaEvent_t e0, e1;
         CYC_CHECK_CUDA(cudaEventCreate(&e0));
         CYC_CHECK_CUDA(cudaEventCreate(&e1));
         CYC_CHECK_CUDA(cudaEventRecord(e0, stream));
-        if (G == 1) launch_model<T, 1>(a, ngroups, stream);
-        else launch_model<T, 8>(a, ngroups, stream);
+        if (G == 1) launch_one_fit(ctl, tol);
+        else launch_eight_fit(ctl, tol);
         CYC_CHECK_CUDA(cudaEventRecord(e1, stream));
         CYC_CHECK_CUDA(cudaEventSynchronize(e1));
         CYC_CHECK_CUDA(cudaEventElapsedTime(ms, e0, e1));
@@ -2229,6 +1857,13 @@ struct BatchRunner {
         const int J = ds.J;
         d_lfix.alloc(lane_fix.size());
         CYC_CHECK_CUDA(cudaMemcpyAsync(d_lfix.get(), lane_fix.data(), lane_fix.size(), cudaMemcpyHostToDevice, stream));
+        if (G == 1) {
+            lists.assign(F, {});
+            for (int f = 0; f < F; ++f)
+                for (int j : all_cols)
+                    if (!(lane_fix[(size_t)f * J + j] & 1)) lists[f].push_back(j);
+            upload_lists();
+        }
         std::vector<int> act(Fp, 0);
         std::copy(running.begin(), running.end(), act.begin());
         CYC_CHECK_CUDA(cudaMemcpyAsync(d_active.get(), act.data(), Fp * sizeof(int), cudaMemcpyHostToDevice, stream));
@@ -2299,6 +1934,29 @@ struct BatchRunner {
         CYC_CHECK_CUDA(cudaMemcpyAsync(counters.data(), d_counters.get(), counters.size() * sizeof(unsigned long long),
                                        cudaMemcpyDeviceToHost, stream));
         CYC_CHECK_CUDA(cudaStreamSynchronize(stream));
+        for (int f = 0; f < F; ++f)
+            CYC_REQUIRE(flags[f] != kTimedOut, CYC_ERR_TIMEOUT, "a wait between the CTAs of a fit ran out");
+        if (G == 1) {
+            // the counts k_batch keeps on the device, from the cycles and the moving steps per column
+            std::vector<unsigned> upd((size_t)F * J);
+            CYC_CHECK_CUDA(cudaMemcpyAsync(upd.data(), d_upd.get(), upd.size() * sizeof(unsigned),
+                                           cudaMemcpyDeviceToHost, stream));
+            CYC_CHECK_CUDA(cudaStreamSynchronize(stream));
+            for (int f = 0; f < F; ++f) {
+                unsigned long long& streamed = counters[3 + f];
+                for (int j : lists[lists.size() > 1 ? f : 0]) {
+                    const int fm = ds.fmt[j];
+                    const unsigned long long n = (unsigned long long)ds.col_len(j), u = upd[(size_t)f * J + j];
+                    const unsigned long long grads = (unsigned long long)iters[f];
+                    const int per = (fm == CYC_DENSE || fm == CYC_INTERCEPT ? 0 : 4) +
+                                    (fm == CYC_INDICATOR || fm == CYC_INTERCEPT ? 0 : 8);
+                    counters[0] += grads * n;
+                    counters[1] += u * n;
+                    counters[2] += grads;
+                    streamed += (grads + u) * n * per;
+                }
+            }
+        }
     }
 };
 
@@ -2437,6 +2095,57 @@ BatchShape tuned_shape(Dataset& ds, cudaStream_t stream, int F, int G, int C, co
     return best;
 }
 
+// ---- one fit to a cluster, or eight to a group ---------------------------------
+// One fit to a cluster (ccd.cu) is faster until the fits outnumber the SMs or
+// their linear predictors outgrow L2; eight to a group (k_batch) keeps eight
+// fits' predictors of a row side by side, and a step costs about 3 us and 2.5
+// more per 1,000 entries of the mean column, whatever its fits.  Measured,
+// grouped against one to a cluster (logistic CV grids): 10k rows, 10 fits 34
+// ms / 11 ms, 160 fits 35 / 13; 50k rows Zipf, 40 fits 19 / 10, 160 fits 22 /
+// 21; 400k rows, 20 fits 36 / 16; 500k rows x 4,000, 40 fits 519 / 427, 200
+// fits 664 / 1,380; 100k rows x 4,000, 200 fits 822 / 1,410.  The rule
+// compares the two modelled cycles, with 0.8 for the models' errors; a solve
+// large enough for the cluster tuner times a cycle of both instead of
+// trusting the model where it favours one to a cluster, and caches the choice
+// per problem shape.  Grouped models (clr, cpr) always run one to a cluster
+// (30 against 8.7 ms at 160 fits of 10k rows, 23 against 15 at 80 fits of 100k).
+std::map<TuneKey, int>& tuned_groups() {
+    static auto* m = new std::map<TuneKey, int>();   // lives to process exit
+    return *m;
+}
+
+int group_size(Dataset& ds, cudaStream_t stream, int F, const cyc_prior& prior, const cyc_fit_spec* specs,
+               const std::vector<double>& beta, const std::vector<double>& hd, const int* d_fold, int n_folds,
+               const std::vector<int>* fit_fold, const cyc_control& ctl, const std::vector<int>& fixed_cols,
+               bool swindle) {
+    if (const char* e = std::getenv("CYC_BATCH_GROUP")) return std::atoi(e) == 8 ? 8 : 1;
+    const double entries = (double)(ds.nnz_idx + ds.nnz_val);
+    const bool large = F >= 16 && F * entries >= 1e8 && default_cluster(ds.K) > 1;
+    if (large && std::getenv("CYC_BATCH_CLUSTER")) return 8;
+    double visits = 0.0;
+    for (int j = 0; j < ds.J; ++j) visits += (double)ds.col_len(j);
+    const double waves8 = std::ceil((double)((F + 7) / 8) * default_cluster(ds.K) / (2.0 * 148));
+    if (ccd_shape(ds, F).cycle_us > 0.8 * (3.0 * ds.J + 0.0025 * visits) * waves8) return 8;
+    if (!large || swindle) return 1;
+    const TuneKey key{ds.model, ds.K, ds.J, F, 0, ctl.precision, d_fold ? n_folds : 0, fixed_cols, ds.nnz_idx};
+    {
+        std::lock_guard<std::mutex> lk(g_tune_mutex);
+        auto it = tuned_groups().find(key);
+        if (it != tuned_groups().end()) return it->second;
+    }
+    auto time = [&](int G) {
+        return ctl.precision == CYC_MIXED
+                   ? probe_cycle<float>(ds, stream, F, G, 0, prior, specs, beta, hd, d_fold, n_folds, fit_fold, ctl,
+                                        fixed_cols)
+                   : probe_cycle<double>(ds, stream, F, G, 0, prior, specs, beta, hd, d_fold, n_folds, fit_fold, ctl,
+                                         fixed_cols);
+    };
+    const int best = time(1) < time(8) ? 1 : 8;
+    std::lock_guard<std::mutex> lk(g_tune_mutex);
+    tuned_groups()[key] = best;
+    return best;
+}
+
 // Fits the persistent kernel does not take -- Cox, whose risk sets follow
 // each fit's weights and are rescanned after every moving coordinate, and
 // fits under the KKT swindle, each with its own active set -- run
@@ -2554,12 +2263,17 @@ void run_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* specs, i
         if (specs[f].start_beta) std::copy(specs[f].start_beta, specs[f].start_beta + J, beta.begin() + (size_t)f * J);
         if (ds.has_offset) beta[(size_t)f * J] = 1.0;
     }
-    const int G = F >= 4 ? 8 : 1;
+    const bool can8 = model_independent(ds.model) && F >= 4;
     // the swindle runs when some column has a Laplace prior (a KKT boundary,
     // JointPrior.h:149-157); otherwise it is findMode itself
     std::vector<int> ptype(J, prior->prior_type);
     for (int i = 0; i < prior->n_exclude; ++i) ptype[prior->exclude[i]] = CYC_PRIOR_NONE;
     const bool swindle = ctl->use_kkt_swindle && std::count(ptype.begin(), ptype.end(), (int)CYC_PRIOR_LAPLACE) > 0;
+    int G = 1;
+    if (can8) {
+        NvtxRange range("cyclops batch: group choice");
+        G = group_size(ds, stream, F, *prior, specs, beta, hd, d_fold, n_folds, fit_fold, *ctl, fixed_cols, swindle);
+    }
     std::vector<int> iters, flags;
     std::vector<unsigned long long> ctr;
     cyc_run_stats st{};
@@ -2603,7 +2317,8 @@ void run_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* specs, i
     // the tuners time whole cycles over every column, which an active-set
     // pass does not run: swindle solves keep the defaults
     int C = default_cluster(ds.K);
-    if (!swindle) {
+    if (G == 1) C = ccd_shape(ds, F).C;
+    if (G != 1 && !swindle) {
         NvtxRange range("cyclops batch: cluster tuner");
         C = tuned_cluster(ds, stream, F, G, *prior, specs, beta, hd, d_fold, n_folds, fit_fold, *ctl, fixed_cols);
     }

@@ -1,0 +1,746 @@
+// ccd.cu -- the one-fit persistent CCD: a fit's whole coordinate loop, its
+// convergence test included, in one launch (lr, pr, clr, cpr).
+//
+// CyclicCoordinateDescent::findMode (src/cyclops/CyclicCoordinateDescent.cpp
+// :909-1216) is one serial chain of coordinate steps, so what bounds it is
+// the latency of a step: the entries' row state, exp() and a division, a sum
+// over the threads, the step's division, and the write of the row state.
+// A step has no work for more than a few SMs, and a kernel boundary alone
+// costs as much as a whole step (three launches a coordinate measured 9 us;
+// here a step of a 100-entry column is well under 1 us).  So:
+//  * a fit is one thread-block cluster of C CTAs that split the rows; C is 1
+//    while a column has few entries per CTA, and the cluster's (gradient,
+//    Hessian) sums cross CTAs through distributed shared memory by st.async,
+//    which arrives on the receiver's mbarrier (see ccd_shape for the rule);
+//  * the linear predictors of a CTA's rows live in shared memory for the
+//    launch when they fit, else in global memory through L1 (every access is
+//    to the CTA's own rows); exp(xb) is recomputed, never stored;
+//  * a column's first kR entries per thread stay in registers from the
+//    gradient to the update, and the next column's row ids and values load
+//    while this one's sums cross the CTA;
+//  * every thread computes the coordinate step from the same sums in the
+//    same order, so nothing is broadcast and no second exchange is needed.
+// Independent fits are independent clusters of one launch.
+#include "ccd.cuh"
+
+#include <cooperative_groups.h>
+#include <math_constants.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+#include <type_traits>
+
+#include "row_terms.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace cyc {
+
+namespace {
+
+constexpr int kR = 2;            // entries of a column a thread keeps in registers
+constexpr int kU = 4;            // further entries a thread has in flight
+constexpr int kCh = 128;         // coordinates staged at a time
+constexpr int kWarps = kCcdThreads / 32;
+
+// the row's mean under the model; a logistic row whose exp(xb) overflows is NaN
+// when `strict`, as exb / (1 + exb) is in the per-coordinate engine
+template <class T, int MODEL>
+__device__ __forceinline__ T fit_mean(T v, bool strict) {
+    if constexpr (MODEL == CYC_LR && sizeof(T) == 8) {
+        const double a = strict && v > 709.782712893384 ? CUDART_NAN : -v;
+        return 1.0 / (1.0 + exp(a));
+    } else {
+        return row_mean<T, MODEL>(v);
+    }
+}
+
+template <class T, int WM>
+struct RowWeight {
+    const T* w;
+    const signed char* fold;
+    int held;
+    __device__ __forceinline__ T by_fold(int v) const { return v != held ? T(1) : T(0); }
+    __device__ __forceinline__ T operator()(int k) const {
+        if (WM == 0) return T(1);
+        if (WM == 1) return by_fold((int)__ldg(fold + k));
+        return __ldg(w + k);
+    }
+};
+
+// a column of the current chunk, in this CTA's rows
+struct ColMeta {
+    const int* ci;       // row ids of its entries, null for dense columns (entry i is row r0 + i)
+    const double* cv;    // values, null for indicators
+    const int* es;       // strata of its entries (grouped models)
+    const signed char* ef;   // fold ids of its entries (CV folds)
+    int n;               // entries
+    int pt;              // prior type
+};
+
+// what a column's step needs besides its sums, prepared when the chunk is
+// staged so that selections and one division are left after the sums arrive
+struct ColStep {
+    double beta, bound, xjy;
+    double pre, iv, lam;     // added to g, added to h, the Laplace rate (0: another prior)
+    int s;                   // sign of beta (2: not a Laplace prior)
+};
+
+// T: state type.  MODEL: cyc_model.  WM: row weights (0 ones, 1 CV folds, 2 a
+// vector).  SM: the linear predictors of the CTA's rows are in shared memory.
+//
+// A column's entries are dealt to the threads in rounds of NT; up to kR
+// rounds stay in registers from the gradient to the update.  The code of a
+// round is straight-line (one round and kR rounds as separate instances): with
+// one warp per scheduler the instructions of a step are latency too.
+// ---- the cluster exchange: 16 bytes to a peer's shared memory, counted on its mbarrier
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned peer_addr(unsigned addr, int rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void push16(unsigned dst, unsigned mbar, double a, double b) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(dst),
+                 "l"(__double_as_longlong(a)), "l"(__double_as_longlong(b)), "r"(mbar)
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_init(unsigned mbar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(unsigned mbar, int bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(unsigned mbar, int phase) {
+    unsigned ok;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(mbar), "r"(phase)
+        : "memory");
+    return ok != 0;
+}
+// A peer is at most one column's work away (well under a millisecond); a wait
+// that outlasts this many clocks (about two seconds) gives up.
+constexpr long long kWaitClocks = 4000000000ll;
+
+template <class T, int MODEL, int WM, bool SM>
+__global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
+    constexpr bool kGrouped = (MODEL == CYC_CLR || MODEL == CYC_CPR);
+    cg::cluster_group cluster = cg::this_cluster();
+    const int C = A.C;
+    const int rank = C > 1 ? (int)cluster.block_rank() : 0;
+    const int f = blockIdx.x / C;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int NT = blockDim.x, NW = NT >> 5;
+    if (A.active && !A.active[f]) {              // the whole cluster leaves
+        if (rank == 0 && tid == 0) { A.out_iter[f] = 0; A.out_flag[f] = CYC_SUCCESS; }
+        return;
+    }
+    const int r0 = A.rpart[rank], r1 = A.rpart[rank + 1], nr = r1 - r0;
+    // this CTA's rows; row ids are made relative to r0
+    T* const xg = (T*)A.xb + (size_t)f * A.K + r0;
+    const RowWeight<T, WM> weight{WM == 2 ? (const T*)A.w + (size_t)f * A.K + r0 : nullptr,
+                                  WM == 1 ? A.fold + r0 : nullptr, WM == 1 ? A.fitfold[f] : 0};
+    double* const dg = kGrouped ? A.denom + (size_t)f * A.S : nullptr;
+    const double* const ng = kGrouped ? A.nw + (size_t)f * A.S : nullptr;
+    const size_t fj = (size_t)f * A.J;
+    const double var = A.variance[f];
+    const double lam = sqrt(2.0 / var);          // LaplacePrior rate, CovariatePrior.h:282-292
+    const double ivar = 1.0 / var;
+    const bool strict = A.strict_mean != 0;
+
+    __shared__ double2 s_part[2][kWarps];        // the warps' sums, by parity
+    __shared__ __align__(16) double2 s_cl[2][kCcdCluster];   // the CTAs' sums, by parity
+    __shared__ __align__(8) unsigned long long s_mb[2];      // their arrival
+    __shared__ double2 s_all;                    // the cluster's sums
+    __shared__ int s_dead;                       // a wait for the peers ran out
+    __shared__ ColMeta c_m[kCh + 1];             // one empty column after the last
+    __shared__ ColStep c_s[kCh];
+    __shared__ double c_ob[kCh], c_oh[kCh];
+    __shared__ int c_j[kCh], c_up[kCh];
+    extern __shared__ __align__(16) unsigned char dyn_smem[];
+    T* const sx = reinterpret_cast<T*>(dyn_smem);
+    auto get = [&](int k) -> T { return SM ? sx[k] : xg[k]; };
+    auto put = [&](int k, T v) {
+        if (SM) sx[k] = v;
+        else xg[k] = v;
+    };
+    if (SM)
+        for (int i = tid; i < nr; i += blockDim.x) sx[i] = xg[i];
+    if (tid == 0) {
+        s_dead = 0;
+        mbar_init(smem_addr(&s_mb[0]));
+        mbar_init(smem_addr(&s_mb[1]));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (C > 1) cluster.sync();
+    else __syncthreads();
+
+    int par = 0, phase = 0;                      // of the next exchange: parity of its slots, of their mbarrier
+    // (a, b) summed over the cluster's threads, the same in every thread.
+    // Warp sums by shuffles (a in the lower
+    // half-warp, b in the upper), then over the warps, then over the CTAs, in
+    // fixed orders.  It has at least one __syncthreads, which also orders the
+    // caller's earlier reads before its later writes.
+    auto combine = [&](double& a, double& b) {
+        constexpr unsigned full = 0xffffffffu;
+        {
+            const bool up = (lane & 16) != 0;
+            double v = up ? b : a;
+            v += __shfl_xor_sync(full, up ? a : b, 16);
+            v += __shfl_xor_sync(full, v, 8);
+            v += __shfl_xor_sync(full, v, 4);
+            v += __shfl_xor_sync(full, v, 2);
+            v += __shfl_xor_sync(full, v, 1);
+            if ((lane & 15) == 0) (&s_part[par][warp].x)[lane >> 4] = v;
+        }
+        __syncthreads();
+        auto total = [&](const double2* src, int n) {
+            double2 t[4] = {};
+            #pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (i < n) t[i] = src[i];
+            if (n > 4) {
+                #pragma unroll
+                for (int i = 4; i < kCcdCluster; ++i)
+                    if (i < n) { t[i & 3].x += src[i].x; t[i & 3].y += src[i].y; }
+            }
+            a = (t[0].x + t[1].x) + (t[2].x + t[3].x);
+            b = (t[0].y + t[1].y) + (t[2].y + t[3].y);
+        };
+        if (C == 1) {
+            total(s_part[par], NW);
+            par ^= 1;
+            return;
+        }
+        // slots and mbarriers alternate: a peer writes slot `par` again only
+        // two exchanges on, after this CTA has sent the one between, which it
+        // does after reading this one
+        if (warp == 0) {
+            const unsigned mb = smem_addr(&s_mb[par]);
+            total(s_part[par], NW);
+            if (lane == 0) mbar_expect(mb, 16 * C);
+            if (lane < C) push16(peer_addr(smem_addr(&s_cl[par][rank]), lane), peer_addr(mb, lane), a, b);
+            if (!s_dead && !mbar_try(mb, phase)) {
+                const long long t0 = clock64();
+                while (!mbar_try(mb, phase))
+                    if (clock64() - t0 > kWaitClocks) { s_dead = 1; break; }
+            }
+            total(s_cl[par], C);
+            if (lane == 0) s_all = make_double2(a, b);
+        }
+        __syncthreads();
+        a = s_all.x;
+        b = s_all.y;
+        phase ^= par;
+        par ^= 1;
+    };
+
+    // the convergence objective (getGradientObjective, getLogLikelihood, with
+    // the log prior for Lange; 0 for ONE_STEP), or the Zhang-Oles criterion
+    // (computeZhangOlesConvergenceCriterion, CyclicCoordinateDescent.cpp
+    // :560-579, renewing xb_save), the same in every thread
+    auto objective = [&]() -> double {
+        if (A.conv == CYC_CONV_ONE_STEP) return 0.0;
+        double a = 0.0, b = 0.0;
+        if (A.conv == CYC_CONV_ZHANG_OLES) {
+            T* save = (T*)A.xb_save + (size_t)f * A.K + r0;
+            for (int k = tid; k < nr; k += NT) {
+                const double v = (double)get(k), w = (double)weight(k);
+                a += fabs(v - (double)save[k]) * w;
+                b += fabs(v) * w;
+                save[k] = get(k);
+            }
+        } else {
+            const bool use_ll = A.conv != CYC_CONV_GRADIENT;
+            #pragma unroll 4
+            for (int k = tid; k < nr; k += NT) {
+                const double v = (double)get(k), wt = (double)weight(k), yk = A.y[r0 + k];
+                if (!use_ll) {
+                    a += v * yk * wt;
+                } else {
+                    double c = (int)yk * v * wt;                    // logLikeNumeratorContrib(int, RealType)
+                    if (MODEL == CYC_LR) c -= wt * log(1.0 + exp(v));
+                    if (MODEL == CYC_PR) c -= wt * exp(v);
+                    a += c;
+                }
+            }
+            if (use_ll && kGrouped && nr > 0) {
+                const int s0 = A.strat[r0], s1 = r1 >= A.K ? A.S : A.strat[r1];
+                for (int s = s0 + tid; s < s1; s += NT) a -= ng[s] * log(dg[s]);
+            }
+            if (A.conv == CYC_CONV_LANGE && rank == 0)
+                for (int j = tid; j < A.J; j += NT) b += log_density(A.ptype[j], var, A.beta[fj + j]);
+        }
+        combine(a, b);
+        if (A.conv == CYC_CONV_ZHANG_OLES) return a / (1.0 + b);
+        if (A.conv != CYC_CONV_GRADIENT && (MODEL == CYC_PR || MODEL == CYC_CPR)) a += A.llfixed[f];
+        return A.conv == CYC_CONV_LANGE ? a + b : a;
+    };
+
+    // ccdUpdateBeta (:1394-1413) with the priors' getDelta (as prior_delta_rate)
+    auto step = [&](const ColStep& p, double g, double h) -> double {
+        if (h < 0.0) { g = 0.0; h = 0.0; }                          // :1407-1410
+        const double base = g + p.pre, up = base + p.lam, down = base - p.lam;
+        const double zero = down > 0 ? down : (up < 0 ? up : 0.0);
+        const double num = p.s == 0 ? zero : (p.s < 0 ? down : up);
+        double delta = -num / (h + p.iv);
+        if (p.s == 0) delta = (num != 0.0 && delta == delta) ? delta : 0.0;
+        else if (p.s != 2 && sgn(p.beta + delta) != p.s) delta = -p.beta;
+        if (delta < -p.bound) delta = -p.bound;                     // applyBounds :1503-1520
+        else if (delta > p.bound) delta = p.bound;
+        return delta;
+    };
+    auto next_bound = [](double bound, double delta) { return std_max(std_max(fabs(delta) * 2, bound / 2), 1E-3); };
+
+    double last = A.conv == CYC_CONV_ZHANG_OLES ? 0.0 : objective();   // findMode :949-953
+    const int* cols = A.cols + (size_t)f * A.cols_stride;
+    const int ncols = A.ncols[(size_t)f * A.ncols_stride];
+    int it = 0, flag = CYC_SUCCESS;
+    for (;;) {
+        for (int base = 0; base < ncols; base += kCh) {
+            const int jn = min(kCh, ncols - base);
+            __syncthreads();                     // the last chunk's arrays have been read
+            if (tid == 0) c_m[jn] = ColMeta{A.idx, nullptr, A.strat, A.fold, 0, 0};
+            for (int q = tid; q < jn; q += blockDim.x) {
+                const int j = cols[base + q];
+                const int fm = A.fmt[j];
+                const bool dn = (fm == CYC_DENSE || fm == CYC_INTERCEPT);
+                const int e0 = dn ? r0 : A.split[j * (C + 1) + rank];
+                const int e1 = dn ? r1 : A.split[j * (C + 1) + rank + 1];
+                ColMeta m;
+                m.ci = dn ? nullptr : A.idx + A.col_ptr[j] + e0;
+                m.cv = (fm == CYC_SPARSE || fm == CYC_DENSE) ? A.val + A.val_ptr[j] + e0 : nullptr;
+                m.es = !kGrouped ? nullptr : (dn ? A.strat + r0 : A.entry_strat + A.col_ptr[j] + e0);
+                m.ef = WM != 1 ? nullptr : (dn ? A.fold + r0 : A.entry_fold + A.col_ptr[j] + e0);
+                m.n = e1 - e0;
+                m.pt = A.ptype[j];
+                c_m[q] = m;
+                c_j[q] = j;
+                const double beta = A.beta[fj + j];
+                ColStep p{beta, A.hdelta[fj + j], A.xjy[fj + j], 0.0, 0.0, 0.0, 2};
+                if (m.pt == CYC_PRIOR_NORMAL) {
+                    p.pre = beta / var;
+                    p.iv = ivar;
+                } else if (m.pt == CYC_PRIOR_LAPLACE) {
+                    p.lam = lam;
+                    p.s = sgn(beta);
+                }
+                c_s[q] = p;
+            }
+            __syncthreads();
+            // the next column and its first kR rounds, as loaded (nothing here
+            // waits for a load): row ids (-1: no entry), values, and for grouped
+            // models the strata of the entry and of its neighbours (-1: none)
+            ColMeta nm = c_m[0];
+            int nk[kR], nf[kR], ns[kR], np[kR], nn[kR];
+            double nx[kR];
+            auto fetch = [&](int r) {
+                const int i = tid + r * NT;
+                nk[r] = ns[r] = np[r] = nn[r] = -1;
+                nx[r] = 1.0;
+                nf[r] = 0;
+                if (i < nm.n) {
+                    if (WM == 1) nf[r] = (int)__ldg(nm.ef + i);
+                    if (nm.ci) nk[r] = __ldg(nm.ci + i);
+                    else nk[r] = r0 + i;
+                    if (nm.cv) nx[r] = __ldg(nm.cv + i);
+                    if (kGrouped) {
+                        ns[r] = __ldg(nm.es + i);
+                        if (i > 0) np[r] = __ldg(nm.es + i - 1);
+                        if (i + 1 < nm.n) nn[r] = __ldg(nm.es + i + 1);
+                    }
+                }
+            };
+            auto prefetch = [&](int q) {
+                nm = c_m[q];
+                fetch(0);
+                if (nm.n > NT) {
+                    #pragma unroll
+                    for (int r = 1; r < kR; ++r) fetch(r);
+                }
+            };
+            prefetch(0);
+            for (int q = 0; q < jn; ++q) {
+                const ColMeta m = nm;
+                const bool ind = m.cv == nullptr;
+                const ColStep p = c_s[q];
+                double dl;
+                // the step from the sums, written down by one thread
+                auto finish = [&](double g, double h) {
+                    dl = step(p, g - p.xjy, h);                             // :1181-1183
+                    if (tid == 0) {
+                        c_oh[q] = next_bound(p.bound, dl);
+                        c_ob[q] = dl != 0.0 ? p.beta + dl : p.beta;
+                        c_up[q] = dl != 0.0;
+                    }
+                };
+                if constexpr (!kGrouped) {
+                    auto column = [&](auto rounds) {
+                        constexpr int R = decltype(rounds)::value;
+                        int kk[R];
+                        T xx[R], vv[R], ww[R];
+                        #pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            kk[r] = nk[r] - r0;              // negative: no entry
+                            xx[r] = (T)nx[r];
+                            vv[r] = kk[r] >= 0 ? get(kk[r]) : T(0);
+                            ww[r] = kk[r] < 0 ? T(0) : (WM == 1 ? weight.by_fold(nf[r]) : weight(kk[r]));
+                        }
+                        prefetch(q + 1);
+                        Kahan<T> ag, ah;
+                        // (lanes without an entry compute too: fewer branches are fewer cycles here)
+                        #pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            T gi, hi;
+                            mean_terms<T, MODEL>(fit_mean<T, MODEL>(vv[r], strict), xx[r], WM == 2 ? ww[r] : T(1), ind,
+                                                 gi, hi);
+                            ag.add(ww[r] != T(0) ? gi : T(0));
+                            ah.add(ww[r] != T(0) ? hi : T(0));
+                        }
+                        if (R == kR)
+                            for (int b0 = kR * NT + tid; b0 < m.n; b0 += kU * NT) {
+                                int k2[kU];
+                                T x2[kU], v2[kU], w2[kU];
+                                #pragma unroll
+                                for (int u = 0; u < kU; ++u) {
+                                    const int i = b0 + u * NT;
+                                    k2[u] = i < m.n ? (m.ci ? __ldg(m.ci + i) - r0 : i) : -1;
+                                    x2[u] = (i < m.n && m.cv) ? (T)__ldg(m.cv + i) : T(1);
+                                }
+                                #pragma unroll
+                                for (int u = 0; u < kU; ++u) {
+                                    v2[u] = k2[u] >= 0 ? get(k2[u]) : T(0);
+                                    w2[u] = k2[u] < 0 ? T(0)
+                                            : WM == 1 ? weight.by_fold((int)__ldg(m.ef + b0 + u * NT))
+                                                      : weight(k2[u]);
+                                }
+                                #pragma unroll
+                                for (int u = 0; u < kU; ++u) {
+                                    T gi, hi;
+                                    mean_terms<T, MODEL>(fit_mean<T, MODEL>(v2[u], strict), x2[u],
+                                                         WM == 2 ? w2[u] : T(1), ind, gi, hi);
+                                    ag.add(w2[u] != T(0) ? gi : T(0));
+                                    ah.add(w2[u] != T(0) ? hi : T(0));
+                                }
+                            }
+                        double g = ag.value(), h = ah.value();
+                        combine(g, h);
+                        finish(g, h);
+                        if (dl == 0.0) return;               // nothing moved: no write to order
+                        const T d = (T)dl;                   // updateXBeta
+                        #pragma unroll
+                        for (int r = 0; r < R; ++r)
+                            if (kk[r] >= 0) put(kk[r], vv[r] + d * xx[r]);
+                        if (R == kR)
+                            for (int b0 = kR * NT + tid; b0 < m.n; b0 += kU * NT) {
+                                int k2[kU];
+                                T x2[kU], v2[kU];
+                                #pragma unroll
+                                for (int u = 0; u < kU; ++u) {
+                                    const int i = b0 + u * NT;
+                                    k2[u] = i < m.n ? (m.ci ? __ldg(m.ci + i) - r0 : i) : -1;
+                                    x2[u] = (i < m.n && m.cv) ? (T)__ldg(m.cv + i) : T(1);
+                                }
+                                #pragma unroll
+                                for (int u = 0; u < kU; ++u) v2[u] = k2[u] >= 0 ? get(k2[u]) : T(0);
+                                #pragma unroll
+                                for (int u = 0; u < kU; ++u)
+                                    if (k2[u] >= 0) put(k2[u], v2[u] + d * x2[u]);
+                            }
+                        __syncthreads();
+                    };
+                    if (m.n <= NT) column(std::integral_constant<int, 1>{});
+                    else column(std::integral_constant<int, kR>{});
+                } else {
+                    // the first entry of each run of one stratum takes the run
+                    // (ConditionalLogisticRegression::incrementGradientAndHessian,
+                    // ModelSpecifics.h:820-837)
+                    auto column = [&](auto rounds) {
+                        constexpr int R = decltype(rounds)::value;
+                        int kk[R], ss[R], bb[R];
+                        T xx[R], vv[R], ex[R];
+                        double dd[R], ev[R];
+                        #pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            kk[r] = nk[r] - r0;              // negative: no entry
+                            xx[r] = (T)nx[r];
+                            ss[r] = ns[r];
+                            // bit 0: the entry starts its stratum's run; bit 1: the run goes on
+                            bb[r] = ss[r] >= 0 ? (np[r] != ss[r] ? 1 : 0) | (nn[r] == ss[r] ? 2 : 0) : 0;
+                            vv[r] = kk[r] >= 0 ? get(kk[r]) : T(0);
+                            dd[r] = (bb[r] & 1) ? dg[ss[r]] : 1.0;
+                            ev[r] = (bb[r] & 1) ? __ldg(ng + ss[r]) : 0.0;
+                        }
+                        prefetch(q + 1);
+                        Kahan<T> ag, ah;
+                        auto row = [&](int i) { return m.ci ? __ldg(m.ci + i) - r0 : i; };
+                        auto rest = [&](int i, int s, T& n1, T& n2) {      // the run's further entries
+                            for (++i; i < m.n && __ldg(m.es + i) == s; ++i) {
+                                const T x = ind ? T(1) : (T)__ldg(m.cv + i);
+                                const T e = fexp(get(row(i)));
+                                n1 += e * x;
+                                if (!ind) n2 += e * x * x;
+                            }
+                        };
+                        auto add = [&](T n1, T n2, double d, double nwk) {
+                            const double t = (double)n1 / d;
+                            const double gg = nwk * t;
+                            ag.add((T)gg);
+                            ah.add((T)(ind ? gg * (1.0 - t) : nwk * ((double)n2 / d - t * t)));
+                        };
+                        #pragma unroll
+                        for (int r = 0; r < R; ++r) ex[r] = fexp(vv[r]);
+                        #pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            T n1 = ex[r] * xx[r], n2 = ind ? T(0) : n1 * xx[r];
+                            if ((bb[r] & 3) == 3) rest(tid + r * NT, ss[r], n1, n2);
+                            add(n1, n2, dd[r], ev[r]);       // ev is 0 where no run starts
+                        }
+                        if (R == kR)
+                            for (int i = kR * NT + tid; i < m.n; i += NT) {
+                                const int s = __ldg(m.es + i);
+                                if (__ldg(m.es + i - 1) == s) continue;
+                                const T x = ind ? T(1) : (T)__ldg(m.cv + i);
+                                const T e = fexp(get(row(i)));
+                                T n1 = e * x, n2 = ind ? T(0) : n1 * x;
+                                rest(i, s, n1, n2);
+                                add(n1, n2, dg[s], ng[s]);
+                            }
+                        double g = ag.value(), h = ah.value();
+                        combine(g, h);
+                        finish(g, h);
+                        if (dl == 0.0) return;
+                        const T d = (T)dl;                   // updateXBeta and the strata's denominators
+                        auto move = [&](int i, int s, double& acc) {
+                            for (; i < m.n && __ldg(m.es + i) == s; ++i) {
+                                const T x = ind ? T(1) : (T)__ldg(m.cv + i);
+                                const int k = row(i);
+                                const T old = get(k), nv = old + d * x;
+                                put(k, nv);
+                                acc += (double)fexp(nv) - (double)fexp(old);
+                            }
+                        };
+                        #pragma unroll
+                        for (int r = 0; r < R; ++r)
+                            if (bb[r] & 1) {
+                                const T nv = vv[r] + d * xx[r];
+                                put(kk[r], nv);
+                                double acc = dd[r] + ((double)fexp(nv) - (double)ex[r]);
+                                if (bb[r] & 2) move(tid + r * NT + 1, ss[r], acc);
+                                dg[ss[r]] = acc;
+                            }
+                        if (R == kR)
+                            for (int i = kR * NT + tid; i < m.n; i += NT) {
+                                const int s = __ldg(m.es + i);
+                                if (__ldg(m.es + i - 1) == s) continue;
+                                double acc = dg[s];
+                                move(i, s, acc);
+                                dg[s] = acc;
+                            }
+                        __syncthreads();
+                    };
+                    if (m.n <= NT) column(std::integral_constant<int, 1>{});
+                    else column(std::integral_constant<int, kR>{});
+                }
+            }
+            __syncthreads();
+            if (rank == 0)
+                for (int q = tid; q < jn; q += blockDim.x) {
+                    const size_t o = fj + c_j[q];
+                    A.beta[o] = c_ob[q];
+                    A.hdelta[o] = c_oh[q];
+                    if (c_up[q]) A.col_updates[o] += 1u;
+                }
+        }
+        // ---- performCheckConvergence (:839-906)
+        ++it;
+        __syncthreads();
+        // rank 0's coefficients are staged by every CTA in the next cycle
+        if (C > 1) cluster.sync();
+        const double o = objective();
+        double conv;
+        int ill = 0;
+        if (A.conv == CYC_CONV_ZHANG_OLES) {
+            conv = o;
+        } else {
+            if (o != o) { conv = 0.0; ill = 1; }
+            else conv = fabs(o - last) / (fabs(o) + 1.0);
+            last = o;
+        }
+        if (s_dead) { flag = kTimedOut; break; }   // the same in every thread: read after a barrier
+        if (A.tol > 0 && conv < A.tol) { flag = ill ? CYC_ILLCONDITIONED : CYC_SUCCESS; break; }
+        if (it == A.max_iter) { flag = CYC_MAX_ITERATIONS; break; }
+    }
+    if (SM) {
+        __syncthreads();
+        for (int i = tid; i < nr; i += blockDim.x) xg[i] = sx[i];
+    }
+    if (C > 1) cluster.sync();   // no CTA leaves while others may still write its shared memory
+    if (rank == 0 && tid == 0) {
+        A.out_iter[f] = it;
+        A.out_flag[f] = flag;
+    }
+}
+
+// linear predictors of a CTA's rows in shared memory while they fit beside the
+// static arrays; the rest of the 256 KB stays L1
+constexpr size_t kRowBytes = 200 * 1024;
+
+template <class T, int MODEL, int WM, bool SM>
+void launch_one(const CcdArgs& a, size_t dyn, cudaStream_t stream) {
+    auto kern = k_ccd<T, MODEL, WM, SM>;
+    if (SM) CYC_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowBytes));
+    if (a.C > 8) CYC_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.F * a.C);
+    cfg.blockDim = dim3(a.threads);
+    cfg.dynamicSmemBytes = dyn;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = a.C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CYC_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, (const CcdArgs)a));
+    count_launch();
+}
+
+template <class T, int MODEL, int WM>
+void launch_rows(const CcdArgs& a, const std::vector<int>& rpart, cudaStream_t stream) {
+    int rows = 0;
+    for (int r = 0; r < a.C; ++r) rows = std::max(rows, rpart[r + 1] - rpart[r]);
+    const size_t bytes = (size_t)rows * sizeof(T);
+    const char* xs = std::getenv("CYC_BATCH_XB_SMEM");      // 0: global memory
+    const bool fits = bytes <= kRowBytes && !(xs && std::atoi(xs) == 0);
+    if constexpr (sizeof(T) == 8) {
+        if (fits) return launch_one<T, MODEL, WM, true>(a, bytes, stream);
+    }
+    launch_one<T, MODEL, WM, false>(a, 0, stream);
+}
+
+template <class T, int MODEL>
+void launch_weights(const CcdArgs& a, const std::vector<int>& rpart, cudaStream_t stream) {
+    switch (a.weights) {
+    case 0: launch_rows<T, MODEL, 0>(a, rpart, stream); break;
+    case 1: launch_rows<T, MODEL, 1>(a, rpart, stream); break;
+    default: launch_rows<T, MODEL, 2>(a, rpart, stream); break;
+    }
+}
+
+__global__ void k_entry_folds(long long n, const int* __restrict__ idx, const signed char* __restrict__ fold,
+                              signed char* __restrict__ out) {
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
+        out[e] = fold[idx[e]];
+}
+
+}  // namespace
+
+template <class T>
+void launch_ccd(const CcdArgs& a, const std::vector<int>& rpart, cudaStream_t stream) {
+    switch (a.model) {
+    case CYC_LR: launch_weights<T, CYC_LR>(a, rpart, stream); break;
+    case CYC_PR: launch_weights<T, CYC_PR>(a, rpart, stream); break;
+    case CYC_CLR: launch_weights<T, CYC_CLR>(a, rpart, stream); break;
+    case CYC_CPR: launch_weights<T, CYC_CPR>(a, rpart, stream); break;
+    default: throw Error{CYC_ERR_UNSUPPORTED, "the persistent solver supports lr, pr, clr, cpr"};
+    }
+}
+template void launch_ccd<double>(const CcdArgs&, const std::vector<int>&, cudaStream_t);
+template void launch_ccd<float>(const CcdArgs&, const std::vector<int>&, cudaStream_t);
+
+// clusters of this shape the device holds at once (as one representative of the
+// kernel's instances is held: their register counts differ little)
+static int resident_fits(int C, int threads, size_t dyn) {
+    auto kern = k_ccd<double, CYC_LR, 1, true>;
+    CYC_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowBytes));
+    CYC_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = dyn;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    CYC_CHECK_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
+    return n;
+}
+
+// The shape with the least modelled time of a cycle.  Measured here: a step
+// takes 0.84 us with 128 threads a CTA and 0.95 with 256 (more warps at every
+// barrier), 0.2 to 0.3 more when its sums cross a cluster, and 0.4 or 0.5 us
+// for every further round of the threads over a CTA's share of the column; fits
+// whose clusters the device does not hold side by side wait their turn.
+// (10k rows, 1,000 columns of 100 entries: 35 ms for 41 cycles with one CTA,
+// 43 to 48 with clusters; 100k rows, 600 Zipf columns and 4 dense ones: 116 ms
+// for 40 cycles with one CTA of 256 threads, 46 with four, 30 with sixteen.)
+CcdShape ccd_shape(const Dataset& ds, int F) {
+    const double cross[] = {0.0, 0.2, 0.22, 0.26, 0.3};
+    CcdShape best{1, 128, 0.0};
+    int log2c = 0;
+    for (int C = 1; C <= kCcdCluster; C *= 2, ++log2c) {
+        for (int threads = 128; threads <= kCcdThreads; threads *= 2) {
+            const size_t bytes = ((size_t)ds.K + C - 1) / C * sizeof(double);
+            const int slots = resident_fits(C, threads, bytes <= kRowBytes ? bytes : 0);
+            if (slots < 1) continue;
+            // predictors of the fits in flight that neither shared memory nor
+            // L2 holds come from HBM, a row at a time
+            const bool far = bytes > kRowBytes && (double)std::min(F, slots) * ds.K * sizeof(double) > 100e6;
+            const double round = far ? 1.2 : (threads == 128 ? 0.4 : 0.5);
+            double us = 0.0;
+            for (int j = 0; j < ds.J; ++j) {
+                const double rounds = std::ceil((double)ds.col_len(j) / (C * threads));
+                us += (threads == 128 ? 0.84 : 0.95) + (far ? 0.5 : 0.0) + cross[log2c] + round * std::max(0.0, rounds - 1.0);
+            }
+            us *= (F + slots - 1) / slots;
+            if (best.cycle_us == 0.0 || us < best.cycle_us) best = {C, threads, us};
+        }
+    }
+    // CYC_BATCH_CLUSTER="CTAs[,threads]" fixes the shape
+    if (const char* e = std::getenv("CYC_BATCH_CLUSTER")) {
+        int c = best.C, t = best.threads;
+        std::sscanf(e, "%d,%d", &c, &t);
+        best.C = std::max(1, std::min(kCcdCluster, c));
+        best.threads = std::max(32, std::min(kCcdThreads, t / 32 * 32));
+    }
+    return best;
+}
+
+std::vector<int> ccd_rows(const Dataset& ds, int C) {
+    std::vector<int> rpart(C + 1, ds.K);
+    for (int r = 0; r < C; ++r) {
+        int b = (int)((long long)ds.K * r / C);
+        if (model_grouped(ds.model)) {
+            auto it = std::lower_bound(ds.strat_ptr.begin(), ds.strat_ptr.end(), b);
+            b = (it == ds.strat_ptr.end()) ? ds.K : *it;
+        }
+        rpart[r] = b;
+    }
+    for (int r = 1; r <= C; ++r) rpart[r] = std::max(rpart[r], rpart[r - 1]);
+    return rpart;
+}
+
+void ccd_splits(const Dataset& ds, int C, const int* d_rpart, int* d_split, cudaStream_t stream) {
+    launch(k_splits, (ds.J * (C + 1) + 255) / 256, 256, 0, stream, ds.J, C, ds.d_fmt.get(), ds.d_col_ptr.get(),
+           ds.d_idx.get(), d_rpart, d_split);
+}
+
+void ccd_entry_folds(const Dataset& ds, const signed char* d_fold, signed char* d_out, cudaStream_t stream) {
+    if (ds.nnz_idx)
+        launch(k_entry_folds, grid_for(ds.nnz_idx, 4), kThreads, 0, stream, ds.nnz_idx, (const int*)ds.d_idx.get(),
+               d_fold, d_out);
+}
+
+}  // namespace cyc

@@ -1,0 +1,76 @@
+// ccd.cuh -- the one-fit persistent CCD kernel (ccd.cu): arguments, launch
+// shape and launch.
+#pragma once
+#include "internal.cuh"
+
+namespace cyc {
+
+constexpr int kCcdThreads = 256;   // most threads a CTA has
+constexpr int kCcdCluster = 16;    // most CTAs a fit has (the non-portable cluster limit)
+// out_flag of a fit whose CTAs lost one another (a bounded wait ran out)
+constexpr int kTimedOut = -1;
+
+// F fits over one dataset, each a thread-block cluster of C CTAs that split
+// the rows.  Arrays marked [F] hold one element per fit.
+struct CcdArgs {
+    int model, K, J, S, F, C;
+    int threads;                  // per CTA, a multiple of 32 up to kCcdThreads
+    int weights;                  // 0: all ones; 1: CV folds; 2: `w`
+    int strict_mean;              // logistic mean as exb / (1 + exb), NaN where exb overflows (as the
+                                  // per-coordinate engine), else 1 / (1 + exp(-xb))
+    const int* fmt;
+    const long long* col_ptr;
+    const long long* val_ptr;
+    const int* idx;
+    const double* val;
+    const int* entry_strat;       // stratum of every entry of idx (grouped models)
+    const int* split;             // J x (C+1): first entry of rank r's rows, relative to the column
+    const int* rpart;             // C+1 row boundaries
+    const double* y;
+    const int* strat;             // K (grouped)
+    const int* cols;              // the columns a fit steps through, in order; fit f's at f * cols_stride
+    const int* ncols;             // their number; fit f's at f * ncols_stride
+    int cols_stride, ncols_stride;
+    const int* ptype;             // J
+    void* xb;                     // [F][K] T linear predictors, current on entry and exit
+    void* xb_save;                // [F][K] T (Zhang-Oles convergence)
+    const void* w;                // [F][K] T row weights (weights == 2)
+    const signed char* fold;      // K fold id per row (weights == 1)
+    const signed char* entry_fold;   // fold id of every entry of idx (weights == 1)
+    const int* fitfold;           // [F] held-out fold
+    double* denom;                // [F][S] (grouped), current on entry
+    const double* nw;             // [F][S] (grouped)
+    const double* xjy;            // [F][J]
+    double* beta;                 // [F][J]
+    double* hdelta;               // [F][J]
+    const double* variance;       // [F]
+    const double* llfixed;        // [F]
+    const int* active;            // [F] 0: the fit is left alone; null: all run
+    unsigned* col_updates;        // [F][J] steps that moved a coefficient, added to
+    int conv;
+    double tol;
+    int max_iter;
+    int* out_iter;                // [F]
+    int* out_flag;                // [F]
+};
+
+// CTAs a fit and threads a CTA for F one-fit solves of a dataset, and the
+// modelled time of a cycle of them all
+struct CcdShape {
+    int C, threads;
+    double cycle_us;
+};
+CcdShape ccd_shape(const Dataset& ds, int F);
+// row boundaries of C CTAs, at stratum starts for grouped models
+std::vector<int> ccd_rows(const Dataset& ds, int C);
+// the split of every column's entries over those boundaries
+void ccd_splits(const Dataset& ds, int C, const int* d_rpart, int* d_split, cudaStream_t stream);
+
+// fold ids of the entries of idx (CV folds), so that a column's load beside its row ids
+void ccd_entry_folds(const Dataset& ds, const signed char* d_fold, signed char* d_out, cudaStream_t stream);
+
+// one launch of the F fits (T: double, or float with compensated sums)
+template <class T>
+void launch_ccd(const CcdArgs& a, const std::vector<int>& rpart, cudaStream_t stream);
+
+}  // namespace cyc

@@ -17,6 +17,7 @@
 // reference's column-by-column axpy order.
 #include "internal.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -82,7 +83,7 @@ void prepare_pool(int device) {
 size_t Dataset::device_bytes() const {
     return d_fmt.bytes() + d_col_ptr.bytes() + d_val_ptr.bytes() + d_idx.bytes() + d_val.bytes() +
            d_y.bytes() + d_time.bytes() + d_strat.bytes() + d_strat_ptr.bytes() + d_row_ptr.bytes() +
-           d_row_col.bytes() + d_row_val.bytes();
+           d_row_col.bytes() + d_row_val.bytes() + d_entry_strat.bytes();
 }
 
 // on the calling thread's allocation stream (the dataset's, during uploads)
@@ -133,6 +134,24 @@ void Dataset::ensure_csr() {
     upload(d_row_val, rv.data(), rv.size());
     CYC_CHECK_CUDA(cudaStreamSynchronize(stream));   // usable from every stream
     have_csr = true;
+}
+
+__global__ void k_entry_strata(long long n, const int* __restrict__ idx, const int* __restrict__ strat,
+                               int* __restrict__ out) {
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
+        out[e] = strat[idx[e]];
+}
+
+void Dataset::ensure_entry_strata() {
+    std::lock_guard<std::mutex> lock(csr_mutex);
+    if (have_entry_strata) return;
+    StreamScope scope(stream);
+    d_entry_strat.alloc(std::max<long long>(1, nnz_idx));
+    if (nnz_idx)
+        launch(k_entry_strata, grid_for(nnz_idx, 4), kThreads, 0, stream, nnz_idx, (const int*)d_idx.get(),
+               (const int*)d_strat.get(), d_entry_strat.get());
+    CYC_CHECK_CUDA(cudaStreamSynchronize(stream));   // usable from every stream
+    have_entry_strata = true;
 }
 
 }  // namespace cyc

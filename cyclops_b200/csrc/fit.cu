@@ -8,6 +8,7 @@
 // one-thread kernel between the gradient and update kernels, beta / the trust
 // region / delta stay in device memory, and one cycle is replayed as CUDA
 // graphs.  The host reads two flags per cycle (the convergence test).
+#include "ccd.cuh"
 #include "engine.cuh"
 #include "solver_common.cuh"
 
@@ -71,6 +72,10 @@ __global__ void k_zhang_oles(int K, const double* __restrict__ xb, double* __res
         b += fabs(xb[k]) * w;
     }
     grid_sum2_finalize(a, b, partial, ticket, [&](double A, double B) { *out = A / (1.0 + B); });
+}
+
+__global__ void k_fill(int n, double v, double* __restrict__ out) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = v;
 }
 
 __global__ void k_copy(int K, const double* __restrict__ src, double* __restrict__ dst) {
@@ -201,13 +206,77 @@ struct FitRunner {
         CYC_CHECK_LAUNCH();
     }
 
+    // ---- lr, pr, clr, cpr: findMode as one launch of the persistent kernel
+    std::vector<int> rpart, cols_fix;
+    DevBuf<int> d_rpart, d_split, d_cols, d_ncols, d_out;
+    DevBuf<double> d_variance;
+    CcdArgs ccd{};
+
+    void prepare_ccd() {
+        Dataset& ds = *e.ds;
+        const CcdShape shape = ccd_shape(ds, 1);
+        rpart = ccd_rows(ds, shape.C);
+        d_rpart.alloc(shape.C + 1); d_split.alloc((size_t)J * (shape.C + 1)); d_cols.alloc(J); d_ncols.alloc(1);
+        d_out.alloc(2); d_variance.alloc(1);
+        CYC_CHECK_CUDA(cudaMemcpyAsync(d_rpart.get(), rpart.data(), (shape.C + 1) * sizeof(int), cudaMemcpyHostToDevice,
+                                       e.stream));
+        CYC_CHECK_CUDA(cudaMemcpyAsync(d_variance.get(), &variance, sizeof(double), cudaMemcpyHostToDevice, e.stream));
+        ccd_splits(ds, shape.C, d_rpart.get(), d_split.get(), e.stream);
+        if (model_grouped(ds.model)) ds.ensure_entry_strata();
+        ccd.model = ds.model; ccd.K = ds.K; ccd.J = J; ccd.S = ds.S; ccd.F = 1; ccd.C = shape.C;
+        ccd.threads = shape.threads;
+        ccd.weights = e.use_w ? 2 : 0;
+        ccd.strict_mean = 1;
+        ccd.fmt = ds.d_fmt.get(); ccd.col_ptr = ds.d_col_ptr.get(); ccd.val_ptr = ds.d_val_ptr.get();
+        ccd.idx = ds.d_idx.get(); ccd.val = ds.d_val.get(); ccd.entry_strat = ds.d_entry_strat.get();
+        ccd.split = d_split.get(); ccd.rpart = d_rpart.get(); ccd.y = ds.d_y.get(); ccd.strat = ds.d_strat.get();
+        ccd.cols = d_cols.get(); ccd.ncols = d_ncols.get();
+        ccd.ptype = ptype.get(); ccd.xb = e.xb.get(); ccd.w = e.kw.get();
+        ccd.denom = e.denom.get(); ccd.nw = e.nw.get(); ccd.xjy = e.xjy.get();
+        ccd.beta = beta.get(); ccd.hdelta = hdelta.get(); ccd.variance = d_variance.get();
+        ccd.llfixed = e.ll_fixed.get(); ccd.col_updates = col_updates.get();
+        ccd.out_iter = d_out.get(); ccd.out_flag = d_out.get() + 1;
+    }
+
+    int find_mode_ccd(double bound, int* iterations) {
+        launch(k_fill, grid_for(J, 1), kThreads, 0, e.stream, J, bound, hdelta.get());     // resetBounds
+        if (cols_fix != fixb) {                      // the columns not fixed now
+            std::vector<int> cols;
+            for (int j = 0; j < J; ++j)
+                if (!fixb[j]) cols.push_back(j);
+            const int n = (int)cols.size();
+            cols.push_back(n);
+            CYC_CHECK_CUDA(cudaMemcpyAsync(d_cols.get(), cols.data(), n * sizeof(int), cudaMemcpyHostToDevice, e.stream));
+            CYC_CHECK_CUDA(cudaMemcpyAsync(d_ncols.get(), cols.data() + n, sizeof(int), cudaMemcpyHostToDevice, e.stream));
+            e.sync();                                // the host list goes away
+            cols_fix = fixb;
+        }
+        ccd.conv = ctl.convergence_type;
+        ccd.tol = ctl.tolerance;
+        ccd.max_iter = ctl.max_iterations;
+        if (ccd.conv == CYC_CONV_ZHANG_OLES) {       // saveXBeta
+            e.xb_save.alloc(e.ds->K);
+            launch(k_copy, grid_for(e.ds->K, 1), kThreads, 0, e.stream, e.ds->K, e.xb.get(), e.xb_save.get());
+            ccd.xb_save = e.xb_save.get();
+        }
+        launch_ccd<double>(ccd, rpart, e.stream);
+        // exp(xbeta) and the denominators follow the linear predictors
+        e.remaining_statistics(true);
+        CYC_CHECK_CUDA(cudaMemcpyAsync(h_flags, d_out.get(), 2 * sizeof(int), cudaMemcpyDeviceToHost, e.stream));
+        e.sync();
+        CYC_REQUIRE(h_flags[1] != kTimedOut, CYC_ERR_TIMEOUT, "a wait between the CTAs of a fit ran out");
+        *iterations = h_flags[0];
+        return h_flags[1];
+    }
+
     // findMode (CyclicCoordinateDescent.cpp:909-1216), cyclic branch
     int find_mode(double bound, int* iterations) {
-        std::vector<double> hd(J, bound);                       // resetBounds
-        CYC_CHECK_CUDA(cudaMemcpyAsync(hdelta.get(), hd.data(), J * sizeof(double), cudaMemcpyHostToDevice, e.stream));
         const int conv = ctl.convergence_type;
         CYC_REQUIRE(conv >= CYC_CONV_GRADIENT && conv <= CYC_CONV_ZHANG_OLES, CYC_ERR_ARGUMENT,
                     "Unknown convergence criterion");
+        if (!model_cumulative(e.model)) return find_mode_ccd(bound, iterations);
+        std::vector<double> hd(J, bound);                       // resetBounds
+        CYC_CHECK_CUDA(cudaMemcpyAsync(hdelta.get(), hd.data(), J * sizeof(double), cudaMemcpyHostToDevice, e.stream));
         const int K = e.ds->K;
         if (conv < CYC_CONV_ZHANG_OLES) {
             launch_objective(conv);
@@ -279,7 +348,7 @@ struct FitRunner {
             flag = CYC_SUCCESS;
             if (n_active > 0) {
                 for (int j = 0; j < J; ++j) fixb[j] = !active[j];
-                build_graphs();
+                if (model_cumulative(e.model)) build_graphs();
                 flag = find_mode(bound, iterations);
             }
             if (n_inactive == 0 || flag != CYC_SUCCESS) break;
@@ -308,8 +377,9 @@ struct FitRunner {
 
     bool swindle = false;
 
-    // the graphs replay one cycle over the columns not fixed now
+    // cox: the graphs replay one cycle over the columns not fixed now
     void ensure_graphs() {
+        if (!model_cumulative(e.model)) return;
         if (graphs.empty() || graphs_fix != fixb) build_graphs();
     }
 
@@ -337,6 +407,7 @@ struct FitRunner {
     }
 
     void prepare() {
+        if (!model_cumulative(e.model)) prepare_ccd();
         e.fixed_terms_ll(true);
         e.fixed_terms_gh(true);
         set_beta(h_start);

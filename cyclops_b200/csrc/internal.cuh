@@ -205,8 +205,7 @@ struct ColView {
 // column batches of the batched solver (planned on the host, batch.cu)
 // ---------------------------------------------------------------------------
 struct RunPlan {
-    int C = 0, G = 0;
-    int batch_rows = 0;         // cap on a batch's entries in any one CTA's rows (0: none)
+    int C = 0;
     int cap = 0, dmax = 0, max_levels = 0;   // the batch shape it was planned with (short-column
                                              // bound, shared rows, replay levels)
     std::vector<int> fixed;     // columns held fixed besides the offset (ascending)
@@ -253,7 +252,11 @@ struct Dataset {
     DevBuf<int> d_row_col;
     DevBuf<double> d_row_val;
 
-    // column batches of the batched solver, cached per (cluster size, fits per group)
+    // stratum of every entry of d_idx (grouped models), built on first use
+    bool have_entry_strata = false;
+    DevBuf<int> d_entry_strat;
+
+    // column batches of the batched solver, cached per cluster size and shape
     std::vector<RunPlan> run_plans;
 
     long long col_len(int j) const {
@@ -269,6 +272,7 @@ struct Dataset {
     }
     size_t device_bytes() const;
     void ensure_csr();
+    void ensure_entry_strata();
 };
 
 // ---------------------------------------------------------------------------

@@ -28,16 +28,19 @@ __host__ __device__ inline double prior_delta_rate(int type, double variance, do
                                                    double h) {
     if (type == CYC_PRIOR_NONE) return -(g / h);
     if (type == CYC_PRIOR_NORMAL) return -(g + (beta / variance)) / (h + (1.0 / variance));
-    const double neg = -(g - lambda) / h;
-    const double pos = -(g + lambda) / h;
+    // of the two candidate steps -(g -+ lambda) / h the signs choose one before
+    // the division (the division sits on the solvers' serial chain): from
+    // beta = 0 the step down exists when g > lambda, the one up when
+    // g < -lambda; a NaN quotient takes neither
     const int s = sgn(beta);
     double delta;
     if (s == 0) {
-        if (neg < 0) delta = neg;
-        else if (pos > 0) delta = pos;
-        else delta = 0;
+        const double up = g + lambda, down = g - lambda;
+        const double num = down > 0 ? down : (up < 0 ? up : 0.0);
+        const double step = -num / h;
+        delta = (num != 0.0 && step == step) ? step : 0.0;
     } else {
-        delta = s < 0 ? neg : pos;
+        delta = -(s < 0 ? g - lambda : g + lambda) / h;
         if (sgn(beta + delta) != s) delta = -beta;
     }
     return delta;
