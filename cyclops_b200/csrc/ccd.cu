@@ -32,6 +32,7 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include "mbar.cuh"
 #include "row_terms.cuh"
 
 namespace cg = cooperative_groups;
@@ -95,39 +96,6 @@ struct ColStep {
 // rounds stay in registers from the gradient to the update.  The code of a
 // round is straight-line (one round and kR rounds as separate instances): with
 // one warp per scheduler the instructions of a step are latency too.
-// ---- the cluster exchange: 16 bytes to a peer's shared memory, counted on its mbarrier
-__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned peer_addr(unsigned addr, int rank) {
-    unsigned r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void push16(unsigned dst, unsigned mbar, double a, double b) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(dst),
-                 "l"(__double_as_longlong(a)), "l"(__double_as_longlong(b)), "r"(mbar)
-                 : "memory");
-}
-__device__ __forceinline__ void mbar_init(unsigned mbar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
-}
-__device__ __forceinline__ void mbar_expect(unsigned mbar, int bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(unsigned mbar, int phase) {
-    unsigned ok;
-    asm volatile(
-        "{\n.reg .pred p;\n"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(mbar), "r"(phase)
-        : "memory");
-    return ok != 0;
-}
-// A peer is at most one column's work away (well under a millisecond); a wait
-// that outlasts this many clocks (about two seconds) gives up.
-constexpr long long kWaitClocks = 4000000000ll;
-
 template <class T, int MODEL, int WM, bool SM>
 __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
     constexpr bool kGrouped = (MODEL == CYC_CLR || MODEL == CYC_CPR);
@@ -176,7 +144,7 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
         s_dead = 0;
         mbar_init(smem_addr(&s_mb[0]));
         mbar_init(smem_addr(&s_mb[1]));
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mbar_init_fence();
     }
     if (C > 1) cluster.sync();
     else __syncthreads();
@@ -226,11 +194,7 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
             total(s_part[par], NW);
             if (lane == 0) mbar_expect(mb, 16 * C);
             if (lane < C) push16(peer_addr(smem_addr(&s_cl[par][rank]), lane), peer_addr(mb, lane), a, b);
-            if (!s_dead && !mbar_try(mb, phase)) {
-                const long long t0 = clock64();
-                while (!mbar_try(mb, phase))
-                    if (clock64() - t0 > kWaitClocks) { s_dead = 1; break; }
-            }
+            if (!s_dead && !mbar_wait(mb, phase)) s_dead = 1;
             total(s_cl[par], C);
             if (lane == 0) s_all = make_double2(a, b);
         }

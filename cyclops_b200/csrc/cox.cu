@@ -1,0 +1,1066 @@
+// cox.cu -- the persistent Breslow Cox CCD: a fit's whole coordinate loop in
+// one launch.
+//
+// With n_e events and risk-set sum D_e at event group e, and A_e / B_e the sums
+// of a column's w exp(xb) x / x^2 over the rows at risk at e, the reference
+// walks every group for (ModelSpecifics.hpp:904-962)
+//     g = sum_e n_e A_e / D_e,   h = sum_e n_e (B_e / D_e - (A_e / D_e)^2).
+// A_e is a running sum of the column's entries, so the sums turn over:
+//     g = sum_k v_k S1(e_k),  h = sum_k v_k x_k S1(e_k) - sum_k v_k (2 A'_k + v_k) S2(e_k)
+// with v_k = w exp(xb) x of entry k, e_k its slot, A'_k the running sum before
+// it, and S1, S2 the suffix sums (within the stratum) of n/D and n/D^2.  Every
+// term of S1 and S2 has one sign and nothing is differenced, so FP64 sums in
+// tree order carry no more error than D itself.  A column then costs a pass
+// over its own entries; only a step that moves a coefficient renews the sums:
+// one pass over the event groups (about a third of the rows here), not over
+// every row, and nothing but S1 and S2 is written.
+//
+// What bounds a step is latency at small sizes (block scans, two exchanges a
+// cluster) and one division per event group at large ones, so a fit is one
+// cluster of up to 16 CTAs that split the event groups in order; their carries
+// cross by st.async on mbarriers.  The per-slot arrays stay in shared memory
+// where they fit, S1 and S2 alone where only those do, else in L2.  (Before:
+// seven launches a coordinate that rewrote nine arrays over all rows, 35 us a
+// coordinate at 20k rows and 56 us at 500k.)
+#include "cox.cuh"
+
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <cstdio>
+#include <cstdlib>
+
+#include "ccd.cuh"
+#include "mbar.cuh"
+#include "row_terms.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace cyc {
+
+namespace {
+
+constexpr int kCh = 64;           // coordinates staged at a time
+// slots of a thread taken at a time, without branches: every thread of a CTA
+// runs the same number of blocks, past its last slot on zeros
+constexpr int kB = 4;
+constexpr int kMaxC = kCcdCluster;
+// in an entry's slot position: the slot's stratum goes on past the slots of its
+// CTA (kTailBit), past those of its thread (kThreadBit)
+constexpr int kTailBit = 1 << 30, kThreadBit = 1 << 29, kPosMask = kThreadBit - 1;
+constexpr unsigned kFull = 0xffffffffu;
+
+// ---- the risk sets ------------------------------------------------------------
+
+constexpr int kTileItems = 8;
+constexpr int kTile = kThreads * kTileItems;
+
+// inclusive scan over the rows in three launches: tile totals, their scan, the
+// rows.  `item(k)` is the row's value, `op` max or plus.
+struct OpMax {
+    static constexpr int kZero = -1;
+    __device__ int operator()(int a, int b) const { return max(a, b); }
+};
+struct OpSum {
+    static constexpr int kZero = 0;
+    __device__ int operator()(int a, int b) const { return a + b; }
+};
+
+template <class Op>
+__device__ int block_scan(int v, int* s_w) {      // inclusive over the block's threads
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    Op op;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(kFull, v, o);
+        if (lane >= o) v = op(u, v);
+    }
+    if (lane == 31) s_w[w] = v;
+    __syncthreads();
+    int pre = Op::kZero;
+    for (int q = 0; q < w; ++q) pre = op(pre, s_w[q]);
+    __syncthreads();
+    return op(pre, v);
+}
+
+template <class Op, class Item>
+__global__ void k_rows_totals(int K, Item item, int* __restrict__ tiles) {
+    __shared__ int s_w[kThreads / 32];
+    const int k0 = blockIdx.x * kTile + threadIdx.x * kTileItems;
+    Op op;
+    int v = Op::kZero;
+    for (int i = 0; i < kTileItems; ++i)
+        if (k0 + i < K) v = op(v, item(k0 + i));
+    v = block_scan<Op>(v, s_w);
+    if (threadIdx.x == kThreads - 1) tiles[blockIdx.x] = v;
+}
+
+template <class Op>
+__global__ void k_tiles_scan(int n, int* __restrict__ tiles) {       // one block: exclusive, in place
+    __shared__ int s_w[kThreads / 32];
+    __shared__ int s_carry;
+    Op op;
+    if (threadIdx.x == 0) s_carry = Op::kZero;
+    __syncthreads();
+    for (int b = 0; b < n; b += kThreads) {
+        const int i = b + threadIdx.x;
+        const int v = i < n ? tiles[i] : Op::kZero;
+        const int inc = op(s_carry, block_scan<Op>(v, s_w));
+        __syncthreads();
+        int ex = __shfl_up_sync(kFull, inc, 1);
+        if ((threadIdx.x & 31) == 31) s_w[threadIdx.x >> 5] = inc;
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) ex = threadIdx.x == 0 ? s_carry : s_w[(threadIdx.x >> 5) - 1];
+        if (i < n) tiles[i] = ex;
+        __syncthreads();
+        if (threadIdx.x == kThreads - 1) s_carry = inc;
+        __syncthreads();
+    }
+}
+
+template <class Op, class Item>
+__global__ void k_rows_scan(int K, Item item, const int* __restrict__ tiles, int* __restrict__ out) {
+    __shared__ int s_w[kThreads / 32];
+    const int k0 = blockIdx.x * kTile + threadIdx.x * kTileItems;
+    Op op;
+    int v[kTileItems];
+    int t = Op::kZero;
+    for (int i = 0; i < kTileItems; ++i) {
+        t = op(t, k0 + i < K ? item(k0 + i) : Op::kZero);
+        v[i] = t;
+    }
+    const int inc = block_scan<Op>(t, s_w);
+    int pre = __shfl_up_sync(kFull, inc, 1);
+    if ((threadIdx.x & 31) == 31) s_w[threadIdx.x >> 5] = inc;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) pre = threadIdx.x == 0 ? Op::kZero : s_w[(threadIdx.x >> 5) - 1];
+    pre = op(tiles[blockIdx.x], pre);
+    for (int i = 0; i < kTileItems; ++i)
+        if (k0 + i < K) out[k0 + i] = op(pre, v[i]);
+}
+
+struct LastWeighted {                // the row itself where it has weight
+    const double* w;
+    __device__ int operator()(int k) const { return w[k] != 0.0 ? k : -1; }
+};
+// 1 where a row starts an event group (setPidForAccumulation's rule,
+// ModelSpecifics.hpp:1809-1868: consecutive weighted rows share a group when
+// both are events at one time of one stratum)
+struct GroupStart {
+    const double *w, *y, *time;
+    const int *strat, *last;         // last weighted row up to each row (null: every row)
+    __device__ int operator()(int k) const {
+        if (y[k] == 0.0 || (w && w[k] == 0.0)) return 0;
+        const int p = k == 0 ? -1 : (last ? last[k - 1] : k - 1);
+        if (p < 0 || strat[p] != strat[k]) return 1;
+        return !(y[p] == 1.0 && time[p] == time[k] && y[p] == y[k]);
+    }
+};
+
+__global__ void k_slot_rows(int K, const double* __restrict__ w, const double* __restrict__ y,
+                            const int* __restrict__ strat, const int* __restrict__ cnt, int* __restrict__ first,
+                            int* __restrict__ end, int* __restrict__ sstr, int* __restrict__ total) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x) {
+        if (k == K - 1) *total = cnt[k];
+        if (y[k] == 0.0 || (w && w[k] == 0.0)) continue;
+        const int e = cnt[k] - 1;
+        atomicMax(end + e, k);
+        if (k == 0 || cnt[k - 1] == e) {
+            first[e] = k;
+            sstr[e] = strat[k];
+        }
+    }
+}
+
+// the split of the slots over the CTAs, and the rows that go with it (a CTA's
+// rows end with its last slot's last event; the last CTA takes the rest)
+__global__ void k_slot_parts(int K, int C, const int* __restrict__ total, const int* __restrict__ end,
+                             int* __restrict__ spart, int* __restrict__ rpart) {
+    const int E = *total;
+    for (int r = threadIdx.x; r <= C; r += blockDim.x) {
+        const int s = (int)((long long)E * r / C);
+        spart[r] = s;
+        rpart[r] = r == 0 ? 0 : (r == C ? K : (s == 0 ? 0 : end[s - 1] + 1));
+    }
+}
+
+__device__ __forceinline__ int slot_position(int e, int C, int nt, const int* spart, int& r) {
+    r = 0;
+    while (r + 1 < C && e >= spart[r + 1]) ++r;
+    const int s0 = spart[r], ns = spart[r + 1] - s0, m = (ns + nt - 1) / nt;
+    const int q = e - s0;
+    return (q % m) * nt + q / m;
+}
+
+// per slot (a warp each): events, first row, flags
+__global__ void k_slots(int C, int nt, int per_cta, const int* __restrict__ total, const int* __restrict__ spart,
+                        const int* __restrict__ first, const int* __restrict__ end, const int* __restrict__ sstr,
+                        const int* __restrict__ strat_ptr, const double* __restrict__ w, const double* __restrict__ y,
+                        int* __restrict__ lo, unsigned char* __restrict__ flag, double* __restrict__ n) {
+    const int E = *total, lane = threadIdx.x & 31;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < E; e += nwarps) {
+        double a = 0.0;
+        for (int k = first[e] + lane; k <= end[e]; k += 32) a += y[k] * (w ? w[k] : 1.0);
+        for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(kFull, a, o);
+        if (lane == 0) {
+            const int s = sstr[e];
+            const bool starts = e == 0 || sstr[e - 1] != s, ends = e + 1 == E || sstr[e + 1] != s;
+            lo[e] = starts ? strat_ptr[s] : end[e - 1] + 1;
+            int r;
+            const int p = slot_position(e, C, nt, spart, r);
+            n[(size_t)r * per_cta + p] = a;
+            flag[(size_t)r * per_cta + p] = (unsigned char)((starts ? 1 : 0) | (ends ? 2 : 0));
+        }
+    }
+}
+
+// sums of w exp(xb) over each slot's rows (a warp each)
+__global__ void k_slot_increments(int C, int nt, int per_cta, const int* __restrict__ total, const int* __restrict__ spart,
+                                  const int* __restrict__ lo, const int* __restrict__ end,
+                                  const double* __restrict__ w, const double* __restrict__ xb,
+                                  double* __restrict__ d) {
+    const int E = *total, lane = threadIdx.x & 31;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < E; e += nwarps) {
+        double a = 0.0;
+        for (int k = lo[e] + lane; k <= end[e]; k += 32) {
+            const double wk = w ? w[k] : 1.0;
+            if (wk != 0.0) a += wk * exp(xb[k]);
+        }
+        for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(kFull, a, o);
+        if (lane == 0) {
+            int r;
+            const int p = slot_position(e, C, nt, spart, r);
+            d[(size_t)r * per_cta + p] = a;
+        }
+    }
+}
+
+// every row's slot position in its CTA (-1: none), with kTailBit and kThreadBit.
+// Rows of weight zero get the slot their
+// place in the order gives (they add nothing), so a column's slots ascend.
+__global__ void k_row_slots(int K, int C, int nt, const int* __restrict__ total, const int* __restrict__ spart,
+                            const int* __restrict__ sstr, const int* __restrict__ end,
+                            const int* __restrict__ strat, const int* __restrict__ cnt, int* __restrict__ out) {
+    const int E = *total;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x) {
+        int o = -1;
+        const int e = cnt[k] > 0 && end[cnt[k] - 1] >= k ? cnt[k] - 1 : cnt[k];
+        if (e < E && sstr[e] == strat[k]) {
+            int r;
+            o = slot_position(e, C, nt, spart, r);
+            const int s0 = spart[r], next = spart[r + 1], m = (next - s0 + nt - 1) / nt;
+            const int after = min(next, s0 + ((e - s0) / m + 1) * m);       // first slot past its thread's
+            if (next < E && sstr[next] == sstr[e]) o |= kTailBit;
+            if (after < E && sstr[after] == sstr[e]) o |= kThreadBit;
+        }
+        out[k] = o;
+    }
+}
+
+__global__ void k_entry_slots(long long nnz, const int* __restrict__ idx, const int* __restrict__ rowslot,
+                              int* __restrict__ out) {
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nnz; e += (long long)gridDim.x * blockDim.x)
+        out[e] = rowslot[idx[e]];
+}
+
+// ---- the solver ------------------------------------------------------------------
+
+struct ColMeta {
+    const int* ci;       // row ids (null for dense columns: entry i is row r0 + i)
+    const double* cv;    // values (null for indicators)
+    const int* es;       // slot positions of the entries
+    const int* st;       // strata of the entries (null: one stratum)
+    int n;
+    int before;          // the column has entries before this CTA's rows
+};
+
+// WHERE the per-slot arrays live: 0 all in shared memory, 1 S1 and S2 (and the
+// flags), 2 global memory.  kNT threads: few while a thread has few slots (the
+// scans cost every warp the same, so warps without work only take issue slots;
+// 512 threads took 26 ms where 128 take 13 at 20k rows x 500 columns).  SEG:
+// more than one stratum, so sums restart at their boundaries.
+template <int WHERE, int kNT, bool SEG>
+__global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs A) {
+    constexpr int kNW = kNT / 32;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int C = A.C;
+    const int rank = C > 1 ? (int)cluster.block_rank() : 0;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int r0 = A.rpart[rank], nr = A.rpart[rank + 1] - r0;
+    const int ns = A.spart[rank + 1] - A.spart[rank];
+    const int m = (ns + kNT - 1) / kNT;                   // slots of a thread
+    const int mine = max(0, min(m, ns - tid * m));
+    double* const xg = A.xb + r0;                         // this CTA's rows, relative to r0
+    const double* const wg = A.weighted ? A.w + r0 : nullptr;
+    const double var = A.variance;
+    const double lam = sqrt(2.0 / var);                   // LaplacePrior rate, CovariatePrior.h:282-292
+    const size_t base_slot = (size_t)rank * A.per_cta;
+
+    extern __shared__ __align__(16) unsigned char dyn_smem[];
+    double* const sm = reinterpret_cast<double*>(dyn_smem);
+    const int nb = (m + kB - 1) / kB;                     // blocks of kB slots of a thread
+    const int np = nb * kB * kNT;                         // positions in use
+    double* const S1 = WHERE <= 1 ? sm : A.S1 + base_slot;
+    double* const S2 = WHERE <= 1 ? sm + np : A.S2 + base_slot;
+    double* const dd = WHERE == 0 ? sm + 2 * np : A.d + base_slot;
+    double* const nn = WHERE == 0 ? sm + 3 * np : const_cast<double*>(A.n) + base_slot;
+    // the sums before each block of kB slots of a thread
+    double* const bp = WHERE <= 1 ? sm + (WHERE == 0 ? 4 : 2) * np : A.bp + base_slot / kB;
+    unsigned char* const fl = WHERE <= 1 ? reinterpret_cast<unsigned char*>(bp + nb * kNT)
+                                         : const_cast<unsigned char*>(A.flag) + base_slot;
+
+    __shared__ double s_a[2][kNW], s_b[2][kNW];           // warp totals of a scan, by parity
+    __shared__ int s_f[2][kNW];
+    __shared__ double s_sum[5][kNW];                      // a column's sums by warp
+    // exchanges: A (risk-set totals), B (a column's sums, three pieces), C (suffix totals)
+    __shared__ __align__(16) double2 x_a[2][kMaxC], x_c[2][kMaxC], x_b[2][3][kMaxC];
+    __shared__ __align__(8) unsigned long long s_mb[3][2];
+    __shared__ double s_carry, s_c1, s_c2, s_dl;
+    __shared__ int s_dead;
+    __shared__ int s_hasend[kMaxC];
+    __shared__ ColMeta c_m[kCh + 1];
+    __shared__ double c_beta[kCh], c_hd[kCh], c_xjy[kCh], c_ob[kCh], c_oh[kCh];
+    __shared__ int c_j[kCh], c_pt[kCh], c_up[kCh];
+    __shared__ double s_mv[kNT];                          // the entries' changes of their slots
+    __shared__ int s_ms[kNT];                             // and the slots
+    __shared__ double s_post1[kNT], s_post2[kNT];         // what follows each thread's slots in S1 and S2
+
+    if (tid == 0) {
+        s_dead = 0;
+        s_carry = s_c1 = s_c2 = 0.0;
+        for (int i = 0; i < 6; ++i) mbar_init(smem_addr(&s_mb[i / 2][i % 2]));
+        mbar_init_fence();
+    }
+    if (WHERE <= 1)
+        for (int p = tid; p < np; p += kNT) {
+            if (SEG) fl[p] = A.flag[base_slot + p];
+            if (WHERE == 0) {
+                dd[p] = A.d[base_slot + p];
+                nn[p] = A.n[base_slot + p];
+            }
+        }
+    __syncthreads();
+    auto starts = [&](int p) { return SEG && (fl[p] & 1); };
+    auto ends = [&](int p) { return SEG && (fl[p] & 2); };
+    // this thread's first slot that starts a stratum, whether one ends in its
+    // slots, and whether one ends in the CTA's
+    int first_start = m, has_end = 0;
+    if (SEG)
+        for (int i = mine - 1; i >= 0; --i) {
+            if (starts(i * kNT + tid)) first_start = i;
+            has_end |= ends(i * kNT + tid);
+        }
+    const int my_end = __syncthreads_or(has_end);
+    if (C > 1) {
+        cluster.sync();                                   // mbarriers are ready, peers are here
+        if (tid < C) *cluster.map_shared_rank(&s_hasend[rank], tid) = my_end;
+        cluster.sync();
+    }
+
+    int use[3] = {0, 0, 0};                               // exchanges of each kind so far
+    auto wait = [&](int kind) {                           // warp 0
+        const int i = use[kind];
+        if (!s_dead && !mbar_wait(smem_addr(&s_mb[kind][i & 1]), (i >> 1) & 1)) s_dead = 1;
+    };
+    int par = 0;                                          // of the next block scan
+
+    // exclusive segmented sum over the threads in order: (f, a) of this thread
+    // becomes the sum since the last segment start before it (f: there is one);
+    // the block's own total in (tf, ta).  One __syncthreads.
+    auto warp_up = [&](int& f, double& a) {               // inclusive, within the warp
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int uf = SEG ? __shfl_up_sync(kFull, f, o) : 0;
+            const double ua = __shfl_up_sync(kFull, a, o);
+            if (lane >= o) {
+                if (!SEG || !f) a = ua + a;
+                f |= uf;
+            }
+        }
+    };
+    // sum of v over the lanes [lo, hi) of the warps' totals (hi <= kNW)
+    auto among = [&](double v, int lo, int hi) {
+        v = lane >= lo && lane < hi ? v : 0.0;
+        #pragma unroll
+        for (int o = kNW / 2; o; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+        return __shfl_sync(kFull, v, 0);
+    };
+    auto scan_up = [&](int& f, double& a, int& tf, double& ta) {
+        warp_up(f, a);
+        if (lane == 31) { s_f[par][warp] = f; s_a[par][warp] = a; }
+        int ef = SEG ? __shfl_up_sync(kFull, f, 1) : 0;
+        double ea = __shfl_up_sync(kFull, a, 1);
+        if (lane == 0) { ef = 0; ea = 0.0; }
+        __syncthreads();
+        if constexpr (kNW <= 8) {                         // few totals: in order
+            int pf = 0, qf = 0;
+            double pa = 0.0, qa = 0.0;
+            #pragma unroll
+            for (int w = 0; w < kNW; ++w) {
+                if (w == warp) { pf = qf; pa = qa; }
+                const int wf = SEG ? s_f[par][w] : 0;
+                qa = SEG && wf ? s_a[par][w] : qa + s_a[par][w];
+                qf |= wf;
+            }
+            tf = qf;
+            ta = qa;
+            a = ef ? ea : pa + ea;
+            f = ef | pf;
+            par ^= 1;
+            return;
+        }
+        const double wa = s_a[par][lane & (kNW - 1)];
+        const unsigned fm = SEG ? __ballot_sync(kFull, lane < kNW && s_f[par][lane & (kNW - 1)]) : 0u;
+        const unsigned before = fm & ((1u << warp) - 1u);
+        const double pa = among(wa, before ? 31 - __clz(before) : 0, warp);
+        if (C > 1 && warp == 0) {                         // the block's total, for the peers
+            tf = fm != 0;
+            ta = among(wa, fm ? 31 - __clz(fm) : 0, kNW);
+        }
+        a = ef ? ea : pa + ea;
+        f = ef | (before != 0);
+        par ^= 1;
+    };
+    // the same over the threads in reverse, for two sums (f: a segment ends)
+    auto scan_down = [&](int f, double& a, double& b, double& ta, double& tb) {
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int uf = SEG ? __shfl_down_sync(kFull, f, o) : 0;
+            const double ua = __shfl_down_sync(kFull, a, o), ub = __shfl_down_sync(kFull, b, o);
+            if (lane + o < 32) {
+                if (!SEG || !f) { a += ua; b += ub; }
+                f |= uf;
+            }
+        }
+        if (lane == 0) { s_f[par][warp] = f; s_a[par][warp] = a; s_b[par][warp] = b; }
+        int ef = SEG ? __shfl_down_sync(kFull, f, 1) : 0;
+        double ea = __shfl_down_sync(kFull, a, 1), eb = __shfl_down_sync(kFull, b, 1);
+        if (lane == 31) { ef = 0; ea = eb = 0.0; }
+        __syncthreads();
+        if constexpr (kNW <= 8) {
+            double pa = 0.0, pb = 0.0, qa = 0.0, qb = 0.0;
+            #pragma unroll
+            for (int w = kNW - 1; w >= 0; --w) {
+                if (w == warp) { pa = qa; pb = qb; }
+                const int wf = SEG ? s_f[par][w] : 0;
+                qa = SEG && wf ? s_a[par][w] : qa + s_a[par][w];
+                qb = SEG && wf ? s_b[par][w] : qb + s_b[par][w];
+            }
+            ta = qa;
+            tb = qb;
+            a = ef ? ea : ea + pa;
+            b = ef ? eb : eb + pb;
+            par ^= 1;
+            return;
+        }
+        const double wa = s_a[par][lane & (kNW - 1)], wb = s_b[par][lane & (kNW - 1)];
+        const unsigned fm = SEG ? __ballot_sync(kFull, lane < kNW && s_f[par][lane & (kNW - 1)]) : 0u;
+        const unsigned after = fm & ~((2u << warp) - 1u);
+        const int hi = after ? __ffs(after) : kNW;        // the first later warp with an end, included
+        const double pa = among(wa, warp + 1, hi), pb = among(wb, warp + 1, hi);
+        if (C > 1 && warp == 0) {
+            const int h0 = fm ? __ffs(fm) : kNW;
+            ta = among(wa, 0, h0);
+            tb = among(wb, 0, h0);
+        }
+        a = ef ? ea : ea + pa;
+        b = ef ? eb : eb + pb;
+        par ^= 1;
+    };
+
+    // The risk-set sum before this thread's first slot (where no stratum starts
+    // in between); leaves the sums before each block of its slots in `bp` and
+    // the last block's increments in dv.
+    double dv[kB];
+    auto risk_prefix = [&]() -> double {
+        double a = 0.0, nx[kB];
+        #pragma unroll
+        for (int u = 0; u < kB; ++u) nx[u] = nb > 0 ? dd[u * kNT + tid] : 0.0;
+        for (int b = 0; b < nb; ++b) {
+            #pragma unroll
+            for (int u = 0; u < kB; ++u) dv[u] = nx[u];
+            if (b + 1 < nb) {
+                #pragma unroll
+                for (int u = 0; u < kB; ++u) nx[u] = dd[((b + 1) * kB + u) * kNT + tid];
+            }
+            bp[b * kNT + tid] = a;
+            #pragma unroll
+            for (int u = 0; u < kB; ++u) a = starts((b * kB + u) * kNT + tid) ? dv[u] : a + dv[u];
+        }
+        int f = SEG && first_start < mine, tf = 0;
+        double ta = 0.0;
+        scan_up(f, a, tf, ta);
+        if (C > 1) {
+            if (warp == 0) {
+                const int i = use[0] & 1;
+                const unsigned mb = smem_addr(&s_mb[0][i]);
+                if (lane == 0) mbar_expect(mb, 16 * C);
+                if (lane < C) push16(peer_addr(smem_addr(&x_a[i][rank]), lane), peer_addr(mb, lane), ta, tf ? 1.0 : 0.0);
+                wait(0);
+                double c = 0.0;
+                for (int r = 0; r < rank; ++r) {
+                    const double2 t = x_a[i][r];
+                    c = t.y != 0.0 ? t.x : c + t.x;
+                }
+                if (lane == 0) s_carry = c;
+            }
+            ++use[0];
+            __syncthreads();
+            if (!f) a = s_carry + a;
+        }
+        return a;
+    };
+    // the risk-set sums of block b's slots in `out` from the increments `in` (1
+    // past the thread's last slot)
+    auto risk_sums = [&](int b, double pre, const double (&in)[kB], double (&out)[kB]) {
+        double run = bp[b * kNT + tid];
+        #pragma unroll
+        for (int u = 0; u < kB; ++u) {
+            const int i = b * kB + u;
+            run = starts(i * kNT + tid) ? in[u] : run + in[u];
+            out[u] = i >= mine ? 1.0 : (!SEG || i < first_start ? pre + run : run);
+        }
+    };
+
+    // S1, S2 from the risk-set increments (computeAccumlatedDenominator and the
+    // n/D terms, ModelSpecifics.hpp:1670-1694), the thread's slots from the last
+    // to the first; what follows them in the stratum is left in s_post1/2 (later
+    // threads) and s_c1/2 (later CTAs) for the entries to add.
+    auto renew = [&]() {
+        const double pre = risk_prefix();
+        double a1 = 0.0, a2 = 0.0;
+        double nv[kB];
+        #pragma unroll
+        for (int u = 0; u < kB; ++u) nv[u] = nb > 0 ? nn[((nb - 1) * kB + u) * kNT + tid] : 0.0;
+        for (int b = nb - 1; b >= 0; --b) {
+            double D[kB], q1[kB], dx[kB], nx[kB];
+            if (b > 0) {                                  // the next block's loads are in flight
+                #pragma unroll
+                for (int u = 0; u < kB; ++u) {
+                    const int p = ((b - 1) * kB + u) * kNT + tid;
+                    dx[u] = dd[p];
+                    nx[u] = nn[p];
+                }
+            }
+            risk_sums(b, pre, dv, D);
+            #pragma unroll
+            for (int u = 0; u < kB; ++u) {
+                D[u] = 1.0 / D[u];                        // one division for both terms
+                q1[u] = nv[u] * D[u];
+            }
+            #pragma unroll
+            for (int u = kB - 1; u >= 0; --u) {
+                const int p = (b * kB + u) * kNT + tid;
+                const double q2 = q1[u] * D[u];
+                const bool en = ends(p);
+                a1 = en ? q1[u] : a1 + q1[u];
+                a2 = en ? q2 : a2 + q2;
+                S1[p] = a1;
+                S2[p] = a2;
+            }
+            #pragma unroll
+            for (int u = 0; u < kB; ++u) {
+                dv[u] = dx[u];
+                nv[u] = nx[u];
+            }
+        }
+        double t1 = 0.0, t2 = 0.0;
+        scan_down(has_end, a1, a2, t1, t2);
+        s_post1[tid] = a1;
+        s_post2[tid] = a2;
+        if (C > 1 && warp == 0) {                         // what follows in the later CTAs
+            const int ic = use[2] & 1;
+            const unsigned mb = smem_addr(&s_mb[2][ic]);
+            if (lane == 0) mbar_expect(mb, 16 * C);
+            if (lane < C) push16(peer_addr(smem_addr(&x_c[ic][rank]), lane), peer_addr(mb, lane), t1, t2);
+            wait(2);
+            double c1 = 0.0, c2 = 0.0;
+            for (int r = C - 1; r > rank; --r) {
+                const double2 t = x_c[ic][r];
+                if (SEG && s_hasend[r]) { c1 = t.x; c2 = t.y; }
+                else { c1 += t.x; c2 += t.y; }
+            }
+            if (lane == 0) { s_c1 = c1; s_c2 = c2; }
+        }
+        ++use[2];
+        __syncthreads();
+    };
+
+    // (a, b) summed over the cluster's threads, the same in every thread
+    auto sum2 = [&](double& a, double& b) {
+        for (int o = 16; o; o >>= 1) {
+            a += __shfl_xor_sync(kFull, a, o);
+            b += __shfl_xor_sync(kFull, b, o);
+        }
+        __syncthreads();
+        if (lane == 0) { s_sum[0][warp] = a; s_sum[1][warp] = b; }
+        __syncthreads();
+        a = b = 0.0;
+        for (int q = 0; q < kNW; ++q) { a += s_sum[0][q]; b += s_sum[1][q]; }
+        if (C > 1) {
+            const int i = use[0] & 1;
+            if (warp == 0) {
+                const unsigned mb = smem_addr(&s_mb[0][i]);
+                if (lane == 0) mbar_expect(mb, 16 * C);
+                if (lane < C) push16(peer_addr(smem_addr(&x_a[i][rank]), lane), peer_addr(mb, lane), a, b);
+                wait(0);
+            }
+            ++use[0];
+            __syncthreads();
+            a = b = 0.0;
+            for (int r = 0; r < C; ++r) { a += x_a[i][r].x; b += x_a[i][r].y; }
+        }
+        __syncthreads();
+    };
+
+    // getLogLikelihood (ModelSpecifics.hpp:605-650)
+    auto log_likelihood = [&]() -> double {
+        const double pre = risk_prefix();
+        double a = 0.0, b = 0.0;
+        for (int g = 0; g < nb; ++g) {
+            double D[kB];
+            #pragma unroll
+            for (int u = 0; u < kB; ++u) dv[u] = dd[(g * kB + u) * kNT + tid];
+            risk_sums(g, pre, dv, D);
+            #pragma unroll
+            for (int u = 0; u < kB; ++u) b += nn[(g * kB + u) * kNT + tid] * log(D[u]);
+        }
+        for (int k = tid; k < nr; k += kNT)
+            if ((int)A.y[r0 + k] == 1) a += wg ? xg[k] * wg[k] : xg[k];
+        sum2(a, b);
+        return a - b;
+    };
+    auto objective = [&]() -> double {
+        double a = 0.0, b = 0.0;
+        switch (A.conv) {
+        case CYC_CONV_GRADIENT:
+            for (int k = tid; k < nr; k += kNT) a += xg[k] * A.y[r0 + k] * (wg ? wg[k] : 1.0);
+            sum2(a, b);
+            return a;
+        case CYC_CONV_MITTAL: return log_likelihood();
+        case CYC_CONV_LANGE:
+            a = log_likelihood();
+            {
+                double p = 0.0, u = 0.0;
+                if (rank == 0)
+                    for (int j = tid; j < A.J; j += kNT) p += log_density(A.ptype[j], var, A.beta[j]);
+                sum2(p, u);
+                return a + p;
+            }
+        case CYC_CONV_ZHANG_OLES:                         // renews xb_save
+            for (int k = tid; k < nr; k += kNT) {
+                const double w = wg ? wg[k] : 1.0, v = xg[k];
+                a += fabs(v - A.xb_save[r0 + k]) * w;
+                b += fabs(v) * w;
+                A.xb_save[r0 + k] = v;
+            }
+            sum2(a, b);
+            return a / (1.0 + b);
+        default: return 0.0;                              // ONE_STEP
+        }
+    };
+
+    if (A.max_iter == 0 && !A.score) {
+        const double ll = log_likelihood();
+        if (rank == 0 && tid == 0) {
+            *A.out_ll = ll;
+            *A.out_iter = 0;
+            *A.out_flag = s_dead ? kTimedOut : CYC_SUCCESS;
+        }
+        if (C > 1) cluster.sync();
+        return;
+    }
+    double last = A.conv == CYC_CONV_ZHANG_OLES || A.score ? 0.0 : objective();
+    renew();
+    const int ncols = *A.ncols;
+    int it = 0, flag = CYC_SUCCESS;
+    for (;;) {
+        for (int base = 0; base < ncols; base += kCh) {
+            const int jn = min(kCh, ncols - base);
+            __syncthreads();
+            if (tid == 0) c_m[jn] = ColMeta{A.idx, nullptr, A.rowslot, nullptr, 0, 0};
+            for (int q = tid; q < jn; q += kNT) {
+                const int j = A.cols[base + q];
+                const int fm = A.fmt[j];
+                const bool dn = (fm == CYC_DENSE || fm == CYC_INTERCEPT);
+                const int e0 = dn ? r0 : A.split[j * (C + 1) + rank];
+                const int e1 = dn ? r0 + nr : A.split[j * (C + 1) + rank + 1];
+                ColMeta c;
+                c.ci = dn ? nullptr : A.idx + A.col_ptr[j] + e0;
+                c.cv = (fm == CYC_SPARSE || fm == CYC_DENSE) ? A.val + A.val_ptr[j] + e0 : nullptr;
+                c.es = dn ? A.rowslot + r0 : A.entry + A.col_ptr[j] + e0;
+                c.st = !A.entry_strat ? nullptr : (dn ? A.strat + r0 : A.entry_strat + A.col_ptr[j] + e0);
+                c.n = e1 - e0;
+                c.before = e0 > 0;
+                c_m[q] = c;
+                c_j[q] = j;
+                c_pt[q] = A.ptype[j];
+                c_beta[q] = A.beta[j];
+                c_hd[q] = A.hdelta[j];
+                c_xjy[q] = A.xjy[j];
+            }
+            __syncthreads();
+            // Columns of at most kNT - 32 entries in this CTA have one entry a
+            // thread, from the second warp on: the first combines the sums and
+            // takes the step while the others load the next column: its entry's
+            // row, value, slot (and the one before), whether it starts a
+            // stratum's entries; then the row's state.
+            const int te = tid - 32;
+            ColMeta nm = c_m[0];
+            int nk = -1, nslot = -1, npslot = -1, nst = -1, npst = -1;
+            double nx = 1.0, nxb = 0.0, nw = 1.0;
+            auto load_ids = [&](int q) {
+                nm = c_m[q];
+                nk = nslot = npslot = nst = npst = -1;
+                nx = 1.0;
+                if (nm.n <= kNT - 32 && te >= 0 && te < nm.n) {
+                    if (nm.ci) nk = __ldg(nm.ci + te);
+                    else nk = r0 + te;
+                    if (nm.cv) nx = __ldg(nm.cv + te);
+                    nslot = __ldg(nm.es + te);
+                    if (te > 0) npslot = __ldg(nm.es + te - 1);
+                    if (SEG) {
+                        nst = __ldg(nm.st + te);
+                        if (te > 0 || nm.before) npst = __ldg(nm.st + te - 1);
+                    }
+                }
+            };
+            auto load_rows = [&]() {
+                if (nk >= 0) {
+                    nxb = xg[nk - r0];
+                    if (wg) nw = __ldg(wg + nk - r0);
+                }
+            };
+            load_ids(0);
+            load_rows();
+            for (int q = 0; q < jn; ++q) {
+                const ColMeta c = nm;
+                const bool one = c.n <= kNT - 32;         // one entry a thread at most
+                const int per = (c.n + kNT - 1) / kNT;    // entries a thread otherwise, in order
+                const int i0 = tid * per, i1 = min(c.n, i0 + per);
+                const int k1 = nk - r0, slot1 = nslot, pslot1 = npslot;
+                const double x1 = nx, xb1 = nxb, w1 = nw;
+                const bool start1 = SEG && nst != npst;
+                const bool ind = c.cv == nullptr;
+                const double c1 = s_c1, c2 = s_c2;
+                // ---- the column's sums
+                double g = 0.0, h = 0.0, a = 0.0, vh2 = 0.0, ex1 = 0.0;
+                int f = 0;
+                auto entry = [&](double v, double x, int slot, bool start) {
+                    if (SEG && start) { f = 1; a = 0.0; }
+                    if (slot >= 0) {
+                        const int p = slot & kPosMask;
+                        const int t = p & (kNT - 1);      // the slot's thread
+                        const double o1 = (slot & kThreadBit ? s_post1[t] : 0.0) + (slot & kTailBit ? c1 : 0.0);
+                        const double o2 = (slot & kThreadBit ? s_post2[t] : 0.0) + (slot & kTailBit ? c2 : 0.0);
+                        const double t1 = S1[p] + o1, t2 = S2[p] + o2;
+                        g += v * t1;
+                        h += v * x * t1 - v * (2.0 * a + v) * t2;
+                        if (!SEG || !f) vh2 += v * t2;
+                        a += v;
+                    }
+                };
+                if (one) {
+                    if (k1 >= 0) {
+                        ex1 = exp(xb1);
+                        const double w = wg ? w1 : 1.0;
+                        entry(w != 0.0 ? w * ex1 * x1 : 0.0, x1, slot1, start1);
+                    }
+                } else {
+                    for (int i = i0; i < i1; ++i) {
+                        const int k = (c.ci ? __ldg(c.ci + i) - r0 : i);
+                        const double x = ind ? 1.0 : __ldg(c.cv + i);
+                        const bool st = SEG && ((i == 0 && !c.before) || __ldg(c.st + i) != __ldg(c.st + i - 1));
+                        const int slot = __ldg(c.es + i);
+                        const double w = wg ? __ldg(wg + k) : 1.0;
+                        entry(slot >= 0 && w != 0.0 ? w * exp(xg[k]) * x : 0.0, x, slot, st);
+                    }
+                }
+                // the threads' sums to the warp's: what precedes a thread in its
+                // warp enters through the running sum, as what precedes a warp in
+                // its CTA and a CTA in the cluster does below
+                {
+                    int wf = f;
+                    double wa = a;
+                    warp_up(wf, wa);
+                    int ef = SEG ? __shfl_up_sync(kFull, wf, 1) : 0;
+                    double ea = __shfl_up_sync(kFull, wa, 1);
+                    if (lane == 0) { ef = 0; ea = 0.0; }
+                    h -= 2.0 * ea * vh2;
+                    if (SEG && ef) vh2 = 0.0;             // not reached by what precedes the warp
+                    if (lane == 31) { s_sum[3][warp] = wa; s_sum[4][warp] = wf ? 1.0 : 0.0; }
+                    // three sums at once: lanes keep (g, vh2) or h, then one value
+                    const bool up = (lane & 16) != 0;
+                    double u0 = up ? h : g, u1 = up ? 0.0 : vh2;
+                    u0 += __shfl_xor_sync(kFull, up ? g : h, 16);
+                    u1 += __shfl_xor_sync(kFull, up ? vh2 : 0.0, 16);
+                    const bool up8 = (lane & 8) != 0;
+                    double u = up8 ? u1 : u0;
+                    u += __shfl_xor_sync(kFull, up8 ? u0 : u1, 8);
+                    u += __shfl_xor_sync(kFull, u, 4);
+                    u += __shfl_xor_sync(kFull, u, 2);
+                    u += __shfl_xor_sync(kFull, u, 1);
+                    if (lane == 0) s_sum[0][warp] = u;
+                    if (lane == 16) s_sum[1][warp] = u;
+                    if (lane == 8) s_sum[2][warp] = u;
+                }
+                __syncthreads();
+                const int ib = use[1] & 1;
+                if (warp == 0) {
+                    g = h = vh2 = 0.0;
+                    double pre = 0.0;                     // the running sum that reaches warp w
+                    int tf = 0;
+                    #pragma unroll
+                    for (int w = 0; w < kNW; ++w) {
+                        const double wa = s_sum[3][w], v2 = s_sum[2][w];
+                        const bool wf = SEG && s_sum[4][w] != 0.0;
+                        g += s_sum[0][w];
+                        h += s_sum[1][w] - 2.0 * pre * v2;
+                        if (!tf) vh2 += v2;
+                        tf |= wf;
+                        pre = wf ? wa : pre + wa;
+                    }
+                    if (C > 1) {
+                        const unsigned mb = smem_addr(&s_mb[1][ib]);
+                        if (lane == 0) mbar_expect(mb, 48 * C);
+                        if (lane < C) {
+                            const unsigned pm = peer_addr(mb, lane);
+                            push16(peer_addr(smem_addr(&x_b[ib][0][rank]), lane), pm, g, h);
+                            push16(peer_addr(smem_addr(&x_b[ib][1][rank]), lane), pm, vh2, pre);
+                            push16(peer_addr(smem_addr(&x_b[ib][2][rank]), lane), pm, tf ? 1.0 : 0.0, 0.0);
+                        }
+                        wait(1);
+                        g = h = pre = 0.0;
+                        for (int r = 0; r < C; ++r) {
+                            const double2 b0 = x_b[ib][0][r], b1 = x_b[ib][1][r];
+                            g += b0.x;
+                            h += b0.y - 2.0 * pre * b1.x;
+                            pre = SEG && x_b[ib][2][r].x != 0.0 ? b1.y : pre + b1.y;
+                        }
+                    }
+                    // ---- the coordinate step (ccdUpdateBeta :1394-1413, applyBounds :1503-1520)
+                    g -= c_xjy[q];                        // :1181-1183
+                    if (lane == 0) {
+                        if (A.score) {
+                            s_dl = 0.0;
+                            if (rank == 0) A.score[base + q] = fabs(g);
+                        } else {
+                            if (h < 0.0) { g = 0.0; h = 0.0; }
+                            const double b = c_beta[q];
+                            double hd = c_hd[q];
+                            double dl = prior_delta_rate(c_pt[q], var, lam, b, g, h);
+                            dl = apply_bounds(&hd, dl);
+                            s_dl = dl;
+                            c_oh[q] = hd;
+                            c_ob[q] = dl != 0.0 ? b + dl : b;
+                            c_up[q] = dl != 0.0;
+                        }
+                    }
+                }
+                ++use[1];
+                load_ids(q + 1);
+                load_rows();                              // as they are if nothing moves
+                __syncthreads();
+                const double dl = s_dl;
+                if (dl == 0.0) continue;
+                // ---- updateXBeta: the first entry of each run of one slot takes the
+                // run, with its change of the slot's increment
+                auto move = [&](int i, int slot, double acc) {
+                    for (; i < c.n && __ldg(c.es + i) == slot; ++i) {
+                        const int k = c.ci ? __ldg(c.ci + i) - r0 : i;
+                        const double x = ind ? 1.0 : __ldg(c.cv + i), w = wg ? __ldg(wg + k) : 1.0;
+                        const double old = xg[k], v = add_mul_rn(old, dl, x);
+                        xg[k] = v;
+                        if (w != 0.0) acc += w * exp(v) - w * exp(old);
+                    }
+                    dd[slot & kPosMask] = acc;
+                };
+                if (one) {
+                    if (k1 >= 0) {
+                        const double v = add_mul_rn(xb1, dl, x1), w = wg ? w1 : 1.0;
+                        xg[k1] = v;
+                        s_mv[tid] = w != 0.0 ? w * exp(v) - w * ex1 : 0.0;
+                        s_ms[tid] = slot1;
+                    }
+                    __syncthreads();
+                    if (k1 >= 0 && slot1 >= 0 && slot1 != pslot1) {
+                        double acc = dd[slot1 & kPosMask];
+                        for (int i = tid; i < 32 + c.n && s_ms[i] == slot1; ++i) acc += s_mv[i];
+                        dd[slot1 & kPosMask] = acc;
+                    }
+                } else {
+                    for (int i = i0; i < i1; ++i) {
+                        const int slot = __ldg(c.es + i);
+                        if (slot < 0) {
+                            const int k = c.ci ? __ldg(c.ci + i) - r0 : i;
+                            xg[k] = add_mul_rn(xg[k], dl, ind ? 1.0 : __ldg(c.cv + i));
+                        } else if (i == 0 || __ldg(c.es + i - 1) != slot) {
+                            move(i, slot, dd[slot & kPosMask]);
+                        }
+                    }
+                }
+                __syncthreads();
+                load_rows();                              // while the suffix sums are renewed
+                renew();
+            }
+            __syncthreads();
+            if (rank == 0 && !A.score)
+                for (int q = tid; q < jn; q += kNT) {
+                    const int j = c_j[q];
+                    A.beta[j] = c_ob[q];
+                    A.hdelta[j] = c_oh[q];
+                    if (c_up[q]) A.col_updates[j] += 1u;
+                }
+        }
+        if (A.score) { flag = s_dead ? kTimedOut : CYC_SUCCESS; break; }
+        // ---- performCheckConvergence (:839-906)
+        ++it;
+        __syncthreads();
+        if (C > 1) cluster.sync();    // rank 0's coefficients are staged by every CTA in the next cycle
+        const double o = objective();
+        double conv;
+        int ill = 0;
+        if (A.conv == CYC_CONV_ZHANG_OLES) {
+            conv = o;
+        } else {
+            if (o != o) { conv = 0.0; ill = 1; }
+            else conv = fabs(o - last) / (fabs(o) + 1.0);
+            last = o;
+        }
+        __syncthreads();
+        if (s_dead) { flag = kTimedOut; break; }          // the same in every thread of the CTA
+        if (A.tol > 0 && conv < A.tol) { flag = ill ? CYC_ILLCONDITIONED : CYC_SUCCESS; break; }
+        if (it == A.max_iter) { flag = CYC_MAX_ITERATIONS; break; }
+    }
+    const double ll = A.score ? 0.0 : log_likelihood();
+    if (C > 1) cluster.sync();       // no CTA leaves while others may still write its shared memory
+    if (rank == 0 && tid == 0) {
+        *A.out_ll = ll;
+        *A.out_iter = it;
+        *A.out_flag = flag;
+    }
+}
+
+constexpr size_t kSmemBytes = 200 * 1024;
+
+template <int WHERE, int kNT, bool SEG>
+void launch_where(const CoxArgs& a, size_t dyn, cudaStream_t stream) {
+    auto kern = k_cox<WHERE, kNT, SEG>;
+    CYC_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+    if (a.C > 8) CYC_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.C);
+    cfg.blockDim = dim3(kNT);
+    cfg.dynamicSmemBytes = dyn;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = a.C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CYC_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, (const CoxArgs)a));
+    count_launch();
+}
+
+}  // namespace
+
+// shared bytes of a CTA of `threads` with room for `per_cta` slots: all per-slot
+// arrays, or S1 and S2 alone, the block sums and the flags
+static size_t cox_bytes(int threads, int per_cta, bool all) {
+    const size_t m = (size_t)per_cta / threads;
+    return threads * (m * (all ? 32 : 16) + m / kB * sizeof(double) + m);
+}
+
+template <bool SEG>
+static void launch_seg(const CoxArgs& a, cudaStream_t stream) {
+    const size_t all = cox_bytes(a.threads, a.per_cta, true), sums = cox_bytes(a.threads, a.per_cta, false);
+    if (a.threads == 128) launch_where<0, 128, SEG>(a, all, stream);
+    else if (a.threads == 256) launch_where<0, 256, SEG>(a, all, stream);
+    else if (all <= kSmemBytes) launch_where<0, 512, SEG>(a, all, stream);
+    else if (sums <= kSmemBytes) launch_where<1, 512, SEG>(a, sums, stream);
+    else launch_where<2, 512, SEG>(a, 0, stream);
+}
+
+void launch_cox(const CoxArgs& a, cudaStream_t stream) {
+    if (a.entry_strat) launch_seg<true>(a, stream);
+    else launch_seg<false>(a, stream);
+}
+
+CoxShape cox_shape(Dataset& ds) {
+    const int events = ds.event_rows();
+    CoxShape s{1, 128};
+    while (s.C < kMaxC && events > 128 * 8 * s.C) s.C *= 2;
+    while (s.threads < kCoxThreads && events > s.threads * 12 * s.C) s.threads *= 2;
+    // CYC_COX_CLUSTER="CTAs[,threads]" fixes the shape
+    if (const char* e = std::getenv("CYC_COX_CLUSTER")) {
+        int c = s.C, t = s.threads;
+        std::sscanf(e, "%d,%d", &c, &t);
+        s.C = std::max(1, std::min(kMaxC, c));
+        s.threads = t <= 128 ? 128 : t <= 256 ? 256 : 512;
+    }
+    // 128 and 256 threads keep every per-slot array in shared memory
+    while (s.threads < kCoxThreads && cox_bytes(s.threads, (events / s.C + kB * s.threads) / (kB * s.threads) * (kB * s.threads), true) > kSmemBytes) s.threads *= 2;
+    return s;
+}
+
+CoxSlots::CoxSlots(Dataset& d_, CoxShape shape) : ds(d_), C(shape.C), threads(shape.threads) {
+    cap = std::max(1, ds.event_rows());
+    per_cta = ((cap + C - 1) / C + kB * threads - 1) / (kB * threads) * (kB * threads);
+    const int K = ds.K;
+    cnt.alloc(K);
+    tiles.alloc((K + kTile - 1) / kTile);
+    end.alloc(cap); first.alloc(cap); lo.alloc(cap); sstr.alloc(cap);
+    rowslot.alloc(K); rpart.alloc(C + 1); spart.alloc(C + 1); total.alloc(1);
+    split.alloc((size_t)ds.J * (C + 1));
+    entry.alloc(std::max<long long>(1, ds.nnz_idx));
+    const size_t n_ = (size_t)C * per_cta;
+    flag.alloc(n_); n.alloc(n_); d.alloc(n_); S1.alloc(n_); S2.alloc(n_);
+    bp.alloc(n_ / kB);
+}
+
+void CoxSlots::build(const double* d_w, cudaStream_t stream) {
+    const int K = ds.K, nt = (K + kTile - 1) / kTile;
+    const double* y = ds.d_y.get();
+    const int* strat = ds.d_strat.get();
+    const int* lastp = nullptr;
+    if (d_w) {
+        last.alloc(K);
+        const LastWeighted item{d_w};
+        launch(k_rows_totals<OpMax, LastWeighted>, nt, kThreads, 0, stream, K, item, tiles.get());
+        launch(k_tiles_scan<OpMax>, 1, kThreads, 0, stream, nt, tiles.get());
+        launch(k_rows_scan<OpMax, LastWeighted>, nt, kThreads, 0, stream, K, item, (const int*)tiles.get(), last.get());
+        lastp = last.get();
+    }
+    const GroupStart item{d_w, y, ds.d_time.get(), strat, lastp};
+    launch(k_rows_totals<OpSum, GroupStart>, nt, kThreads, 0, stream, K, item, tiles.get());
+    launch(k_tiles_scan<OpSum>, 1, kThreads, 0, stream, nt, tiles.get());
+    launch(k_rows_scan<OpSum, GroupStart>, nt, kThreads, 0, stream, K, item, (const int*)tiles.get(), cnt.get());
+    CYC_CHECK_CUDA(cudaMemsetAsync(end.get(), 0xff, cap * sizeof(int), stream));
+    // positions past the slots read as empty
+    CYC_CHECK_CUDA(cudaMemsetAsync(n.get(), 0, n.bytes(), stream));
+    CYC_CHECK_CUDA(cudaMemsetAsync(d.get(), 0, d.bytes(), stream));
+    CYC_CHECK_CUDA(cudaMemsetAsync(flag.get(), 0, flag.bytes(), stream));
+    launch(k_slot_rows, grid_for(K, 1), kThreads, 0, stream, K, d_w, y, strat, (const int*)cnt.get(), first.get(),
+           end.get(), sstr.get(), total.get());
+    launch(k_slot_parts, 1, 32, 0, stream, K, C, (const int*)total.get(), (const int*)end.get(), spart.get(),
+           rpart.get());
+    launch(k_slots, grid_for(32ll * cap, 1), kThreads, 0, stream, C, threads, per_cta, (const int*)total.get(),
+           (const int*)spart.get(), (const int*)first.get(), (const int*)end.get(), (const int*)sstr.get(),
+           (const int*)ds.d_strat_ptr.get(), d_w, y, lo.get(), flag.get(), n.get());
+    launch(k_row_slots, grid_for(K, 1), kThreads, 0, stream, K, C, threads, (const int*)total.get(), (const int*)spart.get(),
+           (const int*)sstr.get(), (const int*)end.get(), strat, (const int*)cnt.get(), rowslot.get());
+    if (ds.nnz_idx)
+        launch(k_entry_slots, grid_for(ds.nnz_idx, 4), kThreads, 0, stream, ds.nnz_idx, (const int*)ds.d_idx.get(),
+               (const int*)rowslot.get(), entry.get());
+    ccd_splits(ds, C, rpart.get(), split.get(), stream);
+}
+
+void CoxSlots::increments(const double* d_xb, const double* d_w, cudaStream_t stream) {
+    launch(k_slot_increments, grid_for(32ll * cap, 1), kThreads, 0, stream, C, threads, per_cta, (const int*)total.get(),
+           (const int*)spart.get(), (const int*)lo.get(), (const int*)end.get(), d_w, d_xb, d.get());
+}
+
+}  // namespace cyc

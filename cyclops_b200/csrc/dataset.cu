@@ -142,6 +142,12 @@ __global__ void k_entry_strata(long long n, const int* __restrict__ idx, const i
         out[e] = strat[idx[e]];
 }
 
+int Dataset::event_rows() {
+    std::lock_guard<std::mutex> lock(csr_mutex);
+    if (n_event_rows < 0) n_event_rows = (int)(K - std::count(y.begin(), y.end(), 0.0));
+    return n_event_rows;
+}
+
 void Dataset::ensure_entry_strata() {
     std::lock_guard<std::mutex> lock(csr_mutex);
     if (have_entry_strata) return;

@@ -36,9 +36,7 @@ Engine::Engine(Dataset* d) : ds(d), device(d->device) {
     CYC_CHECK_CUDA(cudaMemsetAsync(ticket.get(), 0, sizeof(unsigned), stream));
     CYC_CHECK_CUDA(cudaMemsetAsync(xb.get(), 0, K * sizeof(double), stream));
     CYC_CHECK_CUDA(cudaMemsetAsync(ll_fixed.get(), 0, sizeof(double), stream));
-    if (model_cumulative(model)) {
-        regroup(nullptr);                                // setPidForAccumulation(nullptr)
-    } else {
+    if (!model_cumulative(model)) {                      // cox: ensure_groups()
         N = model_grouped(model) ? ds->S : K;
         alloc_denominators();
     }
@@ -185,7 +183,13 @@ void Engine::set_weights(const double* w, bool use_cv) {
     const bool had_stats = stats_known;
     use_w = use_cv && w != nullptr;
     const double* wp = use_w ? w : nullptr;
-    if (model_cumulative(model)) regroup(wp);
+    if (model_cumulative(model)) {
+        CYC_REQUIRE(!wp || std::any_of(wp, wp + K, [](double v) { return v != 0.0; }), CYC_ERR_ARGUMENT,
+                    "all weights are zero");
+        h_weights.clear();
+        if (wp) h_weights.assign(wp, wp + K);
+        groups_current = false;
+    }
     if (wp) {
         weights_buf.alloc(K);
         CYC_CHECK_CUDA(cudaMemcpyAsync(weights_buf.get(), wp, K * sizeof(double), cudaMemcpyHostToDevice, stream));
@@ -194,6 +198,16 @@ void Engine::set_weights(const double* w, bool use_cv) {
     } else {
         launch(k_set_kw, grid_for(K, 1), kThreads, 0, stream, K, nullptr, kw.get());
     }
+    if (!model_cumulative(model)) group_weights();
+    if (model_cumulative(model)) {
+        if (had_stats) remaining_statistics(true);
+        else stats_known = false;
+    }
+}
+
+// the groups' weights (setWeights, hNWeight)
+void Engine::group_weights() {
+    const int K = ds->K;
     CYC_CHECK_CUDA(cudaMemsetAsync(nw.get(), 0, (N + 1) * sizeof(double), stream));
     if (model_independent(model)) {
         launch(k_nw_independent, grid_for(K, 1), kThreads, 0, stream, K, kw.get(), nw.get());
@@ -201,10 +215,15 @@ void Engine::set_weights(const double* w, bool use_cv) {
         launch(k_nw_grouped, grid_for(N, 1), kThreads, 0, stream, N, group_rows(), ds->d_y.get(), kw.get(), nw.get());
     }
     CYC_CHECK_LAUNCH();
-    if (model_cumulative(model)) {
-        if (had_stats) remaining_statistics(true);
-        else stats_known = false;
-    }
+}
+
+// cox: the risk-set groups of the current weights, built by the first call
+// that needs them (the device-resident solver has its own, cox.cu)
+void Engine::ensure_groups() {
+    if (!model_cumulative(model) || groups_current) return;
+    regroup(h_weights.empty() ? nullptr : h_weights.data());
+    group_weights();
+    groups_current = true;
 }
 
 void Engine::fixed_terms_ll(bool use_cv) {
@@ -258,13 +277,9 @@ void Engine::compute_xbeta_device(const double* d_beta) {
     stats_known = false;
 }
 
-void Engine::cox_rescan(int lo) {
-    if (lo >= N) return;
-    cox_rescan_gated(nullptr, lo);
-}
-
 // computeRemainingStatistics (ModelSpecifics.hpp:1588-1633)
 void Engine::remaining_statistics(bool use_weights) {
+    ensure_groups();
     const int K = ds->K;
     if (model_independent(model)) {
         launch(k_rs_independent, grid_for(K, 1), kThreads, 0, stream, K, model, xb.get(), exb.get(), denom.get());
@@ -282,6 +297,7 @@ void Engine::numerator_for_gradient(int j, bool use_weights) {
     if (!model_cumulative(model)) return;
     ColView c = ds->view(j);
     if (c.n == 0) return;
+    ensure_groups();
     const int blocks = grid_for(c.n, 4);
     if (c.indicator())
         launch(k_cox_numerator<true>, blocks, kThreads, 0, stream, c, group.get(), exb.get(), kw.get(),
@@ -299,6 +315,7 @@ void Engine::launch_gradient(int j, bool use_weights, double* out) {
         CYC_CHECK_CUDA(cudaMemsetAsync(out, 0, 2 * sizeof(double), stream));
         return;
     }
+    ensure_groups();
     const int blocks = grid_for(c.n, 4);
     const bool uw = use_weights && use_w;
     if (model_independent(model)) {
@@ -341,47 +358,45 @@ void Engine::gradient_hessian(int j, bool use_weights, double* g, double* h) {
     *h = h_result[1];
 }
 
-// updateXBeta (ModelSpecifics.hpp:1466-1586); delta either a host value or a
-// device pointer (the device-resident solver)
-void Engine::launch_update(int j, bool use_weights, const double* d_delta, double delta) {
+// updateXBeta (ModelSpecifics.hpp:1466-1586)
+void Engine::launch_update(int j, bool use_weights, double delta) {
     ColView c = ds->view(j);
-    if (c.n == 0) return;
+    if (c.n == 0 || delta == 0.0) return;
+    ensure_groups();
     const int blocks = grid_for(c.n, 4);
     if (model_independent(model)) {
-        launch(k_update_independent, blocks, kThreads, 0, stream, c, d_delta, delta, xb.get(), exb.get(), denom.get());
+        launch(k_update_independent, blocks, kThreads, 0, stream, c, delta, xb.get(), exb.get(), denom.get());
     } else {
-        launch(k_update_grouped, blocks, kThreads, 0, stream, c, d_delta, delta, groups(), kw.get(),
+        launch(k_update_grouped, blocks, kThreads, 0, stream, c, delta, groups(), kw.get(),
                                                           model_cumulative(model) && use_weights && use_w,
                                                           xb.get(), exb.get(), denom.get());
-        if (model_cumulative(model)) cox_rescan_gated(d_delta, first_group(j));
+        if (model_cumulative(model)) cox_rescan(h_first_group[j]);
     }
     CYC_CHECK_LAUNCH();
 }
 
-int Engine::first_group(int j) const { return h_first_group[j]; }
-
-// D / P1 / P2 over groups [lo, N); `gate` (device) skips the work when the
-// coordinate step it points at is zero
-void Engine::cox_rescan_gated(const double* gate, int lo) {
+// D / P1 / P2 over groups [lo, N)
+void Engine::cox_rescan(int lo) {
     if (lo >= N) return;
     const int hi = N;
     // tiles start at lo rounded down to a multiple of kScanItems (aligned loads)
     const int ntiles = (hi - scan_base(lo) + kScanTile - 1) / kScanTile;
-    launch(k_scanD_tiles, ntiles, kThreads, 0, stream, gate, lo, hi, gstart.get(), denom.get(), aggD.get());
-    launch(k_scanD_write, ntiles, kThreads, 0, stream, gate, lo, hi, gstart.get(), denom.get(), nw.get(),
+    launch(k_scanD_tiles, ntiles, kThreads, 0, stream, lo, hi, gstart.get(), denom.get(), aggD.get());
+    launch(k_scanD_write, ntiles, kThreads, 0, stream, lo, hi, gstart.get(), denom.get(), nw.get(),
                                                    (const SegD*)aggD.get(), D.get(), R1.get(), R2.get(), aggP.get());
-    launch(k_scanP_write, ntiles, kThreads, 0, stream, gate, lo, hi, gstart.get(), (const double*)R1.get(),
+    launch(k_scanP_write, ntiles, kThreads, 0, stream, lo, hi, gstart.get(), (const double*)R1.get(),
                                                    (const double*)R2.get(), (const SegP*)aggP.get(),
                                                    P1h.get(), P1l.get(), P2h.get(), P2l.get());
     CYC_CHECK_LAUNCH();
 }
 
 void Engine::update_xbeta(double delta, int j, bool use_weights) {
-    launch_update(j, use_weights, nullptr, delta);
+    launch_update(j, use_weights, delta);
     sync();
 }
 
 void Engine::launch_loglik(bool use_cv, double* out) {
+    ensure_groups();
     const int K = ds->K;
     const int M = std::max(K, N);
     const double* den = model_cumulative(model) ? D.get() : denom.get();
@@ -414,6 +429,7 @@ double Engine::gradient_objective(bool use_cv) {
 
 // getPredictiveLogLikelihood (ModelSpecifics.hpp:652-690)
 double Engine::predictive_log_likelihood(const double* w) {
+    ensure_groups();
     const int K = ds->K;
     std::vector<double> saved;
     if (model_cumulative(model)) {
@@ -505,10 +521,9 @@ void Engine::fisher_information(const int* cols, int n, double* out) {
 }
 
 // computeKktConditions (CyclicCoordinateDescent.cpp:817-837): |gradient| of
-// columns cols[0..n) (host ids; d_cols the same ids on the device) into
-// d_out[0..n) at the current state.  lr / pr / clr / cpr score every column
-// in one launch; cox walks its risk sets column by column.
-void Engine::kkt_scores(const int* cols, const int* d_cols, int n, bool use_weights, double* d_out) {
+// columns d_cols[0..n) into d_out[0..n) at the current state, in one launch (lr,
+// pr, clr, cpr; cox scores in its solver, cox.cu)
+void Engine::kkt_scores(const int* d_cols, int n, bool use_weights, double* d_out) {
     if (n == 0) return;
     const bool uw = use_weights && use_w;
     const int K = ds->K;
@@ -527,18 +542,11 @@ void Engine::kkt_scores(const int* cols, const int* d_cols, int n, bool use_weig
             launch(k_kkt_independent<CYC_PR>, blocks, kThreads, 0, stream, n, d_cols, K, fmt, cp, vp, ix, vl,
                    (const double*)exb.get(), (const double*)denom.get(), (const double*)nw.get(), uw ? 1 : 0,
                    (const double*)xjy.get(), d_out);
-    } else if (model_grouped(model)) {
+    } else {
+        CYC_REQUIRE(model_grouped(model), CYC_ERR_UNSUPPORTED, "cox columns are scored by the solver");
         launch(k_kkt_grouped, blocks, kThreads, 0, stream, n, d_cols, K, fmt, cp, vp, ix, vl, groups(),
                (const double*)exb.get(), (const double*)denom.get(), (const double*)nw.get(),
                (const double*)xjy.get(), d_out);
-    } else {
-        DevBuf<double> gh;
-        gh.alloc(2 * (size_t)n);
-        for (int i = 0; i < n; ++i) {
-            numerator_for_gradient(cols[i], use_weights);
-            launch_gradient(cols[i], use_weights, gh.get() + 2 * (size_t)i);
-        }
-        launch(k_abs_gradients, grid_for(n, 1), kThreads, 0, stream, n, (const double*)gh.get(), d_out);
     }
     CYC_CHECK_LAUNCH();
 }
@@ -671,6 +679,9 @@ extern "C" int cyc_engine_fisher_information(cyc_engine* e, const int* columns, 
 extern "C" int cyc_engine_get_n(const cyc_engine* e, int* n) {
     return guarded([&] {
         CYC_REQUIRE(e && n, CYC_ERR_ARGUMENT, "null argument");
+        CYC_CHECK_CUDA(cudaSetDevice(e->eng->ds->device));
+        StreamScope scope(e->eng->stream);
+        e->eng->ensure_groups();
         *n = e->eng->N;
     });
 }

@@ -38,13 +38,16 @@ struct Engine {
     DevBuf<SegP> aggP;
     std::vector<long long> h_glist_ptr;
     std::vector<int> h_first_group;
+    std::vector<double> h_weights;     // the weights the groups are to follow (empty: none)
+    bool groups_current = false;
 
     void sync();
     void alloc_denominators();
     const int* groups() const;
     const int* group_rows() const;
     void regroup(const double* w);
-    int first_group(int j) const;
+    void group_weights();
+    void ensure_groups();
 
     void set_weights(const double* w, bool use_cv);
     void fixed_terms_ll(bool use_cv);
@@ -57,10 +60,9 @@ struct Engine {
     void numerator_for_gradient(int j, bool use_weights);
     void launch_gradient(int j, bool use_weights, double* out);
     void gradient_hessian(int j, bool use_weights, double* g, double* h);
-    void launch_update(int j, bool use_weights, const double* d_delta, double delta);
+    void launch_update(int j, bool use_weights, double delta);
     void update_xbeta(double delta, int j, bool use_weights);
     void cox_rescan(int lo);
-    void cox_rescan_gated(const double* gate, int lo);
     void launch_loglik(bool use_cv, double* out);
     double log_likelihood(bool use_cv);
     void launch_gradient_objective(bool use_cv, double* out);
@@ -69,7 +71,7 @@ struct Engine {
     void predictive_estimates(double* y, const double* w);
     void get_xbeta(double* out);
     void fisher_information(const int* cols, int n, double* out);
-    void kkt_scores(const int* cols, const int* d_cols, int n, bool use_weights, double* d_out);
+    void kkt_scores(const int* d_cols, int n, bool use_weights, double* d_out);
     void save_xbeta();
     void get_xbeta_save(double* out);
 };

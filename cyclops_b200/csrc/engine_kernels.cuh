@@ -496,19 +496,12 @@ __global__ void k_kkt_grouped(int n_cols, const int* __restrict__ cols, int K, c
     }
 }
 
-// |gh[2i]| -> out[i]
-__global__ void k_abs_gradients(int n, const double* __restrict__ gh, double* __restrict__ out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = fabs(gh[2 * i]);
-}
-
 // ---- updateXBeta (ModelSpecifics.hpp:1524-1586) -----------------------------
 
 // independent rows: each row is its own denominator
-__global__ void k_update_independent(ColView c, const double* delta_ptr, double delta_val,
+__global__ void k_update_independent(ColView c, double delta,
                                      double* __restrict__ xb, double* __restrict__ exb,
                                      double* __restrict__ denom) {
-    const double delta = delta_ptr ? *delta_ptr : delta_val;
-    if (delta == 0.0) return;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < c.n;
          e += (long long)gridDim.x * blockDim.x) {
         const int k = c.row(e);
@@ -523,12 +516,10 @@ __global__ void k_update_independent(ColView c, const double* delta_ptr, double 
 
 // grouped / cumulative rows: the first entry of each run updates the run and
 // adds its denominator change (weighted for cox when use_w)
-__global__ void k_update_grouped(ColView c, const double* delta_ptr, double delta_val,
+__global__ void k_update_grouped(ColView c, double delta,
                                  const int* __restrict__ group, const double* __restrict__ kw,
                                  int weighted, double* __restrict__ xb, double* __restrict__ exb,
                                  double* __restrict__ denom) {
-    const double delta = delta_ptr ? *delta_ptr : delta_val;
-    if (delta == 0.0) return;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < c.n;
          e += (long long)gridDim.x * blockDim.x) {
         const int key = group[c.row(e)];
@@ -694,10 +685,8 @@ __device__ __forceinline__ void load_items(int i0, int lo, int hi, const int* __
 // first group of the tiling: lo rounded down to a multiple of 8
 __host__ __device__ __forceinline__ int scan_base(int lo) { return lo & ~(kScanItems - 1); }
 
-// `gate`: when non-null and *gate == 0 (a zero coordinate step), nothing changed
-__global__ void __launch_bounds__(kThreads, 4) k_scanD_tiles(const double* gate, int lo, int hi, const int* __restrict__ gstart,
+__global__ void __launch_bounds__(kThreads, 4) k_scanD_tiles(int lo, int hi, const int* __restrict__ gstart,
                               const double* __restrict__ denom, SegD* __restrict__ agg) {
-    if (gate && *gate == 0.0) return;
     __shared__ SegD s_w[kThreads / 32];
     const int i0 = scan_base(lo) + blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     int f[kScanItems];
@@ -750,11 +739,10 @@ __device__ __forceinline__ SegP carry_init_P(int lo, const int* __restrict__ gst
 }
 
 // writes D and the P terms r1 = n/D, r2 = n/D^2 (R1, R2) for the P pass
-__global__ void __launch_bounds__(kThreads, 3) k_scanD_write(const double* gate, int lo, int hi, const int* __restrict__ gstart,
+__global__ void __launch_bounds__(kThreads, 3) k_scanD_write(int lo, int hi, const int* __restrict__ gstart,
                               const double* __restrict__ denom, const double* __restrict__ nw,
                               const SegD* __restrict__ aggD, double* __restrict__ D, double* __restrict__ R1,
                               double* __restrict__ R2, SegP* __restrict__ aggP) {
-    if (gate && *gate == 0.0) return;
     __shared__ SegD s_w[kThreads / 32];
     __shared__ SegP s_wp[kThreads / 32];
     const SegD carry = tile_carry(aggD, (int)blockIdx.x, carry_init_D(lo, gstart, D), s_w);
@@ -787,11 +775,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_scanD_write(const double* gate,
     if (threadIdx.x == 0) aggP[blockIdx.x] = totp;
 }
 
-__global__ void __launch_bounds__(kThreads, 3) k_scanP_write(const double* gate, int lo, int hi, const int* __restrict__ gstart,
+__global__ void __launch_bounds__(kThreads, 3) k_scanP_write(int lo, int hi, const int* __restrict__ gstart,
                               const double* __restrict__ R1, const double* __restrict__ R2,
                               const SegP* __restrict__ aggP, double* __restrict__ P1h, double* __restrict__ P1l,
                               double* __restrict__ P2h, double* __restrict__ P2l) {
-    if (gate && *gate == 0.0) return;
     __shared__ SegP s_wp[kThreads / 32];
     const SegP carry = tile_carry(aggP, (int)blockIdx.x, carry_init_P(lo, gstart, P1h, P1l, P2h, P2l), s_wp);
     const int i0 = scan_base(lo) + blockIdx.x * kScanTile + threadIdx.x * kScanItems;

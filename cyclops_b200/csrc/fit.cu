@@ -2,13 +2,13 @@
 //
 // The reference runs the loop on the host (CyclicCoordinateDescent::findMode,
 // src/cyclops/CyclicCoordinateDescent.cpp:909-1216) and crosses into the
-// engine three times per coordinate.  Here the coordinate step
-// (ccdUpdateBeta + prior getDelta + applyBounds, :1394-1413, :1503-1520,
-// src/cyclops/priors/CovariatePrior.h:186-188, 240-273, 410-415) runs in a
-// one-thread kernel between the gradient and update kernels, beta / the trust
-// region / delta stay in device memory, and one cycle is replayed as CUDA
-// graphs.  The host reads two flags per cycle (the convergence test).
+// engine three times per coordinate.  Here findMode is one launch of a
+// persistent kernel (ccd.cu for lr, pr, clr and cpr, cox.cu for cox) on the
+// engine's linear predictors; the host reads the cycle count and the return
+// flag when it ends, and runs the restarts, the active-set passes and the
+// profile searches around it.
 #include "ccd.cuh"
+#include "cox.cuh"
 #include "engine.cuh"
 #include "solver_common.cuh"
 
@@ -23,56 +23,6 @@ namespace cyc {
 static thread_local cyc_run_stats g_stats{};
 
 namespace {
-
-__global__ void k_step(int j, const double* __restrict__ gh, StepState st) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double g = gh[0], h = gh[1];
-    if (h < 0.0) { g = 0.0; h = 0.0; }                     // ccdUpdateBeta :1407-1410
-    const double beta = st.beta[j];
-    double delta = prior_delta(st.prior_type[j], st.variance, beta, g, h);
-    delta = apply_bounds(st.hdelta + j, delta);
-    if (delta != 0.0) st.beta[j] = beta + delta;
-    *st.delta = delta;
-    if (delta != 0.0) {
-        atomicAdd(st.n_updates, 1ull);
-        if (st.col_updates) st.col_updates[j] += 1u;
-    }
-}
-
-// performCheckConvergence (CyclicCoordinateDescent.cpp:839-906) for the
-// objective-based criteria; flags[0] = done, flags[1] = ill-conditioned
-__global__ void k_check(const double* __restrict__ obj, double* __restrict__ last, double tol,
-                        int iteration, int max_iter, int zhang_oles, int* __restrict__ flags) {
-    if (threadIdx.x != 0) return;
-    double conv;
-    int ill = 0;
-    const double o = *obj;
-    if (!zhang_oles) {
-        if (o != o) { conv = 0.0; ill = 1; }
-        else conv = fabs(o - *last) / (fabs(o) + 1.0);
-        *last = o;
-    } else {
-        conv = o;
-    }
-    int done = 0;
-    if (tol > 0 && conv < tol) done = 1;
-    else if (iteration == max_iter) done = 2;
-    flags[0] = done;
-    flags[1] = ill;
-}
-
-// computeZhangOlesConvergenceCriterion (CyclicCoordinateDescent.cpp:560-579), then saveXBeta
-__global__ void k_zhang_oles(int K, const double* __restrict__ xb, double* __restrict__ xb_save,
-                             const double* __restrict__ kw, int use_w, double2* partial,
-                             unsigned* ticket, double* out) {
-    double a = 0.0, b = 0.0;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x) {
-        const double w = use_w ? kw[k] : 1.0;
-        a += fabs(xb[k] - xb_save[k]) * w;
-        b += fabs(xb[k]) * w;
-    }
-    grid_sum2_finalize(a, b, partial, ticket, [&](double A, double B) { *out = A / (1.0 + B); });
-}
 
 __global__ void k_fill(int n, double v, double* __restrict__ out) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = v;
@@ -100,7 +50,7 @@ struct FitRunner {
     Engine& e;
     const cyc_control& ctl;
     int J;
-    std::vector<int> fixb, base_fix, pt, graphs_fix;
+    std::vector<int> fixb, base_fix, pt;
     DevBuf<double> beta, hdelta, gh, delta, obj, last;
     DevBuf<int> ptype, flags;
     DevBuf<unsigned long long> n_updates;
@@ -108,7 +58,6 @@ struct FitRunner {
     double variance;
     PinnedBlock h_block;                 // two flags read back per cycle (pinned, pooled)
     int* h_flags = h_block.as<int>();
-    std::vector<cudaGraphExec_t> graphs;
     std::vector<double> h_start;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
@@ -139,21 +88,8 @@ struct FitRunner {
         e.sync();
     }
     ~FitRunner() {
-        for (auto g : graphs) cudaGraphExecDestroy(g);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
-    }
-
-    StepState step_state() {
-        StepState s;
-        s.beta = beta.get();
-        s.hdelta = hdelta.get();
-        s.delta = delta.get();
-        s.prior_type = ptype.get();
-        s.variance = variance;
-        s.n_updates = n_updates.get();
-        s.col_updates = col_updates.get();
-        return s;
     }
 
     void set_beta(const std::vector<double>& b) {
@@ -163,47 +99,6 @@ struct FitRunner {
         if (std::all_of(b.begin(), b.end(), [](double v) { return v == 0.0; })) e.zero_xbeta();
         else e.compute_xbeta_device(beta.get());
         e.sync();
-    }
-
-    void launch_coordinate(int j) {
-        e.numerator_for_gradient(j, true);
-        e.launch_gradient(j, true, gh.get());
-        launch(k_step, 1, 32, 0, e.stream, j, gh.get(), step_state());
-        CYC_CHECK_LAUNCH();
-        e.launch_update(j, true, delta.get(), 0.0);
-    }
-
-    // one cycle as a list of graphs of at most `chunk` coordinates each
-    void build_graphs() {
-        for (auto g : graphs) CYC_CHECK_CUDA(cudaGraphExecDestroy(g));
-        graphs.clear();
-        graphs_fix = fixb;
-        const int chunk = 4096;
-        for (int b = 0; b < J; b += chunk) {
-            cudaGraph_t g;
-            CYC_CHECK_CUDA(cudaStreamBeginCapture(e.stream, cudaStreamCaptureModeThreadLocal));
-            for (int j = b; j < std::min(J, b + chunk); ++j)
-                if (!fixb[j]) launch_coordinate(j);
-            CYC_CHECK_CUDA(cudaStreamEndCapture(e.stream, &g));
-            cudaGraphExec_t x;
-            CYC_CHECK_CUDA(cudaGraphInstantiate(&x, g, 0));
-            CYC_CHECK_CUDA(cudaGraphDestroy(g));
-            graphs.push_back(x);
-        }
-    }
-
-    void launch_objective(int conv) {
-        if (conv == CYC_CONV_GRADIENT) {
-            e.launch_gradient_objective(true, obj.get());
-        } else if (conv == CYC_CONV_MITTAL) {
-            e.launch_loglik(true, obj.get());
-        } else if (conv == CYC_CONV_LANGE) {
-            e.launch_loglik(true, obj.get());
-            launch(k_add_logprior, 1, kThreads, 0, e.stream, J, beta.get(), ptype.get(), variance, obj.get(), obj.get());
-        } else if (conv == CYC_CONV_ONE_STEP) {
-            CYC_CHECK_CUDA(cudaMemsetAsync(obj.get(), 0, sizeof(double), e.stream));
-        }
-        CYC_CHECK_LAUNCH();
     }
 
     // ---- lr, pr, clr, cpr: findMode as one launch of the persistent kernel
@@ -238,27 +133,37 @@ struct FitRunner {
         ccd.out_iter = d_out.get(); ccd.out_flag = d_out.get() + 1;
     }
 
-    int find_mode_ccd(double bound, int* iterations) {
-        launch(k_fill, grid_for(J, 1), kThreads, 0, e.stream, J, bound, hdelta.get());     // resetBounds
-        if (cols_fix != fixb) {                      // the columns not fixed now
+    // a list of columns and its length on the device
+    void upload_list(const std::vector<int>& list, DevBuf<int>& d_list, DevBuf<int>& d_n) {
+        const int n = (int)list.size();
+        CYC_CHECK_CUDA(cudaMemcpyAsync(d_list.get(), list.data(), n * sizeof(int), cudaMemcpyHostToDevice, e.stream));
+        CYC_CHECK_CUDA(cudaMemcpyAsync(d_n.get(), &n, sizeof(int), cudaMemcpyHostToDevice, e.stream));
+        e.sync();                                    // the host list goes away
+    }
+
+    // fresh trust regions (resetBounds), the list of the columns not fixed now,
+    // and the linear predictors saved for the Zhang-Oles criterion
+    void prepare_pass(double bound) {
+        launch(k_fill, grid_for(J, 1), kThreads, 0, e.stream, J, bound, hdelta.get());
+        if (cols_fix != fixb) {
             std::vector<int> cols;
             for (int j = 0; j < J; ++j)
                 if (!fixb[j]) cols.push_back(j);
-            const int n = (int)cols.size();
-            cols.push_back(n);
-            CYC_CHECK_CUDA(cudaMemcpyAsync(d_cols.get(), cols.data(), n * sizeof(int), cudaMemcpyHostToDevice, e.stream));
-            CYC_CHECK_CUDA(cudaMemcpyAsync(d_ncols.get(), cols.data() + n, sizeof(int), cudaMemcpyHostToDevice, e.stream));
-            e.sync();                                // the host list goes away
+            upload_list(cols, d_cols, d_ncols);
             cols_fix = fixb;
         }
+        if (ctl.convergence_type == CYC_CONV_ZHANG_OLES) {
+            e.xb_save.alloc(e.ds->K);
+            launch(k_copy, grid_for(e.ds->K, 1), kThreads, 0, e.stream, e.ds->K, e.xb.get(), e.xb_save.get());
+        }
+    }
+
+    int find_mode_ccd(double bound, int* iterations) {
+        prepare_pass(bound);
         ccd.conv = ctl.convergence_type;
         ccd.tol = ctl.tolerance;
         ccd.max_iter = ctl.max_iterations;
-        if (ccd.conv == CYC_CONV_ZHANG_OLES) {       // saveXBeta
-            e.xb_save.alloc(e.ds->K);
-            launch(k_copy, grid_for(e.ds->K, 1), kThreads, 0, e.stream, e.ds->K, e.xb.get(), e.xb_save.get());
-            ccd.xb_save = e.xb_save.get();
-        }
+        ccd.xb_save = e.xb_save.get();
         launch_ccd<double>(ccd, rpart, e.stream);
         // exp(xbeta) and the denominators follow the linear predictors
         e.remaining_statistics(true);
@@ -269,45 +174,77 @@ struct FitRunner {
         return h_flags[1];
     }
 
+    // ---- cox: the same with the risk sets of the fit's weights (cox.cu)
+    std::unique_ptr<CoxSlots> slots;
+    CoxArgs cox{};
+    DevBuf<int> d_score_cols, d_score_n;
+
+    const double* cox_weights() const { return e.use_w ? e.kw.get() : nullptr; }
+
+    void prepare_cox() {
+        Dataset& ds = *e.ds;
+        slots.reset(new CoxSlots(ds, cox_shape(ds)));
+        slots->build(cox_weights(), e.stream);
+        d_cols.alloc(J); d_ncols.alloc(1); d_out.alloc(2);
+        if (ds.S > 1) ds.ensure_entry_strata();
+        CoxSlots& s = *slots;
+        cox.K = ds.K; cox.J = J; cox.C = s.C; cox.threads = s.threads; cox.per_cta = s.per_cta; cox.weighted = e.use_w;
+        cox.fmt = ds.d_fmt.get(); cox.col_ptr = ds.d_col_ptr.get(); cox.val_ptr = ds.d_val_ptr.get();
+        cox.idx = ds.d_idx.get(); cox.val = ds.d_val.get();
+        cox.entry = s.entry.get(); cox.rowslot = s.rowslot.get();
+        cox.entry_strat = ds.S > 1 ? ds.d_entry_strat.get() : nullptr; cox.strat = ds.d_strat.get();
+        cox.split = s.split.get(); cox.rpart = s.rpart.get(); cox.spart = s.spart.get(); cox.flag = s.flag.get();
+        cox.n = s.n.get(); cox.d = s.d.get(); cox.S1 = s.S1.get(); cox.S2 = s.S2.get(); cox.bp = s.bp.get();
+        cox.y = ds.d_y.get(); cox.w = e.kw.get(); cox.xb = e.xb.get();
+        cox.cols = d_cols.get(); cox.ncols = d_ncols.get();
+        cox.ptype = ptype.get(); cox.variance = variance; cox.xjy = e.xjy.get();
+        cox.beta = beta.get(); cox.hdelta = hdelta.get(); cox.col_updates = col_updates.get();
+        cox.out_iter = d_out.get(); cox.out_flag = d_out.get() + 1; cox.out_ll = obj.get();
+    }
+
+    // one launch on the current linear predictors; its flags in h_flags
+    void launch_cox_pass(const CoxArgs& a) {
+        slots->increments(e.xb.get(), cox_weights(), e.stream);
+        launch_cox(a, e.stream);
+        CYC_CHECK_CUDA(cudaMemcpyAsync(h_flags, d_out.get(), 2 * sizeof(int), cudaMemcpyDeviceToHost, e.stream));
+        e.sync();
+        CYC_REQUIRE(h_flags[1] != kTimedOut, CYC_ERR_TIMEOUT, "a wait between the CTAs of a fit ran out");
+    }
+
+    int find_mode_cox(double bound, int* iterations) {
+        prepare_pass(bound);
+        cox.conv = ctl.convergence_type;
+        cox.tol = ctl.tolerance;
+        cox.max_iter = ctl.max_iterations != 0 ? ctl.max_iterations : -1;    // 0: no limit (0 there: evaluate only)
+        cox.xb_save = e.xb_save.get();
+        launch_cox_pass(cox);
+        ll_current = true;
+        *iterations = h_flags[0];
+        return h_flags[1];
+    }
+
+    // the log likelihood of the current linear predictors is in `obj` (cox)
+    bool ll_current = false;
+
+    // statistics that follow the linear predictors between passes (cox has none)
+    void refresh_statistics() {
+        ll_current = false;
+        if (!model_cumulative(e.model)) e.remaining_statistics(true);
+    }
+
+    // beta_j += delta, through the linear predictors
+    void move_coordinate(int j, double delta) {
+        ll_current = false;
+        if (model_cumulative(e.model)) e.axpy_xbeta(delta, j);
+        else e.launch_update(j, true, delta);
+    }
+
     // findMode (CyclicCoordinateDescent.cpp:909-1216), cyclic branch
     int find_mode(double bound, int* iterations) {
         const int conv = ctl.convergence_type;
         CYC_REQUIRE(conv >= CYC_CONV_GRADIENT && conv <= CYC_CONV_ZHANG_OLES, CYC_ERR_ARGUMENT,
                     "Unknown convergence criterion");
-        if (!model_cumulative(e.model)) return find_mode_ccd(bound, iterations);
-        std::vector<double> hd(J, bound);                       // resetBounds
-        CYC_CHECK_CUDA(cudaMemcpyAsync(hdelta.get(), hd.data(), J * sizeof(double), cudaMemcpyHostToDevice, e.stream));
-        const int K = e.ds->K;
-        if (conv < CYC_CONV_ZHANG_OLES) {
-            launch_objective(conv);
-            launch(k_copy, 1, 1, 0, e.stream, 1, obj.get(), last.get());
-            CYC_CHECK_LAUNCH();
-        } else {
-            e.xb_save.alloc(K);
-            launch(k_copy, grid_for(K, 1), kThreads, 0, e.stream, K, e.xb.get(), e.xb_save.get());
-        }
-        e.sync();
-        int it = 0;
-        for (;;) {
-            for (auto g : graphs) CYC_CHECK_CUDA(cudaGraphLaunch(g, e.stream));
-            it++;
-            if (conv < CYC_CONV_ZHANG_OLES) {
-                launch_objective(conv);
-                launch(k_check, 1, 32, 0, e.stream, obj.get(), last.get(), ctl.tolerance, it, ctl.max_iterations, 0, flags.get());
-                CYC_CHECK_LAUNCH();
-            } else {
-                launch(k_zhang_oles, grid_for(K, 4), kThreads, 0, e.stream, K, e.xb.get(), e.xb_save.get(), e.kw.get(),
-                                                                        e.use_w, e.partial.get(), e.ticket.get(), obj.get());
-                launch(k_copy, grid_for(K, 1), kThreads, 0, e.stream, K, e.xb.get(), e.xb_save.get());
-                launch(k_check, 1, 32, 0, e.stream, obj.get(), last.get(), ctl.tolerance, it, ctl.max_iterations, 1, flags.get());
-            }
-            CYC_CHECK_CUDA(cudaMemcpyAsync(h_flags, flags.get(), 2 * sizeof(int), cudaMemcpyDeviceToHost, e.stream));
-            e.sync();
-            if (h_flags[0]) break;
-        }
-        *iterations = it;
-        if (h_flags[0] == 1) return h_flags[1] ? CYC_ILLCONDITIONED : CYC_SUCCESS;
-        return CYC_MAX_ITERATIONS;
+        return model_cumulative(e.model) ? find_mode_cox(bound, iterations) : find_mode_ccd(bound, iterations);
     }
 
     // kktSwindle (CyclicCoordinateDescent.cpp:636-814).  The intercept and
@@ -337,7 +274,7 @@ struct FitRunner {
         for (int j = 0; j < J; ++j) {
             if (base_fix[j] || active[j] || hb[j] == 0.0) continue;
             CYC_CHECK_CUDA(cudaMemsetAsync(beta.get() + j, 0, sizeof(double), e.stream));
-            e.launch_update(j, true, nullptr, 0.0 - hb[j]);
+            move_coordinate(j, 0.0 - hb[j]);
         }
         std::vector<int> inactive;
         DevBuf<int> d_inactive;
@@ -348,7 +285,6 @@ struct FitRunner {
             flag = CYC_SUCCESS;
             if (n_active > 0) {
                 for (int j = 0; j < J; ++j) fixb[j] = !active[j];
-                if (model_cumulative(e.model)) build_graphs();
                 flag = find_mode(bound, iterations);
             }
             if (n_inactive == 0 || flag != CYC_SUCCESS) break;
@@ -360,8 +296,21 @@ struct FitRunner {
             d_inactive.alloc(n);
             d_score.alloc(n);
             score.resize(n);
-            CYC_CHECK_CUDA(cudaMemcpyAsync(d_inactive.get(), inactive.data(), n * sizeof(int), cudaMemcpyHostToDevice, e.stream));
-            e.kkt_scores(inactive.data(), d_inactive.get(), n, true, d_score.get());
+            if (model_cumulative(e.model)) {
+                d_score_cols.alloc(J);
+                d_score_n.alloc(1);
+                upload_list(inactive, d_score_cols, d_score_n);
+                CoxArgs a = cox;
+                a.cols = d_score_cols.get();
+                a.ncols = d_score_n.get();
+                a.score = d_score.get();
+                a.out_ll = last.get();
+                launch_cox_pass(a);
+            } else {
+                CYC_CHECK_CUDA(cudaMemcpyAsync(d_inactive.get(), inactive.data(), n * sizeof(int), cudaMemcpyHostToDevice,
+                                               e.stream));
+                e.kkt_scores(d_inactive.get(), n, true, d_score.get());
+            }
             CYC_CHECK_CUDA(cudaMemcpyAsync(score.data(), d_score.get(), n * sizeof(double), cudaMemcpyDeviceToHost, e.stream));
             e.sync();
             int moved = 0;
@@ -377,12 +326,6 @@ struct FitRunner {
 
     bool swindle = false;
 
-    // cox: the graphs replay one cycle over the columns not fixed now
-    void ensure_graphs() {
-        if (!model_cumulative(e.model)) return;
-        if (graphs.empty() || graphs_fix != fixb) build_graphs();
-    }
-
     // update (CyclicCoordinateDescent.cpp:586-615): findMode (or the
     // swindle), restarted from beta 0 with a tenfold smaller trust region
     // while ill-conditioned, at most max_bound_count times
@@ -390,7 +333,6 @@ struct FitRunner {
         double bound = ctl.initial_bound;
         int count = 0, flag = CYC_SUCCESS;
         for (;;) {
-            if (!swindle) ensure_graphs();
             flag = swindle ? kkt_swindle(bound, iters) : find_mode(bound, iters);
             ++count;
             if (flag == CYC_ILLCONDITIONED && count < ctl.max_bound_count) {
@@ -398,7 +340,7 @@ struct FitRunner {
                 std::vector<double> b(J, 0.0);                   // resetBeta :256-264
                 if (e.ds->has_offset) b[0] = 1.0;
                 set_beta(b);
-                e.remaining_statistics(true);
+                refresh_statistics();
             } else {
                 break;
             }
@@ -407,19 +349,25 @@ struct FitRunner {
     }
 
     void prepare() {
-        if (!model_cumulative(e.model)) prepare_ccd();
+        if (model_cumulative(e.model)) prepare_cox();
+        else prepare_ccd();
         e.fixed_terms_ll(true);
         e.fixed_terms_gh(true);
         set_beta(h_start);
-        e.remaining_statistics(true);
+        refresh_statistics();
         // the swindle runs when some prior has a KKT boundary (JointPrior.h:149-157)
         swindle = ctl.use_kkt_swindle && std::count(pt.begin(), pt.end(), (int)CYC_PRIOR_LAPLACE) > 0;
-        if (!swindle) ensure_graphs();
     }
 
     // getLogLikelihood and getLogPrior at the current state
     void objective_terms(double* ll, double* lp) {
-        e.launch_loglik(true, obj.get());
+        if (!model_cumulative(e.model)) {
+            e.launch_loglik(true, obj.get());
+        } else if (!ll_current) {
+            CoxArgs a = cox;
+            a.max_iter = 0;
+            launch_cox_pass(a);
+        }
         launch(k_add_logprior, 1, kThreads, 0, e.stream, J, beta.get(), ptype.get(), variance, nullptr, last.get());
         CYC_CHECK_LAUNCH();
         CYC_CHECK_CUDA(cudaMemcpyAsync(&h_block.as<double>()[1], obj.get(), sizeof(double), cudaMemcpyDeviceToHost, e.stream));
@@ -442,17 +390,15 @@ struct FitRunner {
     //   lr / pr   gradient nnz_j (4 + s_x + s + w), update nnz_j (4 + s_x + 3 s);
     //   clr / cpr the same plus 16 B per stratum the column touches (at most
     //             one per entry) for the gradient and for an update;
-    //   cox       numerator scatter nnz_j (4 + s_x + s + w) + 16 g_j, gradient
-    //             32 g_j (the two double-double prefix sums at the g_j groups
-    //             the column touches), update nnz_j (4 + s_x + 3 s + w)
-    //             + 16 g_j and the rescan of the groups from the column's first
-    //             to N at 56 B a group (denominator and group weight read; the
-    //             accumulated denominator and two double-double prefix sums
-    //             written).
+    //   cox       gradient nnz_j (4 + s_x + s + w) + 16 nnz_j (the two suffix
+    //             sums at the entries' slots), update nnz_j (4 + s_x + 3 s + w)
+    //             and 32 B per event group (its increment and events read, the
+    //             two suffix sums written).
     // Gradients count once per cycle for every column not fixed, updates once
     // per step that moved beta; each convergence check reads K (2 s + 8).
     double algorithmic_bytes(int iters, const std::vector<unsigned>& upd) const {
-        const Dataset& ds = *e.ds;
+        Dataset& ds = *e.ds;
+        const double events = model_cumulative(ds.model) ? (double)ds.event_rows() : 0.0;
         const int K = ds.K;
         const double w = e.use_w ? 8.0 : 0.0;
         double bytes = (double)(iters + 1) * K * (2 * 8.0 + 8.0);
@@ -465,9 +411,8 @@ struct FitRunner {
             const double si = dense ? 0.0 : 4.0;
             double grad, upd_b;
             if (model_cumulative(ds.model)) {
-                const double g = (double)(e.h_glist_ptr[j + 1] - e.h_glist_ptr[j]);
-                grad = n * (si + sx + 8.0 + w) + 16.0 * g + 32.0 * g;
-                upd_b = n * (si + sx + 24.0 + w) + 16.0 * g + 56.0 * (double)std::max(0, e.N - e.first_group(j));
+                grad = n * (si + sx + 8.0 + w) + 16.0 * n;
+                upd_b = n * (si + sx + 24.0 + w) + 32.0 * events;
             } else if (model_grouped(ds.model)) {
                 grad = n * (si + sx + 8.0 + w) + 16.0 * n;
                 upd_b = n * (si + sx + 24.0) + 16.0 * n;
@@ -525,7 +470,7 @@ struct FitRunner {
         const double delta = x - hb[0];
         hb[0] += delta;
         CYC_CHECK_CUDA(cudaMemcpyAsync(beta.get() + j, hb, sizeof(double), cudaMemcpyHostToDevice, e.stream));
-        e.launch_update(j, true, nullptr, delta);
+        move_coordinate(j, delta);
         e.sync();
     }
 
@@ -631,7 +576,7 @@ struct FitRunner {
         e.fixed_terms_ll(true);
         e.fixed_terms_gh(true);
         e.compute_xbeta_device(beta.get());
-        e.remaining_statistics(true);
+        refresh_statistics();
         fixb[j] = base_fix[j] = 1;
         update(&iters);
         fixb[j] = base_fix[j] = 0;

@@ -273,6 +273,8 @@ struct Dataset {
     size_t device_bytes() const;
     void ensure_csr();
     void ensure_entry_strata();
+    int n_event_rows = -1;
+    int event_rows();                // rows with a nonzero outcome (counted once)
 };
 
 // ---------------------------------------------------------------------------

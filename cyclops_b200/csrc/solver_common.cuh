@@ -5,16 +5,6 @@
 
 namespace cyc {
 
-struct StepState {
-    double* beta;                    // J
-    double* hdelta;                  // J trust-region half widths
-    double* delta;                   // out: the last step
-    const int* prior_type;           // J (flat prior on excluded columns)
-    double variance;
-    unsigned long long* n_updates;   // steps with delta != 0
-    unsigned* col_updates;           // J: steps with delta != 0 per column (null: not counted)
-};
-
 __host__ __device__ inline int sgn(double x) { return x == 0 ? 0 : (x < 0 ? -1 : 1); }
 
 // std::max(a, b) semantics: returns a unless a < b (NaN in a propagates)
