@@ -40,6 +40,7 @@
 
 #include "engine.cuh"
 #include "ccd.cuh"
+#include "cox.cuh"
 #include "row_terms.cuh"
 #include "variance_search.h"
 
@@ -2146,11 +2147,10 @@ int group_size(Dataset& ds, cudaStream_t stream, int F, const cyc_prior& prior, 
     return best;
 }
 
-// Fits the persistent kernel does not take -- Cox, whose risk sets follow
-// each fit's weights and are rescanned after every moving coordinate, and
-// fits under the KKT swindle, each with its own active set -- run
-// concurrently: one device-resident single-fit CCD (cyc_fit: its own engine,
-// stream and CUDA graphs) per host thread, up to CYC_CONCURRENT_FITS (default
+// Fits under the KKT swindle that no batch kernel takes (cox, grouped models,
+// mixed precision), each with its own active set, run concurrently: one
+// device-resident single-fit CCD (cyc_fit: its own engine and stream) per host
+// thread, up to CYC_CONCURRENT_FITS (default
 // 8) at a time, so their kernels overlap on the device.  Each fit is the one
 // cyc_fit computes alone.
 void run_fits_concurrently(cyc_dataset* dsh, const cyc_prior* prior, const cyc_fit_spec* specs, int F,
@@ -2469,11 +2469,14 @@ extern "C" int cyc_batch_fit(cyc_dataset* dsh, const cyc_prior* prior, const cyc
     return guarded([&] {
         NvtxRange range("cyc_batch_fit");
         CYC_REQUIRE(dsh && prior && specs && ctl && out && F > 0, CYC_ERR_ARGUMENT, "null argument");
-        if (model_cumulative(dsh->ds.model) || (ctl->use_kkt_swindle && !batch_swindle(dsh->ds, ctl))) {
-            // cox fits carry their own risk sets, and swindle fits of grouped
-            // models or mixed precision their own active sets, which one
-            // batch kernel does not share: they run as concurrent cyc_fit calls
+        if (ctl->use_kkt_swindle && !batch_swindle(dsh->ds, ctl)) {
+            // swindle fits of cox, grouped models or mixed precision have their
+            // own active sets, which no batch kernel runs: concurrent cyc_fit calls
             run_fits_concurrently(dsh, prior, specs, F, ctl, out);
+            return;
+        }
+        if (model_cumulative(dsh->ds.model)) {
+            run_cox_batch(dsh->ds, prior, specs, F, ctl, out, nullptr, nullptr);
             return;
         }
         run_batch(dsh->ds, prior, specs, F, ctl, out, nullptr, 0, nullptr, nullptr);
@@ -2748,13 +2751,18 @@ extern "C" int cyc_cv_grid_fit_weighted(cyc_dataset* dsh, const cyc_prior* prior
             specs[i].weights = train.data() + (size_t)(i % n_folds) * K;
             specs[i].variance = variances[i / n_folds];
         }
-        if (model_cumulative(ds.model) || (ctl->use_kkt_swindle && !batch_swindle(ds, ctl))) {
+        const bool cox_batch = model_cumulative(ds.model) && !ctl->use_kkt_swindle;
+        std::vector<double> pll(F);
+        if (cox_batch) {                               // the fits and their scores together
+            std::vector<const double*> held_of(F);
+            for (int i = 0; i < F; ++i) held_of[i] = held.data() + (size_t)(i % n_folds) * K;
+            run_cox_batch(ds, prior, specs.data(), F, ctl, out, held_of.data(), pll.data());
+        } else if (ctl->use_kkt_swindle && !batch_swindle(ds, ctl)) {
             run_fits_concurrently(dsh, prior, specs.data(), F, ctl, out);
         } else {
             run_batch(ds, prior, specs.data(), F, ctl, out, nullptr, 0, nullptr, nullptr);
         }
-        std::vector<double> pll(F);
-        {
+        if (!cox_batch) {
             Engine eng(&ds);
             StreamScope scope(eng.stream);
             for (int i = 0; i < F; ++i) {

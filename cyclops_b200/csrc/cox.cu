@@ -27,10 +27,13 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
+#include <memory>
 
 #include "ccd.cuh"
+#include "engine.cuh"
 #include "mbar.cuh"
 #include "row_terms.cuh"
 
@@ -281,10 +284,14 @@ struct ColMeta {
 // 512 threads took 26 ms where 128 take 13 at 20k rows x 500 columns).  SEG:
 // more than one stratum, so sums restart at their boundaries.
 template <int WHERE, int kNT, bool SEG>
-__global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs A) {
+__global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits, int C) {
     constexpr int kNW = kNT / 32;
     cg::cluster_group cluster = cg::this_cluster();
-    const int C = A.C;
+    __shared__ CoxArgs A;
+    static_assert(sizeof(CoxArgs) % 4 == 0, "copied by words");
+    for (int i = threadIdx.x; i < (int)(sizeof(CoxArgs) / 4); i += kNT)
+        reinterpret_cast<int*>(&A)[i] = reinterpret_cast<const int*>(fits + blockIdx.x / C)[i];
+    __syncthreads();
     const int rank = C > 1 ? (int)cluster.block_rank() : 0;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int r0 = A.rpart[rank], nr = A.rpart[rank + 1] - r0;
@@ -626,8 +633,14 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs A) {
             #pragma unroll
             for (int u = 0; u < kB; ++u) b += nn[(g * kB + u) * kNT + tid] * log(D[u]);
         }
-        for (int k = tid; k < nr; k += kNT)
-            if ((int)A.y[r0 + k] == 1) a += wg ? xg[k] * wg[k] : xg[k];
+        for (int k = tid; k < nr; k += kNT) {
+            if (A.predict) {
+                const double w = wg ? wg[k] : 1.0;
+                if (w != 0.0) a += A.y[r0 + k] * w * xg[k];
+            } else if ((int)A.y[r0 + k] == 1) {
+                a += wg ? xg[k] * wg[k] : xg[k];
+            }
+        }
         sum2(a, b);
         return a - b;
     };
@@ -945,23 +958,23 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs A) {
 constexpr size_t kSmemBytes = 200 * 1024;
 
 template <int WHERE, int kNT, bool SEG>
-void launch_where(const CoxArgs& a, size_t dyn, cudaStream_t stream) {
+void launch_where(const CoxArgs* d_fits, int F, int C, size_t dyn, cudaStream_t stream) {
     auto kern = k_cox<WHERE, kNT, SEG>;
     CYC_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
-    if (a.C > 8) CYC_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    if (C > 8) CYC_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(a.C);
+    cfg.gridDim = dim3(F * C);
     cfg.blockDim = dim3(kNT);
     cfg.dynamicSmemBytes = dyn;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = a.C;
+    attr[0].val.clusterDim.x = C;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    CYC_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, (const CoxArgs)a));
+    CYC_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, d_fits, C));
     count_launch();
 }
 
@@ -974,19 +987,25 @@ static size_t cox_bytes(int threads, int per_cta, bool all) {
     return threads * (m * (all ? 32 : 16) + m / kB * sizeof(double) + m);
 }
 
-template <bool SEG>
-static void launch_seg(const CoxArgs& a, cudaStream_t stream) {
-    const size_t all = cox_bytes(a.threads, a.per_cta, true), sums = cox_bytes(a.threads, a.per_cta, false);
-    if (a.threads == 128) launch_where<0, 128, SEG>(a, all, stream);
-    else if (a.threads == 256) launch_where<0, 256, SEG>(a, all, stream);
-    else if (all <= kSmemBytes) launch_where<0, 512, SEG>(a, all, stream);
-    else if (sums <= kSmemBytes) launch_where<1, 512, SEG>(a, sums, stream);
-    else launch_where<2, 512, SEG>(a, 0, stream);
+static int cox_where(CoxShape s, int per_cta) {
+    if (s.threads < kCoxThreads || cox_bytes(s.threads, per_cta, true) <= kSmemBytes) return 0;
+    return cox_bytes(s.threads, per_cta, false) <= kSmemBytes ? 1 : 2;
 }
 
-void launch_cox(const CoxArgs& a, cudaStream_t stream) {
-    if (a.entry_strat) launch_seg<true>(a, stream);
-    else launch_seg<false>(a, stream);
+template <bool SEG>
+static void launch_seg(const CoxArgs* d_fits, int F, CoxShape s, int per_cta, cudaStream_t stream) {
+    const int where = cox_where(s, per_cta), C = s.C;
+    const size_t dyn = where == 2 ? 0 : cox_bytes(s.threads, per_cta, where == 0);
+    if (s.threads == 128) launch_where<0, 128, SEG>(d_fits, F, C, dyn, stream);
+    else if (s.threads == 256) launch_where<0, 256, SEG>(d_fits, F, C, dyn, stream);
+    else if (where == 0) launch_where<0, 512, SEG>(d_fits, F, C, dyn, stream);
+    else if (where == 1) launch_where<1, 512, SEG>(d_fits, F, C, dyn, stream);
+    else launch_where<2, 512, SEG>(d_fits, F, C, dyn, stream);
+}
+
+void launch_cox(const CoxArgs* d_fits, int F, CoxShape shape, int per_cta, bool strata, cudaStream_t stream) {
+    if (strata) launch_seg<true>(d_fits, F, shape, per_cta, stream);
+    else launch_seg<false>(d_fits, F, shape, per_cta, stream);
 }
 
 CoxShape cox_shape(Dataset& ds) {
@@ -1017,8 +1036,34 @@ CoxSlots::CoxSlots(Dataset& d_, CoxShape shape) : ds(d_), C(shape.C), threads(sh
     split.alloc((size_t)ds.J * (C + 1));
     entry.alloc(std::max<long long>(1, ds.nnz_idx));
     const size_t n_ = (size_t)C * per_cta;
-    flag.alloc(n_); n.alloc(n_); d.alloc(n_); S1.alloc(n_); S2.alloc(n_);
-    bp.alloc(n_ / kB);
+    flag.alloc(n_); n.alloc(n_);
+}
+
+CoxState::CoxState(const CoxSlots& s, int F) : np(s.positions()) {
+    const int where = cox_where(s.shape(), s.per_cta);
+    d.alloc(F * np);
+    if (where == 2) { S1.alloc(F * np); S2.alloc(F * np); bp.alloc(F * np / kB); }
+}
+
+void CoxState::set(CoxArgs& a, int f) const {
+    a.d = d.get() + f * np;
+    if (S1.get()) { a.S1 = S1.get() + f * np; a.S2 = S2.get() + f * np; a.bp = bp.get() + f * np / kB; }
+}
+
+CoxArgs CoxSlots::args() const {
+    CoxArgs a{};
+    a.K = ds.K; a.J = ds.J; a.per_cta = per_cta;
+    a.fmt = ds.d_fmt.get(); a.col_ptr = ds.d_col_ptr.get(); a.val_ptr = ds.d_val_ptr.get();
+    a.idx = ds.d_idx.get(); a.val = ds.d_val.get();
+    a.entry = entry.get(); a.rowslot = rowslot.get();
+    if (ds.S > 1) {
+        ds.ensure_entry_strata();
+        a.entry_strat = ds.d_entry_strat.get();
+    }
+    a.strat = ds.d_strat.get();
+    a.split = split.get(); a.rpart = rpart.get(); a.spart = spart.get(); a.flag = flag.get();
+    a.n = n.get(); a.y = ds.d_y.get();
+    return a;
 }
 
 void CoxSlots::build(const double* d_w, cudaStream_t stream) {
@@ -1041,7 +1086,6 @@ void CoxSlots::build(const double* d_w, cudaStream_t stream) {
     CYC_CHECK_CUDA(cudaMemsetAsync(end.get(), 0xff, cap * sizeof(int), stream));
     // positions past the slots read as empty
     CYC_CHECK_CUDA(cudaMemsetAsync(n.get(), 0, n.bytes(), stream));
-    CYC_CHECK_CUDA(cudaMemsetAsync(d.get(), 0, d.bytes(), stream));
     CYC_CHECK_CUDA(cudaMemsetAsync(flag.get(), 0, flag.bytes(), stream));
     launch(k_slot_rows, grid_for(K, 1), kThreads, 0, stream, K, d_w, y, strat, (const int*)cnt.get(), first.get(),
            end.get(), sstr.get(), total.get());
@@ -1058,9 +1102,238 @@ void CoxSlots::build(const double* d_w, cudaStream_t stream) {
     ccd_splits(ds, C, rpart.get(), split.get(), stream);
 }
 
-void CoxSlots::increments(const double* d_xb, const double* d_w, cudaStream_t stream) {
+void CoxSlots::increments(const double* d_xb, const double* d_w, double* out, cudaStream_t stream) const {
+    CYC_CHECK_CUDA(cudaMemsetAsync(out, 0, positions() * sizeof(double), stream));   // past the slots: empty
     launch(k_slot_increments, grid_for(32ll * cap, 1), kThreads, 0, stream, C, threads, per_cta, (const int*)total.get(),
-           (const int*)spart.get(), (const int*)lo.get(), (const int*)end.get(), d_w, d_xb, d.get());
+           (const int*)spart.get(), (const int*)lo.get(), (const int*)end.get(), d_w, d_xb, out);
+}
+
+// ---- many fits -------------------------------------------------------------------
+
+void run_cox_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* specs, int F, const cyc_control* ctl,
+                   cyc_fit_result* out, const double* const* held, double* pred) {
+    const int K = ds.K, J = ds.J;
+    CYC_REQUIRE(prior->prior_type >= CYC_PRIOR_NONE && prior->prior_type <= CYC_PRIOR_NORMAL, CYC_ERR_ARGUMENT,
+                "Unknown prior type");
+    CYC_REQUIRE(ctl->convergence_type >= CYC_CONV_GRADIENT && ctl->convergence_type <= CYC_CONV_ZHANG_OLES,
+                CYC_ERR_ARGUMENT, "Unknown convergence criterion");
+    std::vector<int> pt(J, prior->prior_type);
+    for (int i = 0; i < prior->n_exclude; ++i) {
+        CYC_REQUIRE(prior->exclude[i] >= 0 && prior->exclude[i] < J, CYC_ERR_ARGUMENT, "exclude index out of range");
+        pt[prior->exclude[i]] = CYC_PRIOR_NONE;
+    }
+    for (int f = 0; f < F; ++f) {
+        CYC_REQUIRE(out[f].beta, CYC_ERR_ARGUMENT, "null argument");
+        CYC_REQUIRE(prior->prior_type == CYC_PRIOR_NONE || specs[f].variance > 0, CYC_ERR_ARGUMENT,
+                    "prior variance must be positive");
+        CYC_REQUIRE(specs[f].n_fixed >= 0 && (specs[f].n_fixed == 0 || specs[f].fixed), CYC_ERR_ARGUMENT,
+                    "bad fixed-column list");
+        for (int i = 0; i < specs[f].n_fixed; ++i)
+            CYC_REQUIRE(specs[f].fixed[i] >= 0 && specs[f].fixed[i] < J, CYC_ERR_ARGUMENT, "fixed column out of range");
+    }
+    CYC_CHECK_CUDA(cudaSetDevice(ds.device));
+    OwnedStream own;
+    CYC_CHECK_CUDA(cudaStreamCreateWithFlags(&own.s, cudaStreamNonBlocking));
+    cudaStream_t stream = own.s;
+    StreamScope scope(stream);
+    const CoxShape shape = cox_shape(ds);
+
+    // one set of risk sets per weight vector of this call
+    struct Weighting {
+        const double* host;
+        DevBuf<double> w, xjy;
+        std::unique_ptr<CoxSlots> slots;
+    };
+    std::vector<std::unique_ptr<Weighting>> sets;
+    auto weighting = [&](const double* h, bool with_xjy) -> Weighting& {
+        for (auto& s : sets)
+            if (s->host == h && (!with_xjy || s->xjy.get())) return *s;
+        sets.emplace_back(new Weighting{h});
+        Weighting& s = *sets.back();
+        if (h) {
+            CYC_REQUIRE(std::any_of(h, h + K, [](double v) { return v != 0.0; }), CYC_ERR_ARGUMENT,
+                        "all weights are zero");
+            s.w.alloc(K);
+            CYC_CHECK_CUDA(cudaMemcpyAsync(s.w.get(), h, K * sizeof(double), cudaMemcpyHostToDevice, stream));
+        }
+        s.slots.reset(new CoxSlots(ds, shape));
+        s.slots->build(s.w.get(), stream);
+        if (with_xjy) {
+            s.xjy.alloc(J);
+            launch_xjy(ds, s.w.get(), s.xjy.get(), stream);
+        }
+        return s;
+    };
+
+    DevBuf<double> xb, xb_save, beta, hdelta, ll;
+    DevBuf<int> ptype, cols, ncols, flags;
+    DevBuf<unsigned> updates;
+    DevBuf<CoxArgs> d_args;
+    xb.alloc((size_t)F * K); beta.alloc((size_t)F * J); hdelta.alloc((size_t)F * J); ll.alloc(F);
+    ptype.alloc(J); cols.alloc((size_t)F * J); ncols.alloc(F); flags.alloc(2 * F); updates.alloc((size_t)F * J);
+    d_args.alloc(F);
+    const bool zhang = ctl->convergence_type == CYC_CONV_ZHANG_OLES;
+    if (zhang) xb_save.alloc((size_t)F * K);
+    CYC_CHECK_CUDA(cudaMemcpyAsync(ptype.get(), pt.data(), J * sizeof(int), cudaMemcpyHostToDevice, stream));
+    CYC_CHECK_CUDA(cudaMemsetAsync(updates.get(), 0, updates.bytes(), stream));
+    std::vector<int> h_cols((size_t)F * J), h_n(F);
+    std::vector<double> h_beta((size_t)F * J, 0.0);
+    std::vector<CoxArgs> args(F);
+    std::vector<Weighting*> of(F);
+    for (int f = 0; f < F; ++f) {
+        std::vector<char> fixed(J, 0);
+        if (ds.has_offset) fixed[0] = 1;
+        for (int i = 0; i < specs[f].n_fixed; ++i) fixed[specs[f].fixed[i]] = 1;
+        for (int j = 0; j < J; ++j)
+            if (!fixed[j]) h_cols[(size_t)f * J + h_n[f]++] = j;
+        double* b = h_beta.data() + (size_t)f * J;
+        if (specs[f].start_beta) std::copy(specs[f].start_beta, specs[f].start_beta + J, b);
+        if (ds.has_offset) b[0] = 1.0;
+        of[f] = &weighting(specs[f].weights, true);
+    }
+    CoxState state(*sets[0]->slots, F);
+    CYC_CHECK_CUDA(cudaMemcpyAsync(cols.get(), h_cols.data(), cols.bytes(), cudaMemcpyHostToDevice, stream));
+    CYC_CHECK_CUDA(cudaMemcpyAsync(ncols.get(), h_n.data(), F * sizeof(int), cudaMemcpyHostToDevice, stream));
+    for (int f = 0; f < F; ++f) {
+        CoxArgs a = of[f]->slots->args();
+        a.weighted = of[f]->host != nullptr;
+        a.w = of[f]->w.get();
+        a.xb = xb.get() + (size_t)f * K;
+        a.xb_save = zhang ? xb_save.get() + (size_t)f * K : nullptr;
+        a.cols = cols.get() + (size_t)f * J;
+        a.ncols = ncols.get() + f;
+        a.ptype = ptype.get();
+        a.variance = specs[f].variance;
+        a.xjy = of[f]->xjy.get();
+        a.beta = beta.get() + (size_t)f * J;
+        a.hdelta = hdelta.get() + (size_t)f * J;
+        a.col_updates = updates.get() + (size_t)f * J;
+        a.conv = ctl->convergence_type;
+        a.tol = ctl->tolerance;
+        a.max_iter = ctl->max_iterations != 0 ? ctl->max_iterations : -1;
+        a.out_iter = flags.get() + 2 * f;
+        a.out_flag = flags.get() + 2 * f + 1;
+        a.out_ll = ll.get() + f;
+        state.set(a, f);
+        args[f] = a;
+    }
+    const bool strata = ds.S > 1;
+    // the fits of `run`: their increments, one launch, the flags read back
+    std::vector<int> h_flags(2 * F);
+    cudaEvent_t e0, e1;
+    CYC_CHECK_CUDA(cudaEventCreate(&e0));
+    CYC_CHECK_CUDA(cudaEventCreate(&e1));
+    struct Events { cudaEvent_t a, b; ~Events() { cudaEventDestroy(a); cudaEventDestroy(b); } } events{e0, e1};
+    cyc_run_stats st{};
+    auto pass = [&](const std::vector<int>& run, const std::vector<CoxArgs>& a, const std::vector<Weighting*>& w) {
+        std::vector<CoxArgs> list;
+        for (int f : run) {
+            w[f]->slots->increments(a[f].xb, w[f]->w.get(), a[f].d, stream);
+            list.push_back(a[f]);
+        }
+        CYC_CHECK_CUDA(cudaMemcpyAsync(d_args.get(), list.data(), list.size() * sizeof(CoxArgs), cudaMemcpyHostToDevice,
+                                       stream));
+        CYC_CHECK_CUDA(cudaEventRecord(e0, stream));
+        launch_cox(d_args.get(), (int)run.size(), shape, sets[0]->slots->per_cta, strata, stream);
+        CYC_CHECK_CUDA(cudaEventRecord(e1, stream));
+        CYC_CHECK_CUDA(cudaMemcpyAsync(h_flags.data(), flags.get(), 2 * F * sizeof(int), cudaMemcpyDeviceToHost, stream));
+        CYC_CHECK_CUDA(cudaStreamSynchronize(stream));
+        float ms = 0.f;
+        CYC_CHECK_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        for (int f : run)
+            CYC_REQUIRE(h_flags[2 * f + 1] != kTimedOut, CYC_ERR_TIMEOUT, "a wait between the CTAs of a fit ran out");
+        return ms;
+    };
+    // update (CyclicCoordinateDescent.cpp:586-615): fits that come back
+    // ill-conditioned restart from beta 0 with a tenfold smaller trust region
+    std::vector<int> run(F);
+    for (int f = 0; f < F; ++f) run[f] = f;
+    double bound = ctl->initial_bound;
+    for (int count = 1; !run.empty(); ++count) {
+        std::vector<double> hd((size_t)J, bound);
+        for (int f : run) {
+            const double* b = h_beta.data() + (size_t)f * J;
+            CYC_CHECK_CUDA(cudaMemcpyAsync(args[f].beta, b, J * sizeof(double), cudaMemcpyHostToDevice, stream));
+            CYC_CHECK_CUDA(cudaMemcpyAsync(args[f].hdelta, hd.data(), J * sizeof(double), cudaMemcpyHostToDevice, stream));
+            if (std::all_of(b, b + J, [](double v) { return v == 0.0; }))
+                CYC_CHECK_CUDA(cudaMemsetAsync(args[f].xb, 0, K * sizeof(double), stream));
+            else
+                launch_xbeta(ds, args[f].beta, args[f].xb, stream);
+            if (zhang)
+                CYC_CHECK_CUDA(cudaMemcpyAsync(args[f].xb_save, args[f].xb, K * sizeof(double), cudaMemcpyDeviceToDevice,
+                                               stream));
+        }
+        CYC_CHECK_CUDA(cudaStreamSynchronize(stream));   // the host arrays go away
+        st.kernel_ms += pass(run, args, of);
+        st.launches += 1;
+        std::vector<int> again;
+        for (int f : run) {
+            out[f].iterations = h_flags[2 * f];
+            out[f].return_flag = h_flags[2 * f + 1];
+            st.cycles += out[f].iterations;
+            if (out[f].return_flag == CYC_ILLCONDITIONED && count < ctl->max_bound_count) {
+                again.push_back(f);
+                double* b = h_beta.data() + (size_t)f * J;
+                std::fill(b, b + J, 0.0);
+                if (ds.has_offset) b[0] = 1.0;
+            }
+        }
+        run.swap(again);
+        bound /= 10.0;
+    }
+    std::vector<double> h_ll(F);
+    std::vector<unsigned> upd((size_t)F * J);
+    CYC_CHECK_CUDA(cudaMemcpyAsync(h_beta.data(), beta.get(), beta.bytes(), cudaMemcpyDeviceToHost, stream));
+    CYC_CHECK_CUDA(cudaMemcpyAsync(h_ll.data(), ll.get(), F * sizeof(double), cudaMemcpyDeviceToHost, stream));
+    CYC_CHECK_CUDA(cudaMemcpyAsync(upd.data(), updates.get(), updates.bytes(), cudaMemcpyDeviceToHost, stream));
+    CYC_CHECK_CUDA(cudaStreamSynchronize(stream));
+    for (int f = 0; f < F; ++f) {
+        const double* b = h_beta.data() + (size_t)f * J;
+        std::copy(b, b + J, out[f].beta);
+        out[f].log_likelihood = h_ll[f];
+        double lp = 0.0;
+        for (int j = 0; j < J; ++j) lp += log_density(pt[j], specs[f].variance, b[j]);
+        out[f].log_prior = lp;
+        for (int i = 0; i < h_n[f]; ++i) {
+            const int j = h_cols[(size_t)f * J + i];
+            const double n = (double)ds.col_len(j);
+            st.gradient_entries += out[f].iterations * n;
+            st.update_entries += upd[(size_t)f * J + j] * n;
+            st.coordinate_steps += out[f].iterations;
+        }
+    }
+    st.phases = 1;
+    st.phase_ms[0] = st.kernel_ms;
+    st.phase_state_bytes[0] = 8;
+    if (pred) {
+        std::vector<CoxArgs> eval = args;
+        std::vector<Weighting*> by(F);
+        std::vector<int> good;
+        for (int f = 0; f < F; ++f) {
+            pred[f] = std::nan("");
+            if (out[f].return_flag != CYC_SUCCESS) continue;   // AbstractCrossValidationDriver.cpp:236-240
+            good.push_back(f);
+            by[f] = &weighting(held[f], false);
+            CoxArgs a = by[f]->slots->args();
+            a.weighted = 1;
+            a.w = by[f]->w.get();
+            a.xb = args[f].xb;
+            a.variance = args[f].variance;
+            a.predict = 1;
+            a.out_iter = args[f].out_iter;
+            a.out_flag = args[f].out_flag;
+            a.out_ll = args[f].out_ll;
+            state.set(a, f);
+            eval[f] = a;
+        }
+        if (!good.empty()) {
+            pass(good, eval, by);
+            CYC_CHECK_CUDA(cudaMemcpyAsync(h_ll.data(), ll.get(), F * sizeof(double), cudaMemcpyDeviceToHost, stream));
+            CYC_CHECK_CUDA(cudaStreamSynchronize(stream));
+            for (int f : good) pred[f] = h_ll[f];
+        }
+    }
+    set_last_stats(st);
 }
 
 }  // namespace cyc

@@ -13,6 +13,8 @@ struct CoxShape {
 };
 CoxShape cox_shape(Dataset& ds);
 
+struct CoxArgs;
+
 // The risk sets of a weighting, reduced to the groups that hold events: slot e
 // is an event group in row order (rows by stratum, then falling time; tied
 // events of a stratum share one).  A row enters the risk sets from the first
@@ -29,18 +31,30 @@ struct CoxSlots {
     DevBuf<int> cnt, last, tiles;  // scans over the rows
     DevBuf<int> end, first, lo, sstr, rowslot, rpart, spart, total, split, entry;
     DevBuf<unsigned char> flag;    // [C][per_cta] bit 0: the slot starts its stratum, bit 1: it ends it
-    DevBuf<double> n, d, S1, S2;   // [C][per_cta] events; risk-set increments; suffix sums of n/D, n/D^2
-    DevBuf<double> bp;             // scratch of the solver
+    DevBuf<double> n;              // [C][per_cta] events
 
     CoxSlots(Dataset& ds, CoxShape shape);
     // for row weights d_w (K, device) or null
     void build(const double* d_w, cudaStream_t stream);
-    // the risk-set increments (sums of w exp(xb) over each slot's rows)
-    void increments(const double* d_xb, const double* d_w, cudaStream_t stream);
+    // the risk-set increments (sums of w exp(xb) over each slot's rows) in `out`
+    void increments(const double* d_xb, const double* d_w, double* out, cudaStream_t stream) const;
+    size_t positions() const { return (size_t)C * per_cta; }
+    CoxShape shape() const { return {C, threads}; }
+    // the arguments that follow from the dataset and the risk sets
+    CoxArgs args() const;
+};
+
+// the solver's per-slot arrays of F fits: risk-set increments, and where shared
+// memory does not hold them the suffix sums and block sums
+struct CoxState {
+    DevBuf<double> d, S1, S2, bp;
+    size_t np;
+    CoxState(const CoxSlots& s, int F);
+    void set(CoxArgs& a, int f) const;
 };
 
 struct CoxArgs {
-    int K, J, C, threads, per_cta;
+    int K, J, per_cta;
     int weighted;                  // use `w`
     const int* fmt;
     const long long* col_ptr;
@@ -73,10 +87,18 @@ struct CoxArgs {
     int conv;
     double tol;
     int max_iter;                  // 0: evaluate the log likelihood only
+    int predict;                   // as getPredictiveLogLikelihood: every outcome at its value
     int* out_iter;
     int* out_flag;                 // kTimedOut (ccd.cuh): the CTAs lost one another
     double* out_ll;
 };
-void launch_cox(const CoxArgs& a, cudaStream_t stream);
+// one launch of F fits of one shape; `d_fits` is their arguments on the device
+void launch_cox(const CoxArgs* d_fits, int F, CoxShape shape, int per_cta, bool strata, cudaStream_t stream);
+
+// F Cox fits as one launch (each the one cyc_fit gives alone), weights per fit;
+// with `held`, the predictive log likelihood of each fit's held-out rows under
+// those weights in `pred` (NaN where the fit did not succeed)
+void run_cox_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* specs, int F, const cyc_control* ctl,
+                   cyc_fit_result* out, const double* const* held, double* pred);
 
 }  // namespace cyc

@@ -235,12 +235,19 @@ void Engine::fixed_terms_ll(bool use_cv) {
     CYC_CHECK_LAUNCH();
 }
 
+void launch_xjy(const Dataset& ds, const double* d_w, double* d_xjy, cudaStream_t stream) {
+    launch(k_xjy, std::min(ds.J, 148 * 16), 128, 0, stream, ds.J, ds.d_fmt.get(), ds.d_col_ptr.get(), ds.d_val_ptr.get(),
+           ds.d_idx.get(), ds.d_val.get(), ds.K, ds.d_y.get(), d_w, d_w != nullptr, d_xjy);
+}
+
+void launch_xbeta(Dataset& ds, const double* d_beta, double* d_xb, cudaStream_t stream) {
+    ds.ensure_csr();
+    launch(k_xbeta_rows, grid_for(ds.K, 1), kThreads, 0, stream, ds.K, ds.d_row_ptr.get(), ds.d_row_col.get(),
+           ds.d_row_val.get(), d_beta, d_xb);
+}
+
 void Engine::fixed_terms_gh(bool use_cv) {
-    const int J = ds->J;
-    launch(k_xjy, std::min(J, 148 * 16), 128, 0, stream, J, ds->d_fmt.get(), ds->d_col_ptr.get(),
-                                                     ds->d_val_ptr.get(), ds->d_idx.get(), ds->d_val.get(),
-                                                     ds->K, ds->d_y.get(), kw.get(), use_cv && use_w, xjy.get());
-    CYC_CHECK_LAUNCH();
+    launch_xjy(*ds, use_cv && use_w ? kw.get() : nullptr, xjy.get(), stream);
 }
 
 void Engine::zero_xbeta() {
@@ -269,11 +276,7 @@ void Engine::compute_xbeta(const double* beta_host) {
 }
 
 void Engine::compute_xbeta_device(const double* d_beta) {
-    ds->ensure_csr();
-    const int K = ds->K;
-    launch(k_xbeta_rows, grid_for(K, 1), kThreads, 0, stream, K, ds->d_row_ptr.get(), ds->d_row_col.get(),
-                                                          ds->d_row_val.get(), d_beta, xb.get());
-    CYC_CHECK_LAUNCH();
+    launch_xbeta(*ds, d_beta, xb.get(), stream);
     stats_known = false;
 }
 
@@ -608,7 +611,7 @@ extern "C" int cyc_engine_clone(const cyc_engine* e, cyc_engine** out) {
 }
 
 extern "C" int cyc_engine_set_weights(cyc_engine* e, const double* w, int use_cv) {
-    return ENGINE_CALL(e, e->eng->set_weights(w, use_cv != 0); e->eng->sync());
+    return ENGINE_CALL(e, e->eng->set_weights(w, use_cv != 0); e->eng->ensure_groups(); e->eng->sync());
 }
 extern "C" int cyc_engine_compute_fixed_terms_ll(cyc_engine* e, int use_cv) {
     return ENGINE_CALL(e, e->eng->fixed_terms_ll(use_cv != 0); e->eng->sync());

@@ -76,6 +76,10 @@ struct Engine {
     void get_xbeta_save(double* out);
 };
 
+// XjY under row weights d_w (null: none), and the linear predictors of d_beta
+void launch_xjy(const Dataset& ds, const double* d_w, double* d_xjy, cudaStream_t stream);
+void launch_xbeta(Dataset& ds, const double* d_beta, double* d_xb, cudaStream_t stream);
+
 }  // namespace cyc
 
 struct cyc_engine {

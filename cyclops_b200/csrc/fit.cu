@@ -176,6 +176,8 @@ struct FitRunner {
 
     // ---- cox: the same with the risk sets of the fit's weights (cox.cu)
     std::unique_ptr<CoxSlots> slots;
+    std::unique_ptr<CoxState> state;
+    DevBuf<CoxArgs> d_cox;
     CoxArgs cox{};
     DevBuf<int> d_score_cols, d_score_n;
 
@@ -186,16 +188,11 @@ struct FitRunner {
         slots.reset(new CoxSlots(ds, cox_shape(ds)));
         slots->build(cox_weights(), e.stream);
         d_cols.alloc(J); d_ncols.alloc(1); d_out.alloc(2);
-        if (ds.S > 1) ds.ensure_entry_strata();
-        CoxSlots& s = *slots;
-        cox.K = ds.K; cox.J = J; cox.C = s.C; cox.threads = s.threads; cox.per_cta = s.per_cta; cox.weighted = e.use_w;
-        cox.fmt = ds.d_fmt.get(); cox.col_ptr = ds.d_col_ptr.get(); cox.val_ptr = ds.d_val_ptr.get();
-        cox.idx = ds.d_idx.get(); cox.val = ds.d_val.get();
-        cox.entry = s.entry.get(); cox.rowslot = s.rowslot.get();
-        cox.entry_strat = ds.S > 1 ? ds.d_entry_strat.get() : nullptr; cox.strat = ds.d_strat.get();
-        cox.split = s.split.get(); cox.rpart = s.rpart.get(); cox.spart = s.spart.get(); cox.flag = s.flag.get();
-        cox.n = s.n.get(); cox.d = s.d.get(); cox.S1 = s.S1.get(); cox.S2 = s.S2.get(); cox.bp = s.bp.get();
-        cox.y = ds.d_y.get(); cox.w = e.kw.get(); cox.xb = e.xb.get();
+        state.reset(new CoxState(*slots, 1));
+        d_cox.alloc(1);
+        cox = slots->args();
+        state->set(cox, 0);
+        cox.weighted = e.use_w; cox.w = e.kw.get(); cox.xb = e.xb.get();
         cox.cols = d_cols.get(); cox.ncols = d_ncols.get();
         cox.ptype = ptype.get(); cox.variance = variance; cox.xjy = e.xjy.get();
         cox.beta = beta.get(); cox.hdelta = hdelta.get(); cox.col_updates = col_updates.get();
@@ -204,8 +201,9 @@ struct FitRunner {
 
     // one launch on the current linear predictors; its flags in h_flags
     void launch_cox_pass(const CoxArgs& a) {
-        slots->increments(e.xb.get(), cox_weights(), e.stream);
-        launch_cox(a, e.stream);
+        slots->increments(e.xb.get(), cox_weights(), a.d, e.stream);
+        CYC_CHECK_CUDA(cudaMemcpyAsync(d_cox.get(), &a, sizeof(CoxArgs), cudaMemcpyHostToDevice, e.stream));
+        launch_cox(d_cox.get(), 1, slots->shape(), slots->per_cta, e.ds->S > 1, e.stream);
         CYC_CHECK_CUDA(cudaMemcpyAsync(h_flags, d_out.get(), 2 * sizeof(int), cudaMemcpyDeviceToHost, e.stream));
         e.sync();
         CYC_REQUIRE(h_flags[1] != kTimedOut, CYC_ERR_TIMEOUT, "a wait between the CTAs of a fit ran out");
