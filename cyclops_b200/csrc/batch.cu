@@ -1589,7 +1589,7 @@ struct BatchRunner {
     DevBuf<unsigned long long> d_counters;
     DevBuf<unsigned char> d_lfix;
     // one-fit groups (ccd.cu): threads a CTA, the column lists and the moving steps per column
-    int threads = 0;
+    int threads = 0, teams = 1;
     DevBuf<int> d_cols, d_ncols, d_out;
     DevBuf<unsigned> d_upd;
     std::vector<std::vector<int>> lists;     // one for all fits, or one a fit (active-set passes)
@@ -1605,6 +1605,7 @@ struct BatchRunner {
             const CcdShape sh1 = ccd_shape(ds, F);
             C = sh1.C;
             threads = sh1.threads;
+            teams = sh1.teams;
         } else {
             C = C_ > 0 ? std::min(kMaxC, C_) : default_cluster(K);
         }
@@ -1794,7 +1795,8 @@ struct BatchRunner {
 
     void launch_one_fit(const cyc_control& ctl, double tol) {
         CcdArgs a{};
-        a.model = ds.model; a.K = ds.K; a.J = ds.J; a.S = ds.S; a.F = F; a.C = C; a.threads = threads;
+        a.model = ds.model; a.K = ds.K; a.J = ds.J; a.S = ds.S; a.F = F; a.C = C;
+        a.threads = threads; a.teams = teams;
         a.weights = d_fold ? 1 : (unit_weights ? 0 : 2);
         a.fmt = ds.d_fmt.get(); a.col_ptr = ds.d_col_ptr.get(); a.val_ptr = ds.d_val_ptr.get();
         a.idx = ds.d_idx.get(); a.val = ds.d_val.get(); a.entry_strat = ds.d_entry_strat.get();

@@ -14,7 +14,8 @@ constexpr int kTimedOut = -1;
 // the rows.  Arrays marked [F] hold one element per fit.
 struct CcdArgs {
     int model, K, J, S, F, C;
-    int threads;                  // per CTA, a multiple of 32 up to kCcdThreads
+    int threads;                  // per CTA, a multiple of 64 up to kCcdThreads
+    int teams;                    // 2: the CTA's threads take the columns in two teams (lr, pr)
     int weights;                  // 0: all ones; 1: CV folds; 2: `w`
     int strict_mean;              // logistic mean as exb / (1 + exb), NaN where exb overflows (as the
                                   // per-coordinate engine), else 1 / (1 + exp(-xb))
@@ -54,10 +55,10 @@ struct CcdArgs {
     int* out_flag;                // [F]
 };
 
-// CTAs a fit and threads a CTA for F one-fit solves of a dataset, and the
-// modelled time of a cycle of them all
+// CTAs a fit, threads and teams a CTA for F one-fit solves of a dataset, and
+// the modelled time of a cycle of them all
 struct CcdShape {
-    int C, threads;
+    int C, threads, teams;
     double cycle_us;
 };
 CcdShape ccd_shape(const Dataset& ds, int F);

@@ -120,6 +120,7 @@ struct FitRunner {
         if (model_grouped(ds.model)) ds.ensure_entry_strata();
         ccd.model = ds.model; ccd.K = ds.K; ccd.J = J; ccd.S = ds.S; ccd.F = 1; ccd.C = shape.C;
         ccd.threads = shape.threads;
+        ccd.teams = shape.teams;
         ccd.weights = e.use_w ? 2 : 0;
         ccd.strict_mean = 1;
         ccd.fmt = ds.d_fmt.get(); ccd.col_ptr = ds.d_col_ptr.get(); ccd.val_ptr = ds.d_val_ptr.get();

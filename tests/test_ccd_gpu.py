@@ -45,7 +45,7 @@ def _oracle(data, prior, variance, weights=None, conv=D.CONV_GRADIENT, tol=1e-6,
     return O.port().fit(data, prior, variance, control=ctl, weights=weights, start=start)
 
 
-@pytest.mark.parametrize("shape", ["1,32", "1,128", "1,256", "3,128", "8,256", "16,128"])
+@pytest.mark.parametrize("shape", ["1,64,1", "1,128,1", "1,256,2", "3,128,2", "8,256,2", "16,256,1"])
 @pytest.mark.parametrize("model", [D.LR, D.PR, D.CLR, D.CPR])
 @pytest.mark.parametrize("K", [40, 1100])
 def test_edge_columns_match_oracle(cuda_lib, monkeypatch, shape, model, K):
@@ -59,7 +59,7 @@ def test_edge_columns_match_oracle(cuda_lib, monkeypatch, shape, model, K):
 
 
 @pytest.mark.parametrize("conv", [D.CONV_LANGE, D.CONV_MITTAL, D.CONV_ONE_STEP, D.CONV_ZHANG_OLES])
-@pytest.mark.parametrize("shape", ["1,128", "4,128"])
+@pytest.mark.parametrize("shape", ["1,128,1", "4,256,2"])
 def test_convergence_rules_match_oracle(cuda_lib, monkeypatch, shape, conv):
     from cyclops_b200 import api
     monkeypatch.setenv("CYC_BATCH_CLUSTER", shape)
