@@ -11,6 +11,7 @@
 #include "engine.cuh"
 #include "engine_kernels.cuh"
 
+#include <atomic>
 #include <algorithm>
 #include <cmath>
 #include <memory>
@@ -32,6 +33,7 @@ Engine::Engine(Dataset* d) : ds(d), device(d->device) {
     partial.alloc(148 * 8);
     ticket.alloc(1);
     result.alloc(8);
+    *h_word = 0;                  // the block may have been another engine's
     ll_fixed.alloc(1);
     CYC_CHECK_CUDA(cudaMemsetAsync(ticket.get(), 0, sizeof(unsigned), stream));
     CYC_CHECK_CUDA(cudaMemsetAsync(xb.get(), 0, K * sizeof(double), stream));
@@ -50,6 +52,31 @@ Engine::~Engine() {
 }
 
 void Engine::sync() { CYC_CHECK_CUDA(cudaStreamSynchronize(stream)); }
+
+// A call of a few microseconds of device work is bounded by how the host
+// learns of its end.  The kernel that ends the call writes the results into
+// pinned memory itself and then a tag that the host polls: the gradient and
+// Hessian of 100 entries took 21.5 us by a copy and a stream synchronisation,
+// 14.5 this way, an update 15.4 and 13.7.  The stream is asked now and then, so
+// that a failed kernel ends the wait with its error.
+HostSignal Engine::signal() {
+    HostSignal sig;
+    sig.word = h_word;
+    sig.tag = ++tag;
+    return sig;
+}
+
+void Engine::await(const HostSignal& sig) {
+    const volatile unsigned* word = sig.word;
+    for (unsigned spin = 1; *word != sig.tag; ++spin) {
+        if (spin % 4096 != 0) continue;
+        const cudaError_t e = cudaStreamQuery(stream);
+        if (e == cudaErrorNotReady) continue;
+        CYC_CHECK_CUDA(e);
+        break;                                        // all of it is done
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+}
 
 void Engine::alloc_denominators() {
     denom.alloc(N + 1);
@@ -311,42 +338,39 @@ void Engine::numerator_for_gradient(int j, bool use_weights) {
     CYC_CHECK_LAUNCH();
 }
 
-// launches the gradient/Hessian of column j into out[0..1] (device)
-void Engine::launch_gradient(int j, bool use_weights, double* out) {
+// launches the gradient/Hessian of column j into out[0..1] and
+// sets `sig` (a column with entries)
+void Engine::launch_gradient(int j, bool use_weights, double* out, const HostSignal& sig) {
     ColView c = ds->view(j);
-    if (c.n == 0) {                                   // ModelSpecifics.hpp:720-723
-        CYC_CHECK_CUDA(cudaMemsetAsync(out, 0, 2 * sizeof(double), stream));
-        return;
-    }
     ensure_groups();
     const int blocks = grid_for(c.n, 4);
     const bool uw = use_weights && use_w;
     if (model_independent(model)) {
         if (model == CYC_LR) {
             if (c.indicator())
-                launch(k_gh_independent<CYC_LR, true>, blocks, kThreads, 0, stream, c, exb.get(), denom.get(), nw.get(), uw, xjy.get(), j, partial.get(), ticket.get(), out);
+                launch(k_gh_independent<CYC_LR, true>, blocks, kThreads, 0, stream, c, exb.get(), denom.get(), nw.get(), uw, xjy.get(), j, partial.get(), ticket.get(), out, sig);
             else
-                launch(k_gh_independent<CYC_LR, false>, blocks, kThreads, 0, stream, c, exb.get(), denom.get(), nw.get(), uw, xjy.get(), j, partial.get(), ticket.get(), out);
+                launch(k_gh_independent<CYC_LR, false>, blocks, kThreads, 0, stream, c, exb.get(), denom.get(), nw.get(), uw, xjy.get(), j, partial.get(), ticket.get(), out, sig);
         } else {
             if (c.indicator())
-                launch(k_gh_independent<CYC_PR, true>, blocks, kThreads, 0, stream, c, exb.get(), denom.get(), nw.get(), uw, xjy.get(), j, partial.get(), ticket.get(), out);
+                launch(k_gh_independent<CYC_PR, true>, blocks, kThreads, 0, stream, c, exb.get(), denom.get(), nw.get(), uw, xjy.get(), j, partial.get(), ticket.get(), out, sig);
             else
-                launch(k_gh_independent<CYC_PR, false>, blocks, kThreads, 0, stream, c, exb.get(), denom.get(), nw.get(), uw, xjy.get(), j, partial.get(), ticket.get(), out);
+                launch(k_gh_independent<CYC_PR, false>, blocks, kThreads, 0, stream, c, exb.get(), denom.get(), nw.get(), uw, xjy.get(), j, partial.get(), ticket.get(), out, sig);
         }
     } else if (model_grouped(model)) {
         if (c.indicator())
-            launch(k_gh_grouped<true>, blocks, kThreads, 0, stream, c, groups(), exb.get(), denom.get(), nw.get(), xjy.get(), j, partial.get(), ticket.get(), out);
+            launch(k_gh_grouped<true>, blocks, kThreads, 0, stream, c, groups(), exb.get(), denom.get(), nw.get(), xjy.get(), j, partial.get(), ticket.get(), out, sig);
         else
-            launch(k_gh_grouped<false>, blocks, kThreads, 0, stream, c, groups(), exb.get(), denom.get(), nw.get(), xjy.get(), j, partial.get(), ticket.get(), out);
+            launch(k_gh_grouped<false>, blocks, kThreads, 0, stream, c, groups(), exb.get(), denom.get(), nw.get(), xjy.get(), j, partial.get(), ticket.get(), out, sig);
     } else {
         const long long b = h_glist_ptr[j], e = h_glist_ptr[j + 1];
         const int L = (int)(e - b);
         if (L == 0) {
-            launch(k_copy_neg_xjy, 1, 1, 0, stream, xjy.get(), j, out);
+            launch(k_copy_neg_xjy, 1, 1, 0, stream, xjy.get(), j, out, sig);
         } else if (c.indicator()) {
-            launch(k_cox_gradient<true>, 1, kThreads, 0, stream, glist.get() + b, L, gstart.get(), gend.get(), numer.get(), numer2.get(), P1h.get(), P1l.get(), P2h.get(), P2l.get(), xjy.get(), j, out);
+            launch(k_cox_gradient<true>, 1, kThreads, 0, stream, glist.get() + b, L, gstart.get(), gend.get(), numer.get(), numer2.get(), P1h.get(), P1l.get(), P2h.get(), P2l.get(), xjy.get(), j, out, sig);
         } else {
-            launch(k_cox_gradient<false>, 1, kThreads, 0, stream, glist.get() + b, L, gstart.get(), gend.get(), numer.get(), numer2.get(), P1h.get(), P1l.get(), P2h.get(), P2l.get(), xjy.get(), j, out);
+            launch(k_cox_gradient<false>, 1, kThreads, 0, stream, glist.get() + b, L, gstart.get(), gend.get(), numer.get(), numer2.get(), P1h.get(), P1l.get(), P2h.get(), P2l.get(), xjy.get(), j, out, sig);
         }
     }
     CYC_CHECK_LAUNCH();
@@ -354,25 +378,31 @@ void Engine::launch_gradient(int j, bool use_weights, double* out) {
 
 void Engine::gradient_hessian(int j, bool use_weights, double* g, double* h) {
     CYC_REQUIRE(stats_known, CYC_ERR_STATE, "Error in state synchronization.");
-    launch_gradient(j, use_weights, result.get());
-    CYC_CHECK_CUDA(cudaMemcpyAsync(h_result, result.get(), 2 * sizeof(double), cudaMemcpyDeviceToHost, stream));
-    sync();
+    if (ds->view(j).n == 0) {                         // ModelSpecifics.hpp:720-723
+        sync();
+        *g = *h = 0.0;
+        return;
+    }
+    const HostSignal sig = signal();
+    launch_gradient(j, use_weights, h_result, sig);
+    await(sig);
     *g = h_result[0];
     *h = h_result[1];
 }
 
 // updateXBeta (ModelSpecifics.hpp:1466-1586)
-void Engine::launch_update(int j, bool use_weights, double delta) {
+void Engine::launch_update(int j, bool use_weights, double delta, const HostSignal& sig) {
     ColView c = ds->view(j);
     if (c.n == 0 || delta == 0.0) return;
     ensure_groups();
     const int blocks = grid_for(c.n, 4);
     if (model_independent(model)) {
-        launch(k_update_independent, blocks, kThreads, 0, stream, c, delta, xb.get(), exb.get(), denom.get());
+        launch(k_update_independent, blocks, kThreads, 0, stream, c, delta, xb.get(), exb.get(), denom.get(),
+               ticket.get(), sig);
     } else {
         launch(k_update_grouped, blocks, kThreads, 0, stream, c, delta, groups(), kw.get(),
                                                           model_cumulative(model) && use_weights && use_w,
-                                                          xb.get(), exb.get(), denom.get());
+                                                          xb.get(), exb.get(), denom.get(), ticket.get(), sig);
         if (model_cumulative(model)) cox_rescan(h_first_group[j]);
     }
     CYC_CHECK_LAUNCH();
@@ -394,39 +424,45 @@ void Engine::cox_rescan(int lo) {
 }
 
 void Engine::update_xbeta(double delta, int j, bool use_weights) {
-    launch_update(j, use_weights, delta);
-    sync();
+    if (model_cumulative(model) || delta == 0.0 || ds->view(j).n == 0) {    // ends in a scan, or in nothing
+        launch_update(j, use_weights, delta);
+        sync();
+        return;
+    }
+    const HostSignal sig = signal();
+    launch_update(j, use_weights, delta, sig);
+    await(sig);
 }
 
-void Engine::launch_loglik(bool use_cv, double* out) {
+void Engine::launch_loglik(bool use_cv, double* out, const HostSignal& sig) {
     ensure_groups();
     const int K = ds->K;
     const int M = std::max(K, N);
     const double* den = model_cumulative(model) ? D.get() : denom.get();
     launch(k_loglik, grid_for(M, 4), kThreads, 0, stream, model, K, N, ds->d_y.get(), xb.get(), kw.get(),
                                                       use_cv && use_w, nw.get(), den, ll_fixed.get(),
-                                                      partial.get(), ticket.get(), out);
+                                                      partial.get(), ticket.get(), out, sig);
     CYC_CHECK_LAUNCH();
 }
 
 double Engine::log_likelihood(bool use_cv) {
-    launch_loglik(use_cv, result.get());
-    CYC_CHECK_CUDA(cudaMemcpyAsync(h_result, result.get(), sizeof(double), cudaMemcpyDeviceToHost, stream));
-    sync();
+    const HostSignal sig = signal();
+    launch_loglik(use_cv, h_result, sig);
+    await(sig);
     return h_result[0];
 }
 
-void Engine::launch_gradient_objective(bool use_cv, double* out) {
+void Engine::launch_gradient_objective(bool use_cv, double* out, const HostSignal& sig) {
     const int K = ds->K;
     launch(k_grad_objective, grid_for(K, 4), kThreads, 0, stream, K, ds->d_y.get(), xb.get(), kw.get(),
-                                                              use_cv && use_w, partial.get(), ticket.get(), out);
+                                                              use_cv && use_w, partial.get(), ticket.get(), out, sig);
     CYC_CHECK_LAUNCH();
 }
 
 double Engine::gradient_objective(bool use_cv) {
-    launch_gradient_objective(use_cv, result.get());
-    CYC_CHECK_CUDA(cudaMemcpyAsync(h_result, result.get(), sizeof(double), cudaMemcpyDeviceToHost, stream));
-    sync();
+    const HostSignal sig = signal();
+    launch_gradient_objective(use_cv, h_result, sig);
+    await(sig);
     return h_result[0];
 }
 

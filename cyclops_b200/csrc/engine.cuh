@@ -26,8 +26,10 @@ struct Engine {
     DevBuf<double2> partial;
     DevBuf<unsigned> ticket;
     DevBuf<double> result, ll_fixed;
-    PinnedBlock h_block;          // results read back (pinned, from the process-wide pool)
+    PinnedBlock h_block;          // results (pinned, from the process-wide pool): kernels write them here
     double* h_result = h_block.as<double>();
+    unsigned* h_word = h_block.as<unsigned>() + 8;      // past the results: the last signal's tag
+    unsigned tag = 0;
 
     // cox
     DevBuf<int> group, grow_ptr, gstart, gend, glist;
@@ -42,6 +44,8 @@ struct Engine {
     bool groups_current = false;
 
     void sync();
+    HostSignal signal();
+    void await(const HostSignal& sig);
     void alloc_denominators();
     const int* groups() const;
     const int* group_rows() const;
@@ -58,14 +62,14 @@ struct Engine {
     void compute_xbeta_device(const double* d_beta);
     void remaining_statistics(bool use_weights);
     void numerator_for_gradient(int j, bool use_weights);
-    void launch_gradient(int j, bool use_weights, double* out);
+    void launch_gradient(int j, bool use_weights, double* out, const HostSignal& sig);
     void gradient_hessian(int j, bool use_weights, double* g, double* h);
-    void launch_update(int j, bool use_weights, double delta);
+    void launch_update(int j, bool use_weights, double delta, const HostSignal& sig = HostSignal{});
     void update_xbeta(double delta, int j, bool use_weights);
     void cox_rescan(int lo);
-    void launch_loglik(bool use_cv, double* out);
+    void launch_loglik(bool use_cv, double* out, const HostSignal& sig = HostSignal{});
     double log_likelihood(bool use_cv);
-    void launch_gradient_objective(bool use_cv, double* out);
+    void launch_gradient_objective(bool use_cv, double* out, const HostSignal& sig);
     double gradient_objective(bool use_cv);
     double predictive_log_likelihood(const double* w);
     void predictive_estimates(double* y, const double* w);

@@ -237,7 +237,7 @@ __global__ void k_fisher_pairs(int n_pairs, const int* __restrict__ pa, const in
 template <int MODEL, bool IND>
 __global__ void k_gh_independent(ColView c, const double* __restrict__ exb, const double* __restrict__ denom,
                                  const double* __restrict__ nw, int use_w, const double* __restrict__ xjy, int j,
-                                 double2* partial, unsigned* ticket, double* out) {
+                                 double2* partial, unsigned* ticket, double* out, HostSignal sig) {
     double g = 0.0, h = 0.0;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < c.n;
          e += (long long)gridDim.x * blockDim.x) {
@@ -259,6 +259,7 @@ __global__ void k_gh_independent(ColView c, const double* __restrict__ exb, cons
     grid_sum2_finalize(g, h, partial, ticket, [&](double G, double H) {
         out[0] = G - xjy[j];
         out[1] = H;
+        sig.set();
     });
 }
 
@@ -269,7 +270,7 @@ template <bool IND>
 __global__ void k_gh_grouped(ColView c, const int* __restrict__ group, const double* __restrict__ exb,
                              const double* __restrict__ denom, const double* __restrict__ nw,
                              const double* __restrict__ xjy, int j, double2* partial, unsigned* ticket,
-                             double* out) {
+                             double* out, HostSignal sig) {
     double g = 0.0, h = 0.0;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < c.n;
          e += (long long)gridDim.x * blockDim.x) {
@@ -293,6 +294,7 @@ __global__ void k_gh_grouped(ColView c, const int* __restrict__ group, const dou
     grid_sum2_finalize(g, h, partial, ticket, [&](double G, double H) {
         out[0] = G - xjy[j];
         out[1] = H;
+        sig.set();
     });
 }
 
@@ -345,7 +347,7 @@ __global__ void k_cox_gradient(const int* __restrict__ list, int L, const int* _
                                const double* __restrict__ numer2, const double* __restrict__ P1h,
                                const double* __restrict__ P1l, const double* __restrict__ P2h,
                                const double* __restrict__ P2l, const double* __restrict__ xjy, int j,
-                               double* out) {
+                               double* out, HostSignal sig) {
     // Each thread takes kItems consecutive groups of the list per tile; the
     // running sums A (and B) restart at every stratum change and carry
     // across tiles; threads' spans are combined by warp shuffles and then
@@ -430,13 +432,15 @@ __global__ void k_cox_gradient(const int* __restrict__ list, int L, const int* _
     if (threadIdx.x == 0) {
         out[0] = g - xjy[j];
         out[1] = h;
+        sig.set();
     }
 }
 
 // a column whose group list is empty: gradient -XjY, Hessian 0 (ModelSpecifics.hpp:906)
-__global__ void k_copy_neg_xjy(const double* __restrict__ xjy, int j, double* out) {
+__global__ void k_copy_neg_xjy(const double* __restrict__ xjy, int j, double* out, HostSignal sig) {
     out[0] = 0.0 - xjy[j];
     out[1] = 0.0;
+    sig.set();
 }
 
 // ---- KKT conditions (CyclicCoordinateDescent.cpp:817-837) ---------------------
@@ -501,7 +505,7 @@ __global__ void k_kkt_grouped(int n_cols, const int* __restrict__ cols, int K, c
 // independent rows: each row is its own denominator
 __global__ void k_update_independent(ColView c, double delta,
                                      double* __restrict__ xb, double* __restrict__ exb,
-                                     double* __restrict__ denom) {
+                                     double* __restrict__ denom, unsigned* ticket, HostSignal sig) {
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < c.n;
          e += (long long)gridDim.x * blockDim.x) {
         const int k = c.row(e);
@@ -512,6 +516,7 @@ __global__ void k_update_independent(ColView c, double delta,
         exb[k] = nw_;
         denom[k] += nw_ - old;
     }
+    grid_signal(sig, ticket);
 }
 
 // grouped / cumulative rows: the first entry of each run updates the run and
@@ -519,7 +524,7 @@ __global__ void k_update_independent(ColView c, double delta,
 __global__ void k_update_grouped(ColView c, double delta,
                                  const int* __restrict__ group, const double* __restrict__ kw,
                                  int weighted, double* __restrict__ xb, double* __restrict__ exb,
-                                 double* __restrict__ denom) {
+                                 double* __restrict__ denom, unsigned* ticket, HostSignal sig) {
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < c.n;
          e += (long long)gridDim.x * blockDim.x) {
         const int key = group[c.row(e)];
@@ -539,6 +544,7 @@ __global__ void k_update_grouped(ColView c, double delta,
         } while (f < c.n && group[c.row(f)] == key);
         denom[key] = d;
     }
+    grid_signal(sig, ticket);
 }
 
 // ---- cox denominator scan (computeAccumlatedDenominator, ModelSpecifics.hpp:1670-1694)
@@ -815,7 +821,7 @@ __device__ __forceinline__ double ll_denom(int model, double n, double d) {
 __global__ void k_loglik(int model, int K, int N, const double* __restrict__ y, const double* __restrict__ xb,
                          const double* __restrict__ kw, int use_cv, const double* __restrict__ nw,
                          const double* __restrict__ den, const double* __restrict__ fixed,
-                         double2* partial, unsigned* ticket, double* out) {
+                         double2* partial, unsigned* ticket, double* out, HostSignal sig) {
     double a = 0.0, b = 0.0;
     const int M = K > N ? K : N;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
@@ -829,17 +835,21 @@ __global__ void k_loglik(int model, int K, int N, const double* __restrict__ y, 
         double ll = A - B;
         if (has_fixed_ll(model)) ll += *fixed;
         *out = ll;
+        sig.set();
     });
 }
 
 // getGradientObjective (ModelSpecifics.hpp:103-120)
 __global__ void k_grad_objective(int K, const double* __restrict__ y, const double* __restrict__ xb,
                                  const double* __restrict__ kw, int use_cv, double2* partial,
-                                 unsigned* ticket, double* out) {
+                                 unsigned* ticket, double* out, HostSignal sig) {
     double a = 0.0;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x)
         a += use_cv ? xb[k] * y[k] * kw[k] : xb[k] * y[k];
-    grid_sum2_finalize(a, 0.0, partial, ticket, [&](double A, double) { *out = A; });
+    grid_sum2_finalize(a, 0.0, partial, ticket, [&](double A, double) {
+        *out = A;
+        sig.set();
+    });
 }
 
 // getPredictiveLogLikelihood (ModelSpecifics.hpp:652-690 and logPredLikeContrib,

@@ -309,10 +309,15 @@ __device__ __forceinline__ void block_sum2(double& a, double& b) {
 // last block to finish (ticket) sums the partials in block order and calls
 // `fin(total_a, total_b)` from thread 0.  `ticket` must be zero on entry and
 // is left at zero.
+// A grid of one block has its total at once.
 template <class Fin>
 __device__ __forceinline__ void grid_sum2_finalize(double a, double b, double2* partial,
                                                    unsigned* ticket, Fin fin) {
     block_sum2(a, b);
+    if (gridDim.x == 1) {
+        if (threadIdx.x == 0) fin(a, b);
+        return;
+    }
     __shared__ bool is_last;
     if (threadIdx.x == 0) {
         partial[blockIdx.x] = make_double2(a, b);
@@ -335,6 +340,33 @@ __device__ __forceinline__ void grid_sum2_finalize(double a, double b, double2* 
             *ticket = 0u;
         }
     }
+}
+
+// Where a kernel tells the waiting host that its work is done: a word of
+// pinned host memory set to `tag` after all of the kernel's writes (null: the
+// host waits for the stream).
+struct HostSignal {
+    unsigned* word = nullptr;
+    unsigned tag = 0;
+    __device__ __forceinline__ void set() const {
+        if (!word) return;
+        __threadfence_system();
+        *static_cast<volatile unsigned*>(word) = tag;
+    }
+};
+
+// set `sig` once every block of the grid is through (called by all threads);
+// `ticket` must be zero on entry and is left at zero
+__device__ __forceinline__ void grid_signal(const HostSignal& sig, unsigned* ticket) {
+    if (!sig.word) return;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    if (gridDim.x > 1) {
+        __threadfence();
+        if (atomicAdd(ticket, 1u) != gridDim.x - 1) return;
+        *ticket = 0u;
+    }
+    sig.set();
 }
 
 inline int grid_for(long long n, int items_per_thread = 4, int max_blocks = 148 * 8) {
