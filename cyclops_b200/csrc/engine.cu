@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cmath>
 #include <memory>
+#include <numeric>
 
 namespace cyc {
 
@@ -528,19 +529,38 @@ void Engine::fisher_information(const int* cols, int n, double* out) {
     if (grouped)
         CYC_REQUIRE((double)n * S <= (double)(1u << 27), CYC_ERR_MEMORY,
                     "too many columns x strata for one Fisher information call");
-    std::vector<int> pa, pb;
+    // the columns by falling length, and tasks of one of them with a run of
+    // later ones of about kTaskEntries entries
+    constexpr long long kTaskEntries = 8192;
+    std::vector<int> order(n);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int x, int y) { return ds->col_len(cols[x]) > ds->col_len(cols[y]); });
+    std::vector<FisherTask> tasks;
     for (int i = 0; i < n; ++i)
-        for (int j = i; j < n; ++j) { pa.push_back(i); pb.push_back(j); }
-    const int np = (int)pa.size();
-    DevBuf<int> d_cols, d_pa, d_pb;
+        for (int j = i; j < n;) {
+            const int j0 = j;
+            for (long long m = 0; j < n && (j == j0 || m < kTaskEntries); ++j) m += ds->col_len(cols[order[j]]);
+            tasks.push_back({i, j0, j});
+        }
+    const int nt = (int)tasks.size();
+    std::vector<int> plan(2 * (size_t)n);            // column ids in that order, then their places in `cols`
+    for (int i = 0; i < n; ++i) { plan[i] = cols[order[i]]; plan[n + i] = order[i]; }
+    // a block's bitmap of one column's rows
+    constexpr size_t kBitmapBytes = 200 * 1024;
+    const size_t bitmap = ((size_t)K + 31) / 32 * sizeof(unsigned);
+    const int words = bitmap <= kBitmapBytes ? (int)(bitmap / sizeof(unsigned)) : 0;
+    DevBuf<int> d_cols, d_plan;
+    DevBuf<FisherTask> d_tasks;
     DevBuf<double> d_v, d_t, d_out;
-    d_cols.alloc(n); d_pa.alloc(np); d_pb.alloc(np); d_v.alloc(K); d_out.alloc(np);
-    CYC_CHECK_CUDA(cudaMemcpyAsync(d_cols.get(), cols, n * sizeof(int), cudaMemcpyHostToDevice, stream));
-    CYC_CHECK_CUDA(cudaMemcpyAsync(d_pa.get(), pa.data(), np * sizeof(int), cudaMemcpyHostToDevice, stream));
-    CYC_CHECK_CUDA(cudaMemcpyAsync(d_pb.get(), pb.data(), np * sizeof(int), cudaMemcpyHostToDevice, stream));
+    d_plan.alloc(plan.size()); d_tasks.alloc(nt); d_v.alloc(K); d_out.alloc((size_t)n * n);
+    CYC_CHECK_CUDA(cudaMemcpyAsync(d_plan.get(), plan.data(), plan.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
+    CYC_CHECK_CUDA(cudaMemcpyAsync(d_tasks.get(), tasks.data(), nt * sizeof(FisherTask), cudaMemcpyHostToDevice, stream));
     launch(k_fisher_row, grid_for(K, 4), kThreads, 0, stream, K, model, (const double*)exb.get(),
            (const double*)denom.get(), (const int*)ds->d_strat.get(), d_v.get());
     if (grouped) {
+        d_cols.alloc(n);
+        CYC_CHECK_CUDA(cudaMemcpyAsync(d_cols.get(), cols, n * sizeof(int), cudaMemcpyHostToDevice, stream));
         d_t.alloc((size_t)n * S);
         CYC_CHECK_CUDA(cudaMemsetAsync(d_t.get(), 0, (size_t)n * S * sizeof(double), stream));
         launch(k_fisher_strata, std::min(n, 148 * 8), kThreads, 0, stream, n, (const int*)d_cols.get(), K, S,
@@ -548,15 +568,17 @@ void Engine::fisher_information(const int* cols, int n, double* out) {
                (const int*)ds->d_idx.get(), (const double*)ds->d_val.get(), (const int*)ds->d_strat.get(),
                (const double*)exb.get(), d_t.get());
     }
-    launch(k_fisher_pairs, std::min(np, 148 * 8), kThreads, 0, stream, np, (const int*)d_pa.get(),
-           (const int*)d_pb.get(), (const int*)d_cols.get(), K, S, grouped ? 1 : 0, (const int*)ds->d_fmt.get(),
-           (const long long*)ds->d_col_ptr.get(), (const long long*)ds->d_val_ptr.get(), (const int*)ds->d_idx.get(),
-           (const double*)ds->d_val.get(), (const double*)d_v.get(), (const int*)ds->d_strat.get(),
-           (const double*)denom.get(), (const double*)d_t.get(), d_out.get());
-    std::vector<double> h(np);
-    CYC_CHECK_CUDA(cudaMemcpyAsync(h.data(), d_out.get(), np * sizeof(double), cudaMemcpyDeviceToHost, stream));
+    const size_t smem = words * sizeof(unsigned);
+    if (smem > 48 * 1024)
+        CYC_CHECK_CUDA(cudaFuncSetAttribute(k_fisher_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    launch(k_fisher_pairs, std::min(nt, 148 * 8), kThreads, smem, stream, nt, (const FisherTask*)d_tasks.get(), n,
+           (const int*)d_plan.get(), (const int*)d_plan.get() + n, words, K, S, grouped ? 1 : 0,
+           (const int*)ds->d_fmt.get(), (const long long*)ds->d_col_ptr.get(),
+           (const long long*)ds->d_val_ptr.get(), (const int*)ds->d_idx.get(), (const double*)ds->d_val.get(),
+           (const double*)d_v.get(), (const int*)ds->d_strat.get(), (const double*)denom.get(),
+           (const double*)d_t.get(), d_out.get());
+    CYC_CHECK_CUDA(cudaMemcpyAsync(out, d_out.get(), (size_t)n * n * sizeof(double), cudaMemcpyDeviceToHost, stream));
     sync();
-    for (int p = 0; p < np; ++p) out[(size_t)pa[p] * n + pb[p]] = out[(size_t)pb[p] * n + pa[p]] = h[p];
 }
 
 // computeKktConditions (CyclicCoordinateDescent.cpp:817-837): |gradient| of
