@@ -50,10 +50,16 @@ namespace cyc {
 
 namespace {
 
-constexpr int kBT = 256;          // threads per CTA
+constexpr int kBT = 256;          // threads per CTA of the set-up kernels
 constexpr int kMaxC = 8;          // CTAs per cluster (portable limit)
-// shared memory per CTA for rows arriving by cp.async (8-fit groups)
-constexpr int kAsyncBytes = 32768;
+
+// what follows from the solver's NT threads a CTA
+template <int NT>
+struct BatchDims {
+    static constexpr int kAsyncBytes = 128 * NT;   // shared memory for rows arriving by cp.async
+    static constexpr int kRunMax = NT / 32;        // columns of a batch: a warp each
+    static constexpr int kDirtyMax = NT / 8;       // rows a batch may share between its columns
+};
 
 struct BatchArgs {
     int model, K, J, C;
@@ -99,7 +105,7 @@ struct BatchArgs {
 
 // sum (a, b) over the CTA's slots that share this thread's fit lane; result
 // for lane f lands in out[f] (threads < G then read it)
-template <int G>
+template <int G, int NT>
 __device__ __forceinline__ void block_reduce_lanes(double a, double b, double2* out, double2 (*scratch)[G]) {
     for (int o = G; o < 32; o <<= 1) {
         a += __shfl_xor_sync(0xffffffffu, a, o);
@@ -110,7 +116,7 @@ __device__ __forceinline__ void block_reduce_lanes(double a, double b, double2* 
     __syncthreads();
     if (threadIdx.x < G) {
         double sa = 0.0, sb = 0.0;
-        for (int q = 0; q < kBT / 32; ++q) {
+        for (int q = 0; q < NT / 32; ++q) {
             sa += scratch[q][threadIdx.x].x;
             sb += scratch[q][threadIdx.x].y;
         }
@@ -127,22 +133,33 @@ __device__ __forceinline__ T row_weight(const T* wg, const signed char* fold, in
     return wg[(size_t)k * G + fl];
 }
 
-template <class T, int MODEL, int G, int WM>
+template <class T, int MODEL, int G, int WM, int NT>
 __device__ __forceinline__ double objective_partial(const BatchArgs& A, int grp, int r0, int r1, const T* xbg, const T* wg, int fitfold, int fl, bool use_ll) {
+    constexpr int kU = 4;                    // rows in flight
     Kahan<double> acc;
-    const int slot = threadIdx.x / G, nslots = kBT / G;
-    for (int k = r0 + slot; k < r1; k += nslots) {
-        const double v = (double)xbg[(size_t)k * G + fl];
-        const double wt = (double)row_weight<T, WM>(wg, A.fold, fitfold, k, G, fl);
-        const double yk = A.y[k];
-        if (!use_ll) {
-            acc.add(v * yk * wt);                                       // getGradientObjective
-        } else {
-            const int yi = (int)yk;                                     // logLikeNumeratorContrib
-            double c = yi * v * wt;
-            if (MODEL == CYC_LR) c -= wt * log(1.0 + exp(v));          // nw * log(denom), denom = 1 + exb
-            if (MODEL == CYC_PR) c -= wt * exp(v);                      // nw * denom
-            acc.add(c);
+    const int slot = threadIdx.x / G, nslots = NT / G;
+    for (int k0 = r0 + slot; k0 < r1; k0 += kU * nslots) {
+        double vv[kU], ww[kU], yy[kU];
+        #pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int k = min(k0 + u * nslots, r1 - 1);
+            vv[u] = (double)xbg[(size_t)k * G + fl];
+            ww[u] = (double)row_weight<T, WM>(wg, A.fold, fitfold, k, G, fl);
+            yy[u] = A.y[k];
+        }
+        #pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            if (k0 + u * nslots >= r1) break;
+            const double v = vv[u], wt = ww[u], yk = yy[u];
+            if (!use_ll) {
+                acc.add(v * yk * wt);                                   // getGradientObjective
+            } else {
+                const int yi = (int)yk;                                 // logLikeNumeratorContrib
+                double c = yi * v * wt;
+                if (MODEL == CYC_LR) c -= wt * log(1.0 + exp(v));      // nw * log(denom), denom = 1 + exb
+                if (MODEL == CYC_PR) c -= wt * exp(v);                  // nw * denom
+                acc.add(c);
+            }
         }
     }
     return acc.value();
@@ -187,20 +204,15 @@ __device__ __forceinline__ void store_row(T* p, const T (&v)[N]) {
 
 // Thread-per-row layout of one group's G fits: a row's linear predictors
 // are split into TPR parts of FPT = 4 fits (16 bytes in FP32, one 32-byte
-// sector in FP64), and each thread holds R = 2 rows' parts at a time.  The
-// layout is a parameter of the caller (a CTA streaming one long column,
-// BLOCK, or a warp taking one short column of a batch); wider parts or more
-// rows per thread measured slower on B200 here: the registers they take make
-// the rest of the persistent kernel spill.
-template <class T, int G, bool BLOCK>
+// sector in FP64); wider parts or more rows per thread measured slower on B200
+// here: the registers they take make the rest of the persistent kernel spill.
+template <class T, int G>
 struct RowLayout {
     static constexpr int FPT = (G % 4 != 0) ? G : 4;
     static constexpr int TPR = G / FPT;
-    static constexpr int R = 2;
-    // row parts in flight per thread when rows arrive by cp.async (their
-    // slots fit in kAsyncBytes per CTA)
+    // row parts in flight per thread when rows arrive by cp.async
     static constexpr int D = 4;
-    static_assert(kBT * D * FPT * sizeof(T) <= kAsyncBytes, "cp.async slots exceed their shared memory");
+    static_assert(D * FPT * sizeof(T) <= BatchDims<32>::kAsyncBytes / 32, "cp.async slots exceed their shared memory");
 };
 
 // 16-byte asynchronous copies global -> shared (L2 only), one group per row
@@ -257,9 +269,9 @@ __device__ __forceinline__ double warp_reduce_rows(const double (&g)[FPT], const
 
 // Block sum of per-thread (g, h) parts into out[f] = (g, h): warp sums, then
 // the warps' sums in warp order.  Deterministic.
-template <int G, int FPT, int TPR>
+template <int G, int FPT, int TPR, int NT>
 __device__ __forceinline__ void block_reduce_rows(const double (&g)[FPT], const double (&h)[FPT], double2* out,
-                                                  double* scr /* [kBT/32][2G] */) {
+                                                  double* scr /* [NT/32][2G] */) {
     const int wid = threadIdx.x >> 5;
     int fit;
     bool is_h, holder;
@@ -268,7 +280,7 @@ __device__ __forceinline__ void block_reduce_rows(const double (&g)[FPT], const 
     __syncthreads();
     if (threadIdx.x < 2 * G) {
         double s = 0.0;
-        for (int q = 0; q < kBT / 32; ++q) s += scr[q * 2 * G + threadIdx.x];
+        for (int q = 0; q < NT / 32; ++q) s += scr[q * 2 * G + threadIdx.x];
         if (threadIdx.x < G) out[threadIdx.x].x = s;
         else out[threadIdx.x - G].y = s;
     }
@@ -309,9 +321,9 @@ struct ColRows {
 template <class T, int MODEL, int G, int WM, int STRIDE>
 __device__ __forceinline__ void rows_gh(const ColRows<T>& c, int t0, const T* xbg, const T* wg,
                                         const signed char* fold, const unsigned char* wmask, unsigned done, T* abuf,
-                                        double (&g)[RowLayout<T, G, STRIDE == kBT>::FPT],
-                                        double (&h)[RowLayout<T, G, STRIDE == kBT>::FPT]) {
-    using Lay = RowLayout<T, G, STRIDE == kBT>;
+                                        double (&g)[RowLayout<T, G>::FPT],
+                                        double (&h)[RowLayout<T, G>::FPT]) {
+    using Lay = RowLayout<T, G>;
     constexpr int FPT = Lay::FPT, TPR = Lay::TPR, D = Lay::D, RS = STRIDE / TPR;
     const int f0 = (t0 % TPR) * FPT;
     const unsigned dn = done >> f0;
@@ -368,7 +380,7 @@ __device__ __forceinline__ void rows_gh(const ColRows<T>& c, int t0, const T* xb
 // from registers)
 template <class T, int G, int STRIDE>
 __device__ __forceinline__ void rows_update(const ColRows<T>& c, int t0, T* xbg, const T (&d)[G], T* abuf) {
-    using Lay = RowLayout<T, G, STRIDE == kBT>;
+    using Lay = RowLayout<T, G>;
     constexpr int FPT = Lay::FPT, TPR = Lay::TPR, D = Lay::D, RS = STRIDE / TPR;
     const int f0 = (t0 % TPR) * FPT;
     bool moved = false;                     // a part whose fits all kept their coefficients stays
@@ -415,22 +427,22 @@ __device__ __forceinline__ void rows_update(const ColRows<T>& c, int t0, T* xbg,
 // for columns without a step), U items per thread in flight.  Entries on the
 // batch's shared rows (`drow`, nd of them) are left to their owner.  No two
 // items touch the same (row, part): a row outside `drow` is in one column.
-template <class T, int G>
+template <class T, int G, int NT>
 __device__ __forceinline__ void batch_update(T* xbg, const int* idx, const double* val, const int* sidx, const T* sx,
                                              const long long* cp, const long long* vp, const int* e0, const int* off,
                                              const int* fmt, int q, int L, const int* boff,
                                              const double (*dr)[G], const int* drow, int nd) {
-    using Lay = RowLayout<T, G, false>;
+    using Lay = RowLayout<T, G>;
     constexpr int FPT = Lay::FPT, TPR = Lay::TPR, U = 4;
     unsigned bloom = 0;
     for (int d = 0; d < nd; ++d) bloom |= 1u << (drow[d] & 31);
     const int items = boff[L] * TPR;
-    for (int i0 = threadIdx.x; i0 < items; i0 += U * kBT) {
+    for (int i0 = threadIdx.x; i0 < items; i0 += U * NT) {
         int k[U], w[U];
         T x[U];
         #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int i = i0 + u * kBT;
+            const int i = i0 + u * NT;
             k[u] = -1;
             w[u] = 0;
             x[u] = T(1);
@@ -461,11 +473,11 @@ __device__ __forceinline__ void batch_update(T* xbg, const int* idx, const doubl
         T v[U][FPT];
         #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (k[u] >= 0) load_row<T, FPT>(xbg + (size_t)k[u] * G + ((i0 + u * kBT) % TPR) * FPT, v[u]);
+            if (k[u] >= 0) load_row<T, FPT>(xbg + (size_t)k[u] * G + ((i0 + u * NT) % TPR) * FPT, v[u]);
         #pragma unroll
         for (int u = 0; u < U; ++u) {
             if (k[u] < 0) continue;
-            const int f0 = ((i0 + u * kBT) % TPR) * FPT;
+            const int f0 = ((i0 + u * NT) % TPR) * FPT;
             #pragma unroll
             for (int f = 0; f < FPT; ++f) v[u][f] = upd_fma((T)dr[w[u]][f0 + f], x[u], v[u][f]);
             store_row<T, FPT>(xbg + (size_t)k[u] * G + f0, v[u]);
@@ -481,13 +493,13 @@ __device__ __forceinline__ void batch_update(T* xbg, const int* idx, const doubl
 // partials then read shared memory and the update writes the new values from
 // it without reading global memory again.  It occupies the bytes the
 // cp.async row slots of the single-column path use (kAsyncBytes).
-template <class T, int G>
+template <class T, int G, int NT>
 struct BatchCache {
     static constexpr int kPieces = (int)(G * sizeof(T)) / 16;          // 16-byte pieces of a row
     static constexpr int kEntryBytes = (int)(G * sizeof(T) + sizeof(int) + sizeof(T) + 1);
-    static constexpr int kRows = (kAsyncBytes / kEntryBytes) / 32 * 32;
+    static constexpr int kRows = (BatchDims<NT>::kAsyncBytes / kEntryBytes) / 32 * 32;
     static_assert(kPieces >= 1 && (G * sizeof(T)) % 16 == 0, "rows are whole 16-byte pieces");
-    static_assert(kRows * kEntryBytes <= kAsyncBytes, "the batch cache exceeds its shared memory");
+    static_assert(kRows * kEntryBytes <= BatchDims<NT>::kAsyncBytes, "the batch cache exceeds its shared memory");
     T* v;                  // [kRows][G] linear predictors at the batch's start
     int* row;              // [kRows] row ids
     T* x;                  // [kRows] values (1 for indicators)
@@ -504,15 +516,15 @@ struct BatchCache {
 // Gather the batch's entries in this CTA's rows (columns q .. q+L-1, entry
 // offsets boff[0..L]) into the cache; returns after every copy has landed
 // and the CTA has synchronised.
-template <class T, int G, int WM>
-__device__ __forceinline__ void batch_gather(const BatchCache<T, G>& bc, const T* xbg, const int* idx,
+template <class T, int G, int WM, int NT>
+__device__ __forceinline__ void batch_gather(const BatchCache<T, G, NT>& bc, const T* xbg, const int* idx,
                                              const double* val, const signed char* fold, const int* sidx,
                                              const long long* cp, const long long* vp, const int* e0,
                                              const int* off, const int* fmt, int q, const int* boff, int L) {
-    constexpr int P = BatchCache<T, G>::kPieces;
+    constexpr int P = BatchCache<T, G, NT>::kPieces;
     constexpr int PV = 16 / (int)sizeof(T);
     const int E = boff[L];
-    for (int i = threadIdx.x; i < E * P; i += kBT) {
+    for (int i = threadIdx.x; i < E * P; i += NT) {
         const int e = i / P, p = i % P;
         int w = 0;
         while (e >= boff[w + 1]) ++w;
@@ -521,7 +533,7 @@ __device__ __forceinline__ void batch_gather(const BatchCache<T, G>& bc, const T
         cp_async16(bc.v + (size_t)e * G + p * PV, xbg + (size_t)k * G + p * PV);
     }
     cp_async_commit();
-    for (int e = threadIdx.x; e < E; e += kBT) {
+    for (int e = threadIdx.x; e < E; e += NT) {
         int w = 0;
         while (e >= boff[w + 1]) ++w;
         const int qq = q + w, el = e - boff[w];
@@ -540,14 +552,14 @@ __device__ __forceinline__ void batch_gather(const BatchCache<T, G>& bc, const T
 // b0 + t / TPR, b0 + t / TPR + STRIDE / TPR, ... and fits part t % TPR of
 // each -- the entries and order rows_gh gives them, so the sums are the
 // same.
-template <class T, int MODEL, int G, int WM, int STRIDE = 32>
-__device__ __forceinline__ void cache_gh(const BatchCache<T, G>& bc, int b0, int b1, bool ind, const T* wg,
+template <class T, int MODEL, int G, int WM, int NT, int STRIDE = 32>
+__device__ __forceinline__ void cache_gh(const BatchCache<T, G, NT>& bc, int b0, int b1, bool ind, const T* wg,
                                          const unsigned char* wmask, unsigned done,
-                                         double (&g)[RowLayout<T, G, STRIDE == kBT>::FPT],
-                                         double (&h)[RowLayout<T, G, STRIDE == kBT>::FPT]) {
-    using Lay = RowLayout<T, G, STRIDE == kBT>;
+                                         double (&g)[RowLayout<T, G>::FPT],
+                                         double (&h)[RowLayout<T, G>::FPT]) {
+    using Lay = RowLayout<T, G>;
     constexpr int FPT = Lay::FPT, TPR = Lay::TPR, RS = STRIDE / TPR;
-    const int lane = STRIDE == kBT ? (int)threadIdx.x : (int)(threadIdx.x & 31);
+    const int lane = STRIDE == NT ? (int)threadIdx.x : (int)(threadIdx.x & 31);
     const int f0 = (lane % TPR) * FPT;
     const unsigned dn = done >> f0;
     Kahan<T> ag[FPT], ah[FPT];
@@ -573,15 +585,15 @@ __device__ __forceinline__ void cache_gh(const BatchCache<T, G>& bc, int b0, int
 // column with a step writes its new values from the cache; entries on the
 // batch's shared rows (`drow`, nd of them) are left to their owner.  No two
 // items touch the same (row, part): a row outside `drow` is in one column.
-template <class T, int G>
-__device__ __forceinline__ void cache_update(const BatchCache<T, G>& bc, T* xbg, const int* boff, int L,
+template <class T, int G, int NT>
+__device__ __forceinline__ void cache_update(const BatchCache<T, G, NT>& bc, T* xbg, const int* boff, int L,
                                              const double (*dr)[G], const int* drow, int nd) {
-    using Lay = RowLayout<T, G, false>;
+    using Lay = RowLayout<T, G>;
     constexpr int FPT = Lay::FPT, TPR = Lay::TPR;
     unsigned bloom = 0;
     for (int d = 0; d < nd; ++d) bloom |= 1u << (drow[d] & 31);
     const int items = boff[L] * TPR;
-    for (int i = threadIdx.x; i < items; i += kBT) {
+    for (int i = threadIdx.x; i < items; i += NT) {
         const int e = i / TPR, f0 = (i % TPR) * FPT;
         int w = 0;
         while (e >= boff[w + 1]) ++w;
@@ -611,28 +623,30 @@ constexpr int kStage = 4096;
 
 // Columns processed together: consecutive short columns form a batch of at
 // most kRunMax; warp w of every CTA takes column w of the batch, and the batch
-// pays for one load round trip and one cluster barrier.
-constexpr int kRunMax = kBT / 32;
-// A batch may share rows between its columns: at most kDirtyMax such rows,
-// replayed serially (see k_batch).  Columns of at most kBatchCap entries in every CTA's rows join.
-constexpr int kDirtyMax = 32;
+// pays for one load round trip and one cluster barrier.  A batch may share
+// rows between its columns: at most kDirtyMax such rows, replayed serially (see
+// k_batch).  Columns of at most kBatchCap entries in every CTA's rows join.
 constexpr int kBatchCap = 256;
 
 // The batch shape of an 8-fit group's plan: columns with at most `cap`
 // entries in every CTA's rows are short (batched, a warp per column; the
 // rest stream through the whole CTA), a batch shares at most `dmax` rows
 // between its columns and replays at most `lvl` levels.  The defaults are
-// the largest the kernel's shared memory allows; the shape tuner
-// (tuned_shape) may pick smaller ones for a problem.
+// the largest the kernel's shared memory allows (dmax: threads / 8); the shape
+// tuner (tuned_shape) may pick smaller ones for a problem.
 struct BatchShape {
     int cap = 256, dmax = 32, lvl = 8;
-    bool operator==(const BatchShape& o) const { return cap == o.cap && dmax == o.dmax && lvl == o.lvl; }
+    int threads = 256;                    // a CTA's (256 or 512): a batch has at most threads / 32 columns
+    bool operator==(const BatchShape& o) const {
+        return cap == o.cap && dmax == o.dmax && lvl == o.lvl && threads == o.threads;
+    }
 };
 // levels of the serial replay a batch may have (each costs a step chain)
-constexpr int kLevelMax = kRunMax;
+constexpr int kLevelMax = 8;
 
-template <class T, int MODEL, int G, int WM>
-__global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
+template <class T, int MODEL, int G, int WM, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) k_batch(const BatchArgs A) {
+    constexpr int kRunMax = BatchDims<NT>::kRunMax, kDirtyMax = BatchDims<NT>::kDirtyMax;
     cg::cluster_group cluster = cg::this_cluster();
     const int C = A.C;
     const int rank = (int)cluster.block_rank();
@@ -640,8 +654,7 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
     const int r0 = A.rpart[rank], r1 = A.rpart[rank + 1];
     // columns stream thread per row (all fits of a row by vector loads) and
     // short columns go in batches
-    using LayW = RowLayout<T, G, false>;   // a warp per column (batches)
-    using LayB = RowLayout<T, G, true>;    // the CTA per column (single columns)
+    using Lay = RowLayout<T, G>;
     T* xbg = (T*)A.xb + (size_t)grp * A.K * G;
     const T* wg = (WM == 0) ? (const T*)A.w + (size_t)grp * A.K * G : nullptr;
     const int fl = threadIdx.x % G;
@@ -649,10 +662,7 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
     const int fg = grp * G;                   // first fit of the group
     const int fitfold = (WM == 1) ? A.fitfold[fg + fl] : 0;
 
-    // every CTA's (g, h) partials, pushed into each CTA of the cluster before
-    // the barrier (double buffered by parity; one slot per column of a run)
-    __shared__ double2 s_part[2][kMaxC][kRunMax][G];
-    __shared__ double2 s_scr[kBT / 32][G];
+    __shared__ double2 s_scr[NT / 32][G];
     __shared__ double2 s_red[G];
     __shared__ double s_obj[2][kMaxC][G];
     __shared__ double s_dr[kRunMax][G];
@@ -690,12 +700,15 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
     int* s_sidx = reinterpret_cast<int*>(dyn_smem + 3 * kChunk * G * sizeof(double));
     // each thread's cp.async row slots; the batch cache shares those bytes
     T* s_slots = reinterpret_cast<T*>(dyn_smem + 3 * kChunk * G * sizeof(double) + kStage * sizeof(int));
-    T* s_abuf = s_slots + (size_t)threadIdx.x * LayB::D * LayB::FPT;
-    const BatchCache<T, G> bcache(s_slots);
+    T* s_abuf = s_slots + (size_t)threadIdx.x * Lay::D * Lay::FPT;
+    const BatchCache<T, G, NT> bcache(s_slots);
     // shared rows of the open batch: as pushed by their owners (by parity; the
     // replay then moves this CTA's copy of the current parity in place), their
     // model means at the batch's start and now, and their weights
-    T* s_dirty = reinterpret_cast<T*>(reinterpret_cast<unsigned char*>(s_slots) + kAsyncBytes);
+    T* s_dirty = reinterpret_cast<T*>(reinterpret_cast<unsigned char*>(s_slots) + BatchDims<NT>::kAsyncBytes);
+    // every CTA's (g, h) partials, pushed into each CTA of the cluster before
+    // the barrier (double buffered by parity; one slot per column of a run)
+    double2 (*s_part)[kMaxC][kRunMax][G] = reinterpret_cast<double2 (*)[kMaxC][kRunMax][G]>(s_dirty + 5 * kDirtyMax * G);
     T (*s_dst)[kDirtyMax][G] = reinterpret_cast<T (*)[kDirtyMax][G]>(s_dirty);
     T (*s_m0)[G] = reinterpret_cast<T (*)[G]>(s_dirty + 2 * kDirtyMax * G);
     T (*s_mc)[G] = reinterpret_cast<T (*)[G]>(s_dirty + 3 * kDirtyMax * G);
@@ -721,8 +734,8 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
     // initial objective (findMode :949-953)
     int opar = 0;
     {
-        const double p = objective_partial<T, MODEL, G, WM>(A, grp, r0, r1, xbg, wg, fitfold, fl, use_ll);
-        block_reduce_lanes<G>(p, 0.0, s_red, s_scr);
+        const double p = objective_partial<T, MODEL, G, WM, NT>(A, grp, r0, r1, xbg, wg, fitfold, fl, use_ll);
+        block_reduce_lanes<G, NT>(p, 0.0, s_red, s_scr);
         if (threadIdx.x < G)
             for (int r = 0; r < C; ++r) *cluster.map_shared_rank(&s_obj[opar][rank][threadIdx.x], r) = s_red[threadIdx.x].x;
         if (C > 1) cluster.sync(); else __syncthreads();
@@ -764,28 +777,23 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
             if (dl != 0.0) c_beta[qq][f] = b + dl;
             return dl;
         };
-        // work counters of L columns from chunk coordinate q0 (deltas in s_dr),
-        // kept by thread 0 of every CTA over the CTA's own entries of each
-        // column (shared memory only: the counters stay off the loads); the
-        // CTAs' counts add up to the group's, the steps are counted by rank 0
-        auto count_run = [&](int q0, int L) {
-            int act = 0;
-            for (int f = 0; f < G; ++f) act += !s_done[f];
-            for (int w = 0; w < L; ++w) {
-                int upd = 0;
-                for (int f = 0; f < G; ++f) upd += (s_dr[w][f] != 0.0);
-                const int fm = c_fmt[q0 + w];
-                const bool dn = (fm == CYC_DENSE || fm == CYC_INTERCEPT);
-                const bool in = (fm == CYC_INDICATOR || fm == CYC_INTERCEPT);
-                const long long nn = c_e1[q0 + w] - c_e0[q0 + w];
-                n_grad += (unsigned long long)(act * nn);
-                n_upd += (unsigned long long)(upd * nn);
-                if (rank == 0) n_steps += act;
-                n_idx += (unsigned long long)(nn * ((dn ? 0 : 4) + (in ? 0 : 8)) * (1 + (upd ? 1 : 0)));
-            }
+        // work counters of a column (chunk coordinate q, `upd` of its steps not
+        // zero) over the CTA's own entries, kept by lane 0 of the warp that took
+        // the steps; the CTAs' counts add up to the group's, the steps are
+        // counted by rank 0
+        const int running = __popc(~done_m & ((1u << G) - 1u));
+        auto count = [&](int q, int upd) {
+            const int fm = c_fmt[q];
+            const bool dn = (fm == CYC_DENSE || fm == CYC_INTERCEPT);
+            const bool in = (fm == CYC_INDICATOR || fm == CYC_INTERCEPT);
+            const long long nn = c_e1[q] - c_e0[q];
+            n_grad += (unsigned long long)(running * nn);
+            n_upd += (unsigned long long)(upd * nn);
+            if (rank == 0) n_steps += running;
+            n_idx += (unsigned long long)(nn * ((dn ? 0 : 4) + (in ? 0 : 8)) * (1 + (upd ? 1 : 0)));
         };
         // ---- stage the chunk (coalesced)
-        for (int q = threadIdx.x; q < jn; q += kBT) {
+        for (int q = threadIdx.x; q < jn; q += NT) {
             const int j = j0 + q;
             const int f0 = A.fmt[j];
             c_fmt[q] = f0;
@@ -804,7 +812,7 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
             c_e0[q] = dn ? r0 : A.split[j * (C + 1) + rank];
             c_e1[q] = dn ? r1 : A.split[j * (C + 1) + rank + 1];
         }
-        for (int q = threadIdx.x; q < jn * G; q += kBT) {
+        for (int q = threadIdx.x; q < jn * G; q += NT) {
             const int ff = q / jn, jj = q % jn;
             const size_t o = (size_t)(fg + ff) * A.J + j0 + jj;
             c_beta[jj][ff] = A.beta[o];
@@ -836,7 +844,7 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
         __syncthreads();
         {
             const int ns = c_ns, total = c_soff[ns];
-            for (int t = threadIdx.x; t < total; t += kBT) {
+            for (int t = threadIdx.x; t < total; t += NT) {
                 int lo = 0, hi = ns - 1;                 // last staged column with offset <= t
                 while (lo < hi) {
                     const int mid = (lo + hi + 1) >> 1;
@@ -866,7 +874,7 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
                 const int de0 = c_de0[q], nde = c_de0[q + L] - de0;
                 // rows shared inside the batch: their owners push them (all G fits)
                 // into every CTA; the weights of those rows are kept locally
-                for (int t = threadIdx.x; t < nd * G; t += kBT) {
+                for (int t = threadIdx.x; t < nd * G; t += NT) {
                     const int d = t / G, f = t % G;
                     const int k = __ldg(A.drow + dr0 + d);
                     if (k >= r0 && k < r1) {
@@ -881,7 +889,7 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
                     }
                 }
                 if (threadIdx.x <= L) s_bde_ptr[threadIdx.x] = c_de0[q + threadIdx.x] - de0;
-                for (int t = threadIdx.x; t < nde; t += kBT) {
+                for (int t = threadIdx.x; t < nde; t += NT) {
                     s_bde_d[t] = __ldg(A.de_d + de0 + t) & 0xff;
                     s_bde_x[t] = __ldg(A.de_x + de0 + t);
                 }
@@ -892,19 +900,19 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
                     s_cbo[threadIdx.x] = o;
                 }
                 __syncthreads();
-                const bool cached = s_cbo[L] <= BatchCache<T, G>::kRows;
+                const bool cached = s_cbo[L] <= BatchCache<T, G, NT>::kRows;
                 if (cached)
-                    batch_gather<T, G, WM>(bcache, xbg, A.idx, A.val, A.fold, s_sidx, c_cp, c_vp, c_e0, c_off, c_fmt,
+                    batch_gather<T, G, WM, NT>(bcache, xbg, A.idx, A.val, A.fold, s_sidx, c_cp, c_vp, c_e0, c_off, c_fmt,
                                            q, s_cbo, L);
                 // gradient partials of every column from the state at the batch's start
                 if (cached) {
                     if (warp < L) {
-                        double g[LayW::FPT], h[LayW::FPT];
-                        cache_gh<T, MODEL, G, WM>(bcache, s_cbo[warp], s_cbo[warp + 1], c_fmt[q + warp] == CYC_INDICATOR,
+                        double g[Lay::FPT], h[Lay::FPT];
+                        cache_gh<T, MODEL, G, WM, NT>(bcache, s_cbo[warp], s_cbo[warp + 1], c_fmt[q + warp] == CYC_INDICATOR,
                                                   wg, s_wmask, done_m, g, h);
                         int fit;
                         bool is_h, holder;
-                        const double v = warp_reduce_rows<LayW::FPT, LayW::TPR>(g, h, fit, is_h, holder);
+                        const double v = warp_reduce_rows<Lay::FPT, Lay::TPR>(g, h, fit, is_h, holder);
                         if (holder) {
                             double* dst = is_h ? &s_part[par][rank][warp][fit].y : &s_part[par][rank][warp][fit].x;
                             for (int r = 0; r < C; ++r) *cluster.map_shared_rank(dst, r) = v;
@@ -912,13 +920,13 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
                     }
                 } else if (warp < L) {
                     const int qq = q + warp, so = c_off[qq];
-                    double g[LayW::FPT], h[LayW::FPT];
+                    double g[Lay::FPT], h[Lay::FPT];
                     const ColRows<T> cr{A.idx + c_cp[qq], A.val + c_vp[qq], so >= 0 ? s_sidx + so : nullptr,
                                         nullptr, c_e0[qq], c_e1[qq], false, c_fmt[qq] == CYC_INDICATOR};
                     rows_gh<T, MODEL, G, WM, 32>(cr, lane, xbg, wg, A.fold, s_wmask, done_m, s_abuf, g, h);
                     int fit;
                     bool is_h, holder;
-                    const double v = warp_reduce_rows<LayW::FPT, LayW::TPR>(g, h, fit, is_h, holder);
+                    const double v = warp_reduce_rows<Lay::FPT, Lay::TPR>(g, h, fit, is_h, holder);
                     if (holder) {
                         double* dst = is_h ? &s_part[par][rank][warp][fit].y : &s_part[par][rank][warp][fit].x;
                         for (int r = 0; r < C; ++r) *cluster.map_shared_rank(dst, r) = v;
@@ -932,7 +940,7 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
                 // The shared rows move in place in s_dst[par]; their means at the
                 // start (s_m0) and now (s_mc) make a correction exp-free.
                 if (nd > 0) {
-                    for (int t = threadIdx.x; t < nd * G; t += kBT) {
+                    for (int t = threadIdx.x; t < nd * G; t += NT) {
                         const T m = row_mean<T, MODEL>(s_dst[par][t / G][t % G]);
                         s_m0[t / G][t % G] = m;
                         s_mc[t / G][t % G] = m;
@@ -987,6 +995,8 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
                             dl = coord_step(qq, lane, g, h);
                             s_dr[warp][lane] = dl;
                         }
+                        const unsigned moved = __ballot_sync(0xffffffffu, dl != 0.0);
+                        if (lane == 0) count(qq, __popc(moved));
                         dl = __shfl_sync(0xffffffffu, dl, fw);
                         if (dl != 0.0)
                             for (int i = i0 + sl; i < i1; i += 32 / G) {
@@ -1005,7 +1015,7 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
                 // coefficients are skipped.  A cached batch writes the new values
                 // from the cache.
                 if (cached) {
-                    cache_update<T, G>(bcache, xbg, s_cbo, L, s_dr, s_drow, nd);
+                    cache_update<T, G, NT>(bcache, xbg, s_cbo, L, s_dr, s_drow, nd);
                 } else {
                     if (threadIdx.x == 0) {
                         int o = 0;
@@ -1018,15 +1028,14 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
                         s_boff[L] = o;
                     }
                     __syncthreads();
-                    batch_update<T, G>(xbg, A.idx, A.val, s_sidx, nullptr, c_cp, c_vp, c_e0, c_off, c_fmt, q, L,
+                    batch_update<T, G, NT>(xbg, A.idx, A.val, s_sidx, nullptr, c_cp, c_vp, c_e0, c_off, c_fmt, q, L,
                                        s_boff, s_dr, s_drow, nd);
                 }
-                for (int t = threadIdx.x; t < nd * G; t += kBT) {
+                for (int t = threadIdx.x; t < nd * G; t += NT) {
                     const int d = t / G, k = s_drow[d];
                     if (k >= r0 && k < r1) xbg[(size_t)k * G + t % G] = s_dst[par][d][t % G];
                 }
                 __syncthreads();
-                if (threadIdx.x == 0) count_run(q, L);
                 par ^= 1;
                 q += L;
                 continue;
@@ -1037,21 +1046,21 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
                 const bool dense = (fmt == CYC_DENSE || fmt == CYC_INTERCEPT);
                 const ColRows<T> cr{A.idx + c_cp[q], A.val + c_vp[q], so >= 0 ? s_sidx + so : nullptr, nullptr,
                                     c_e0[q], c_e1[q], dense, fmt == CYC_INDICATOR || fmt == CYC_INTERCEPT};
-                double g[LayB::FPT], h[LayB::FPT];
+                double g[Lay::FPT], h[Lay::FPT];
                 // a column whose entries in my rows fit the batch cache is
                 // gathered once and updated from the cache
                 const int n1 = c_e1[q] - c_e0[q];
-                const bool cached1 = !dense && n1 <= BatchCache<T, G>::kRows;
+                const bool cached1 = !dense && n1 <= BatchCache<T, G, NT>::kRows;
                 if (cached1) {
                     if (threadIdx.x <= 1) s_cbo[threadIdx.x] = threadIdx.x ? n1 : 0;
                     __syncthreads();
-                    batch_gather<T, G, WM>(bcache, xbg, A.idx, A.val, A.fold, s_sidx, c_cp, c_vp, c_e0, c_off,
+                    batch_gather<T, G, WM, NT>(bcache, xbg, A.idx, A.val, A.fold, s_sidx, c_cp, c_vp, c_e0, c_off,
                                            c_fmt, q, s_cbo, 1);
-                    cache_gh<T, MODEL, G, WM, kBT>(bcache, 0, n1, cr.ind, wg, s_wmask, done_m, g, h);
+                    cache_gh<T, MODEL, G, WM, NT, NT>(bcache, 0, n1, cr.ind, wg, s_wmask, done_m, g, h);
                 } else {
-                    rows_gh<T, MODEL, G, WM, kBT>(cr, threadIdx.x, xbg, wg, A.fold, s_wmask, done_m, s_abuf, g, h);
+                    rows_gh<T, MODEL, G, WM, NT>(cr, threadIdx.x, xbg, wg, A.fold, s_wmask, done_m, s_abuf, g, h);
                 }
-                block_reduce_rows<G, LayB::FPT, LayB::TPR>(g, h, s_red, reinterpret_cast<double*>(s_scr));
+                block_reduce_rows<G, Lay::FPT, Lay::TPR, NT>(g, h, s_red, reinterpret_cast<double*>(s_scr));
                 if (threadIdx.x < G)
                     for (int r = 0; r < C; ++r) *cluster.map_shared_rank(&s_part[par][rank][0][threadIdx.x], r) = s_red[threadIdx.x];
                 if (C > 1) cluster.sync(); else __syncthreads();
@@ -1062,17 +1071,19 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
                         gs += pp.x;
                         hs += pp.y;
                     }
-                    s_dr[0][threadIdx.x] = coord_step(q, threadIdx.x, gs, hs);
+                    const double dl = coord_step(q, threadIdx.x, gs, hs);
+                    s_dr[0][threadIdx.x] = dl;
+                    const unsigned moved = __ballot_sync((1u << G) - 1u, dl != 0.0);
+                    if (threadIdx.x == 0) count(q, __popc(moved));
                 }
                 __syncthreads();
                 T dd[G];
                 bool any = false;
                 #pragma unroll
                 for (int f = 0; f < G; ++f) { dd[f] = (T)s_dr[0][f]; any |= (s_dr[0][f] != 0.0); }
-                if (threadIdx.x == 0) count_run(q, 1);
                 if (any) {
-                    if (cached1) cache_update<T, G>(bcache, xbg, s_cbo, 1, s_dr, s_drow, 0);
-                    else rows_update<T, G, kBT>(cr, threadIdx.x, xbg, dd, s_abuf);
+                    if (cached1) cache_update<T, G, NT>(bcache, xbg, s_cbo, 1, s_dr, s_drow, 0);
+                    else rows_update<T, G, NT>(cr, threadIdx.x, xbg, dd, s_abuf);
                 }
                 __syncthreads();
                 par ^= 1;
@@ -1081,7 +1092,7 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
         }
         // chunk done: rank 0 writes the group's beta and trust regions back
         if (rank == 0)
-            for (int qq = threadIdx.x; qq < jn * G; qq += kBT) {
+            for (int qq = threadIdx.x; qq < jn * G; qq += NT) {
                 const int ff = qq / jn, jj = qq % jn;
                 const size_t o = (size_t)(fg + ff) * A.J + j0 + jj;
                 A.beta[o] = c_beta[jj][ff];
@@ -1090,8 +1101,8 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
         __syncthreads();
       }
         // ---- convergence test (performCheckConvergence)
-        const double p = objective_partial<T, MODEL, G, WM>(A, grp, r0, r1, xbg, wg, fitfold, fl, use_ll);
-        block_reduce_lanes<G>(p, 0.0, s_red, s_scr);
+        const double p = objective_partial<T, MODEL, G, WM, NT>(A, grp, r0, r1, xbg, wg, fitfold, fl, use_ll);
+        block_reduce_lanes<G, NT>(p, 0.0, s_red, s_scr);
         if (threadIdx.x < G)
             for (int r = 0; r < C; ++r) *cluster.map_shared_rank(&s_obj[opar][rank][threadIdx.x], r) = s_red[threadIdx.x].x;
         if (C > 1) cluster.sync(); else __syncthreads();
@@ -1139,7 +1150,7 @@ __global__ void __launch_bounds__(kBT, 2) k_batch(const BatchArgs A) {
         A.out_flag[f] = s_flag[threadIdx.x];
         A.out_obj[f] = s_last[threadIdx.x];
     }
-    if (threadIdx.x == 0) {
+    if (lane == 0) {
         atomicAdd(A.counters + 0, n_grad);
         atomicAdd(A.counters + 1, n_upd);
         if (rank == 0) atomicAdd(A.counters + 2, n_steps);
@@ -1420,8 +1431,8 @@ __global__ void k_batch_llfixed(int K, int G, int F, const double* c, const T* w
 
 // Column batches (see k_batch): walk the columns in order and extend the open
 // batch with the next short column (sparse or indicator, not fixed, at most
-// `cap` entries in every CTA's rows) while it holds fewer than kRunMax
-// columns, the chunk of kChunk coordinates goes on, and the rows shared
+// `cap` entries in every CTA's rows) while it holds fewer than a column a
+// warp, the chunk of kChunk coordinates goes on, and the rows shared
 // between its columns number at most `dmax`; otherwise close it and open a new
 // one.  A column's level is 1 + the highest level of the earlier columns of
 // its batch it shares a row with, so columns of one level touch disjoint
@@ -1496,7 +1507,7 @@ static RunPlan plan_runs(const Dataset& ds, const std::vector<int>& rpart, const
                     fresh += rs[rows[e]].dslot < 0;
                     level = std::max(level, rs[rows[e]].rlvl + 1);
                 }
-        if (start >= 0 && (len == kRunMax || (int)shared.size() + fresh > dmax || level > lvl_max)) {
+        if (start >= 0 && (len == shape.threads / 32 || (int)shared.size() + fresh > dmax || level > lvl_max)) {
             close();
             level = 1;
         }
@@ -1531,14 +1542,21 @@ static RunPlan plan_runs(const Dataset& ds, const std::vector<int>& rpart, const
     return P;
 }
 
-template <class T, int MODEL, int G, int WM>
+template <class T, int G, int NT>
+static size_t batch_smem() {
+    using Dims = BatchDims<NT>;
+    return 3 * kChunk * G * sizeof(double) + kStage * sizeof(int) + (size_t)Dims::kAsyncBytes +
+           5 * Dims::kDirtyMax * G * sizeof(T) + 2 * kMaxC * Dims::kRunMax * G * sizeof(double2);
+}
+
+template <class T, int MODEL, int G, int WM, int NT>
 static void launch_batch(const BatchArgs& a, int ngroups, cudaStream_t stream) {
+    auto kern = k_batch<T, MODEL, G, WM, NT>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ngroups * a.C);
-    cfg.blockDim = dim3(kBT);
-    const size_t dyn = 3 * kChunk * G * sizeof(double) + kStage * sizeof(int) + (size_t)kAsyncBytes +
-                       5 * kDirtyMax * G * sizeof(T);
-    CYC_CHECK_CUDA(cudaFuncSetAttribute(k_batch<T, MODEL, G, WM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    cfg.blockDim = dim3(NT);
+    const size_t dyn = batch_smem<T, G, NT>();
+    CYC_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     cfg.dynamicSmemBytes = dyn;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -1548,18 +1566,24 @@ static void launch_batch(const BatchArgs& a, int ngroups, cudaStream_t stream) {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    CYC_CHECK_CUDA(cudaLaunchKernelEx(&cfg, k_batch<T, MODEL, G, WM>, a));
+    CYC_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
     count_launch();
 }
 
-template <class T, int G>
-static void launch_model(const BatchArgs& a, int ngroups, cudaStream_t stream) {
+template <class T, int G, int NT>
+static void launch_threads(const BatchArgs& a, int ngroups, cudaStream_t stream) {
     const bool cv = a.fold != nullptr;
     switch (a.model) {
-    case CYC_LR: cv ? launch_batch<T, CYC_LR, G, 1>(a, ngroups, stream) : launch_batch<T, CYC_LR, G, 0>(a, ngroups, stream); break;
-    case CYC_PR: cv ? launch_batch<T, CYC_PR, G, 1>(a, ngroups, stream) : launch_batch<T, CYC_PR, G, 0>(a, ngroups, stream); break;
+    case CYC_LR: cv ? launch_batch<T, CYC_LR, G, 1, NT>(a, ngroups, stream) : launch_batch<T, CYC_LR, G, 0, NT>(a, ngroups, stream); break;
+    case CYC_PR: cv ? launch_batch<T, CYC_PR, G, 1, NT>(a, ngroups, stream) : launch_batch<T, CYC_PR, G, 0, NT>(a, ngroups, stream); break;
     default: throw Error{CYC_ERR_UNSUPPORTED, "grouped batches support lr and pr"};
     }
+}
+
+template <class T, int G>
+static void launch_model(const BatchArgs& a, int threads, int ngroups, cudaStream_t stream) {
+    if (threads == 512) launch_threads<T, G, 512>(a, ngroups, stream);
+    else launch_threads<T, G, 256>(a, ngroups, stream);
 }
 
 // One batched solve at precision T over fits [0, F) with starting
@@ -1572,6 +1596,50 @@ static void launch_model(const BatchArgs& a, int ngroups, cudaStream_t stream) {
 static int default_cluster(int K) {
     if (const char* e = std::getenv("CYC_BATCH_CLUSTER")) return std::max(1, std::min(kMaxC, std::atoi(e)));
     return std::max(1, std::min(kMaxC, (K + 8191) / 8192));
+}
+
+// Clusters of C CTAs of 512 threads the device holds at once (one CTA an SM).
+static int resident_groups(int C) {
+    auto kern = k_batch<double, CYC_LR, 8, 1, 512>;
+    const size_t dyn = batch_smem<double, 8, 512>();
+    CYC_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(512);
+    cfg.dynamicSmemBytes = dyn;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    CYC_CHECK_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
+    return n;
+}
+
+// CTAs and threads of an 8-fit group.  Two CTAs of 256 threads fit an SM: 25
+// groups of 8 such CTAs leave 96 SMs with one and 52 with two, and a cluster
+// goes at the pace of its slowest CTA.  A CTA of 512 threads has the SM to
+// itself, its batches hold twice the columns, and its batch cache twice the
+// entries; it is taken with the most CTAs a group that still run all groups at
+// once, when that is 4 or more.  Logistic CV grids, 256 threads (best size)
+// against 512: 500k rows x 4,000, 200 fits 639 / 544 ms at 5 CTAs; 100k x 4,000,
+// 200 fits 799 / 689; 250k x 2,500, 100 fits 799 / 705 at 8; 100k x 400, 80 fits
+// 24.1 / 19.7.  With 400 fits only 2 CTAs a group fit at once and the two are
+// even (500k x 1,000: 182 / 179; 60k x 1,000, Poisson: 212 / 215): those stay
+// with 256.  CYC_BATCH_CLUSTER="CTAs[,512]" fixes both.
+struct GroupShape { int C, threads; };
+static GroupShape group_shape(int K, int ngroups) {
+    const int base = default_cluster(K);
+    if (const char* e = std::getenv("CYC_BATCH_CLUSTER")) {
+        int c = 0, t = 0;
+        return {base, std::sscanf(e, "%d,%d", &c, &t) == 2 && t == 512 ? 512 : 256};
+    }
+    for (int C = base; C >= 4; --C)
+        if (resident_groups(C) >= ngroups) return {C, 512};
+    return {base, 256};
 }
 
 template <class T>
@@ -1664,12 +1732,13 @@ struct BatchRunner {
         } else {
             const RunPlan* plan = nullptr;
             for (auto& pl : ds.run_plans)
-                if (pl.C == C && pl.cap == shape.cap && pl.dmax == shape.dmax && pl.max_levels == shape.lvl &&
+                if (pl.C == C && pl.threads == shape.threads && pl.cap == shape.cap && pl.dmax == shape.dmax && pl.max_levels == shape.lvl &&
                     pl.fixed == fixed_cols)
                     plan = &pl;
             if (!plan) {
                 RunPlan pl = plan_runs(ds, rpart, fixb, shape);
                 pl.C = C;
+                pl.threads = shape.threads;
                 pl.cap = shape.cap;
                 pl.dmax = shape.dmax;
                 pl.max_levels = shape.lvl;
@@ -1835,7 +1904,7 @@ struct BatchRunner {
         a.de_x = d_dex.get();
         a.conv = ctl.convergence_type; a.tol = tol; a.max_iter = ctl.max_iterations;
         a.out_iter = d_iter.get(); a.out_flag = d_flag.get(); a.out_obj = d_obj.get(); a.counters = d_counters.get();
-        launch_model<T, 8>(a, ngroups, stream);
+        launch_model<T, 8>(a, shape.threads, ngroups, stream);
     }
 
     void run(const cyc_control& ctl, double tol, float* ms) {
@@ -2056,16 +2125,18 @@ std::map<std::pair<TuneKey, int>, BatchShape>& tuned_shapes() {
     return *m;
 }
 
-BatchShape tuned_shape(Dataset& ds, cudaStream_t stream, int F, int G, int C, const cyc_prior& prior,
+BatchShape tuned_shape(Dataset& ds, cudaStream_t stream, int F, int G, int C, int threads, const cyc_prior& prior,
                        const cyc_fit_spec* specs, const std::vector<double>& beta, const std::vector<double>& hd,
                        const int* d_fold, int n_folds, const std::vector<int>* fit_fold, const cyc_control& ctl,
                        const std::vector<int>& fixed_cols) {
     BatchShape best;
+    best.threads = threads;
+    best.dmax = threads / 8;
     if (const char* e = std::getenv("CYC_BATCH_SHAPE")) {
         int a = best.cap, b = best.dmax, c = best.lvl;
         if (std::sscanf(e, "%d,%d,%d", &a, &b, &c) == 3) {
             best.cap = std::max(1, std::min(kBatchCap, a));
-            best.dmax = std::max(0, std::min(kDirtyMax, b));
+            best.dmax = std::max(0, std::min(threads / 8, b));
             best.lvl = std::max(1, std::min(kLevelMax, c));
         }
         return best;
@@ -2075,7 +2146,7 @@ BatchShape tuned_shape(Dataset& ds, cudaStream_t stream, int F, int G, int C, co
     const TuneKey key{ds.model, ds.K, ds.J, F, G, ctl.precision, d_fold ? n_folds : 0, fixed_cols, ds.nnz_idx};
     {
         std::lock_guard<std::mutex> lk(g_tune_mutex);
-        auto it = tuned_shapes().find({key, C});
+        auto it = tuned_shapes().find({key, C * 1024 + threads});
         if (it != tuned_shapes().end()) return it->second;
     }
     auto time = [&](const BatchShape& sh) {
@@ -2094,7 +2165,7 @@ BatchShape tuned_shape(Dataset& ds, cudaStream_t stream, int F, int G, int C, co
     { BatchShape sh = best; sh.dmax = 16; consider(sh); }
     { BatchShape sh = best; sh.lvl = 2; consider(sh); }
     std::lock_guard<std::mutex> lk(g_tune_mutex);
-    tuned_shapes()[{key, C}] = best;
+    tuned_shapes()[{key, C * 1024 + threads}] = best;
     return best;
 }
 
@@ -2127,7 +2198,8 @@ int group_size(Dataset& ds, cudaStream_t stream, int F, const cyc_prior& prior, 
     if (large && std::getenv("CYC_BATCH_CLUSTER")) return 8;
     double visits = 0.0;
     for (int j = 0; j < ds.J; ++j) visits += (double)ds.col_len(j);
-    const double waves8 = std::ceil((double)((F + 7) / 8) * default_cluster(ds.K) / (2.0 * 148));
+    const GroupShape gs = swindle ? GroupShape{default_cluster(ds.K), 256} : group_shape(ds.K, (F + 7) / 8);
+    const double waves8 = gs.threads == 512 ? 0.85 : std::ceil((double)((F + 7) / 8) * gs.C / (2.0 * 148));
     if (ccd_shape(ds, F).cycle_us > 0.8 * (3.0 * ds.J + 0.0025 * visits) * waves8) return 8;
     if (!large || swindle) return 1;
     const TuneKey key{ds.model, ds.K, ds.J, F, 0, ctl.precision, d_fold ? n_folds : 0, fixed_cols, ds.nnz_idx};
@@ -2136,12 +2208,15 @@ int group_size(Dataset& ds, cudaStream_t stream, int F, const cyc_prior& prior, 
         auto it = tuned_groups().find(key);
         if (it != tuned_groups().end()) return it->second;
     }
+    BatchShape eight;
+    eight.threads = gs.threads;
+    eight.dmax = gs.threads / 8;
     auto time = [&](int G) {
         return ctl.precision == CYC_MIXED
-                   ? probe_cycle<float>(ds, stream, F, G, 0, prior, specs, beta, hd, d_fold, n_folds, fit_fold, ctl,
-                                        fixed_cols)
-                   : probe_cycle<double>(ds, stream, F, G, 0, prior, specs, beta, hd, d_fold, n_folds, fit_fold, ctl,
-                                         fixed_cols);
+                   ? probe_cycle<float>(ds, stream, F, G, gs.C, prior, specs, beta, hd, d_fold, n_folds, fit_fold, ctl,
+                                        fixed_cols, eight)
+                   : probe_cycle<double>(ds, stream, F, G, gs.C, prior, specs, beta, hd, d_fold, n_folds, fit_fold,
+                                         ctl, fixed_cols, eight);
     };
     const int best = time(1) < time(8) ? 1 : 8;
     std::lock_guard<std::mutex> lk(g_tune_mutex);
@@ -2318,16 +2393,19 @@ void run_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* specs, i
     };
     // the tuners time whole cycles over every column, which an active-set
     // pass does not run: swindle solves keep the defaults
-    int C = default_cluster(ds.K);
+    int C = default_cluster(ds.K), threads = 256;
     if (G == 1) C = ccd_shape(ds, F).C;
     if (G != 1 && !swindle) {
         NvtxRange range("cyclops batch: cluster tuner");
-        C = tuned_cluster(ds, stream, F, G, *prior, specs, beta, hd, d_fold, n_folds, fit_fold, *ctl, fixed_cols);
+        const GroupShape gs = group_shape(ds.K, (F + 7) / 8);
+        threads = gs.threads;
+        C = threads == 512 ? gs.C
+                           : tuned_cluster(ds, stream, F, G, *prior, specs, beta, hd, d_fold, n_folds, fit_fold, *ctl, fixed_cols);
     }
     BatchShape shape;
     if (!swindle) {
         NvtxRange range("cyclops batch: shape tuner");
-        shape = tuned_shape(ds, stream, F, G, C, *prior, specs, beta, hd, d_fold, n_folds, fit_fold, *ctl,
+        shape = tuned_shape(ds, stream, F, G, C, threads, *prior, specs, beta, hd, d_fold, n_folds, fit_fold, *ctl,
                             fixed_cols);
     }
     int phase = 0;

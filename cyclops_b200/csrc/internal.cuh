@@ -205,7 +205,7 @@ struct ColView {
 // column batches of the batched solver (planned on the host, batch.cu)
 // ---------------------------------------------------------------------------
 struct RunPlan {
-    int C = 0;
+    int C = 0, threads = 0;
     int cap = 0, dmax = 0, max_levels = 0;   // the batch shape it was planned with (short-column
                                              // bound, shared rows, replay levels)
     std::vector<int> fixed;     // columns held fixed besides the offset (ascending)
