@@ -15,7 +15,7 @@
 // plus, on first computeXBeta with a nonzero coefficient, a row-major copy
 // (d_row_ptr / d_row_col / d_row_val) whose per-row column order equals the
 // reference's column-by-column axpy order.
-#include "internal.cuh"
+#include "row_terms.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -93,45 +93,160 @@ static void upload(DevBuf<T>& buf, const T* src, size_t n) {
     if (n) CYC_CHECK_CUDA(cudaMemcpyAsync(buf.get(), src, n * sizeof(T), cudaMemcpyHostToDevice, alloc_stream()));
 }
 
+// ---- the row-major copy ----------------------------------------------------------
+//
+// Each row lists its columns ascending (the order of zeroXBeta + axpyXBeta per
+// j, CyclicCoordinateDescent.cpp:1452-1470).  The rows are counted with
+// atomics and scanned; then a warp takes a range of rows and walks the columns
+// in order, 32 at a time: the columns' entries in its rows (k_splits), laid end
+// to end, are placed 32 a step, entries of one row in the order of their
+// lanes.  Bound by a load latency a step: 1.3M entries (100k rows, 600 Zipf
+// columns and 5 dense ones) 21 ms as a counting sort on the host, 0.2 here.
+
+namespace {
+
+constexpr int kCsrRows = 512;          // rows of a warp: its cursors, in shared memory
+constexpr int kCsrWarps = 8;
+
+__global__ void k_csr_count(long long n, const int* __restrict__ idx, int* __restrict__ cnt) {
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
+        atomicAdd(cnt + idx[e], 1);
+}
+
+// row offsets: exclusive sums of cnt + `every` (the dense columns), by one block
+__global__ void k_csr_scan(int K, int every, const int* __restrict__ cnt, long long* __restrict__ rp) {
+    constexpr int kItems = 8;
+    __shared__ long long s_w[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    long long carry = 0;
+    for (long long base = 0; base < K; base += (long long)blockDim.x * kItems) {
+        const long long k0 = base + (long long)threadIdx.x * kItems;
+        int c[kItems];
+        long long sum = 0;
+        #pragma unroll
+        for (int q = 0; q < kItems; ++q) {
+            c[q] = k0 + q < K ? cnt[k0 + q] + every : 0;
+            sum += c[q];
+        }
+        long long in = sum;
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long u = __shfl_up_sync(0xffffffffu, in, o);
+            if (lane >= o) in += u;
+        }
+        if (lane == 31) s_w[warp] = in;
+        __syncthreads();
+        long long at = carry + in - sum;
+        for (int q = 0; q < warp; ++q) at += s_w[q];
+        #pragma unroll
+        for (int q = 0; q < kItems; ++q) {
+            if (k0 + q < K) rp[k0 + q] = at;
+            at += c[q];
+        }
+        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) carry += s_w[q];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) rp[K] = carry;
+}
+
+// rows [part[w], part[w + 1]) by warp w; `split` as k_splits leaves it
+__global__ void __launch_bounds__(32 * kCsrWarps)
+k_csr_fill(int J, int W, const int* __restrict__ part, const int* __restrict__ split, const int* __restrict__ fmt,
+           const long long* __restrict__ col_ptr, const long long* __restrict__ val_ptr, const int* __restrict__ idx,
+           const double* __restrict__ val, const long long* __restrict__ rp, int* __restrict__ rc,
+           double* __restrict__ rv) {
+    __shared__ int s_cur[kCsrWarps][kCsrRows];
+    constexpr unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, w = blockIdx.x * kCsrWarps + (threadIdx.x >> 5);
+    if (w >= W) return;
+    int* cur = s_cur[threadIdx.x >> 5];
+    const int r0 = part[w], r1 = part[w + 1];
+    for (int q = lane; q < r1 - r0; q += 32) cur[q] = 0;
+    __syncwarp();
+    for (int j0 = 0; j0 < J; j0 += 32) {
+        const int j = j0 + lane;
+        int f = CYC_INDICATOR, first = 0, n = 0;
+        long long cp = 0, vp = 0;
+        if (j < J) {
+            f = fmt[j];
+            first = split[(size_t)j * (W + 1) + w];
+            n = split[(size_t)j * (W + 1) + w + 1] - first;
+            cp = col_ptr[j];
+            vp = val_ptr[j];
+        }
+        const bool dense = f == CYC_DENSE || f == CYC_INTERCEPT;
+        // the entry's place in the column's ids and values; no values: 1
+        const long long ci = dense ? -1 : cp + first;
+        const long long vi = f == CYC_SPARSE || f == CYC_DENSE ? vp + first : -1;
+        int in = n;
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(full, in, o);
+            if (lane >= o) in += u;
+        }
+        const int total = __shfl_sync(full, in, 31), before = in - n;
+        for (int t0 = 0; t0 < total; t0 += 32) {
+            const int t = t0 + lane;
+            int src = 0;                       // the column of entry t: columns whose entries end at or before t
+            #pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const int end = __shfl_sync(full, in, src + o - 1);
+                if (end <= t) src += o;
+            }
+            const int e = t - __shfl_sync(full, before, src);
+            const int fs = __shfl_sync(full, first, src);
+            const long long c = __shfl_sync(full, ci, src), v = __shfl_sync(full, vi, src);
+            const bool on = t < total;
+            const int k = !on ? -1 - lane : (c < 0 ? fs + e : __ldg(idx + c + e));
+            const unsigned same = __match_any_sync(full, k);
+            if (on) {
+                const int rank = __popc(same & ((1u << lane) - 1u));
+                const long long p = rp[k] + cur[k - r0] + rank;
+                rc[p] = j0 + src;
+                rv[p] = v < 0 ? 1.0 : __ldg(val + v + e);
+            }
+            __syncwarp();
+            if (on && lane == __ffs(same) - 1) cur[k - r0] += __popc(same);
+            __syncwarp();
+        }
+    }
+}
+
+}  // namespace
+
 void Dataset::ensure_csr() {
     std::lock_guard<std::mutex> lock(csr_mutex);
     if (have_csr) return;
     StreamScope scope(stream);
-    // counting sort by row; columns visited in ascending order, so each row
-    // lists its columns ascending (the order of zeroXBeta + axpyXBeta per j,
-    // CyclicCoordinateDescent.cpp:1452-1470)
-    std::vector<long long> rp(K + 1, 0);
-    for (int j = 0; j < J; ++j) {
-        const long long n = col_len(j);
-        if (fmt[j] == CYC_DENSE || fmt[j] == CYC_INTERCEPT) {
-            for (int k = 0; k < K; ++k) rp[k + 1]++;
-        } else {
-            for (long long e = 0; e < n; ++e) rp[h_idx[col_ptr[j] + e] + 1]++;
-        }
+    int every = 0;
+    for (int j = 0; j < J; ++j) every += fmt[j] == CYC_DENSE || fmt[j] == CYC_INTERCEPT;
+    const size_t total = (size_t)nnz_idx + (size_t)every * K;
+    DevBuf<int> cnt, d_part, d_split;
+    cnt.alloc(std::max(1, K));
+    CYC_CHECK_CUDA(cudaMemsetAsync(cnt.get(), 0, std::max(1, K) * sizeof(int), stream));
+    d_row_ptr.alloc((size_t)K + 1);
+    d_row_col.alloc(total);
+    d_row_val.alloc(total);
+    if (nnz_idx)
+        launch(k_csr_count, grid_for(nnz_idx, 4), kThreads, 0, stream, nnz_idx, (const int*)d_idx.get(), cnt.get());
+    launch(k_csr_scan, 1, 1024, 0, stream, K, every, (const int*)cnt.get(), d_row_ptr.get());
+    // as many warps as fill the device, within 64 MB of splits and kCsrRows
+    // rows a warp; more rows than they hold take turns
+    const int most = 148 * 16 * kCsrWarps / 8;
+    const int W = (int)std::max(1LL, std::min<long long>(most, (1LL << 24) / std::max(1, J) - 1));
+    std::vector<int> part(W + 1);
+    for (long long k0 = 0; k0 < K && total > 0; k0 += (long long)W * kCsrRows) {
+        const long long rows = std::min<long long>((long long)W * kCsrRows, K - k0);
+        for (int w = 0; w <= W; ++w) part[w] = (int)(k0 + rows * w / W);
+        upload(d_part, part.data(), part.size());
+        d_split.alloc((size_t)J * (W + 1));
+        launch(k_splits, grid_for((long long)J * (W + 1), 1, 1 << 30), kThreads, 0, stream, J, W, (const int*)d_fmt.get(),
+               (const long long*)d_col_ptr.get(), (const int*)d_idx.get(), (const int*)d_part.get(), d_split.get());
+        launch(k_csr_fill, (W + kCsrWarps - 1) / kCsrWarps, 32 * kCsrWarps, 0, stream, J, W, (const int*)d_part.get(),
+               (const int*)d_split.get(), (const int*)d_fmt.get(), (const long long*)d_col_ptr.get(),
+               (const long long*)d_val_ptr.get(), (const int*)d_idx.get(), (const double*)d_val.get(),
+               (const long long*)d_row_ptr.get(), d_row_col.get(), d_row_val.get());
     }
-    for (int k = 0; k < K; ++k) rp[k + 1] += rp[k];
-    std::vector<long long> cur(rp.begin(), rp.end() - 1);
-    std::vector<int> rc(rp[K]);
-    std::vector<double> rv(rp[K]);
-    std::vector<double> hval(nnz_val);
-    if (nnz_val) {
-        CYC_CHECK_CUDA(cudaMemcpyAsync(hval.data(), d_val.get(), nnz_val * sizeof(double), cudaMemcpyDeviceToHost, stream));
-        CYC_CHECK_CUDA(cudaStreamSynchronize(stream));
-    }
-    for (int j = 0; j < J; ++j) {
-        const int f = fmt[j];
-        const long long n = col_len(j);
-        for (long long e = 0; e < n; ++e) {
-            const int k = (f == CYC_DENSE || f == CYC_INTERCEPT) ? (int)e : h_idx[col_ptr[j] + e];
-            const double x = (f == CYC_DENSE || f == CYC_SPARSE) ? hval[val_ptr[j] + e] : 1.0;
-            const long long p = cur[k]++;
-            rc[p] = j;
-            rv[p] = x;
-        }
-    }
-    upload(d_row_ptr, rp.data(), rp.size());
-    upload(d_row_col, rc.data(), rc.size());
-    upload(d_row_val, rv.data(), rv.size());
     CYC_CHECK_CUDA(cudaStreamSynchronize(stream));   // usable from every stream
     have_csr = true;
 }
