@@ -1306,7 +1306,11 @@ __global__ void k_init_xb(int K, int G, int F, const long long* __restrict__ row
     }
 }
 
-// per-fit XjY (computeXjY, ModelSpecifics.hpp:486-524): one block per column
+// per-fit XjY (computeXjY, ModelSpecifics.hpp:486-524): one block per column and
+// group.  A block that took a column's groups in turn was bound by the load
+// latencies of the longest column: 24 fits of 300 Zipf columns and an intercept
+// over 50k rows 1,865 us, 53 with the groups side by side and four entries
+// in flight.
 template <class T>
 __global__ void k_batch_xjy(int J, int K, int G, int ngroups, const int* fmt, const long long* col_ptr,
                             const long long* val_ptr, const int* idx, const double* val, const double* y,
@@ -1318,14 +1322,28 @@ __global__ void k_batch_xjy(int J, int K, int G, int ngroups, const int* fmt, co
         const long long n = dense ? K : col_ptr[j + 1] - col_ptr[j];
         const int* c = idx + col_ptr[j];
         const double* v = val + val_ptr[j];
-        for (int grp = 0; grp < ngroups; ++grp) {
+        for (int grp = blockIdx.y; grp < ngroups; grp += gridDim.y) {
             // thread = (lane, slot) over G lanes
+            constexpr int kU = 4;
             const int lane = threadIdx.x % G, slot = threadIdx.x / G, ns = kBT / G;
             double acc = 0.0;
-            for (long long e = slot; e < n; e += ns) {
-                const int k = dense ? (int)e : c[e];
-                const double x = (f == CYC_SPARSE || f == CYC_DENSE) ? v[e] : 1.0;
-                acc += x * y[k] * (double)w[((size_t)grp * K + k) * G + lane];
+            for (long long e0 = slot; e0 < n; e0 += kU * ns) {
+                double xx[kU], yy[kU], ww[kU];
+                int kk[kU];
+                #pragma unroll
+                for (int u = 0; u < kU; ++u) {
+                    const long long e = min(e0 + u * ns, n - 1);
+                    kk[u] = dense ? (int)e : c[e];
+                    xx[u] = (f == CYC_SPARSE || f == CYC_DENSE) ? v[e] : 1.0;
+                }
+                #pragma unroll
+                for (int u = 0; u < kU; ++u) {
+                    yy[u] = y[kk[u]];
+                    ww[u] = (double)w[((size_t)grp * K + kk[u]) * G + lane];
+                }
+                #pragma unroll
+                for (int u = 0; u < kU; ++u)
+                    if (e0 + u * ns < n) acc += xx[u] * yy[u] * ww[u];
             }
             for (int o = G; o < 32; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
             const int l = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1817,7 +1835,7 @@ struct BatchRunner {
                    (const int*)d_fitfold.get(), d_xjy.get());
             CYC_CHECK_CUDA(cudaStreamSynchronize(stream));   // before fs is freed
         } else {
-            launch(k_batch_xjy<T>, std::min(J, 148 * 8), kBT, 0, stream, J, K, G, ngroups, ds.d_fmt.get(),
+            launch(k_batch_xjy<T>, dim3(std::min(J, 148 * 8), std::min(ngroups, 65535)), kBT, 0, stream, J, K, G, ngroups, ds.d_fmt.get(),
                    ds.d_col_ptr.get(), ds.d_val_ptr.get(), ds.d_idx.get(), ds.d_val.get(), ds.d_y.get(),
                    (const T*)d_w.get(), d_xjy.get());
         }
@@ -1838,7 +1856,7 @@ struct BatchRunner {
                 for (int i = 2; i <= (int)ds.y[k]; ++i) c[k] -= std::log((double)i);
             d_fixedc.alloc(K);
             CYC_CHECK_CUDA(cudaMemcpyAsync(d_fixedc.get(), c.data(), K * sizeof(double), cudaMemcpyHostToDevice, stream));
-            launch(k_batch_llfixed<T>, Fp, 256, 0, stream, K, G, Fp, (const double*)d_fixedc.get(), (const T*)d_w.get(),
+            launch(k_batch_llfixed<T>, Fp, 1024, 0, stream, K, G, Fp, (const double*)d_fixedc.get(), (const T*)d_w.get(),
                    (const signed char*)d_fold8.get(), (const int*)d_fitfold.get(), d_llfixed.get());
             CYC_CHECK_LAUNCH();
             CYC_CHECK_CUDA(cudaStreamSynchronize(stream));
@@ -1980,7 +1998,7 @@ struct BatchRunner {
         d_ll.alloc(Fp);
         d_pll.alloc(Fp);
         const bool grouped = model_grouped(ds.model);
-        launch(k_batch_final, Fp, kBT, 0, stream, ds.model, ds.K, ds.S, G, Fp, (const double*)ds.d_y.get(),
+        launch(k_batch_final, Fp, 1024, 0, stream, ds.model, ds.K, ds.S, G, Fp, (const double*)ds.d_y.get(),
                (const double*)d_xb.get(), (const double*)d_w.get(), grouped ? (const double*)d_denom.get() : nullptr,
                grouped ? (const double*)d_nw.get() : nullptr, (const int*)ds.d_strat.get(), d_fold,
                (const int*)d_fitfold.get(), (const double*)d_llfixed.get(), d_ll.get(), d_pll.get());
