@@ -179,10 +179,9 @@ typedef struct {
                                    passes of CyclicCoordinateDescent::kktSwindle
                                    (CyclicCoordinateDescent.cpp:636-814) under a
                                    Laplace prior.  Every fit keeps its own
-                                   active set, so cyc_batch_fit and the CV
-                                   grids run such fits one by one as cyc_fit;
-                                   cyc_cv_auto_search returns
-                                   CYC_ERR_UNSUPPORTED */
+                                   active set; batches of lr and pr fits at
+                                   FP64 run the passes together, others as
+                                   concurrent cyc_fit solves */
 } cyc_control;
 
 /* the prior: one default prior for every column, a flat prior on `exclude`
