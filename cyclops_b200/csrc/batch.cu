@@ -2191,13 +2191,14 @@ BatchShape tuned_shape(Dataset& ds, cudaStream_t stream, int F, int G, int C, in
 // One fit to a cluster (ccd.cu) is faster until the fits outnumber the SMs or
 // their linear predictors outgrow L2; eight to a group (k_batch) keeps eight
 // fits' predictors of a row side by side, and a step costs about 3 us and 2.5
-// more per 1,000 entries of the mean column, whatever its fits.  Measured,
-// grouped against one to a cluster (logistic CV grids): 10k rows, 10 fits 34
-// ms / 11 ms, 160 fits 35 / 13; 50k rows Zipf, 40 fits 19 / 10, 160 fits 22 /
-// 21; 400k rows, 20 fits 36 / 16; 500k rows x 4,000, 40 fits 519 / 427, 200
-// fits 664 / 1,380; 100k rows x 4,000, 200 fits 822 / 1,410.  The rule
-// compares the two modelled cycles, with 0.8 for the models' errors; a solve
-// large enough for the cluster tuner times a cycle of both instead of
+// more per 1,000 entries of the mean column, whatever its fits (0.85 of that
+// with 512 threads).  Measured, grouped against one to a cluster (logistic CV
+// grids): 10k rows, 10 fits 34 / 7.9 ms, 160 fits 35 / 12.7; 50k rows Zipf, 40 fits
+// 16 / 9.9, 160 fits 17.7 / 21.4; 100k x 400, 80 fits 29 / 23, Zipf 19.3 / 21; 400k
+// rows, 20 fits 25 / 15; 500k rows x 4,000, 20 fits 382 / 278, 40 fits 385 / 433,
+// 200 fits 544 / 1,380; 100k rows x 4,000, 80 fits 545 / 618, 200 fits 689 / 1,465.
+// The rule compares the two modelled cycles, with 0.8 for the models' errors; a
+// solve large enough for the cluster tuner times a cycle of both instead of
 // trusting the model where it favours one to a cluster, and caches the choice
 // per problem shape.  Grouped models (clr, cpr) always run one to a cluster
 // (30 against 8.7 ms at 160 fits of 10k rows, 23 against 15 at 80 fits of 100k).

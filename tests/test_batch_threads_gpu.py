@@ -64,3 +64,26 @@ def test_eight_fit_shapes_match_oracle(cuda_lib, monkeypatch, model, shape, weig
         ref = O.port().fit(data, D.PRIOR_LAPLACE, variances[i // 5], control=octl, exclude=[0], weights=w[i])
         assert ref.return_flag == 0
         assert_contract(fits[i], ref, what=i)
+
+
+@pytest.mark.parametrize("model", [D.LR, D.PR])
+@pytest.mark.parametrize("shape", ["1,512", "3,512", "8,512"])
+def test_eight_fit_shapes_mixed_precision(cuda_lib, monkeypatch, model, shape):
+    """FP32 state with compensated sums, then the FP64 polish, both sides
+    converged tightly (Mittal rule, 1e-12): the contract without cycle counts,
+    as a change of 1e-12 is at the rounding of the likelihood's sum."""
+    from cyclops_b200 import api
+    from oracle import oracle as O
+    monkeypatch.setenv("CYC_BATCH_GROUP", "8")
+    monkeypatch.setenv("CYC_BATCH_CLUSTER", shape)
+    data = _data(model, K=20_000, seed=7)
+    masks = api.cv_fold_weights(data.K, 4, 13)
+    variances = [D.laplace_variance(lam) for lam in (2.0, 20.0)]
+    prior = api.PriorSpec(D.PRIOR_LAPLACE, 1.0, [0])
+    ctl = api.create_control(tolerance=1e-12, convergence_type="mittal", precision="mixed", polish_tolerance=1e-5,
+                             max_iterations=5000)
+    res = api.cv_grid_fit(data, prior, api.fold_ids_from_weights(masks), 4, variances, ctl)
+    octl = O.make_control(tolerance=1e-12, convergence_type=D.CONV_MITTAL, max_iterations=5000)
+    for i in (0, 3, 6):
+        ref = O.port().fit(data, D.PRIOR_LAPLACE, variances[i // 4], control=octl, exclude=[0], weights=masks[i % 4])
+        assert_contract(res.fits[i], ref, iterations=False, what=i)
