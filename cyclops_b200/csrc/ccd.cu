@@ -705,18 +705,22 @@ static int resident_fits(int C, int threads, size_t dyn) {
 // The shape with the least modelled time of a cycle.  Measured here (us): a
 // step, what its sums add when they cross a cluster, and every further round
 // of a column's threads over a CTA's share of the column; fits whose clusters
-// the device does not hold side by side wait their turn.  (10k rows, 1,000
+// the device does not hold side by side wait their turn, and CTAs that share an
+// SM slow one another (24 fits of 50k rows: 8 CTAs of 128 threads 6.6 ms, 4 of
+// 256, one an SM, 5.6; 20 CV fits of 100k rows: 9.7 ms at 4 CTAs of 128, 7.2 at 6
+// of 256; 40 fits: 14.6 at 2 CTAs, 12.7 at 3).  (10k rows, 1,000
 // columns of 100 entries: 27 ms for 41 cycles with one CTA of two teams, 31.7
 // of one team, 35 to 38 with clusters; 100k rows, 600 Zipf columns and 4 dense
 // ones: 150 ms for 40 cycles with one CTA, 38 with four, 25 with sixteen; 80
 // CV fits of 100k rows: 19 ms with one team, 29 with two.)
 CcdShape ccd_shape(const Dataset& ds, int F) {
-    const double cross[] = {0.0, 0.19, 0.2, 0.25, 0.26};
+    struct { int C; double cross; } sizes[] = {{1, 0.0}, {2, 0.19}, {3, 0.2}, {4, 0.2}, {5, 0.25},
+                                               {6, 0.25}, {8, 0.25}, {12, 0.26}, {16, 0.26}};
     struct { int teams, threads; double step, round; } kinds[] = {
         {2, 256, 0.67, 0.5}, {1, 256, 0.92, 0.5}, {1, 128, 0.80, 0.4}};
     CcdShape best{1, 128, 1, 0.0};
-    int log2c = 0;
-    for (int C = 1; C <= kCcdCluster; C *= 2, ++log2c) {
+    for (const auto& size : sizes) {
+        const int C = size.C;
         for (const auto& kind : kinds) {
             if (kind.teams == 2 && !model_independent(ds.model)) continue;
             const size_t bytes = ((size_t)ds.K + C - 1) / C * sizeof(double);
@@ -727,10 +731,11 @@ CcdShape ccd_shape(const Dataset& ds, int F) {
             const bool far = bytes > kRowBytes && (double)std::min(F, slots) * ds.K * sizeof(double) > 100e6;
             const int deal = kind.threads / kind.teams;
             const double round = far ? 1.2 : kind.round;
+            const double step = kind.step * (std::min(F, slots) * C > 148 ? 1.25 : 1.0) + (far ? 0.5 : 0.0) + size.cross;
             double us = 0.0;
             for (int j = 0; j < ds.J; ++j) {
                 const double rounds = std::ceil((double)ds.col_len(j) / (C * deal));
-                us += kind.step + (far ? 0.5 : 0.0) + cross[log2c] + round * std::max(0.0, rounds - 1.0);
+                us += step + round * std::max(0.0, rounds - 1.0);
             }
             us *= (F + slots - 1) / slots;
             if (best.cycle_us == 0.0 || us < best.cycle_us) best = {C, kind.threads, kind.teams, us};
