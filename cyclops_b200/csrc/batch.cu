@@ -2194,8 +2194,8 @@ BatchShape tuned_shape(Dataset& ds, cudaStream_t stream, int F, int G, int C, in
 // more per 1,000 entries of the mean column, whatever its fits (0.85 of that
 // with 512 threads).  Measured, grouped against one to a cluster (logistic CV
 // grids): 10k rows, 10 fits 34 / 7.9 ms, 160 fits 35 / 12.7; 50k rows Zipf, 40 fits
-// 16 / 9.9, 160 fits 17.7 / 21.4; 100k x 400, 80 fits 29 / 23, Zipf 19.3 / 21; 400k
-// rows, 20 fits 25 / 15; 500k rows x 4,000, 20 fits 382 / 278, 40 fits 385 / 433,
+// 16 / 9.2, 160 fits 17.7 / 21.4; 100k x 400, 80 fits 29 / 15.9, Zipf 19.3 / 17.7; 400k
+// rows, 20 fits 25 / 13.5; 500k rows x 4,000, 20 fits 382 / 278, 40 fits 385 / 433,
 // 200 fits 544 / 1,380; 100k rows x 4,000, 80 fits 545 / 618, 200 fits 689 / 1,465.
 // The rule compares the two modelled cycles, with 0.8 for the models' errors; a
 // solve large enough for the cluster tuner times a cycle of both instead of
