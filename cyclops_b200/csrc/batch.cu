@@ -1660,6 +1660,12 @@ static GroupShape group_shape(int K, int ngroups) {
     return {base, 256};
 }
 
+// fits a group (8, or 1: one to a cluster of shape `one`)
+struct Grouping {
+    int G;
+    CcdShape one;
+};
+
 template <class T>
 struct BatchRunner {
     Dataset& ds;
@@ -1682,16 +1688,15 @@ struct BatchRunner {
     std::vector<int> all_cols;               // the columns not fixed
     bool unit_weights = false;               // no fit has weights or a fold
 
-    BatchRunner(Dataset& d, cudaStream_t s, int F_, int G_, int C_ = 0, BatchShape sh = BatchShape{})
-        : ds(d), stream(s), F(F_), G(G_), shape(sh) {
+    BatchRunner(Dataset& d, cudaStream_t s, int F_, const Grouping& by, int C_ = 0, BatchShape sh = BatchShape{})
+        : ds(d), stream(s), F(F_), G(by.G), shape(sh) {
         ngroups = (F + G - 1) / G;
         Fp = ngroups * G;
         const int K = ds.K;
         if (G == 1) {
-            const CcdShape sh1 = ccd_shape(ds, F);
-            C = sh1.C;
-            threads = sh1.threads;
-            teams = sh1.teams;
+            C = by.one.C;
+            threads = by.one.threads;
+            teams = by.one.teams;
         } else {
             C = C_ > 0 ? std::min(kMaxC, C_) : default_cluster(K);
         }
@@ -2082,11 +2087,11 @@ std::map<TuneKey, int>& tuned_sizes() {
 }
 
 template <class T>
-float probe_cycle(Dataset& ds, cudaStream_t stream, int F, int G, int C, const cyc_prior& prior,
+float probe_cycle(Dataset& ds, cudaStream_t stream, int F, const Grouping& by, int C, const cyc_prior& prior,
                   const cyc_fit_spec* specs, const std::vector<double>& beta, const std::vector<double>& hd,
                   const int* d_fold, int n_folds, const std::vector<int>* fit_fold, const cyc_control& ctl,
                   const std::vector<int>& fixed_cols, BatchShape shape = BatchShape{}) {
-    BatchRunner<T> r(ds, stream, F, G, C, shape);
+    BatchRunner<T> r(ds, stream, F, by, C, shape);
     if (d_fold) r.set_folds(d_fold, n_folds, *fit_fold);
     r.setup(prior, specs, beta, hd, fixed_cols);
     cyc_control one = ctl;
@@ -2112,9 +2117,9 @@ int tuned_cluster(Dataset& ds, cudaStream_t stream, int F, int G, const cyc_prio
     float best_ms = 0.f;
     for (int c = base; c >= 1 && c >= base / 4; c /= 2) {
         const float ms = ctl.precision == CYC_MIXED
-                             ? probe_cycle<float>(ds, stream, F, G, c, prior, specs, beta, hd, d_fold, n_folds,
+                             ? probe_cycle<float>(ds, stream, F, Grouping{G, {}}, c, prior, specs, beta, hd, d_fold, n_folds,
                                                   fit_fold, ctl, fixed_cols)
-                             : probe_cycle<double>(ds, stream, F, G, c, prior, specs, beta, hd, d_fold, n_folds,
+                             : probe_cycle<double>(ds, stream, F, Grouping{G, {}}, c, prior, specs, beta, hd, d_fold, n_folds,
                                                    fit_fold, ctl, fixed_cols);
         if (c == base || ms < best_ms) {
             best = c;
@@ -2169,9 +2174,9 @@ BatchShape tuned_shape(Dataset& ds, cudaStream_t stream, int F, int G, int C, in
     }
     auto time = [&](const BatchShape& sh) {
         return ctl.precision == CYC_MIXED
-                   ? probe_cycle<float>(ds, stream, F, G, C, prior, specs, beta, hd, d_fold, n_folds, fit_fold, ctl,
+                   ? probe_cycle<float>(ds, stream, F, Grouping{G, {}}, C, prior, specs, beta, hd, d_fold, n_folds, fit_fold, ctl,
                                         fixed_cols, sh)
-                   : probe_cycle<double>(ds, stream, F, G, C, prior, specs, beta, hd, d_fold, n_folds, fit_fold,
+                   : probe_cycle<double>(ds, stream, F, Grouping{G, {}}, C, prior, specs, beta, hd, d_fold, n_folds, fit_fold,
                                          ctl, fixed_cols, sh);
     };
     float best_ms = time(best);
@@ -2198,30 +2203,34 @@ BatchShape tuned_shape(Dataset& ds, cudaStream_t stream, int F, int G, int C, in
 // rows, 20 fits 25 / 13.5; 500k rows x 4,000, 20 fits 382 / 278, 40 fits 385 / 433,
 // 200 fits 544 / 1,380; 100k rows x 4,000, 80 fits 545 / 618, 200 fits 689 / 1,465.
 // The rule compares the two modelled cycles, with 0.8 for the models' errors; a
-// solve large enough for the cluster tuner times a cycle of both instead of
-// trusting the model where it favours one to a cluster, and caches the choice
-// per problem shape.  Grouped models (clr, cpr) always run one to a cluster
+// solve large enough for the cluster tuner times a cycle of eight to a group and
+// of one to a cluster at the tuner's sizes instead of trusting the model where
+// it favours one to a cluster, and caches the choice per problem shape (the model
+// put 40 fits of 100k rows x 2,000 columns of 2,000 entries at 3 CTAs, 1,002 ms;
+// 4 CTAs take 804).  Grouped models (clr, cpr) always run one to a cluster
 // (30 against 8.7 ms at 160 fits of 10k rows, 23 against 15 at 80 fits of 100k).
-std::map<TuneKey, int>& tuned_groups() {
-    static auto* m = new std::map<TuneKey, int>();   // lives to process exit
+std::map<TuneKey, Grouping>& tuned_groups() {
+    static auto* m = new std::map<TuneKey, Grouping>();   // lives to process exit
     return *m;
 }
 
-int group_size(Dataset& ds, cudaStream_t stream, int F, const cyc_prior& prior, const cyc_fit_spec* specs,
-               const std::vector<double>& beta, const std::vector<double>& hd, const int* d_fold, int n_folds,
-               const std::vector<int>* fit_fold, const cyc_control& ctl, const std::vector<int>& fixed_cols,
-               bool swindle) {
-    if (const char* e = std::getenv("CYC_BATCH_GROUP")) return std::atoi(e) == 8 ? 8 : 1;
+Grouping group_size(Dataset& ds, cudaStream_t stream, int F, const cyc_prior& prior, const cyc_fit_spec* specs,
+                    const std::vector<double>& beta, const std::vector<double>& hd, const int* d_fold, int n_folds,
+                    const std::vector<int>* fit_fold, const cyc_control& ctl,
+                    const std::vector<int>& fixed_cols, bool swindle) {
+    const CcdShape one = ccd_shape(ds, F);
+    if (const char* e = std::getenv("CYC_BATCH_GROUP")) return {std::atoi(e) == 8 ? 8 : 1, one};
     const double entries = (double)(ds.nnz_idx + ds.nnz_val);
     const bool large = F >= 16 && F * entries >= 1e8 && default_cluster(ds.K) > 1;
-    if (large && std::getenv("CYC_BATCH_CLUSTER")) return 8;
+    if (large && std::getenv("CYC_BATCH_CLUSTER")) return {8, one};
     double visits = 0.0;
     for (int j = 0; j < ds.J; ++j) visits += (double)ds.col_len(j);
     const GroupShape gs = swindle ? GroupShape{default_cluster(ds.K), 256} : group_shape(ds.K, (F + 7) / 8);
     const double waves8 = gs.threads == 512 ? 0.85 : std::ceil((double)((F + 7) / 8) * gs.C / (2.0 * 148));
-    if (ccd_shape(ds, F).cycle_us > 0.8 * (3.0 * ds.J + 0.0025 * visits) * waves8) return 8;
-    if (!large || swindle) return 1;
-    const TuneKey key{ds.model, ds.K, ds.J, F, 0, ctl.precision, d_fold ? n_folds : 0, fixed_cols, ds.nnz_idx};
+    if (one.cycle_us > 0.8 * (3.0 * ds.J + 0.0025 * visits) * waves8) return {8, one};
+    if (!large || swindle) return {1, one};
+    const bool varied = std::any_of(specs, specs + F, [&](const cyc_fit_spec& s) { return s.variance != specs[0].variance; });
+    const TuneKey key{ds.model, ds.K, ds.J, F, varied, ctl.precision, d_fold ? n_folds : 0, fixed_cols, ds.nnz_idx};
     {
         std::lock_guard<std::mutex> lk(g_tune_mutex);
         auto it = tuned_groups().find(key);
@@ -2230,16 +2239,27 @@ int group_size(Dataset& ds, cudaStream_t stream, int F, const cyc_prior& prior, 
     BatchShape eight;
     eight.threads = gs.threads;
     eight.dmax = gs.threads / 8;
-    auto time = [&](int G) {
+    auto time = [&](const Grouping& by, int C) {
         return ctl.precision == CYC_MIXED
-                   ? probe_cycle<float>(ds, stream, F, G, gs.C, prior, specs, beta, hd, d_fold, n_folds, fit_fold, ctl,
+                   ? probe_cycle<float>(ds, stream, F, by, C, prior, specs, beta, hd, d_fold, n_folds, fit_fold, ctl,
                                         fixed_cols, eight)
-                   : probe_cycle<double>(ds, stream, F, G, gs.C, prior, specs, beta, hd, d_fold, n_folds, fit_fold,
-                                         ctl, fixed_cols, eight);
+                   : probe_cycle<double>(ds, stream, F, by, C, prior, specs, beta, hd, d_fold, n_folds, fit_fold, ctl,
+                                         fixed_cols, eight);
     };
-    const int best = time(1) < time(8) ? 1 : 8;
+    Grouping best{8, one};
+    double best_ms = time(best, gs.C);
+    const int base = default_cluster(ds.K);
+    for (int c = base; c >= 1 && c >= base / 4; c /= 2) {
+        const Grouping by{1, ccd_shape(ds, F, c, varied)};
+        // (a cycle of every fit takes whole turns)
+        const double ms = time(by, 0) * ccd_turns(F, by.one.slots, varied) / ccd_turns(F, by.one.slots, false);
+        if (ms < best_ms) {
+            best = by;
+            best_ms = ms;
+        }
+    }
     std::lock_guard<std::mutex> lk(g_tune_mutex);
-    tuned_groups()[key] = best;
+    tuned_groups().emplace(key, best);
     return best;
 }
 
@@ -2365,11 +2385,12 @@ void run_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* specs, i
     std::vector<int> ptype(J, prior->prior_type);
     for (int i = 0; i < prior->n_exclude; ++i) ptype[prior->exclude[i]] = CYC_PRIOR_NONE;
     const bool swindle = ctl->use_kkt_swindle && std::count(ptype.begin(), ptype.end(), (int)CYC_PRIOR_LAPLACE) > 0;
-    int G = 1;
-    if (can8) {
+    const Grouping by = [&] {
+        if (!can8) return Grouping{1, ccd_shape(ds, F)};
         NvtxRange range("cyclops batch: group choice");
-        G = group_size(ds, stream, F, *prior, specs, beta, hd, d_fold, n_folds, fit_fold, *ctl, fixed_cols, swindle);
-    }
+        return group_size(ds, stream, F, *prior, specs, beta, hd, d_fold, n_folds, fit_fold, *ctl, fixed_cols, swindle);
+    }();
+    const int G = by.G;
     std::vector<int> iters, flags;
     std::vector<unsigned long long> ctr;
     cyc_run_stats st{};
@@ -2413,7 +2434,6 @@ void run_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* specs, i
     // the tuners time whole cycles over every column, which an active-set
     // pass does not run: swindle solves keep the defaults
     int C = default_cluster(ds.K), threads = 256;
-    if (G == 1) C = ccd_shape(ds, F).C;
     if (G != 1 && !swindle) {
         NvtxRange range("cyclops batch: cluster tuner");
         const GroupShape gs = group_shape(ds.K, (F + 7) / 8);
@@ -2431,7 +2451,7 @@ void run_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* specs, i
     if (ctl->precision == CYC_MIXED) {
         // FP32 state + compensated sums to the looser tolerance, then the FP64 polish below
         NvtxRange range("cyclops batch: fp32 phase");
-        BatchRunner<float> r32(ds, stream, F, G, C, shape);
+        BatchRunner<float> r32(ds, stream, F, by, C, shape);
         if (d_fold) r32.set_folds(d_fold, n_folds, *fit_fold);
         r32.setup(*prior, specs, beta, hd, fixed_cols);
         float ms = 0.f;
@@ -2442,7 +2462,7 @@ void run_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* specs, i
         std::fill(hd.begin(), hd.end(), ctl->initial_bound);
     }
     NvtxRange range64("cyclops batch: fp64 phase");
-    BatchRunner<double> r64(ds, stream, F, G, C, shape);
+    BatchRunner<double> r64(ds, stream, F, by, C, shape);
     if (d_fold) r64.set_folds(d_fold, n_folds, *fit_fold);
     float ms = 0.f;
     std::vector<int> it64;
@@ -2552,7 +2572,7 @@ void run_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* specs, i
         out[f].log_prior = lp;
     }
     if (pll) pll->assign(p.begin(), p.begin() + F);
-    st.cluster_ctas = C;
+    st.cluster_ctas = r64.C;
     if (G == 8 && model_independent(ds.model)) {
         st.batch_cap = shape.cap;
         st.batch_shared_rows = shape.dmax;

@@ -713,14 +713,16 @@ static int resident_fits(int C, int threads, size_t dyn) {
 // of one team, 35 to 38 with clusters; 100k rows, 600 Zipf columns and 4 dense
 // ones: 150 ms for 40 cycles with one CTA, 38 with four, 25 with sixteen; 80
 // CV fits of 100k rows: 19 ms with one team, 29 with two.)
-CcdShape ccd_shape(const Dataset& ds, int F) {
+CcdShape ccd_shape(const Dataset& ds, int F, int only, bool varied) {
+    only = std::min(only, kCcdCluster);
     struct { int C; double cross; } sizes[] = {{1, 0.0}, {2, 0.19}, {3, 0.2}, {4, 0.2}, {5, 0.25},
                                                {6, 0.25}, {8, 0.25}, {12, 0.26}, {16, 0.26}};
     struct { int teams, threads; double step, round; } kinds[] = {
         {2, 256, 0.67, 0.5}, {1, 256, 0.92, 0.5}, {1, 128, 0.80, 0.4}};
-    CcdShape best{1, 128, 1, 0.0};
+    CcdShape best{std::max(1, only), 128, 1, 1, 0.0};
     for (const auto& size : sizes) {
-        const int C = size.C;
+        if (only > 0 && (size.C < only || best.cycle_us > 0.0)) continue;
+        const int C = only > 0 ? only : size.C;
         for (const auto& kind : kinds) {
             if (kind.teams == 2 && !model_independent(ds.model)) continue;
             const size_t bytes = ((size_t)ds.K + C - 1) / C * sizeof(double);
@@ -737,8 +739,8 @@ CcdShape ccd_shape(const Dataset& ds, int F) {
                 const double rounds = std::ceil((double)ds.col_len(j) / (C * deal));
                 us += step + round * std::max(0.0, rounds - 1.0);
             }
-            us *= (F + slots - 1) / slots;
-            if (best.cycle_us == 0.0 || us < best.cycle_us) best = {C, kind.threads, kind.teams, us};
+            us *= ccd_turns(F, slots, varied);
+            if (best.cycle_us == 0.0 || us < best.cycle_us) best = {C, kind.threads, kind.teams, slots, us};
         }
     }
     // CYC_BATCH_CLUSTER="CTAs[,threads[,teams]]" fixes the shape

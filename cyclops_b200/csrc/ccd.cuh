@@ -55,13 +55,22 @@ struct CcdArgs {
     int* out_flag;                // [F]
 };
 
-// CTAs a fit, threads and teams a CTA for F one-fit solves of a dataset, and
-// the modelled time of a cycle of them all
+// CTAs a fit, threads and teams a CTA for F one-fit solves of a dataset, the
+// clusters of that shape the device holds at once, and the modelled time of a
+// cycle of the F fits.  `C` > 0 asks for that many CTAs; `varied`: the fits end
+// after different numbers of cycles.
 struct CcdShape {
-    int C, threads, teams;
+    int C, threads, teams, slots;
     double cycle_us;
 };
-CcdShape ccd_shape(const Dataset& ds, int F);
+CcdShape ccd_shape(const Dataset& ds, int F, int C = 0, bool varied = false);
+// cycles' worth of time that F fits take where `slots` run at a time: whole
+// turns, or, when fits end at different times and the next take their places,
+// their share
+inline double ccd_turns(int F, int slots, bool varied) {
+    if (F <= slots) return 1.0;
+    return varied ? (double)F / slots : (double)((F + slots - 1) / slots);
+}
 // row boundaries of C CTAs, at stratum starts for grouped models
 std::vector<int> ccd_rows(const Dataset& ds, int C);
 // the split of every column's entries over those boundaries
