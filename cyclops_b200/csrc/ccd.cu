@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
                             ex[r] = fexp(vv[r]);
                             T n1 = ex[r] * xx[r], n2 = ind ? T(0) : n1 * xx[r];
                             if ((bb[r] & 3) == 3) rest(tid + r * NT, ss[r], n1, n2);
-                            run_terms(n1, n2, dd[r], ev[r], gi[r], hi[r]);   // ev is 0 where no run starts
+                            run_terms(n1, n2, dd[r], ev[r], gi[r], hi[r]);
                         };
                         #pragma unroll
                         for (int r = 0; r < R; ++r) {
@@ -509,11 +509,13 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
                         prefetch(q + kTeams);
                         #pragma unroll
                         for (int r = 0; r < R; ++r) terms(r);
+                        // (the terms of an entry that starts no run mean nothing: without its
+                        // stratum's denominator they overflow where exp(xb) alone is large)
                         Kahan<T> ag, ah;
                         #pragma unroll
                         for (int r = 0; r < R; ++r) {
-                            ag.add(gi[r]);
-                            ah.add(hi[r]);
+                            ag.add((bb[r] & 1) ? gi[r] : T(0));
+                            ah.add((bb[r] & 1) ? hi[r] : T(0));
                         }
                         if (R == kR)
                             for (int i = kR * NT + tid; i < m.n; i += NT) {
