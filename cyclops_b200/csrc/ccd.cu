@@ -178,6 +178,7 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
     // lower half-warp, b in the upper), then over the warps, then over the CTAs,
     // in fixed orders.
     int phases = 0;                              // of the next exchange (bit `which`)
+    bool gone = false;                           // this thread's wait for the peers ran out
     auto combine = [&](double& a, double& b, int which) {
         const int w = which == 2 ? (int)threadIdx.x >> 5 : warp, nw = which == 2 ? kTeams * NW : NW;
         auto sync = [&]() {
@@ -218,9 +219,13 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
         if (w == 0) {
             const unsigned mb = smem_addr(&s_mb[which]);
             total(s_part[which], nw);
-            if (lane == 0) mbar_expect(mb, 16 * C);
-            if (lane < C) push16(peer_addr(smem_addr(&s_cl[which][rank]), lane), peer_addr(mb, lane), a, b);
-            if (!s_dead && !mbar_wait(mb, (phases >> which) & 1)) s_dead = 1;
+            // a warp whose wait ran out exchanges nothing more: its peers' next
+            // waits run out too, and all leave at the end of the cycle (agree)
+            if (!gone) {
+                if (lane == 0) mbar_expect(mb, 16 * C);
+                if (lane < C) push16(peer_addr(smem_addr(&s_cl[which][rank]), lane), peer_addr(mb, lane), a, b);
+                if (!mbar_wait(mb, (phases >> which) & 1, A.wait.of(rank))) { s_dead = 1; gone = true; }
+            }
             total(s_cl[which], C);
             if (lane == 0) s_all[which] = make_double2(a, b);
         }
@@ -284,6 +289,16 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
         if (delta < -p.bound) delta = -p.bound;                     // applyBounds :1503-1520
         else if (delta > p.bound) delta = p.bound;
         return delta;
+    };
+    // whether any CTA of the cluster lost the others, the same in every thread of
+    // them all: they stop together, and none leaves while another may store to it
+    auto agree = [&]() -> bool {
+        if (C > 1) {
+            if (threadIdx.x == 0 && *(volatile int*)&s_dead)
+                for (int r = 0; r < C; ++r) *cluster.map_shared_rank(&s_dead, r) = 1;
+            cluster.sync();
+        }
+        return *(volatile int*)&s_dead != 0;
     };
     auto next_bound = [](double bound, double delta) { return std_max(std_max(fabs(delta) * 2, bound / 2), 1E-3); };
 
@@ -590,7 +605,7 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
             else conv = fabs(o - last) / (fabs(o) + 1.0);
             last = o;
         }
-        if (s_dead) { flag = kTimedOut; break; }     // the same in every thread: read after a barrier
+        if (agree()) { flag = kTimedOut; break; }
         if (A.tol > 0 && conv < A.tol) { flag = ill ? CYC_ILLCONDITIONED : CYC_SUCCESS; break; }
         if (it == A.max_iter) { flag = CYC_MAX_ITERATIONS; break; }
     }
@@ -598,6 +613,7 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
         __syncthreads();
         for (int i = threadIdx.x; i < nr; i += blockDim.x) xg[i] = sx[i];
     }
+    if (flag == kTimedOut) stores_land();
     if (C > 1) cluster.sync();   // no CTA leaves while others may still write its shared memory
     if (rank == 0 && threadIdx.x == 0) {
         A.out_iter[f] = it;
@@ -626,14 +642,15 @@ void launch_one(const CcdArgs& a, size_t dyn, cudaStream_t stream) {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    CYC_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, (const CcdArgs)a));
+    CYC_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
     count_launch();
 }
 
 template <class T, int MODEL, int WM>
-void launch_rows(const CcdArgs& a, const std::vector<int>& rpart, cudaStream_t stream) {
+void launch_rows(CcdArgs a, const std::vector<int>& rpart, cudaStream_t stream) {
     int rows = 0;
     for (int r = 0; r < a.C; ++r) rows = std::max(rows, rpart[r + 1] - rpart[r]);
+    a.wait = wait_limit(rows);
     const size_t bytes = (size_t)rows * sizeof(T);
     const char* xs = std::getenv("CYC_BATCH_XB_SMEM");      // 0: global memory
     const bool fits = bytes <= kRowBytes && !(xs && std::atoi(xs) == 0);

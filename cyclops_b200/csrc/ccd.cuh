@@ -1,7 +1,7 @@
 // ccd.cuh -- the one-fit persistent CCD kernel (ccd.cu): arguments, launch
 // shape and launch.
 #pragma once
-#include "internal.cuh"
+#include "mbar.cuh"
 
 namespace cyc {
 
@@ -51,6 +51,7 @@ struct CcdArgs {
     int conv;
     double tol;
     int max_iter;
+    WaitLimit wait;               // set by launch_ccd
     int* out_iter;                // [F]
     int* out_flag;                // [F]
 };

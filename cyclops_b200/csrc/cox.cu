@@ -366,9 +366,22 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits
     }
 
     int use[3] = {0, 0, 0};                               // exchanges of each kind so far
+    // warp 0 exchanges nothing more once its wait ran out; its peers' next waits
+    // run out too, and all stop together (agree)
+    bool gone = false;
     auto wait = [&](int kind) {                           // warp 0
         const int i = use[kind];
-        if (!s_dead && !mbar_wait(smem_addr(&s_mb[kind][i & 1]), (i >> 1) & 1)) s_dead = 1;
+        if (!mbar_wait(smem_addr(&s_mb[kind][i & 1]), (i >> 1) & 1, A.wait.of(rank))) { s_dead = 1; gone = true; }
+    };
+    // whether any CTA of the cluster lost the others, the same in every thread of them all
+    auto agree = [&]() -> bool {
+        __syncthreads();
+        if (C > 1) {
+            if (tid == 0 && *(volatile int*)&s_dead)
+                for (int r = 0; r < C; ++r) *cluster.map_shared_rank(&s_dead, r) = 1;
+            cluster.sync();
+        }
+        return *(volatile int*)&s_dead != 0;
     };
     int par = 0;                                          // of the next block scan
 
@@ -502,9 +515,12 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits
             if (warp == 0) {
                 const int i = use[0] & 1;
                 const unsigned mb = smem_addr(&s_mb[0][i]);
-                if (lane == 0) mbar_expect(mb, 16 * C);
-                if (lane < C) push16(peer_addr(smem_addr(&x_a[i][rank]), lane), peer_addr(mb, lane), ta, tf ? 1.0 : 0.0);
-                wait(0);
+                if (!gone) {
+                    if (lane == 0) mbar_expect(mb, 16 * C);
+                    if (lane < C)
+                        push16(peer_addr(smem_addr(&x_a[i][rank]), lane), peer_addr(mb, lane), ta, tf ? 1.0 : 0.0);
+                    wait(0);
+                }
                 double c = 0.0;
                 for (int r = 0; r < rank; ++r) {
                     const double2 t = x_a[i][r];
@@ -579,9 +595,11 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits
         if (C > 1 && warp == 0) {                         // what follows in the later CTAs
             const int ic = use[2] & 1;
             const unsigned mb = smem_addr(&s_mb[2][ic]);
-            if (lane == 0) mbar_expect(mb, 16 * C);
-            if (lane < C) push16(peer_addr(smem_addr(&x_c[ic][rank]), lane), peer_addr(mb, lane), t1, t2);
-            wait(2);
+            if (!gone) {
+                if (lane == 0) mbar_expect(mb, 16 * C);
+                if (lane < C) push16(peer_addr(smem_addr(&x_c[ic][rank]), lane), peer_addr(mb, lane), t1, t2);
+                wait(2);
+            }
             double c1 = 0.0, c2 = 0.0;
             for (int r = C - 1; r > rank; --r) {
                 const double2 t = x_c[ic][r];
@@ -609,9 +627,11 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits
             const int i = use[0] & 1;
             if (warp == 0) {
                 const unsigned mb = smem_addr(&s_mb[0][i]);
-                if (lane == 0) mbar_expect(mb, 16 * C);
-                if (lane < C) push16(peer_addr(smem_addr(&x_a[i][rank]), lane), peer_addr(mb, lane), a, b);
-                wait(0);
+                if (!gone) {
+                    if (lane == 0) mbar_expect(mb, 16 * C);
+                    if (lane < C) push16(peer_addr(smem_addr(&x_a[i][rank]), lane), peer_addr(mb, lane), a, b);
+                    wait(0);
+                }
             }
             ++use[0];
             __syncthreads();
@@ -676,11 +696,13 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits
 
     if (A.max_iter == 0 && !A.score) {
         const double ll = log_likelihood();
+        const bool dead = agree();
         if (rank == 0 && tid == 0) {
             *A.out_ll = ll;
             *A.out_iter = 0;
-            *A.out_flag = s_dead ? kTimedOut : CYC_SUCCESS;
+            *A.out_flag = dead ? kTimedOut : CYC_SUCCESS;
         }
+        if (dead) stores_land();
         if (C > 1) cluster.sync();
         return;
     }
@@ -836,14 +858,16 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits
                     }
                     if (C > 1) {
                         const unsigned mb = smem_addr(&s_mb[1][ib]);
-                        if (lane == 0) mbar_expect(mb, 48 * C);
-                        if (lane < C) {
-                            const unsigned pm = peer_addr(mb, lane);
-                            push16(peer_addr(smem_addr(&x_b[ib][0][rank]), lane), pm, g, h);
-                            push16(peer_addr(smem_addr(&x_b[ib][1][rank]), lane), pm, vh2, pre);
-                            push16(peer_addr(smem_addr(&x_b[ib][2][rank]), lane), pm, tf ? 1.0 : 0.0, 0.0);
+                        if (!gone) {
+                            if (lane == 0) mbar_expect(mb, 48 * C);
+                            if (lane < C) {
+                                const unsigned pm = peer_addr(mb, lane);
+                                push16(peer_addr(smem_addr(&x_b[ib][0][rank]), lane), pm, g, h);
+                                push16(peer_addr(smem_addr(&x_b[ib][1][rank]), lane), pm, vh2, pre);
+                                push16(peer_addr(smem_addr(&x_b[ib][2][rank]), lane), pm, tf ? 1.0 : 0.0, 0.0);
+                            }
+                            wait(1);
                         }
-                        wait(1);
                         g = h = pre = 0.0;
                         for (int r = 0; r < C; ++r) {
                             const double2 b0 = x_b[ib][0][r], b1 = x_b[ib][1][r];
@@ -926,7 +950,7 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits
                     if (c_up[q]) A.col_updates[j] += 1u;
                 }
         }
-        if (A.score) { flag = s_dead ? kTimedOut : CYC_SUCCESS; break; }
+        if (A.score) break;
         // ---- performCheckConvergence (:839-906)
         ++it;
         __syncthreads();
@@ -941,12 +965,15 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits
             else conv = fabs(o - last) / (fabs(o) + 1.0);
             last = o;
         }
-        __syncthreads();
-        if (s_dead) { flag = kTimedOut; break; }          // the same in every thread of the CTA
+        if (agree()) break;
         if (A.tol > 0 && conv < A.tol) { flag = ill ? CYC_ILLCONDITIONED : CYC_SUCCESS; break; }
         if (it == A.max_iter) { flag = CYC_MAX_ITERATIONS; break; }
     }
     const double ll = A.score ? 0.0 : log_likelihood();
+    if (agree()) {
+        flag = kTimedOut;
+        stores_land();
+    }
     if (C > 1) cluster.sync();       // no CTA leaves while others may still write its shared memory
     if (rank == 0 && tid == 0) {
         *A.out_ll = ll;
@@ -1063,6 +1090,7 @@ CoxArgs CoxSlots::args() const {
     a.strat = ds.d_strat.get();
     a.split = split.get(); a.rpart = rpart.get(); a.spart = spart.get(); a.flag = flag.get();
     a.n = n.get(); a.y = ds.d_y.get();
+    a.wait = wait_limit(ds.K);
     return a;
 }
 

@@ -1,7 +1,7 @@
 // cox.cuh -- the persistent Breslow Cox solver (cox.cu): the risk sets of one
 // weighting and the kernel's launch.
 #pragma once
-#include "internal.cuh"
+#include "mbar.cuh"
 
 namespace cyc {
 
@@ -88,6 +88,7 @@ struct CoxArgs {
     double tol;
     int max_iter;                  // 0: evaluate the log likelihood only
     int predict;                   // as getPredictiveLogLikelihood: every outcome at its value
+    WaitLimit wait;
     int* out_iter;
     int* out_flag;                 // kTimedOut (ccd.cuh): the CTAs lost one another
     double* out_ll;

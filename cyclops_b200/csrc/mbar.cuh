@@ -1,6 +1,9 @@
 // mbar.cuh -- the exchange between the CTAs of a cluster: 16 bytes stored to a
 // peer's shared memory by st.async, counted on the peer's mbarrier.
 #pragma once
+#include <cstdio>
+#include <cstdlib>
+
 #include "internal.cuh"
 
 namespace cyc {
@@ -34,16 +37,37 @@ __device__ __forceinline__ bool mbar_try(unsigned mbar, int phase) {
         : "memory");
     return ok != 0;
 }
-// A peer is at most one column's work away (well under a millisecond); a wait
-// that outlasts this many clocks (about two seconds) gives up.
-constexpr long long kWaitClocks = 4000000000ll;
-// waits for the phase; false when the bound ran out
-__device__ __forceinline__ bool mbar_wait(unsigned mbar, int phase) {
+// waits for the phase; false when `clocks` ran out (0: without a look)
+__device__ __forceinline__ bool mbar_wait(unsigned mbar, int phase, long long clocks) {
+    if (clocks <= 0) return false;
     if (mbar_try(mbar, phase)) return true;
     const long long t0 = clock64();
     while (!mbar_try(mbar, phase))
-        if (clock64() - t0 > kWaitClocks) return false;
+        if (clock64() - t0 > clocks) return false;
     return true;
+}
+// before the CTAs of a cluster that lost one another leave: stores of 16 bytes
+// that nobody waited for land within a few microseconds; about 50 pass here
+__device__ __forceinline__ void stores_land() {
+    const long long t0 = clock64();
+    while (clock64() - t0 < 100000) {}
+}
+
+// How long a CTA waits for its peers.  A peer is at most one pass over its rows
+// away, and in the worst case (one stratum, one thread) that pass is a chain of
+// dependent loads and exponentials, 1,000 to 1,500 clocks a row; so two seconds
+// and 4,096 clocks a row of the CTA with the most.  CYC_WAIT_CLOCKS="clocks[,rank]"
+// sets the bound, and takes CTA `rank` of every cluster for lost at its first
+// wait (how the tests reach this path).
+struct WaitLimit {
+    long long clocks;
+    int lost;
+    __device__ __forceinline__ long long of(int rank) const { return rank == lost ? 0 : clocks; }
+};
+inline WaitLimit wait_limit(long long rows) {
+    WaitLimit w{4000000000ll + 4096 * rows, -1};
+    if (const char* e = std::getenv("CYC_WAIT_CLOCKS")) std::sscanf(e, "%lld,%d", &w.clocks, &w.lost);
+    return w;
 }
 
 }  // namespace cyc
