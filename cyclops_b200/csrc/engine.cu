@@ -569,8 +569,8 @@ void Engine::fisher_information(const int* cols, int n, double* out) {
                (const double*)exb.get(), d_t.get());
     }
     const size_t smem = words * sizeof(unsigned);
-    if (smem > 48 * 1024)
-        CYC_CHECK_CUDA(cudaFuncSetAttribute(k_fisher_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // (the kernel's limit is the process's: the same whatever this call's rows)
+    CYC_CHECK_CUDA(cudaFuncSetAttribute(k_fisher_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBitmapBytes));
     launch(k_fisher_pairs, std::min(nt, 148 * 8), kThreads, smem, stream, nt, (const FisherTask*)d_tasks.get(), n,
            (const int*)d_plan.get(), (const int*)d_plan.get() + n, words, K, S, grouped ? 1 : 0,
            (const int*)ds->d_fmt.get(), (const long long*)ds->d_col_ptr.get(),
