@@ -13,12 +13,13 @@
 // tree order carry no more error than D itself.  A column then costs a pass
 // over its own entries; only a step that moves a coefficient renews the sums:
 // one pass over the event groups (about a third of the rows here), not over
-// every row, and nothing but S1 and S2 is written.
+// every row, and nothing but S1 and S2 is written.  Groups of many rows are cut
+// into slots (kSlotRows); a slot without events only passes the sums on.
 //
 // What bounds a step is latency at small sizes (block scans, two exchanges a
 // cluster) and one division per event group at large ones, so a fit is one
-// cluster of up to 16 CTAs that split the event groups in order; their carries
-// cross by st.async on mbarriers.  The per-slot arrays stay in shared memory
+// cluster of up to 16 CTAs that split the slots in order, with their rows; their
+// carries cross by st.async on mbarriers.  The per-slot arrays stay in shared memory
 // where they fit, S1 and S2 alone where only those do, else in L2.  (Before:
 // seven launches a coordinate that rewrote nine arrays over all rows, 35 us a
 // coordinate at 20k rows and 56 us at 500k.)
@@ -48,6 +49,13 @@ constexpr int kCh = 64;           // coordinates staged at a time
 // runs the same number of blocks, past its last slot on zeros
 constexpr int kB = 4;
 constexpr int kMaxC = kCcdCluster;
+// A slot's rows at most.  Rows between two events are one event group's, and a
+// group can hold most of a cohort (everybody censored at the end of a fixed
+// follow-up enters with the first event): groups are cut so that no thread walks
+// a long run, and the CTAs' rows can be balanced.  100k rows, 87 % of them
+// censored at one time, 100 indicator columns of 2,000 rows, 6 cycles: 441 ms
+// uncut, 10.5 cut.
+constexpr int kSlotRows = 32;
 // in an entry's slot position: the slot's stratum goes on past the slots of its
 // CTA (kTailBit), past those of its thread (kThreadBit)
 constexpr int kTailBit = 1 << 30, kThreadBit = 1 << 29, kPosMask = kThreadBit - 1;
@@ -174,16 +182,99 @@ __global__ void k_slot_rows(int K, const double* __restrict__ w, const double* _
     }
 }
 
-// the split of the slots over the CTAs, and the rows that go with it (a CTA's
-// rows end with its last slot's last event; the last CTA takes the rest)
-__global__ void k_slot_parts(int K, int C, const int* __restrict__ total, const int* __restrict__ end,
-                             int* __restrict__ spart, int* __restrict__ rpart) {
-    const int E = *total;
-    for (int r = threadIdx.x; r <= C; r += blockDim.x) {
-        const int s = (int)((long long)E * r / C);
-        spart[r] = s;
-        rpart[r] = r == 0 ? 0 : (r == C ? K : (s == 0 ? 0 : end[s - 1] + 1));
+// the first row of each event group's rows (those that enter the risk sets with it)
+__global__ void k_group_rows(const int* __restrict__ groups, const int* __restrict__ gend, const int* __restrict__ gstr,
+                             const int* __restrict__ strat_ptr, int* __restrict__ glo) {
+    const int E = *groups;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < E; e += gridDim.x * blockDim.x)
+        glo[e] = e == 0 || gstr[e - 1] != gstr[e] ? strat_ptr[gstr[e]] : gend[e - 1] + 1;
+}
+struct Pieces {                      // the slots of an event group
+    const int *groups, *glo, *gend;
+    __device__ int operator()(int e) const { return e < *groups ? (gend[e] - glo[e]) / kSlotRows + 1 : 0; }
+};
+
+// the event groups as the row kernels read them
+struct Groups {
+    const int *groups;               // their number
+    const int *cnt;                  // by row: groups that start at it or before
+    const int *glo, *gend, *gstr;    // rows and stratum of each
+    const int *gcum;                 // slots up to and with each
+    __device__ int first_slot(int e) const { return e > 0 ? gcum[e - 1] : 0; }
+    // the group whose rows hold row k, or the next one
+    __device__ int of(int k) const { const int c = cnt[k]; return c > 0 && gend[c - 1] >= k ? c - 1 : c; }
+    // slots whose rows all precede row b; b itself goes down to the slot's
+    // first row where it would cut one
+    __device__ int before(int& b) const {
+        if (b == 0) return 0;
+        const int c = cnt[b - 1], e = c > 0 && gend[c - 1] >= b ? c - 1 : c;
+        int s = first_slot(e);
+        if (e < *groups && glo[e] < b) {
+            const int q = (b - glo[e]) / kSlotRows;
+            s += q;
+            b = glo[e] + q * kSlotRows;
+        }
+        return s;
     }
+};
+
+// rows and stratum of every slot (a warp per group)
+__global__ void k_slot_fill(Groups G, int* __restrict__ lo, int* __restrict__ end, int* __restrict__ sstr) {
+    const int E = *G.groups, lane = threadIdx.x & 31;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < E; e += nwarps) {
+        const int s0 = G.first_slot(e), s1 = G.gcum[e];
+        for (int s = s0 + lane; s < s1; s += 32) {
+            const int k = G.glo[e] + (s - s0) * kSlotRows;
+            lo[s] = k;
+            end[s] = min(G.gend[e], k + kSlotRows - 1);
+            sstr[s] = G.gstr[e];
+        }
+    }
+}
+
+// The split of rows and slots over the CTAs: each CTA's share of the rows and its
+// share of the slots add up to 2 / C, and none has more than `room` slots.  (Slots
+// are what a moving step renews, rows what the columns' entries follow: events
+// may lie anywhere among the rows.)  Boundaries fall between slots.  A warp finds
+// a boundary, 32 candidates at a time.
+__global__ void k_slot_parts(int K, int C, int S, int room, Groups G, const int* __restrict__ end,
+                             int* __restrict__ spart, int* __restrict__ rpart) {
+    __shared__ int s_s[kMaxC + 1], s_b[kMaxC + 1];
+    const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (r < C) {
+        const double want = 2.0 * r / C;
+        int lo = 0, hi = K;                               // the share is below `want` at lo, not at hi
+        while (hi - lo > 1) {
+            const int b = lo + (int)((long long)(hi - lo) * (lane + 1) / 33);
+            int at = b;
+            const int s = G.before(at);
+            const unsigned m = __ballot_sync(kFull, (double)b / K + (double)s / max(1, S) >= want);
+            const int f = m ? __ffs(m) - 1 : 32;
+            const int up = __shfl_sync(kFull, b, min(f, 31)), down = __shfl_sync(kFull, b, max(f - 1, 0));
+            if (f < 32) hi = up;
+            if (f > 0) lo = down;
+        }
+        if (lane == 0) {
+            int b = r == 0 ? 0 : hi;
+            s_s[r] = G.before(b);
+            s_b[r] = b;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    s_s[C] = S;
+    s_b[C] = K;
+    for (int q = 1; q < C; ++q) {
+        const int least = max(s_s[q - 1], S - (C - q) * room), most = s_s[q - 1] + room;
+        const int s = min(max(s_s[q], least), most);
+        if (s != s_s[q]) {
+            s_s[q] = s;
+            s_b[q] = end[s - 1] + 1;
+        }
+        s_b[q] = max(s_b[q], s_b[q - 1]);
+    }
+    for (int q = 0; q <= C; ++q) { spart[q] = s_s[q]; rpart[q] = s_b[q]; }
 }
 
 __device__ __forceinline__ int slot_position(int e, int C, int nt, const int* spart, int& r) {
@@ -194,37 +285,35 @@ __device__ __forceinline__ int slot_position(int e, int C, int nt, const int* sp
     return (q % m) * nt + q / m;
 }
 
-// per slot (a warp each): events, first row, flags
-__global__ void k_slots(int C, int nt, int per_cta, const int* __restrict__ total, const int* __restrict__ spart,
-                        const int* __restrict__ first, const int* __restrict__ end, const int* __restrict__ sstr,
-                        const int* __restrict__ strat_ptr, const double* __restrict__ w, const double* __restrict__ y,
-                        int* __restrict__ lo, unsigned char* __restrict__ flag, double* __restrict__ n) {
-    const int E = *total, lane = threadIdx.x & 31;
+// per event group (a warp each): its events, which its last slot has, and its slots' flags
+__global__ void k_slots(int C, int nt, int per_cta, Groups G, const int* __restrict__ spart,
+                        const int* __restrict__ first, const double* __restrict__ w, const double* __restrict__ y,
+                        unsigned char* __restrict__ flag, double* __restrict__ n) {
+    const int E = *G.groups, lane = threadIdx.x & 31;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     for (int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < E; e += nwarps) {
         double a = 0.0;
-        for (int k = first[e] + lane; k <= end[e]; k += 32) a += y[k] * (w ? w[k] : 1.0);
+        for (int k = first[e] + lane; k <= G.gend[e]; k += 32) a += y[k] * (w ? w[k] : 1.0);
         for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(kFull, a, o);
-        if (lane == 0) {
-            const int s = sstr[e];
-            const bool starts = e == 0 || sstr[e - 1] != s, ends = e + 1 == E || sstr[e + 1] != s;
-            lo[e] = starts ? strat_ptr[s] : end[e - 1] + 1;
+        const int s0 = G.first_slot(e), s1 = G.gcum[e], str = G.gstr[e];
+        const bool starts = e == 0 || G.gstr[e - 1] != str, ends = e + 1 == E || G.gstr[e + 1] != str;
+        for (int s = s0 + lane; s < s1; s += 32) {
             int r;
-            const int p = slot_position(e, C, nt, spart, r);
-            n[(size_t)r * per_cta + p] = a;
-            flag[(size_t)r * per_cta + p] = (unsigned char)((starts ? 1 : 0) | (ends ? 2 : 0));
+            const int p = slot_position(s, C, nt, spart, r);
+            n[(size_t)r * per_cta + p] = s == s1 - 1 ? a : 0.0;
+            flag[(size_t)r * per_cta + p] = (unsigned char)((s == s0 && starts ? 1 : 0) | (s == s1 - 1 && ends ? 2 : 0));
         }
     }
 }
 
 // sums of w exp(xb) over each slot's rows (a warp each)
-__global__ void k_slot_increments(int C, int nt, int per_cta, const int* __restrict__ total, const int* __restrict__ spart,
+__global__ void k_slot_increments(int C, int nt, int per_cta, int S, const int* __restrict__ spart,
                                   const int* __restrict__ lo, const int* __restrict__ end,
                                   const double* __restrict__ w, const double* __restrict__ xb,
                                   double* __restrict__ d) {
-    const int E = *total, lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < E; e += nwarps) {
+    for (int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < S; e += nwarps) {
         double a = 0.0;
         for (int k = lo[e] + lane; k <= end[e]; k += 32) {
             const double wk = w ? w[k] : 1.0;
@@ -242,20 +331,20 @@ __global__ void k_slot_increments(int C, int nt, int per_cta, const int* __restr
 // every row's slot position in its CTA (-1: none), with kTailBit and kThreadBit.
 // Rows of weight zero get the slot their
 // place in the order gives (they add nothing), so a column's slots ascend.
-__global__ void k_row_slots(int K, int C, int nt, const int* __restrict__ total, const int* __restrict__ spart,
-                            const int* __restrict__ sstr, const int* __restrict__ end,
-                            const int* __restrict__ strat, const int* __restrict__ cnt, int* __restrict__ out) {
-    const int E = *total;
+__global__ void k_row_slots(int K, int C, int nt, int S, Groups G, const int* __restrict__ spart,
+                            const int* __restrict__ sstr, const int* __restrict__ strat, int* __restrict__ out) {
+    const int E = *G.groups;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x) {
         int o = -1;
-        const int e = cnt[k] > 0 && end[cnt[k] - 1] >= k ? cnt[k] - 1 : cnt[k];
-        if (e < E && sstr[e] == strat[k]) {
+        const int g = G.of(k);
+        if (g < E && G.gstr[g] == strat[k]) {
+            const int s = G.first_slot(g) + (k - G.glo[g]) / kSlotRows;
             int r;
-            o = slot_position(e, C, nt, spart, r);
+            o = slot_position(s, C, nt, spart, r);
             const int s0 = spart[r], next = spart[r + 1], m = (next - s0 + nt - 1) / nt;
-            const int after = min(next, s0 + ((e - s0) / m + 1) * m);       // first slot past its thread's
-            if (next < E && sstr[next] == sstr[e]) o |= kTailBit;
-            if (after < E && sstr[after] == sstr[e]) o |= kThreadBit;
+            const int after = min(next, s0 + ((s - s0) / m + 1) * m);       // first slot past its thread's
+            if (next < S && sstr[next] == sstr[s]) o |= kTailBit;
+            if (after < S && sstr[after] == sstr[s]) o |= kThreadBit;
         }
         out[k] = o;
     }
@@ -569,7 +658,8 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits
             risk_sums(b, pre, dv, D);
             #pragma unroll
             for (int u = 0; u < kB; ++u) {
-                D[u] = 1.0 / D[u];                        // one division for both terms
+                const double inv = 1.0 / D[u];            // one division for both terms
+                D[u] = nv[u] != 0.0 ? inv : 0.0;          // (without events D may be anything)
                 q1[u] = nv[u] * D[u];
             }
             #pragma unroll
@@ -651,7 +741,10 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits
             for (int u = 0; u < kB; ++u) dv[u] = dd[(g * kB + u) * kNT + tid];
             risk_sums(g, pre, dv, D);
             #pragma unroll
-            for (int u = 0; u < kB; ++u) b += nn[(g * kB + u) * kNT + tid] * log(D[u]);
+            for (int u = 0; u < kB; ++u) {
+                const double n = nn[(g * kB + u) * kNT + tid], l = n * log(D[u]);
+                if (n != 0.0) b += l;
+            }
         }
         for (int k = tid; k < nr; k += kNT) {
             if (A.predict) {
@@ -706,6 +799,42 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits
         if (C > 1) cluster.sync();
         return;
     }
+    // The increments formed again from the predictors, once a cycle: a step adds
+    // its change of a slot to them, and the rounding adds up.  A warp takes 32
+    // rows; the last of a slot's rows in it adds their sum.  A slot's rows lie in
+    // two warps at most, so the order of the two does not matter.  (A thread
+    // walking its slots' rows took 65 us a cycle at 20k rows and 350 at 500k;
+    // 15 and 54 this way.)
+    auto reform = [&]() {
+        for (int p = tid; p < np; p += kNT) dd[p] = 0.0;
+        __syncthreads();
+        constexpr int kU = 4;
+        for (int k0 = warp * 32; k0 < nr; k0 += kU * kNT) {
+            int slot[kU];
+            double v[kU], w[kU];
+            #pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                const int k = k0 + u * kNT + lane;
+                slot[u] = k < nr ? __ldg(A.rowslot + r0 + k) : -1;
+                v[u] = k < nr ? xg[k] : 0.0;
+                w[u] = k < nr && wg ? __ldg(wg + k) : 1.0;
+            }
+            #pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                const int p = slot[u] >= 0 ? slot[u] & kPosMask : -1 - lane;
+                double a = slot[u] >= 0 && w[u] != 0.0 ? w[u] * exp(v[u]) : 0.0;
+                #pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int up = __shfl_up_sync(kFull, p, o);
+                    const double ua = __shfl_up_sync(kFull, a, o);
+                    if (lane >= o && up == p) a += ua;
+                }
+                const int next = __shfl_down_sync(kFull, p, 1);
+                if (p >= 0 && (lane == 31 || next != p)) atomicAdd(dd + p, a);
+            }
+        }
+        __syncthreads();
+    };
     double last = A.conv == CYC_CONV_ZHANG_OLES || A.score ? 0.0 : objective();
     renew();
     const int ncols = *A.ncols;
@@ -955,6 +1084,7 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits
         ++it;
         __syncthreads();
         if (C > 1) cluster.sync();    // rank 0's coefficients are staged by every CTA in the next cycle
+        reform();
         const double o = objective();
         double conv;
         int ill = 0;
@@ -1014,15 +1144,16 @@ static size_t cox_bytes(int threads, int per_cta, bool all) {
     return threads * (m * (all ? 32 : 16) + m / kB * sizeof(double) + m);
 }
 
-static int cox_where(CoxShape s, int per_cta) {
-    if (s.threads < kCoxThreads || cox_bytes(s.threads, per_cta, true) <= kSmemBytes) return 0;
-    return cox_bytes(s.threads, per_cta, false) <= kSmemBytes ? 1 : 2;
+// 0: all per-slot arrays in shared memory, 1: S1 and S2, 2: none
+static int cox_where(CoxShape s) {
+    if (cox_bytes(s.threads, s.per_cta, true) <= kSmemBytes) return 0;
+    return s.threads == kCoxThreads && cox_bytes(s.threads, s.per_cta, false) <= kSmemBytes ? 1 : 2;
 }
 
 template <bool SEG>
-static void launch_seg(const CoxArgs* d_fits, int F, CoxShape s, int per_cta, cudaStream_t stream) {
-    const int where = cox_where(s, per_cta), C = s.C;
-    const size_t dyn = where == 2 ? 0 : cox_bytes(s.threads, per_cta, where == 0);
+static void launch_seg(const CoxArgs* d_fits, int F, CoxShape s, cudaStream_t stream) {
+    const int where = cox_where(s), C = s.C;
+    const size_t dyn = where == 2 ? 0 : cox_bytes(s.threads, s.per_cta, where == 0);
     if (s.threads == 128) launch_where<0, 128, SEG>(d_fits, F, C, dyn, stream);
     else if (s.threads == 256) launch_where<0, 256, SEG>(d_fits, F, C, dyn, stream);
     else if (where == 0) launch_where<0, 512, SEG>(d_fits, F, C, dyn, stream);
@@ -1030,16 +1161,17 @@ static void launch_seg(const CoxArgs* d_fits, int F, CoxShape s, int per_cta, cu
     else launch_where<2, 512, SEG>(d_fits, F, C, dyn, stream);
 }
 
-void launch_cox(const CoxArgs* d_fits, int F, CoxShape shape, int per_cta, bool strata, cudaStream_t stream) {
-    if (strata) launch_seg<true>(d_fits, F, shape, per_cta, stream);
-    else launch_seg<false>(d_fits, F, shape, per_cta, stream);
+void launch_cox(const CoxArgs* d_fits, int F, CoxShape shape, bool strata, cudaStream_t stream) {
+    if (strata) launch_seg<true>(d_fits, F, shape, stream);
+    else launch_seg<false>(d_fits, F, shape, stream);
 }
 
-CoxShape cox_shape(Dataset& ds) {
-    const int events = ds.event_rows();
+// (the slots count rows as well as events: 2M rows with 1,000 events are 63,000
+// slots and take 16 CTAs of 512 threads, 103 -> 32 ms for 4 cycles of 22 columns)
+CoxShape cox_shape(int slots) {
     CoxShape s{1, 128};
-    while (s.C < kMaxC && events > 128 * 8 * s.C) s.C *= 2;
-    while (s.threads < kCoxThreads && events > s.threads * 12 * s.C) s.threads *= 2;
+    while (s.C < kMaxC && slots > 128 * 8 * s.C) s.C *= 2;
+    while (s.threads < kCoxThreads && slots > s.threads * 12 * s.C) s.threads *= 2;
     // CYC_COX_CLUSTER="CTAs[,threads]" fixes the shape
     if (const char* e = std::getenv("CYC_COX_CLUSTER")) {
         int c = s.C, t = s.threads;
@@ -1048,56 +1180,25 @@ CoxShape cox_shape(Dataset& ds) {
         s.threads = t <= 128 ? 128 : t <= 256 ? 256 : 512;
     }
     // 128 and 256 threads keep every per-slot array in shared memory
-    while (s.threads < kCoxThreads && cox_bytes(s.threads, (events / s.C + kB * s.threads) / (kB * s.threads) * (kB * s.threads), true) > kSmemBytes) s.threads *= 2;
+    const auto round_up = [&](int n) { return (n + kB * s.threads - 1) / (kB * s.threads) * (kB * s.threads); };
+    const int even = std::max(1, (slots + s.C - 1) / s.C);
+    while (s.threads < kCoxThreads && cox_bytes(s.threads, round_up(even), true) > kSmemBytes) s.threads *= 2;
+    // room for up to twice the even share of the slots, as far as the arrays stay where the even share's are
+    s.per_cta = round_up(2 * even);
+    while (s.per_cta > round_up(even) && cox_where(s) != cox_where({s.C, s.threads, round_up(even)}))
+        s.per_cta -= kB * s.threads;
     return s;
 }
 
-CoxSlots::CoxSlots(Dataset& d_, CoxShape shape) : ds(d_), C(shape.C), threads(shape.threads) {
-    cap = std::max(1, ds.event_rows());
-    per_cta = ((cap + C - 1) / C + kB * threads - 1) / (kB * threads) * (kB * threads);
-    const int K = ds.K;
-    cnt.alloc(K);
-    tiles.alloc((K + kTile - 1) / kTile);
-    end.alloc(cap); first.alloc(cap); lo.alloc(cap); sstr.alloc(cap);
-    rowslot.alloc(K); rpart.alloc(C + 1); spart.alloc(C + 1); total.alloc(1);
-    split.alloc((size_t)ds.J * (C + 1));
-    entry.alloc(std::max<long long>(1, ds.nnz_idx));
-    const size_t n_ = (size_t)C * per_cta;
-    flag.alloc(n_); n.alloc(n_);
-}
-
-CoxState::CoxState(const CoxSlots& s, int F) : np(s.positions()) {
-    const int where = cox_where(s.shape(), s.per_cta);
-    d.alloc(F * np);
-    if (where == 2) { S1.alloc(F * np); S2.alloc(F * np); bp.alloc(F * np / kB); }
-}
-
-void CoxState::set(CoxArgs& a, int f) const {
-    a.d = d.get() + f * np;
-    if (S1.get()) { a.S1 = S1.get() + f * np; a.S2 = S2.get() + f * np; a.bp = bp.get() + f * np / kB; }
-}
-
-CoxArgs CoxSlots::args() const {
-    CoxArgs a{};
-    a.K = ds.K; a.J = ds.J; a.per_cta = per_cta;
-    a.fmt = ds.d_fmt.get(); a.col_ptr = ds.d_col_ptr.get(); a.val_ptr = ds.d_val_ptr.get();
-    a.idx = ds.d_idx.get(); a.val = ds.d_val.get();
-    a.entry = entry.get(); a.rowslot = rowslot.get();
-    if (ds.S > 1) {
-        ds.ensure_entry_strata();
-        a.entry_strat = ds.d_entry_strat.get();
-    }
-    a.strat = ds.d_strat.get();
-    a.split = split.get(); a.rpart = rpart.get(); a.spart = spart.get(); a.flag = flag.get();
-    a.n = n.get(); a.y = ds.d_y.get();
-    a.wait = wait_limit(ds.K);
-    return a;
-}
-
-void CoxSlots::build(const double* d_w, cudaStream_t stream) {
+void CoxSlots::find(const double* d_w, cudaStream_t stream) {
     const int K = ds.K, nt = (K + kTile - 1) / kTile;
     const double* y = ds.d_y.get();
     const int* strat = ds.d_strat.get();
+    const int events = std::max(1, ds.event_rows());
+    cnt.alloc(K);
+    tiles.alloc(nt);
+    gend.alloc(events); first.alloc(events); glo.alloc(events); gstr.alloc(events); gcum.alloc(events);
+    groups.alloc(1);
     const int* lastp = nullptr;
     if (d_w) {
         last.alloc(K);
@@ -1111,19 +1212,40 @@ void CoxSlots::build(const double* d_w, cudaStream_t stream) {
     launch(k_rows_totals<OpSum, GroupStart>, nt, kThreads, 0, stream, K, item, tiles.get());
     launch(k_tiles_scan<OpSum>, 1, kThreads, 0, stream, nt, tiles.get());
     launch(k_rows_scan<OpSum, GroupStart>, nt, kThreads, 0, stream, K, item, (const int*)tiles.get(), cnt.get());
-    CYC_CHECK_CUDA(cudaMemsetAsync(end.get(), 0xff, cap * sizeof(int), stream));
+    CYC_CHECK_CUDA(cudaMemsetAsync(gend.get(), 0xff, events * sizeof(int), stream));
+    launch(k_slot_rows, grid_for(K, 1), kThreads, 0, stream, K, d_w, y, strat, (const int*)cnt.get(), first.get(),
+           gend.get(), gstr.get(), groups.get());
+    // each group's rows, and the slots they are cut into
+    launch(k_group_rows, grid_for(events, 1), kThreads, 0, stream, (const int*)groups.get(), (const int*)gend.get(),
+           (const int*)gstr.get(), (const int*)ds.d_strat_ptr.get(), glo.get());
+    const Pieces pieces{groups.get(), glo.get(), gend.get()};
+    const int gt = (events + kTile - 1) / kTile;          // (no more tiles than the rows have)
+    launch(k_rows_totals<OpSum, Pieces>, gt, kThreads, 0, stream, events, pieces, tiles.get());
+    launch(k_tiles_scan<OpSum>, 1, kThreads, 0, stream, gt, tiles.get());
+    launch(k_rows_scan<OpSum, Pieces>, gt, kThreads, 0, stream, events, pieces, (const int*)tiles.get(), gcum.get());
+    CYC_CHECK_CUDA(cudaMemcpyAsync(&n_slots, gcum.get() + events - 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
+}
+
+void CoxSlots::build(CoxShape s, const double* d_w, cudaStream_t stream) {
+    shape = s;
+    const int K = ds.K, C = shape.C, threads = shape.threads, room = std::max(1, n_slots);
+    lo.alloc(room); end.alloc(room); sstr.alloc(room);
+    rowslot.alloc(K); rpart.alloc(C + 1); spart.alloc(C + 1);
+    split.alloc((size_t)ds.J * (C + 1));
+    entry.alloc(std::max<long long>(1, ds.nnz_idx));
+    flag.alloc(positions()); n.alloc(positions());
     // positions past the slots read as empty
     CYC_CHECK_CUDA(cudaMemsetAsync(n.get(), 0, n.bytes(), stream));
     CYC_CHECK_CUDA(cudaMemsetAsync(flag.get(), 0, flag.bytes(), stream));
-    launch(k_slot_rows, grid_for(K, 1), kThreads, 0, stream, K, d_w, y, strat, (const int*)cnt.get(), first.get(),
-           end.get(), sstr.get(), total.get());
-    launch(k_slot_parts, 1, 32, 0, stream, K, C, (const int*)total.get(), (const int*)end.get(), spart.get(),
+    const Groups G{groups.get(), cnt.get(), glo.get(), gend.get(), gstr.get(), gcum.get()};
+    const int events = std::max(1, ds.event_rows());
+    launch(k_slot_fill, grid_for(32ll * events, 1), kThreads, 0, stream, G, lo.get(), end.get(), sstr.get());
+    launch(k_slot_parts, 1, 32 * kMaxC, 0, stream, K, C, n_slots, shape.per_cta, G, (const int*)end.get(), spart.get(),
            rpart.get());
-    launch(k_slots, grid_for(32ll * cap, 1), kThreads, 0, stream, C, threads, per_cta, (const int*)total.get(),
-           (const int*)spart.get(), (const int*)first.get(), (const int*)end.get(), (const int*)sstr.get(),
-           (const int*)ds.d_strat_ptr.get(), d_w, y, lo.get(), flag.get(), n.get());
-    launch(k_row_slots, grid_for(K, 1), kThreads, 0, stream, K, C, threads, (const int*)total.get(), (const int*)spart.get(),
-           (const int*)sstr.get(), (const int*)end.get(), strat, (const int*)cnt.get(), rowslot.get());
+    launch(k_slots, grid_for(32ll * events, 1), kThreads, 0, stream, C, threads, shape.per_cta, G,
+           (const int*)spart.get(), (const int*)first.get(), d_w, (const double*)ds.d_y.get(), flag.get(), n.get());
+    launch(k_row_slots, grid_for(K, 1), kThreads, 0, stream, K, C, threads, n_slots, G, (const int*)spart.get(),
+           (const int*)sstr.get(), (const int*)ds.d_strat.get(), rowslot.get());
     if (ds.nnz_idx)
         launch(k_entry_slots, grid_for(ds.nnz_idx, 4), kThreads, 0, stream, ds.nnz_idx, (const int*)ds.d_idx.get(),
                (const int*)rowslot.get(), entry.get());
@@ -1132,8 +1254,37 @@ void CoxSlots::build(const double* d_w, cudaStream_t stream) {
 
 void CoxSlots::increments(const double* d_xb, const double* d_w, double* out, cudaStream_t stream) const {
     CYC_CHECK_CUDA(cudaMemsetAsync(out, 0, positions() * sizeof(double), stream));   // past the slots: empty
-    launch(k_slot_increments, grid_for(32ll * cap, 1), kThreads, 0, stream, C, threads, per_cta, (const int*)total.get(),
-           (const int*)spart.get(), (const int*)lo.get(), (const int*)end.get(), d_w, d_xb, out);
+    launch(k_slot_increments, grid_for(32ll * std::max(1, n_slots), 1), kThreads, 0, stream, shape.C, shape.threads,
+           shape.per_cta, n_slots, (const int*)spart.get(), (const int*)lo.get(), (const int*)end.get(), d_w, d_xb, out);
+}
+
+CoxState::CoxState(const CoxSlots& s, int F) : np(s.positions()) {
+    const int where = cox_where(s.shape);
+    d.alloc(F * np);
+    if (where == 2) { S1.alloc(F * np); S2.alloc(F * np); bp.alloc(F * np / kB); }
+}
+
+void CoxState::set(CoxArgs& a, int f) const {
+    a.d = d.get() + f * np;
+    if (S1.get()) { a.S1 = S1.get() + f * np; a.S2 = S2.get() + f * np; a.bp = bp.get() + f * np / kB; }
+}
+
+CoxArgs CoxSlots::args() const {
+    CoxArgs a{};
+    a.K = ds.K; a.J = ds.J; a.per_cta = shape.per_cta;
+    a.fmt = ds.d_fmt.get(); a.col_ptr = ds.d_col_ptr.get(); a.val_ptr = ds.d_val_ptr.get();
+    a.idx = ds.d_idx.get(); a.val = ds.d_val.get();
+    a.entry = entry.get(); a.rowslot = rowslot.get();
+    if (ds.S > 1) {
+        ds.ensure_entry_strata();
+        a.entry_strat = ds.d_entry_strat.get();
+    }
+    a.strat = ds.d_strat.get();
+    a.split = split.get(); a.rpart = rpart.get(); a.spart = spart.get();
+    a.flag = flag.get();
+    a.n = n.get(); a.y = ds.d_y.get();
+    a.wait = wait_limit(ds.K);
+    return a;
 }
 
 // ---- many fits -------------------------------------------------------------------
@@ -1164,7 +1315,6 @@ void run_cox_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* spec
     CYC_CHECK_CUDA(cudaStreamCreateWithFlags(&own.s, cudaStreamNonBlocking));
     cudaStream_t stream = own.s;
     StreamScope scope(stream);
-    const CoxShape shape = cox_shape(ds);
 
     // one set of risk sets per weight vector of this call
     struct Weighting {
@@ -1184,13 +1334,22 @@ void run_cox_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* spec
             s.w.alloc(K);
             CYC_CHECK_CUDA(cudaMemcpyAsync(s.w.get(), h, K * sizeof(double), cudaMemcpyHostToDevice, stream));
         }
-        s.slots.reset(new CoxSlots(ds, shape));
-        s.slots->build(s.w.get(), stream);
+        s.slots.reset(new CoxSlots(ds));
+        s.slots->find(s.w.get(), stream);
         if (with_xjy) {
             s.xjy.alloc(J);
             launch_xjy(ds, s.w.get(), s.xjy.get(), stream);
         }
         return s;
+    };
+    // the slots of the weightings from `first` on, for one launch
+    auto build = [&](size_t first) -> CoxShape {
+        CYC_CHECK_CUDA(cudaStreamSynchronize(stream));
+        int slots = 0;
+        for (size_t i = first; i < sets.size(); ++i) slots = std::max(slots, sets[i]->slots->n_slots);
+        const CoxShape shape = cox_shape(slots);
+        for (size_t i = first; i < sets.size(); ++i) sets[i]->slots->build(shape, sets[i]->w.get(), stream);
+        return shape;
     };
 
     DevBuf<double> xb, xb_save, beta, hdelta, ll;
@@ -1219,7 +1378,8 @@ void run_cox_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* spec
         if (ds.has_offset) b[0] = 1.0;
         of[f] = &weighting(specs[f].weights, true);
     }
-    CoxState state(*sets[0]->slots, F);
+    CoxShape shape = build(0);
+    std::unique_ptr<CoxState> state(new CoxState(*sets[0]->slots, F));
     CYC_CHECK_CUDA(cudaMemcpyAsync(cols.get(), h_cols.data(), cols.bytes(), cudaMemcpyHostToDevice, stream));
     CYC_CHECK_CUDA(cudaMemcpyAsync(ncols.get(), h_n.data(), F * sizeof(int), cudaMemcpyHostToDevice, stream));
     for (int f = 0; f < F; ++f) {
@@ -1242,7 +1402,7 @@ void run_cox_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* spec
         a.out_iter = flags.get() + 2 * f;
         a.out_flag = flags.get() + 2 * f + 1;
         a.out_ll = ll.get() + f;
-        state.set(a, f);
+        state->set(a, f);
         args[f] = a;
     }
     const bool strata = ds.S > 1;
@@ -1262,7 +1422,7 @@ void run_cox_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* spec
         CYC_CHECK_CUDA(cudaMemcpyAsync(d_args.get(), list.data(), list.size() * sizeof(CoxArgs), cudaMemcpyHostToDevice,
                                        stream));
         CYC_CHECK_CUDA(cudaEventRecord(e0, stream));
-        launch_cox(d_args.get(), (int)run.size(), shape, sets[0]->slots->per_cta, strata, stream);
+        launch_cox(d_args.get(), (int)run.size(), shape, strata, stream);
         CYC_CHECK_CUDA(cudaEventRecord(e1, stream));
         CYC_CHECK_CUDA(cudaMemcpyAsync(h_flags.data(), flags.get(), 2 * F * sizeof(int), cudaMemcpyDeviceToHost, stream));
         CYC_CHECK_CUDA(cudaStreamSynchronize(stream));
@@ -1334,14 +1494,22 @@ void run_cox_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* spec
     st.phase_ms[0] = st.kernel_ms;
     st.phase_state_bytes[0] = 8;
     if (pred) {
-        std::vector<CoxArgs> eval = args;
+        std::vector<CoxArgs> eval(F);
         std::vector<Weighting*> by(F);
         std::vector<int> good;
+        state.reset();
+        sets.clear();                                          // the training risk sets go
         for (int f = 0; f < F; ++f) {
             pred[f] = std::nan("");
             if (out[f].return_flag != CYC_SUCCESS) continue;   // AbstractCrossValidationDriver.cpp:236-240
             good.push_back(f);
             by[f] = &weighting(held[f], false);
+        }
+        if (!good.empty()) {
+            shape = build(0);
+            state.reset(new CoxState(*sets[0]->slots, F));
+        }
+        for (int f : good) {
             CoxArgs a = by[f]->slots->args();
             a.weighted = 1;
             a.w = by[f]->w.get();
@@ -1351,7 +1519,7 @@ void run_cox_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* spec
             a.out_iter = args[f].out_iter;
             a.out_flag = args[f].out_flag;
             a.out_ll = args[f].out_ll;
-            state.set(a, f);
+            state->set(a, f);
             eval[f] = a;
         }
         if (!good.empty()) {

@@ -7,39 +7,44 @@ namespace cyc {
 
 constexpr int kCoxThreads = 512;
 
-// CTAs of a Cox fit and threads of a CTA
+// CTAs of a Cox fit, threads of a CTA, and the slots a CTA has room for (a
+// multiple of 4 threads)
 struct CoxShape {
     int C, threads;                // threads: 128, 256 or 512
+    int per_cta = 0;
 };
-CoxShape cox_shape(Dataset& ds);
+// for fits of at most `slots` slots each
+CoxShape cox_shape(int slots);
 
 struct CoxArgs;
 
-// The risk sets of a weighting, reduced to the groups that hold events: slot e
-// is an event group in row order (rows by stratum, then falling time; tied
-// events of a stratum share one).  A row enters the risk sets from the first
-// event group at or after it in its stratum on: that group is the row's slot,
-// and a row after its stratum's last event has none.
+// The risk sets of a weighting, reduced to slots of at most kSlotRows rows.  Rows
+// are sorted by stratum, then falling time; tied events of a stratum are an event
+// group, whose rows are those after the group before, to its last event: they
+// enter the risk sets with it.  Rows after their stratum's last event have no
+// group.  A group's rows are cut into slots, of which the last has its events.
 // Slots are split over C CTAs in order; CTA r's slots are dealt to its threads
 // in contiguous runs of `m` (slot t * m + i of the CTA at position i * threads
 // + t), which is the order all per-slot arrays have.
 struct CoxSlots {
     Dataset& ds;
-    int C, threads;
-    int cap;                       // at least the number of slots
-    int per_cta;                   // positions a CTA has room for (a multiple of 4 `threads`)
+    CoxShape shape{1, 128};
+    int n_slots = 0;
     DevBuf<int> cnt, last, tiles;  // scans over the rows
-    DevBuf<int> end, first, lo, sstr, rowslot, rpart, spart, total, split, entry;
+    DevBuf<int> first, glo, gend, gstr, gcum, groups;      // the event groups
+    DevBuf<int> lo, end, sstr, rowslot, rpart, spart, split, entry;
     DevBuf<unsigned char> flag;    // [C][per_cta] bit 0: the slot starts its stratum, bit 1: it ends it
     DevBuf<double> n;              // [C][per_cta] events
 
-    CoxSlots(Dataset& ds, CoxShape shape);
-    // for row weights d_w (K, device) or null
-    void build(const double* d_w, cudaStream_t stream);
+    explicit CoxSlots(Dataset& d) : ds(d) {}
+    // the event groups and the number of slots for row weights d_w (K, device)
+    // or null; n_slots is known once the stream is through
+    void find(const double* d_w, cudaStream_t stream);
+    // the slots, for a launch of this shape
+    void build(CoxShape s, const double* d_w, cudaStream_t stream);
     // the risk-set increments (sums of w exp(xb) over each slot's rows) in `out`
     void increments(const double* d_xb, const double* d_w, double* out, cudaStream_t stream) const;
-    size_t positions() const { return (size_t)C * per_cta; }
-    CoxShape shape() const { return {C, threads}; }
+    size_t positions() const { return (size_t)shape.C * shape.per_cta; }
     // the arguments that follow from the dataset and the risk sets
     CoxArgs args() const;
 };
@@ -62,7 +67,7 @@ struct CoxArgs {
     const int* idx;
     const double* val;
     const int* entry;              // slot position of every entry of idx (-1: none; bit 30: see k_cox)
-    const int* rowslot;            // the same by row (dense columns)
+    const int* rowslot;            // the same by row
     const int* entry_strat;        // stratum of every entry (null: one stratum)
     const int* strat;              // by row
     const int* split;              // J x (C+1)
@@ -94,7 +99,7 @@ struct CoxArgs {
     double* out_ll;
 };
 // one launch of F fits of one shape; `d_fits` is their arguments on the device
-void launch_cox(const CoxArgs* d_fits, int F, CoxShape shape, int per_cta, bool strata, cudaStream_t stream);
+void launch_cox(const CoxArgs* d_fits, int F, CoxShape shape, bool strata, cudaStream_t stream);
 
 // F Cox fits as one launch (each the one cyc_fit gives alone), weights per fit;
 // with `held`, the predictive log likelihood of each fit's held-out rows under

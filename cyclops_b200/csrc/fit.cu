@@ -186,8 +186,10 @@ struct FitRunner {
 
     void prepare_cox() {
         Dataset& ds = *e.ds;
-        slots.reset(new CoxSlots(ds, cox_shape(ds)));
-        slots->build(cox_weights(), e.stream);
+        slots.reset(new CoxSlots(ds));
+        slots->find(cox_weights(), e.stream);
+        e.sync();
+        slots->build(cox_shape(slots->n_slots), cox_weights(), e.stream);
         d_cols.alloc(J); d_ncols.alloc(1); d_out.alloc(2);
         state.reset(new CoxState(*slots, 1));
         d_cox.alloc(1);
@@ -204,7 +206,7 @@ struct FitRunner {
     void launch_cox_pass(const CoxArgs& a) {
         slots->increments(e.xb.get(), cox_weights(), a.d, e.stream);
         CYC_CHECK_CUDA(cudaMemcpyAsync(d_cox.get(), &a, sizeof(CoxArgs), cudaMemcpyHostToDevice, e.stream));
-        launch_cox(d_cox.get(), 1, slots->shape(), slots->per_cta, e.ds->S > 1, e.stream);
+        launch_cox(d_cox.get(), 1, slots->shape, e.ds->S > 1, e.stream);
         CYC_CHECK_CUDA(cudaMemcpyAsync(h_flags, d_out.get(), 2 * sizeof(int), cudaMemcpyDeviceToHost, e.stream));
         e.sync();
         CYC_REQUIRE(h_flags[1] != kTimedOut, CYC_ERR_TIMEOUT, "a wait between the CTAs of a fit ran out");
