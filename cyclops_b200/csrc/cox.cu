@@ -32,6 +32,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <memory>
+#include <set>
 
 #include "ccd.cuh"
 #include "engine.cuh"
@@ -1289,32 +1290,11 @@ CoxArgs CoxSlots::args() const {
 
 // ---- many fits -------------------------------------------------------------------
 
-void run_cox_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* specs, int F, const cyc_control* ctl,
-                   cyc_fit_result* out, const double* const* held, double* pred) {
+// the fits of one launch: their risk sets, the fits, the scores of `held`
+static void run_cox_fits(Dataset& ds, const std::vector<int>& pt, const cyc_fit_spec* specs, int F,
+                         const cyc_control* ctl, cyc_fit_result* out, const double* const* held, double* pred,
+                         cudaStream_t stream, cyc_run_stats& st) {
     const int K = ds.K, J = ds.J;
-    CYC_REQUIRE(prior->prior_type >= CYC_PRIOR_NONE && prior->prior_type <= CYC_PRIOR_NORMAL, CYC_ERR_ARGUMENT,
-                "Unknown prior type");
-    CYC_REQUIRE(ctl->convergence_type >= CYC_CONV_GRADIENT && ctl->convergence_type <= CYC_CONV_ZHANG_OLES,
-                CYC_ERR_ARGUMENT, "Unknown convergence criterion");
-    std::vector<int> pt(J, prior->prior_type);
-    for (int i = 0; i < prior->n_exclude; ++i) {
-        CYC_REQUIRE(prior->exclude[i] >= 0 && prior->exclude[i] < J, CYC_ERR_ARGUMENT, "exclude index out of range");
-        pt[prior->exclude[i]] = CYC_PRIOR_NONE;
-    }
-    for (int f = 0; f < F; ++f) {
-        CYC_REQUIRE(out[f].beta, CYC_ERR_ARGUMENT, "null argument");
-        CYC_REQUIRE(prior->prior_type == CYC_PRIOR_NONE || specs[f].variance > 0, CYC_ERR_ARGUMENT,
-                    "prior variance must be positive");
-        CYC_REQUIRE(specs[f].n_fixed >= 0 && (specs[f].n_fixed == 0 || specs[f].fixed), CYC_ERR_ARGUMENT,
-                    "bad fixed-column list");
-        for (int i = 0; i < specs[f].n_fixed; ++i)
-            CYC_REQUIRE(specs[f].fixed[i] >= 0 && specs[f].fixed[i] < J, CYC_ERR_ARGUMENT, "fixed column out of range");
-    }
-    CYC_CHECK_CUDA(cudaSetDevice(ds.device));
-    OwnedStream own;
-    CYC_CHECK_CUDA(cudaStreamCreateWithFlags(&own.s, cudaStreamNonBlocking));
-    cudaStream_t stream = own.s;
-    StreamScope scope(stream);
 
     // one set of risk sets per weight vector of this call
     struct Weighting {
@@ -1412,7 +1392,6 @@ void run_cox_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* spec
     CYC_CHECK_CUDA(cudaEventCreate(&e0));
     CYC_CHECK_CUDA(cudaEventCreate(&e1));
     struct Events { cudaEvent_t a, b; ~Events() { cudaEventDestroy(a); cudaEventDestroy(b); } } events{e0, e1};
-    cyc_run_stats st{};
     auto pass = [&](const std::vector<int>& run, const std::vector<CoxArgs>& a, const std::vector<Weighting*>& w) {
         std::vector<CoxArgs> list;
         for (int f : run) {
@@ -1490,9 +1469,6 @@ void run_cox_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* spec
             st.coordinate_steps += out[f].iterations;
         }
     }
-    st.phases = 1;
-    st.phase_ms[0] = st.kernel_ms;
-    st.phase_state_bytes[0] = 8;
     if (pred) {
         std::vector<CoxArgs> eval(F);
         std::vector<Weighting*> by(F);
@@ -1529,6 +1505,76 @@ void run_cox_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* spec
             for (int f : good) pred[f] = h_ll[f];
         }
     }
+}
+
+// device bytes of a weighting's risk sets, and of a fit on them
+static void cox_bytes_of(Dataset& ds, double* weighting, double* fit) {
+    const double K = ds.K, J = ds.J, events = ds.event_rows();
+    const CoxShape s = cox_shape((int)std::min(2e9, events + K / kSlotRows + 1));
+    const double positions = (double)s.C * s.per_cta;
+    *weighting = K * 20 + events * 20 + (events + K / kSlotRows) * 12 + J * (4 * (s.C + 1) + 8) +
+                 (double)ds.nnz_idx * 4 + positions * 9;
+    *fit = K * 16 + J * 24 + positions * (cox_where(s) == 2 ? 26 : 8);
+}
+
+void run_cox_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* specs, int F, const cyc_control* ctl,
+                   cyc_fit_result* out, const double* const* held, double* pred) {
+    const int J = ds.J;
+    CYC_REQUIRE(prior->prior_type >= CYC_PRIOR_NONE && prior->prior_type <= CYC_PRIOR_NORMAL, CYC_ERR_ARGUMENT,
+                "Unknown prior type");
+    CYC_REQUIRE(ctl->convergence_type >= CYC_CONV_GRADIENT && ctl->convergence_type <= CYC_CONV_ZHANG_OLES,
+                CYC_ERR_ARGUMENT, "Unknown convergence criterion");
+    std::vector<int> pt(J, prior->prior_type);
+    for (int i = 0; i < prior->n_exclude; ++i) {
+        CYC_REQUIRE(prior->exclude[i] >= 0 && prior->exclude[i] < J, CYC_ERR_ARGUMENT, "exclude index out of range");
+        pt[prior->exclude[i]] = CYC_PRIOR_NONE;
+    }
+    for (int f = 0; f < F; ++f) {
+        CYC_REQUIRE(out[f].beta, CYC_ERR_ARGUMENT, "null argument");
+        CYC_REQUIRE(prior->prior_type == CYC_PRIOR_NONE || specs[f].variance > 0, CYC_ERR_ARGUMENT,
+                    "prior variance must be positive");
+        CYC_REQUIRE(specs[f].n_fixed >= 0 && (specs[f].n_fixed == 0 || specs[f].fixed), CYC_ERR_ARGUMENT,
+                    "bad fixed-column list");
+        for (int i = 0; i < specs[f].n_fixed; ++i)
+            CYC_REQUIRE(specs[f].fixed[i] >= 0 && specs[f].fixed[i] < J, CYC_ERR_ARGUMENT, "fixed column out of range");
+    }
+    CYC_CHECK_CUDA(cudaSetDevice(ds.device));
+    OwnedStream own;
+    CYC_CHECK_CUDA(cudaStreamCreateWithFlags(&own.s, cudaStreamNonBlocking));
+    StreamScope scope(own.s);
+    // Fits run as many at a time as half of the device's free memory holds
+    // (what the pool keeps counts as free): 1,000 bootstrap replicates of 2M rows
+    // and 50M entries want 270 GB.  CYC_COX_BATCH_BYTES sets the bound.
+    double per_weighting, per_fit;
+    cox_bytes_of(ds, &per_weighting, &per_fit);
+    double bound = 1e9;
+    if (const char* e = std::getenv("CYC_COX_BATCH_BYTES")) {
+        bound = std::atof(e);
+    } else if (F * (per_weighting + per_fit) > bound) {
+        size_t free_bytes = 0, total_bytes = 0;
+        unsigned long long reserved = 0, used = 0;
+        cudaMemPool_t pool;
+        CYC_CHECK_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+        CYC_CHECK_CUDA(cudaDeviceGetDefaultMemPool(&pool, ds.device));
+        CYC_CHECK_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+        CYC_CHECK_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+        bound = 0.5 * ((double)free_bytes + (double)reserved - (double)used);
+    }
+    cyc_run_stats st{};
+    for (int f0 = 0; f0 < F;) {
+        std::set<const double*> weightings;
+        int n = 0;
+        for (; f0 + n < F; ++n) {
+            weightings.insert(specs[f0 + n].weights);
+            if (n > 0 && per_weighting * weightings.size() + per_fit * (n + 1) > bound) break;
+        }
+        run_cox_fits(ds, pt, specs + f0, n, ctl, out + f0, held ? held + f0 : nullptr, pred ? pred + f0 : nullptr, own.s,
+                     st);
+        f0 += n;
+    }
+    st.phases = 1;
+    st.phase_ms[0] = st.kernel_ms;
+    st.phase_state_bytes[0] = 8;
     set_last_stats(st);
 }
 

@@ -75,6 +75,10 @@ def request_bytes(data: D.CyclopsData, fits: int = 1) -> int:
     nnz_val = int(data.col_val.size)
     dataset = nnz_idx * 4 + nnz_val * 8 + J * 24 + K * 24 + (nnz_idx + nnz_val) * 12 + K * 8
     state = fits * (K * 8 * 6 + J * 8 * 4)
+    if data.model == D.COX:                  # the risk sets of the fits' weights, and the solver's arrays on them
+        events = int(np.count_nonzero(data.y))
+        slots = events + K // 32
+        state += fits * (nnz_idx * 4 + K * 28 + J * 76 + events * 20 + slots * 12 + (2 * slots + 65536) * 35)
     return int(1.25 * (dataset + state)) + (1 << 20)
 
 
