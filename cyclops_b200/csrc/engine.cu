@@ -391,17 +391,18 @@ void Engine::gradient_hessian(int j, bool use_weights, double* g, double* h) {
     *h = h_result[1];
 }
 
-// updateXBeta (ModelSpecifics.hpp:1466-1586)
-void Engine::launch_update(int j, bool use_weights, double delta, const HostSignal& sig) {
+// updateXBeta (ModelSpecifics.hpp:1466-1586) by `delta`, or by what `d_delta`
+// holds when the kernel runs (not for cox)
+void Engine::launch_update(int j, bool use_weights, double delta, const HostSignal& sig, const double* d_delta) {
     ColView c = ds->view(j);
-    if (c.n == 0 || delta == 0.0) return;
+    if (c.n == 0 || (!d_delta && delta == 0.0)) return;
     ensure_groups();
     const int blocks = grid_for(c.n, 4);
     if (model_independent(model)) {
-        launch(k_update_independent, blocks, kThreads, 0, stream, c, delta, xb.get(), exb.get(), denom.get(),
+        launch(k_update_independent, blocks, kThreads, 0, stream, c, d_delta, delta, xb.get(), exb.get(), denom.get(),
                ticket.get(), sig);
     } else {
-        launch(k_update_grouped, blocks, kThreads, 0, stream, c, delta, groups(), kw.get(),
+        launch(k_update_grouped, blocks, kThreads, 0, stream, c, d_delta, delta, groups(), kw.get(),
                                                           model_cumulative(model) && use_weights && use_w,
                                                           xb.get(), exb.get(), denom.get(), ticket.get(), sig);
         if (model_cumulative(model)) cox_rescan(h_first_group[j]);

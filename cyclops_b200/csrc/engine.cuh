@@ -64,7 +64,8 @@ struct Engine {
     void numerator_for_gradient(int j, bool use_weights);
     void launch_gradient(int j, bool use_weights, double* out, const HostSignal& sig);
     void gradient_hessian(int j, bool use_weights, double* g, double* h);
-    void launch_update(int j, bool use_weights, double delta, const HostSignal& sig = HostSignal{});
+    void launch_update(int j, bool use_weights, double delta, const HostSignal& sig = HostSignal{},
+                       const double* d_delta = nullptr);
     void update_xbeta(double delta, int j, bool use_weights);
     void cox_rescan(int lo);
     void launch_loglik(bool use_cv, double* out, const HostSignal& sig = HostSignal{});

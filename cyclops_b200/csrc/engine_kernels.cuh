@@ -588,11 +588,15 @@ __global__ void k_kkt_grouped(int n_cols, const int* __restrict__ cols, int K, c
 }
 
 // ---- updateXBeta (ModelSpecifics.hpp:1524-1586) -----------------------------
+// The step comes by value, or from `d_delta` where a kernel before took it (zero:
+// nothing moves).
 
 // independent rows: each row is its own denominator
-__global__ void k_update_independent(ColView c, double delta,
+__global__ void k_update_independent(ColView c, const double* d_delta, double delta,
                                      double* __restrict__ xb, double* __restrict__ exb,
                                      double* __restrict__ denom, unsigned* ticket, HostSignal sig) {
+    if (d_delta) delta = *d_delta;
+    if (delta == 0.0) return;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < c.n;
          e += (long long)gridDim.x * blockDim.x) {
         const int k = c.row(e);
@@ -608,10 +612,12 @@ __global__ void k_update_independent(ColView c, double delta,
 
 // grouped / cumulative rows: the first entry of each run updates the run and
 // adds its denominator change (weighted for cox when use_w)
-__global__ void k_update_grouped(ColView c, double delta,
+__global__ void k_update_grouped(ColView c, const double* d_delta, double delta,
                                  const int* __restrict__ group, const double* __restrict__ kw,
                                  int weighted, double* __restrict__ xb, double* __restrict__ exb,
                                  double* __restrict__ denom, unsigned* ticket, HostSignal sig) {
+    if (d_delta) delta = *d_delta;
+    if (delta == 0.0) return;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < c.n;
          e += (long long)gridDim.x * blockDim.x) {
         const int key = group[c.row(e)];

@@ -6,7 +6,9 @@
 // persistent kernel (ccd.cu for lr, pr, clr and cpr, cox.cu for cox) on the
 // engine's linear predictors; the host reads the cycle count and the return
 // flag when it ends, and runs the restarts, the active-set passes and the
-// profile searches around it.
+// profile searches around it.  Fits of mostly very long columns, which want more
+// SMs than a cluster has, run the engine's kernels over the whole device instead
+// (long_columns).
 #include "ccd.cuh"
 #include "cox.cuh"
 #include "engine.cuh"
@@ -15,6 +17,8 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <cstdlib>
+#include <cstring>
 #include <memory>
 #include <string>
 
@@ -24,12 +28,58 @@ static thread_local cyc_run_stats g_stats{};
 
 namespace {
 
+constexpr int kGoesOn = -2;
+
 __global__ void k_fill(int n, double v, double* __restrict__ out) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = v;
 }
 
 __global__ void k_copy(int K, const double* __restrict__ src, double* __restrict__ dst) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x) dst[k] = src[k];
+}
+
+// the coordinate step of the device-wide route (ccdUpdateBeta, CyclicCoordinateDescent.cpp
+// :1394-1413, with the priors' getDelta and applyBounds, :1503-1520)
+__global__ void k_step(int j, const double* __restrict__ gh, const int* __restrict__ ptype, double variance,
+                       double* __restrict__ beta, double* __restrict__ hdelta, double* __restrict__ delta,
+                       unsigned* __restrict__ col_updates) {
+    double g = gh[0], h = gh[1];
+    if (h < 0.0) { g = 0.0; h = 0.0; }
+    const double d = apply_bounds(hdelta + j, prior_delta(ptype[j], variance, beta[j], g, h));
+    if (d != 0.0) {
+        beta[j] += d;
+        col_updates[j] += 1u;
+    }
+    *delta = d;
+}
+
+// performCheckConvergence (CyclicCoordinateDescent.cpp:839-906): out[0] = the
+// cycles, out[1] = the return flag, -2 while the fit goes on
+__global__ void k_check(const double* __restrict__ obj, double* __restrict__ last, double tol, int iteration,
+                        int max_iter, int zhang_oles, int* __restrict__ out) {
+    const double o = *obj;
+    double conv = o;
+    bool ill = false;
+    if (!zhang_oles) {
+        ill = o != o;
+        conv = ill ? 0.0 : fabs(o - *last) / (fabs(o) + 1.0);
+        *last = o;
+    }
+    out[0] = iteration;
+    out[1] = tol > 0 && conv < tol ? (ill ? CYC_ILLCONDITIONED : CYC_SUCCESS)
+                                   : (iteration == max_iter ? CYC_MAX_ITERATIONS : kGoesOn);
+}
+
+// computeZhangOlesConvergenceCriterion (CyclicCoordinateDescent.cpp:560-579), renewing xb_save
+__global__ void k_zhang_oles(int K, const double* __restrict__ xb, double* __restrict__ xb_save,
+                             const double* __restrict__ kw, double2* partial, unsigned* ticket, double* out) {
+    double a = 0.0, b = 0.0;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x) {
+        a += fabs(xb[k] - xb_save[k]) * kw[k];
+        b += fabs(xb[k]) * kw[k];
+        xb_save[k] = xb[k];
+    }
+    grid_sum2_finalize(a, b, partial, ticket, [&](double A, double B) { *out = A / (1.0 + B); });
 }
 
 // LANGE objective: log likelihood + log prior
@@ -44,6 +94,30 @@ __global__ void k_add_logprior(int J, const double* __restrict__ beta, const int
     if (threadIdx.x == 0) out[0] = (ll ? *ll : 0.0) + a;
 }
 
+// Whether a fit runs over the whole device, a column at a time, instead of in one
+// cluster of `shape`: the modelled cycles of both.  A cluster takes a column in
+// rounds of its threads, at most 4,096 entries each; the engine's three kernels
+// take 13 to 30 us for any column and then go at the device's bandwidth.  Us a
+// column, device / cluster: logistic, dense 200k rows 15.5 / 18.3, 1M 29 / 121, 2.5M
+// 69 / 334; indicators of 30 % 400k rows 20 / 12, 1M 25 / 53, of 3 % 1M 20 / 12, 2.5M
+// 24 / 30; matched sets of 5, dense 60k rows 32 / 47, 1M 62 / 1,045, 30 % 200k 31 / 41,
+// 1M 34 / 309, 3 % 1M 28 / 27, 2.5M 29 / 68 (a thread walks a set's entries).
+// CYC_FIT_ROUTE: "columns" or "cluster".
+bool long_columns(const Dataset& ds, const CcdShape& shape) {
+    if (const char* e = std::getenv("CYC_FIT_ROUTE")) return std::strcmp(e, "columns") == 0;
+    const bool grouped = model_grouped(ds.model);
+    const bool local = (double)ds.K / shape.C * sizeof(double) <= 200 * 1024;      // predictors in shared memory
+    const double deal = (double)shape.C * shape.threads / shape.teams;
+    double cluster = 3.2e-3 * ds.K / shape.C, device = 12.0 + 8e-6 * ds.K;          // the objective
+    for (int j = 0; j < ds.J; ++j) {
+        const bool dense = ds.fmt[j] == CYC_DENSE || ds.fmt[j] == CYC_INTERCEPT;
+        const double n = (double)ds.col_len(j), round = grouped ? 3.3 : local ? 0.36 : dense ? 0.5 : 0.7;
+        cluster += 1.0 + round * std::max(0.0, std::ceil(n / deal) - 1.0);
+        device += grouped ? 30.0 + 35e-6 * n : dense ? 13.0 + 14e-6 * n : 18.0 + 22e-6 * n;
+    }
+    return device < 0.95 * cluster;
+}
+
 }  // namespace
 
 struct FitRunner {
@@ -52,8 +126,7 @@ struct FitRunner {
     int J;
     std::vector<int> fixb, base_fix, pt;
     DevBuf<double> beta, hdelta, gh, delta, obj, last;
-    DevBuf<int> ptype, flags;
-    DevBuf<unsigned long long> n_updates;
+    DevBuf<int> ptype;
     DevBuf<unsigned> col_updates;        // per column: coordinate steps that moved beta
     double variance;
     PinnedBlock h_block;                 // two flags read back per cycle (pinned, pooled)
@@ -79,15 +152,15 @@ struct FitRunner {
             pt[prior.exclude[i]] = CYC_PRIOR_NONE;
         }
         beta.alloc(J); hdelta.alloc(J); gh.alloc(2); delta.alloc(1); obj.alloc(1); last.alloc(1);
-        ptype.alloc(J); flags.alloc(2); n_updates.alloc(1); col_updates.alloc(J);
+        ptype.alloc(J); col_updates.alloc(J);
         CYC_CHECK_CUDA(cudaMemcpyAsync(ptype.get(), pt.data(), J * sizeof(int), cudaMemcpyHostToDevice, e.stream));
-        CYC_CHECK_CUDA(cudaMemsetAsync(n_updates.get(), 0, sizeof(unsigned long long), e.stream));
         CYC_CHECK_CUDA(cudaMemsetAsync(col_updates.get(), 0, J * sizeof(unsigned), e.stream));
         CYC_CHECK_CUDA(cudaEventCreate(&ev0));
         CYC_CHECK_CUDA(cudaEventCreate(&ev1));
         e.sync();
     }
     ~FitRunner() {
+        drop_graphs();
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
     }
@@ -110,6 +183,7 @@ struct FitRunner {
     void prepare_ccd() {
         Dataset& ds = *e.ds;
         const CcdShape shape = ccd_shape(ds, 1);
+        by_column = long_columns(ds, shape);
         rpart = ccd_rows(ds, shape.C);
         d_rpart.alloc(shape.C + 1); d_split.alloc((size_t)J * (shape.C + 1)); d_cols.alloc(J); d_ncols.alloc(1);
         d_out.alloc(2); d_variance.alloc(1);
@@ -156,6 +230,81 @@ struct FitRunner {
         if (ctl.convergence_type == CYC_CONV_ZHANG_OLES) {
             e.xb_save.alloc(e.ds->K);
             launch(k_copy, grid_for(e.ds->K, 1), kThreads, 0, e.stream, e.ds->K, e.xb.get(), e.xb_save.get());
+        }
+    }
+
+    // ---- the same with the engine's kernels over the whole device, a column at a
+    // time: gradient, step, update, the step left on the device
+    bool by_column = false;
+
+    void launch_objective() {
+        switch (ctl.convergence_type) {
+        case CYC_CONV_GRADIENT: e.launch_gradient_objective(true, obj.get(), HostSignal{}); break;
+        case CYC_CONV_MITTAL: e.launch_loglik(true, obj.get()); break;
+        case CYC_CONV_LANGE:
+            e.launch_loglik(true, obj.get());
+            launch(k_add_logprior, 1, kThreads, 0, e.stream, J, beta.get(), ptype.get(), variance, obj.get(), obj.get());
+            break;
+        case CYC_CONV_ZHANG_OLES:
+            launch(k_zhang_oles, grid_for(e.ds->K, 4), kThreads, 0, e.stream, e.ds->K, e.xb.get(), e.xb_save.get(),
+                   e.kw.get(), e.partial.get(), e.ticket.get(), obj.get());
+            break;
+        default: CYC_CHECK_CUDA(cudaMemsetAsync(obj.get(), 0, sizeof(double), e.stream));   // ONE_STEP
+        }
+    }
+
+    // the columns not fixed now as graphs (a launch from the host costs more than
+    // a short column's kernel), of at most kGraphColumns each
+    static constexpr int kGraphColumns = 4096;
+    std::vector<cudaGraphExec_t> graphs;
+    std::vector<int> graphs_fix;
+
+    void capture_columns() {
+        if (!graphs.empty() && graphs_fix == fixb) return;
+        drop_graphs();
+        for (int b = 0; b < J; b += kGraphColumns) {
+            cudaGraph_t g;
+            CYC_CHECK_CUDA(cudaStreamBeginCapture(e.stream, cudaStreamCaptureModeThreadLocal));
+            for (int j = b; j < std::min(J, b + kGraphColumns); ++j) {
+                if (fixb[j]) continue;
+                if (e.ds->col_len(j) > 0) e.launch_gradient(j, true, gh.get(), HostSignal{});
+                else CYC_CHECK_CUDA(cudaMemsetAsync(gh.get(), 0, 2 * sizeof(double), e.stream));
+                launch(k_step, 1, 1, 0, e.stream, j, gh.get(), ptype.get(), variance, beta.get(), hdelta.get(),
+                       delta.get(), col_updates.get());
+                e.launch_update(j, true, 0.0, HostSignal{}, delta.get());
+            }
+            CYC_CHECK_CUDA(cudaStreamEndCapture(e.stream, &g));
+            cudaGraphExec_t x;
+            const cudaError_t made = cudaGraphInstantiate(&x, g, 0);
+            CYC_CHECK_CUDA(cudaGraphDestroy(g));
+            CYC_CHECK_CUDA(made);
+            graphs.push_back(x);
+        }
+        graphs_fix = fixb;
+    }
+    void drop_graphs() {
+        for (auto& g : graphs) cudaGraphExecDestroy(g);
+        graphs.clear();
+    }
+
+    int find_mode_columns(double bound, int* iterations) {
+        prepare_pass(bound);
+        const bool zhang = ctl.convergence_type == CYC_CONV_ZHANG_OLES;
+        if (!zhang) {
+            launch_objective();
+            launch(k_copy, 1, 1, 0, e.stream, 1, obj.get(), last.get());
+        }
+        capture_columns();
+        for (int it = 1;; ++it) {
+            for (auto& g : graphs) CYC_CHECK_CUDA(cudaGraphLaunch(g, e.stream));
+            launch_objective();
+            launch(k_check, 1, 1, 0, e.stream, obj.get(), last.get(), ctl.tolerance, it, ctl.max_iterations, zhang ? 1 : 0,
+                   d_out.get());
+            CYC_CHECK_CUDA(cudaMemcpyAsync(h_flags, d_out.get(), 2 * sizeof(int), cudaMemcpyDeviceToHost, e.stream));
+            e.sync();
+            if (h_flags[1] == kGoesOn) continue;
+            *iterations = h_flags[0];
+            return h_flags[1];
         }
     }
 
@@ -245,7 +394,8 @@ struct FitRunner {
         const int conv = ctl.convergence_type;
         CYC_REQUIRE(conv >= CYC_CONV_GRADIENT && conv <= CYC_CONV_ZHANG_OLES, CYC_ERR_ARGUMENT,
                     "Unknown convergence criterion");
-        return model_cumulative(e.model) ? find_mode_cox(bound, iterations) : find_mode_ccd(bound, iterations);
+        if (model_cumulative(e.model)) return find_mode_cox(bound, iterations);
+        return by_column ? find_mode_columns(bound, iterations) : find_mode_ccd(bound, iterations);
     }
 
     // kktSwindle (CyclicCoordinateDescent.cpp:636-814).  The intercept and
