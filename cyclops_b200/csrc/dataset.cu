@@ -101,7 +101,10 @@ static void upload(DevBuf<T>& buf, const T* src, size_t n) {
 // in order, 32 at a time: the columns' entries in its rows (k_splits), laid end
 // to end, are placed 32 a step, entries of one row in the order of their
 // lanes.  Bound by a load latency a step: 1.3M entries (100k rows, 600 Zipf
-// columns and 5 dense ones) 21 ms as a counting sort on the host, 0.2 here.
+// columns and 5 dense ones) 21 ms as a counting sort on the host, 0.2 here.  The
+// splits of all columns over all warps may be large, so columns go in parts, and
+// the rows' cursors wait in memory between them (fewer warps instead: 1M columns
+// of 10 entries over 100k rows 321 ms; 170 on the host, 37 in parts).
 
 namespace {
 
@@ -149,9 +152,10 @@ __global__ void k_csr_scan(int K, int every, const int* __restrict__ cnt, long l
     if (threadIdx.x == 0) rp[K] = carry;
 }
 
-// rows [part[w], part[w + 1]) by warp w; `split` as k_splits leaves it
+// rows [part[w], part[w + 1]) by warp w; `split` as k_splits leaves it; the J
+// columns are `col0` and the ones after it, `placed` the entries of each row so far
 __global__ void __launch_bounds__(32 * kCsrWarps)
-k_csr_fill(int J, int W, const int* __restrict__ part, const int* __restrict__ split, const int* __restrict__ fmt,
+k_csr_fill(int J, int col0, int W, int* __restrict__ placed, const int* __restrict__ part, const int* __restrict__ split, const int* __restrict__ fmt,
            const long long* __restrict__ col_ptr, const long long* __restrict__ val_ptr, const int* __restrict__ idx,
            const double* __restrict__ val, const long long* __restrict__ rp, int* __restrict__ rc,
            double* __restrict__ rv) {
@@ -161,7 +165,7 @@ k_csr_fill(int J, int W, const int* __restrict__ part, const int* __restrict__ s
     if (w >= W) return;
     int* cur = s_cur[threadIdx.x >> 5];
     const int r0 = part[w], r1 = part[w + 1];
-    for (int q = lane; q < r1 - r0; q += 32) cur[q] = 0;
+    for (int q = lane; q < r1 - r0; q += 32) cur[q] = placed[r0 + q];
     __syncwarp();
     for (int j0 = 0; j0 < J; j0 += 32) {
         const int j = j0 + lane;
@@ -202,7 +206,7 @@ k_csr_fill(int J, int W, const int* __restrict__ part, const int* __restrict__ s
             if (on) {
                 const int rank = __popc(same & ((1u << lane) - 1u));
                 const long long p = rp[k] + cur[k - r0] + rank;
-                rc[p] = j0 + src;
+                rc[p] = col0 + j0 + src;
                 rv[p] = v < 0 ? 1.0 : __ldg(val + v + e);
             }
             __syncwarp();
@@ -210,6 +214,7 @@ k_csr_fill(int J, int W, const int* __restrict__ part, const int* __restrict__ s
             __syncwarp();
         }
     }
+    for (int q = lane; q < r1 - r0; q += 32) placed[r0 + q] = cur[q];
 }
 
 }  // namespace
@@ -230,22 +235,27 @@ void Dataset::ensure_csr() {
     if (nnz_idx)
         launch(k_csr_count, grid_for(nnz_idx, 4), kThreads, 0, stream, nnz_idx, (const int*)d_idx.get(), cnt.get());
     launch(k_csr_scan, 1, 1024, 0, stream, K, every, (const int*)cnt.get(), d_row_ptr.get());
-    // as many warps as fill the device, within 64 MB of splits and kCsrRows
-    // rows a warp; more rows than they hold take turns
-    const int most = 148 * 16 * kCsrWarps / 8;
-    const int W = (int)std::max(1LL, std::min<long long>(most, (1LL << 24) / std::max(1, J) - 1));
+    CYC_CHECK_CUDA(cudaMemsetAsync(cnt.get(), 0, std::max(1, K) * sizeof(int), stream));
+    // as many warps as fill the device, kCsrRows rows a warp (more rows than they
+    // hold take turns), and 64 MB of splits (more columns go in parts)
+    const int W = 148 * 16;
+    const int cols = std::min(J, (1 << 24) / (W + 1));
     std::vector<int> part(W + 1);
+    d_split.alloc((size_t)cols * (W + 1));
     for (long long k0 = 0; k0 < K && total > 0; k0 += (long long)W * kCsrRows) {
         const long long rows = std::min<long long>((long long)W * kCsrRows, K - k0);
         for (int w = 0; w <= W; ++w) part[w] = (int)(k0 + rows * w / W);
         upload(d_part, part.data(), part.size());
-        d_split.alloc((size_t)J * (W + 1));
-        launch(k_splits, grid_for((long long)J * (W + 1), 1, 1 << 30), kThreads, 0, stream, J, W, (const int*)d_fmt.get(),
-               (const long long*)d_col_ptr.get(), (const int*)d_idx.get(), (const int*)d_part.get(), d_split.get());
-        launch(k_csr_fill, (W + kCsrWarps - 1) / kCsrWarps, 32 * kCsrWarps, 0, stream, J, W, (const int*)d_part.get(),
-               (const int*)d_split.get(), (const int*)d_fmt.get(), (const long long*)d_col_ptr.get(),
-               (const long long*)d_val_ptr.get(), (const int*)d_idx.get(), (const double*)d_val.get(),
-               (const long long*)d_row_ptr.get(), d_row_col.get(), d_row_val.get());
+        for (int j = 0; j < J; j += cols) {
+            const int n = std::min(cols, J - j);
+            const int* fm = d_fmt.get() + j;
+            const long long *cp = d_col_ptr.get() + j, *vp = d_val_ptr.get() + j;
+            launch(k_splits, grid_for((long long)n * (W + 1), 1, 1 << 30), kThreads, 0, stream, n, W, fm, cp,
+                   (const int*)d_idx.get(), (const int*)d_part.get(), d_split.get());
+            launch(k_csr_fill, (W + kCsrWarps - 1) / kCsrWarps, 32 * kCsrWarps, 0, stream, n, j, W, cnt.get(),
+                   (const int*)d_part.get(), (const int*)d_split.get(), fm, cp, vp, (const int*)d_idx.get(),
+                   (const double*)d_val.get(), (const long long*)d_row_ptr.get(), d_row_col.get(), d_row_val.get());
+        }
     }
     CYC_CHECK_CUDA(cudaStreamSynchronize(stream));   // usable from every stream
     have_csr = true;
