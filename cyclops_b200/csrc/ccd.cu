@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
     const double var = A.variance[f];
     const double lam = sqrt(2.0 / var);          // LaplacePrior rate, CovariatePrior.h:282-292
     const double ivar = 1.0 / var;
-    const bool strict = A.strict_mean != 0;
+    const bool strict = A.strict != 0;
 
     // by parity of the column (the two teams'): the warps' sums, the CTAs' sums
     // with their arrival, and the cluster's; [2] are the whole CTA's (the objective)
@@ -397,6 +397,7 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
                         constexpr int R = decltype(rounds)::value;
                         int kk[R];
                         T xx[R], vv[R], ww[R], gi[R], hi[R];
+                        bool on[R];                          // the entry enters the sums
                         auto terms = [&](int r) {
                             mean_terms<T, MODEL>(fit_mean<T, MODEL>(vv[r], strict), xx[r], WM == 2 ? ww[r] : T(1), ind,
                                                  gi[r], hi[r]);
@@ -407,6 +408,7 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
                             xx[r] = (T)nx[r];
                             vv[r] = kk[r] >= 0 ? get(kk[r]) : T(0);
                             ww[r] = kk[r] < 0 ? T(0) : (WM == 1 ? weight.by_fold(nf[r]) : weight(kk[r]));
+                            on[r] = WM == 2 && strict ? kk[r] >= 0 : ww[r] != T(0);
                         }
                         prefetch(q + kTeams);
                         // (lanes without an entry compute too: fewer branches are fewer cycles here)
@@ -424,8 +426,8 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
                         Kahan<T> ag, ah;
                         #pragma unroll
                         for (int r = 0; r < R; ++r) {
-                            ag.add(ww[r] != T(0) ? gi[r] : T(0));
-                            ah.add(ww[r] != T(0) ? hi[r] : T(0));
+                            ag.add(on[r] ? gi[r] : T(0));
+                            ah.add(on[r] ? hi[r] : T(0));
                         }
                         if (R == kR)
                             for (int b0 = kR * NT + tid; b0 < m.n; b0 += kU * NT) {
@@ -449,8 +451,9 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
                                     T g1, h1;
                                     mean_terms<T, MODEL>(fit_mean<T, MODEL>(v2[u], strict), x2[u],
                                                          WM == 2 ? w2[u] : T(1), ind, g1, h1);
-                                    ag.add(w2[u] != T(0) ? g1 : T(0));
-                                    ah.add(w2[u] != T(0) ? h1 : T(0));
+                                    const bool on = WM == 2 && strict ? k2[u] >= 0 : w2[u] != T(0);
+                                    ag.add(on ? g1 : T(0));
+                                    ah.add(on ? h1 : T(0));
                                 }
                             }
                         finish(ag.value(), ah.value());

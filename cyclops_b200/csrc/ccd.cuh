@@ -17,8 +17,8 @@ struct CcdArgs {
     int threads;                  // per CTA, a multiple of 64 up to kCcdThreads
     int teams;                    // 2: the CTA's threads take the columns in two teams (lr, pr)
     int weights;                  // 0: all ones; 1: CV folds; 2: `w`
-    int strict_mean;              // logistic mean as exb / (1 + exb), NaN where exb overflows (as the
-                                  // per-coordinate engine), else 1 / (1 + exp(-xb))
+    int strict;                   // as the per-coordinate engine: a logistic row whose exb overflows is NaN,
+                                  // and a row of weight zero that is NaN or infinite makes the sums NaN
     const int* fmt;
     const long long* col_ptr;
     const long long* val_ptr;

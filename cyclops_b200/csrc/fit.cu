@@ -196,7 +196,7 @@ struct FitRunner {
         ccd.threads = shape.threads;
         ccd.teams = shape.teams;
         ccd.weights = e.use_w ? 2 : 0;
-        ccd.strict_mean = 1;
+        ccd.strict = 1;
         ccd.fmt = ds.d_fmt.get(); ccd.col_ptr = ds.d_col_ptr.get(); ccd.val_ptr = ds.d_val_ptr.get();
         ccd.idx = ds.d_idx.get(); ccd.val = ds.d_val.get(); ccd.entry_strat = ds.d_entry_strat.get();
         ccd.split = d_split.get(); ccd.rpart = d_rpart.get(); ccd.y = ds.d_y.get(); ccd.strat = ds.d_strat.get();
