@@ -61,6 +61,8 @@ constexpr int kSlotRows = 32;
 // CTA (kTailBit), past those of its thread (kThreadBit)
 constexpr int kTailBit = 1 << 30, kThreadBit = 1 << 29, kPosMask = kThreadBit - 1;
 constexpr unsigned kFull = 0xffffffffu;
+// relative bound on the rounding of a column's sums
+constexpr double kZero = 0x1p-45;
 
 // ---- the risk sets ------------------------------------------------------------
 
@@ -307,6 +309,20 @@ __global__ void k_slots(int C, int nt, int per_cta, Groups G, const int* __restr
     }
 }
 
+// 1 / the sum of all events (one block)
+__global__ void __launch_bounds__(1024) k_per_event(int np, const double* __restrict__ n, double* __restrict__ out) {
+    __shared__ double s_w[32];
+    double a = 0.0;
+    #pragma unroll 4
+    for (int p = threadIdx.x; p < np; p += 1024) a += n[p];
+    for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(kFull, a, o);
+    if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = a;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < 32; ++w) a += s_w[w];
+    *out = a > 0.0 ? 1.0 / a : 0.0;
+}
+
 // sums of w exp(xb) over each slot's rows (a warp each)
 __global__ void k_slot_increments(int C, int nt, int per_cta, int S, const int* __restrict__ spart,
                                   const int* __restrict__ lo, const int* __restrict__ end,
@@ -414,6 +430,7 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits
     __shared__ __align__(16) double2 x_a[2][kMaxC], x_c[2][kMaxC], x_b[2][3][kMaxC];
     __shared__ __align__(8) unsigned long long s_mb[3][2];
     __shared__ double s_carry, s_c1, s_c2, s_dl;
+    __shared__ double s_per_event;                        // 1 / the weight of the events
     __shared__ int s_dead;
     __shared__ int s_hasend[kMaxC];
     __shared__ ColMeta c_m[kCh + 1];
@@ -426,6 +443,7 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits
     if (tid == 0) {
         s_dead = 0;
         s_carry = s_c1 = s_c2 = 0.0;
+        s_per_event = *A.per_event;
         for (int i = 0; i < 6; ++i) mbar_init(smem_addr(&s_mb[i / 2][i % 2]));
         mbar_init_fence();
     }
@@ -1007,8 +1025,17 @@ __global__ void __launch_bounds__(kNT, 1) k_cox(const CoxArgs* __restrict__ fits
                         }
                     }
                     // ---- the coordinate step (ccdUpdateBeta :1394-1413, applyBounds :1503-1520)
-                    g -= c_xjy[q];                        // :1181-1183
+                    // A column that is constant in every risk set has g = h = 0, which
+                    // these sums give to their rounding only (A / D is x there where it is
+                    // formed), and -g / h of two such numbers is any step.  Their scales:
+                    // sum v S1, and sum v x S1 or, for values, its bound (sum v S1)^2 / events.
                     if (lane == 0) {
+                        const double sum = g;
+                        g -= c_xjy[q];                    // :1181-1183
+                        const double near = kZero * (fabs(sum) + fabs(c_xjy[q]));
+                        if (fabs(g) <= near && near <= 1e300 &&
+                            h <= kZero * (c_m[q].cv ? sum * sum * s_per_event : fabs(sum)))
+                            g = h = 0.0;
                         if (A.score) {
                             s_dl = 0.0;
                             if (rank == 0) A.score[base + q] = fabs(g);
@@ -1234,7 +1261,7 @@ void CoxSlots::build(CoxShape s, const double* d_w, cudaStream_t stream) {
     rowslot.alloc(K); rpart.alloc(C + 1); spart.alloc(C + 1);
     split.alloc((size_t)ds.J * (C + 1));
     entry.alloc(std::max<long long>(1, ds.nnz_idx));
-    flag.alloc(positions()); n.alloc(positions());
+    flag.alloc(positions()); n.alloc(positions()); per_event.alloc(1);
     // positions past the slots read as empty
     CYC_CHECK_CUDA(cudaMemsetAsync(n.get(), 0, n.bytes(), stream));
     CYC_CHECK_CUDA(cudaMemsetAsync(flag.get(), 0, flag.bytes(), stream));
@@ -1245,6 +1272,7 @@ void CoxSlots::build(CoxShape s, const double* d_w, cudaStream_t stream) {
            rpart.get());
     launch(k_slots, grid_for(32ll * events, 1), kThreads, 0, stream, C, threads, shape.per_cta, G,
            (const int*)spart.get(), (const int*)first.get(), d_w, (const double*)ds.d_y.get(), flag.get(), n.get());
+    launch(k_per_event, 1, 1024, 0, stream, (int)positions(), (const double*)n.get(), per_event.get());
     launch(k_row_slots, grid_for(K, 1), kThreads, 0, stream, K, C, threads, n_slots, G, (const int*)spart.get(),
            (const int*)sstr.get(), (const int*)ds.d_strat.get(), rowslot.get());
     if (ds.nnz_idx)
@@ -1283,7 +1311,7 @@ CoxArgs CoxSlots::args() const {
     a.strat = ds.d_strat.get();
     a.split = split.get(); a.rpart = rpart.get(); a.spart = spart.get();
     a.flag = flag.get();
-    a.n = n.get(); a.y = ds.d_y.get();
+    a.n = n.get(); a.per_event = per_event.get(); a.y = ds.d_y.get();
     a.wait = wait_limit(ds.K);
     return a;
 }

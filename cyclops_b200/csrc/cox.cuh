@@ -34,7 +34,7 @@ struct CoxSlots {
     DevBuf<int> first, glo, gend, gstr, gcum, groups;      // the event groups
     DevBuf<int> lo, end, sstr, rowslot, rpart, spart, split, entry;
     DevBuf<unsigned char> flag;    // [C][per_cta] bit 0: the slot starts its stratum, bit 1: it ends it
-    DevBuf<double> n;              // [C][per_cta] events
+    DevBuf<double> n, per_event;   // [C][per_cta] events; 1 / their sum
 
     explicit CoxSlots(Dataset& d) : ds(d) {}
     // the event groups and the number of slots for row weights d_w (K, device)
@@ -75,6 +75,7 @@ struct CoxArgs {
     const int* spart;              // C+1 slot boundaries
     const unsigned char* flag;
     const double* n;
+    const double* per_event;
     double *d, *S1, *S2, *bp;
     const double* y;
     const double* w;               // K
