@@ -72,6 +72,7 @@ _SIGS = {
     "cyc_dataset_destroy": [C.c_void_p],
     "cyc_dataset_info": [C.c_void_p, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_longlong),
                          C.POINTER(C.c_size_t)],
+    "cyc_dataset_set_sharing": [C.c_void_p, C.c_int],
     "cyc_engine_create": [C.c_void_p, C.POINTER(C.c_void_p)],
     "cyc_engine_destroy": [C.c_void_p],
     "cyc_engine_clone": [C.c_void_p, C.POINTER(C.c_void_p)],

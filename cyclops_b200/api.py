@@ -114,6 +114,12 @@ class Dataset:
         N.check(N.lib().cyc_dataset_info(self.handle, C.byref(K), C.byref(J), C.byref(nnz), C.byref(b)))
         return {"K": K.value, "J": J.value, "nnz": nnz.value, "device_bytes": b.value}
 
+    def share(self, calls: int) -> "Dataset":
+        """`calls` fits are expected to run on the device at once, each in a
+        call of its own: size this dataset's fits so that they run side by side."""
+        N.check(N.lib().cyc_dataset_set_sharing(self.handle, int(calls)))
+        return self
+
     def close(self):
         if getattr(self, "handle", None):
             N.lib().cyc_dataset_destroy(self.handle)

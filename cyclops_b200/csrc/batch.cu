@@ -2228,7 +2228,7 @@ Grouping group_size(Dataset& ds, cudaStream_t stream, int F, const cyc_prior& pr
     const GroupShape gs = swindle ? GroupShape{default_cluster(ds.K), 256} : group_shape(ds.K, (F + 7) / 8);
     const double waves8 = gs.threads == 512 ? 0.85 : std::ceil((double)((F + 7) / 8) * gs.C / (2.0 * 148));
     if (one.cycle_us > 0.8 * (3.0 * ds.J + 0.0025 * visits) * waves8) return {8, one};
-    if (!large || swindle) return {1, one};
+    if (!large || swindle) return {1, ds.share > 1 ? ccd_shape(ds, F + ds.share - 1) : one};
     const bool varied = std::any_of(specs, specs + F, [&](const cyc_fit_spec& s) { return s.variance != specs[0].variance; });
     const TuneKey key{ds.model, ds.K, ds.J, F, varied, ctl.precision, d_fold ? n_folds : 0, fixed_cols, ds.nnz_idx};
     {
@@ -2386,7 +2386,7 @@ void run_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* specs, i
     for (int i = 0; i < prior->n_exclude; ++i) ptype[prior->exclude[i]] = CYC_PRIOR_NONE;
     const bool swindle = ctl->use_kkt_swindle && std::count(ptype.begin(), ptype.end(), (int)CYC_PRIOR_LAPLACE) > 0;
     const Grouping by = [&] {
-        if (!can8) return Grouping{1, ccd_shape(ds, F)};
+        if (!can8) return Grouping{1, ccd_shape(ds, F + ds.share - 1)};
         NvtxRange range("cyclops batch: group choice");
         return group_size(ds, stream, F, *prior, specs, beta, hd, d_fold, n_folds, fit_fold, *ctl, fixed_cols, swindle);
     }();

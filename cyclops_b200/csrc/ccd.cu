@@ -735,6 +735,9 @@ static int resident_fits(int C, int threads, size_t dyn) {
 // of one team, 35 to 38 with clusters; 100k rows, 600 Zipf columns and 4 dense
 // ones: 150 ms for 40 cycles with one CTA, 38 with four, 25 with sixteen; 80
 // CV fits of 100k rows: 19 ms with one team, 29 with two.)
+// Callers add the calls that share the device to F: 8 fits of 500k rows, one a
+// call and all at once, take 214 ms with the 16 CTAs that are best alone (102 ms) and
+// 150 with 8 (125 alone); 16 fits 346 and 315.
 CcdShape ccd_shape(const Dataset& ds, int F, int only, bool varied) {
     only = std::min(only, kCcdCluster);
     struct { int C; double cross; } sizes[] = {{1, 0.0}, {2, 0.19}, {3, 0.2}, {4, 0.2}, {5, 0.25},

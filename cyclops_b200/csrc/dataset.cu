@@ -414,3 +414,11 @@ extern "C" int cyc_dataset_info(const cyc_dataset* ds, int* K, int* J, long long
         if (bytes) *bytes = ds->ds.device_bytes();
     });
 }
+
+extern "C" int cyc_dataset_set_sharing(cyc_dataset* ds, int calls) {
+    return guarded([&] {
+        CYC_REQUIRE(ds, CYC_ERR_ARGUMENT, "null dataset");
+        CYC_REQUIRE(calls >= 1, CYC_ERR_ARGUMENT, "at least one call uses the device");
+        ds->ds.share = calls;
+    });
+}

@@ -182,7 +182,7 @@ struct FitRunner {
 
     void prepare_ccd() {
         Dataset& ds = *e.ds;
-        const CcdShape shape = ccd_shape(ds, 1);
+        const CcdShape shape = ccd_shape(ds, ds.share);
         by_column = long_columns(ds, shape);
         rpart = ccd_rows(ds, shape.C);
         d_rpart.alloc(shape.C + 1); d_split.alloc((size_t)J * (shape.C + 1)); d_cols.alloc(J); d_ncols.alloc(1);

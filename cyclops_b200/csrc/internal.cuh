@@ -273,6 +273,7 @@ struct Dataset {
     size_t device_bytes() const;
     void ensure_csr();
     void ensure_entry_strata();
+    int share = 1;                   // calls expected on the device at once (cyc_dataset_set_sharing)
     int n_event_rows = -1;
     int event_rows();                // rows with a nonzero outcome (counted once)
 };

@@ -104,7 +104,7 @@ class Server:
     def _run_job(self, job: List[Request], admitted: float, t0: float) -> List[Response]:
         out = []
         try:
-            ds = api.Dataset(job[0].data, self.device)
+            ds = api.Dataset(job[0].data, self.device).share(self.slots)
             try:
                 if len(job) == 1 and not _persistent_ok(job[0]):
                     r = job[0]

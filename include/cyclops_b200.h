@@ -114,6 +114,12 @@ int cyc_dataset_create(const cyc_data_desc* desc, int device, cyc_dataset** out)
 int cyc_dataset_destroy(cyc_dataset* ds);
 /* rows, columns, stored indices, device bytes held */
 int cyc_dataset_info(const cyc_dataset* ds, int* K, int* J, long long* nnz, size_t* device_bytes);
+/* How many calls of cyc_fit or cyc_batch_fit, on this and other datasets, are
+ * expected to run on the device at once (default 1).  A fit that has the device
+ * to itself takes up to 16 SMs, and not many such fits run side by side; with
+ * `calls` > 1 fits take what lets that many.  Set before the fits; the
+ * results depend on it by the rounding of sums alone. */
+int cyc_dataset_set_sharing(cyc_dataset* ds, int calls);
 
 /* ---- engine: the AbstractModelSpecifics surface ------------------------- */
 
