@@ -1179,6 +1179,8 @@ __global__ void k_fold_to_i8(int K, const int* __restrict__ fold, signed char* _
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x) out[k] = (signed char)fold[k];
 }
 
+const KernelFile g_kernels((const void*)(&k_fold_to_i8));
+
 // per fit: log likelihood under its training weights (getLogLikelihood,
 // ModelSpecifics.hpp:605-650) and, for a CV grid, the predictive log
 // likelihood of its held-out rows (getPredictiveLogLikelihood, :652-690 with

@@ -687,6 +687,8 @@ __global__ void k_entry_folds(long long n, const int* __restrict__ idx, const si
         out[e] = fold[idx[e]];
 }
 
+const KernelFile g_kernels((const void*)(&k_entry_folds));
+
 }  // namespace
 
 template <class T>

@@ -192,6 +192,8 @@ __global__ void k_group_rows(const int* __restrict__ groups, const int* __restri
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < E; e += gridDim.x * blockDim.x)
         glo[e] = e == 0 || gstr[e - 1] != gstr[e] ? strat_ptr[gstr[e]] : gend[e - 1] + 1;
 }
+
+const KernelFile g_kernels((const void*)(&k_group_rows));
 struct Pieces {                      // the slots of an event group
     const int *groups, *glo, *gend;
     __device__ int operator()(int e) const { return e < *groups ? (gend[e] - glo[e]) / kSlotRows + 1 : 0; }

@@ -19,6 +19,8 @@
 
 namespace cyc {
 
+const KernelFile g_kernels((const void*)(&k_set_kw));
+
 Engine::Engine(Dataset* d) : ds(d), device(d->device) {
     CYC_CHECK_CUDA(cudaSetDevice(ds->device));
     CYC_CHECK_CUDA(cudaStreamCreateWithFlags(&own.s, cudaStreamNonBlocking));

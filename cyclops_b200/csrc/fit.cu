@@ -34,6 +34,8 @@ __global__ void k_fill(int n, double v, double* __restrict__ out) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = v;
 }
 
+const KernelFile g_kernels((const void*)(&k_fill));
+
 __global__ void k_copy(int K, const double* __restrict__ src, double* __restrict__ dst) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x) dst[k] = src[k];
 }

@@ -50,6 +50,8 @@ __global__ void k_iota(long long n, int* out) {
         out[i] = (int)i;
 }
 
+const KernelFile g_kernels((const void*)(&k_iota));
+
 // position of each covariate row's outcome: the last of the outcome rows
 // with its rowId (okey sorted, opos their positions, ascending within a
 // run of equal keys), -1 when there is none

@@ -92,6 +92,11 @@ int guarded(F&& f) {
 // Without a scope a buffer falls back to cudaMalloc / cudaFree.
 cudaStream_t& alloc_stream();          // per thread
 void prepare_pool(int device);         // keeps freed memory cached in the device's pool
+// Each source file names one of its kernels, by which all of them can be loaded
+// (load_kernels, dataset.cu).
+struct KernelFile {
+    explicit KernelFile(const void* kernel);
+};
 
 struct StreamScope {
     cudaStream_t prev;

@@ -73,6 +73,8 @@ __global__ void k_gh_independent_noalloc(ColView c, const double* __restrict__ e
     });
 }
 
+const KernelFile g_kernels((const void*)(&k_gh_independent_noalloc<CYC_LR, true>));
+
 NoAllocScratch* scratch_for_current_device() {
     int dev = 0;
     CYC_CHECK_CUDA(cudaGetDevice(&dev));

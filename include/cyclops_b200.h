@@ -117,8 +117,10 @@ int cyc_dataset_info(const cyc_dataset* ds, int* K, int* J, long long* nnz, size
 /* How many calls of cyc_fit or cyc_batch_fit, on this and other datasets, are
  * expected to run on the device at once (default 1).  A fit that has the device
  * to itself takes up to 16 SMs, and not many such fits run side by side; with
- * `calls` > 1 fits take what lets that many.  Set before the fits; the
- * results depend on it by the rounding of sums alone. */
+ * `calls` > 1 fits take what lets that many, and the library's kernels are
+ * loaded at once (0.55 s, the first time on a device) rather than at their first
+ * launch, where a caller would wait for the others' fits.  Set before the fits;
+ * the results depend on it by the rounding of sums alone. */
 int cyc_dataset_set_sharing(cyc_dataset* ds, int calls);
 
 /* ---- engine: the AbstractModelSpecifics surface ------------------------- */
