@@ -1668,6 +1668,18 @@ struct Grouping {
     CcdShape one;
 };
 
+// The runs of the columns not held fixed, planned once per dataset and fixed set.
+// `local`: a fit's predictors fit one CTA's shared memory.
+static std::shared_ptr<const CcdRuns> runs_of(Dataset& ds, const std::vector<int>& fixed, const std::vector<int>& cols) {
+    std::lock_guard<std::mutex> lock(ds.csr_mutex);
+    for (auto& p : ds.disjoint_runs)
+        if (p.first == fixed) return p.second;
+    auto plan = std::make_shared<const CcdRuns>(ccd_runs(ds, cols, ds.K * sizeof(double) <= 200 * 1024));
+    if (ds.disjoint_runs.size() >= 8) ds.disjoint_runs.erase(ds.disjoint_runs.begin());
+    ds.disjoint_runs.emplace_back(fixed, plan);
+    return plan;
+}
+
 template <class T>
 struct BatchRunner {
     Dataset& ds;
@@ -1684,6 +1696,9 @@ struct BatchRunner {
     DevBuf<unsigned char> d_lfix;
     // one-fit groups (ccd.cu): threads a CTA, the column lists and the moving steps per column
     int threads = 0, teams = 1;
+    bool runs = false;                       // the columns in runs (ccd_runs)
+    std::shared_ptr<const CcdRuns> plan;
+    DevBuf<unsigned char> d_runs;
     DevBuf<int> d_cols, d_ncols, d_out;
     DevBuf<unsigned> d_upd;
     std::vector<std::vector<int>> lists;     // one for all fits, or one a fit (active-set passes)
@@ -1699,6 +1714,7 @@ struct BatchRunner {
             C = by.one.C;
             threads = by.one.threads;
             teams = by.one.teams;
+            runs = by.one.runs;
         } else {
             C = C_ > 0 ? std::min(kMaxC, C_) : default_cluster(K);
         }
@@ -1747,6 +1763,12 @@ struct BatchRunner {
             all_cols = lists[0];
             unit_weights = !d_fold && std::all_of(specs, specs + F, [](const cyc_fit_spec& sp) { return !sp.weights; });
             upload_lists();
+            if (runs && !all_cols.empty()) {
+                plan = runs_of(ds, fixed_cols, all_cols);
+                d_runs.alloc(plan->len.size());
+                CYC_CHECK_CUDA(cudaMemcpyAsync(d_runs.get(), plan->len.data(), plan->len.size(), cudaMemcpyHostToDevice,
+                                               stream));
+            }
             d_upd.alloc((size_t)Fp * J);
             CYC_CHECK_CUDA(cudaMemsetAsync(d_upd.get(), 0, (size_t)Fp * J * sizeof(unsigned), stream));
             if (model_grouped(ds.model)) ds.ensure_entry_strata();
@@ -1891,6 +1913,7 @@ struct BatchRunner {
         CcdArgs a{};
         a.model = ds.model; a.K = ds.K; a.J = ds.J; a.S = ds.S; a.F = F; a.C = C;
         a.threads = threads; a.teams = teams;
+        a.runs = lists.size() == 1 ? d_runs.get() : nullptr;     // (active-set passes have lists of their own)
         a.weights = d_fold ? 1 : (unit_weights ? 0 : 2);
         a.fmt = ds.d_fmt.get(); a.col_ptr = ds.d_col_ptr.get(); a.val_ptr = ds.d_val_ptr.get();
         a.idx = ds.d_idx.get(); a.val = ds.d_val.get(); a.entry_strat = ds.d_entry_strat.get();
@@ -2388,7 +2411,19 @@ void run_batch(Dataset& ds, const cyc_prior* prior, const cyc_fit_spec* specs, i
     for (int i = 0; i < prior->n_exclude; ++i) ptype[prior->exclude[i]] = CYC_PRIOR_NONE;
     const bool swindle = ctl->use_kkt_swindle && std::count(ptype.begin(), ptype.end(), (int)CYC_PRIOR_LAPLACE) > 0;
     const Grouping by = [&] {
-        if (!can8) return Grouping{1, ccd_shape(ds, F + ds.share - 1)};
+        if (!can8) {
+            CcdShape one = ccd_shape(ds, F + ds.share - 1);
+            // very short columns: in runs of disjoint ones where that is faster
+            if (model_independent(ds.model) && !swindle && !std::getenv("CYC_BATCH_CLUSTER") &&
+                ds.nnz_idx <= 256ll * J) {
+                std::vector<int> cols;
+                for (int j = ds.has_offset ? 1 : 0; j < J; ++j)
+                    if (!std::binary_search(fixed_cols.begin(), fixed_cols.end(), j)) cols.push_back(j);
+                const double us = cols.empty() ? one.cycle_us : runs_of(ds, fixed_cols, cols)->cycle_us;
+                if (us < 0.9 * one.cycle_us) one = CcdShape{1, 256, 1, 1, us, true};
+            }
+            return Grouping{1, one};
+        }
         NvtxRange range("cyclops batch: group choice");
         return group_size(ds, stream, F, *prior, specs, beta, hd, d_fold, n_folds, fit_fold, *ctl, fixed_cols, swindle);
     }();

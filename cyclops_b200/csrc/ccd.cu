@@ -45,6 +45,7 @@ constexpr int kR = 2;            // entries of a column a thread keeps in regist
 constexpr int kU = 4;            // further entries a thread has in flight
 constexpr int kCh = 128;         // coordinates staged at a time
 constexpr int kWarps = kCcdThreads / 32;
+constexpr int kRunRounds = 8;    // rounds of a warp over a column of a run
 
 // the row's mean under the model; a logistic row whose exp(xb) overflows is NaN
 // when `strict`, as exb / (1 + exb) is in the per-coordinate engine
@@ -112,6 +113,12 @@ __device__ __forceinline__ void bar_arrive(int id, int n) {
 // which the column before changes much more often (20k matched rows: 7.1 ms
 // with one team, 9.2 with two).
 //
+// TEAMS = 0 (independent rows, one CTA): runs of short columns that share no row
+// (ccd_runs) are taken at once, a warp a column: each sees the state that the
+// serial loop would show it, and a run costs one barrier.  The other columns go
+// as with one team.  63,000 columns of 3.5 entries over 3k rows: 0.16 us a column
+// against 0.65; 25,000 of 162 over 705k rows 0.47 against 0.97.
+//
 // A column's entries are dealt to the team's threads in rounds of NT; up to kR
 // rounds stay in registers from the gradient to the update.  The code of a
 // round is straight-line (one round and kR rounds as separate instances): with
@@ -124,7 +131,8 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
     const int C = A.C;
     const int rank = C > 1 ? (int)cluster.block_rank() : 0;
     const int f = blockIdx.x / C;
-    constexpr int kTeams = TEAMS;
+    constexpr bool kRuns = TEAMS == 0;
+    constexpr int kTeams = kRuns ? 1 : TEAMS;
     const int NT = blockDim.x / kTeams, NW = NT >> 5;
     const int lane = threadIdx.x & 31;
     const int team = threadIdx.x >= NT, tid = threadIdx.x - team * NT, warp = tid >> 5;
@@ -156,6 +164,7 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
     __shared__ ColStep c_s[kCh];
     __shared__ double c_ob[kCh], c_oh[kCh];
     __shared__ int c_j[kCh], c_up[kCh];
+    __shared__ unsigned char c_len[kRuns ? kCh : 1];   // runs by place
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     T* const sx = reinterpret_cast<T*>(dyn_smem);
     auto get = [&](int k) -> T { return SM ? sx[k] : xg[k]; };
@@ -337,6 +346,7 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
                     p.s = sgn(beta);
                 }
                 c_s[q] = p;
+                if (kRuns) c_len[q] = A.runs[base + q];
             }
             __syncthreads();
             // the team's next column and its first kR rounds, as loaded (nothing
@@ -363,17 +373,105 @@ __global__ void __launch_bounds__(kCcdThreads, 1) k_ccd(const CcdArgs A) {
                     }
                 }
             };
+            int nq = -1;                         // the column loaded (runs)
             auto prefetch = [&](int q) {
                 nm = c_m[q];
+                nq = q;
                 fetch(0);
                 if (nm.n > NT) {
                     #pragma unroll
                     for (int r = 1; r < kR; ++r) fetch(r);
                 }
             };
+            // a run: this warp's column of it, as loaded
+            int rk[kRunRounds], rf[kRunRounds], rq = -1;
+            double rx[kRunRounds];
+            auto load_run = [&](int q) {
+                rq = q;
+                const int L = q < jn ? c_len[kRuns ? q : 0] : 0;
+                const bool mine = L > 1 && warp < L;
+                const ColMeta m = c_m[mine ? q + warp : jn];
+                #pragma unroll
+                for (int r = 0; r < kRunRounds; ++r) {
+                    const int i = lane + 32 * r;
+                    rk[r] = -1;
+                    rx[r] = 1.0;
+                    rf[r] = 0;
+                    if (i < m.n) {
+                        rk[r] = __ldg(m.ci + i);
+                        if (m.cv) rx[r] = __ldg(m.cv + i);
+                        if (WM == 1) rf[r] = (int)__ldg(m.ef + i);
+                    }
+                }
+            };
+            auto run = [&](int q, int L) {
+                if (rq != q) load_run(q);
+                int kk[kRunRounds], ff[kRunRounds];
+                double x8[kRunRounds];
+                #pragma unroll
+                for (int r = 0; r < kRunRounds; ++r) { kk[r] = rk[r] - r0; x8[r] = rx[r]; ff[r] = rf[r]; }
+                load_run(q + L);
+                auto column = [&](auto rounds) {
+                    constexpr int R = decltype(rounds)::value;
+                    const ColStep p = c_s[q + warp];
+                    const bool ind = c_m[q + warp].cv == nullptr;
+                    T vv[R], xx[R];
+                    Kahan<T> ag, ah;
+                    #pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        xx[r] = (T)x8[r];
+                        vv[r] = kk[r] >= 0 ? get(kk[r]) : T(0);
+                    }
+                    #pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const T w = kk[r] < 0 ? T(0) : (WM == 1 ? weight.by_fold(ff[r]) : weight(kk[r]));
+                        const bool on = WM == 2 && strict ? kk[r] >= 0 : w != T(0);
+                        T gi, hi;
+                        mean_terms<T, MODEL>(fit_mean<T, MODEL>(vv[r], strict), xx[r], WM == 2 ? w : T(1), ind, gi, hi);
+                        ag.add(on ? gi : T(0));
+                        ah.add(on ? hi : T(0));
+                    }
+                    const bool up = (lane & 16) != 0;
+                    const double a = ag.value(), b = ah.value();
+                    double v = up ? b : a;
+                    v += __shfl_xor_sync(full, up ? a : b, 16);
+                    v += __shfl_xor_sync(full, v, 8);
+                    v += __shfl_xor_sync(full, v, 4);
+                    v += __shfl_xor_sync(full, v, 2);
+                    v += __shfl_xor_sync(full, v, 1);
+                    const double g = __shfl_sync(full, v, 0), h = __shfl_sync(full, v, 16);
+                    const double dl = step(p, g - p.xjy, h);
+                    if (lane == 0) {
+                        c_oh[q + warp] = next_bound(p.bound, dl);
+                        c_ob[q + warp] = dl != 0.0 ? p.beta + dl : p.beta;
+                        c_up[q + warp] = dl != 0.0;
+                    }
+                    if (dl != 0.0) {
+                        #pragma unroll
+                        for (int r = 0; r < R; ++r)
+                            if (kk[r] >= 0) put(kk[r], vv[r] + (T)dl * xx[r]);
+                    }
+                };
+                if (warp < L) {
+                    const int n = c_m[q + warp].n;
+                    if (n <= 32) column(std::integral_constant<int, 1>{});
+                    else if (n <= 96) column(std::integral_constant<int, 3>{});
+                    else column(std::integral_constant<int, kRunRounds>{});
+                }
+                __syncthreads();
+            };
             const int first = kTeams == 2 ? team ^ off : 0;
             prefetch(min(first, jn));
             for (int q = first; q < jn; q += kTeams) {
+                if constexpr (kRuns) {
+                    const int L = c_len[q];
+                    if (L > 1) {
+                        run(q, L);
+                        q += L - 1;
+                        continue;
+                    }
+                    if (nq != q) prefetch(q);
+                }
                 const ColMeta m = nm;
                 const bool ind = m.cv == nullptr;
                 const ColStep p = c_s[q];
@@ -657,14 +755,18 @@ void launch_rows(CcdArgs a, const std::vector<int>& rpart, cudaStream_t stream) 
     const size_t bytes = (size_t)rows * sizeof(T);
     const char* xs = std::getenv("CYC_BATCH_XB_SMEM");      // 0: global memory
     const bool fits = bytes <= kRowBytes && !(xs && std::atoi(xs) == 0);
-    constexpr bool two = sizeof(T) == 8 && (MODEL == CYC_LR || MODEL == CYC_PR);
+    constexpr bool rows1 = MODEL == CYC_LR || MODEL == CYC_PR, two = sizeof(T) == 8 && rows1;
     if constexpr (sizeof(T) == 8) {
         if (fits) {
             if constexpr (two) {
+                if (a.runs) return launch_one<T, MODEL, WM, true, 0>(a, bytes, stream);
                 if (a.teams == 2) return launch_one<T, MODEL, WM, true, 2>(a, bytes, stream);
             }
             return launch_one<T, MODEL, WM, true, 1>(a, bytes, stream);
         }
+    }
+    if constexpr (rows1) {
+        if (a.runs) return launch_one<T, MODEL, WM, false, 0>(a, 0, stream);
     }
     if constexpr (two) {
         if (a.teams == 2) return launch_one<T, MODEL, WM, false, 2>(a, 0, stream);
@@ -770,15 +872,55 @@ CcdShape ccd_shape(const Dataset& ds, int F, int only, bool varied) {
             if (best.cycle_us == 0.0 || us < best.cycle_us) best = {C, kind.threads, kind.teams, slots, us};
         }
     }
-    // CYC_BATCH_CLUSTER="CTAs[,threads[,teams]]" fixes the shape
+    // CYC_BATCH_CLUSTER="CTAs[,threads[,teams]]" fixes the shape (teams 0: runs)
     if (const char* e = std::getenv("CYC_BATCH_CLUSTER")) {
         int c = best.C, t = best.threads, n = best.teams;
         std::sscanf(e, "%d,%d,%d", &c, &t, &n);
         best.C = std::max(1, std::min(kCcdCluster, c));
         best.teams = n == 2 && model_independent(ds.model) ? 2 : 1;
         best.threads = std::max(64, std::min(kCcdThreads, t / 64 * 64));
+        best.runs = n == 0 && model_independent(ds.model);
+        if (best.runs) { best.C = 1; best.threads = kCcdThreads; }       // a warp for each column of a run
     }
     return best;
+}
+
+CcdRuns ccd_runs(const Dataset& ds, const std::vector<int>& cols, bool local) {
+    CcdRuns r{std::vector<unsigned char>(cols.size(), 1), 0.0};
+    std::vector<int> seen(ds.K, -1);             // the last run with the row
+    int start = 0, id = -1;
+    auto close = [&](int end) {
+        const int len = end - start;
+        for (int i = start; i < end; ++i) r.len[i] = i == start ? (unsigned char)len : 0;
+        long long n = 0;                         // the longest column
+        for (int i = start; i < end; ++i) n = std::max(n, ds.col_len(cols[i]));
+        if (len > 1) {
+            r.cycle_us += n <= 32 ? (local ? 1.15 : 1.5) : n <= 96 ? (local ? 1.4 : 1.9) : (local ? 2.0 : 3.0);
+        } else if (len == 1) {
+            const double rounds = std::ceil((double)n / kCcdThreads);
+            r.cycle_us += (local ? 1.05 : 1.35) + (local ? 0.5 : 0.7) * std::max(0.0, rounds - 1.0);
+        }
+        start = end;
+    };
+    for (int i = 0; i < (int)cols.size(); ++i) {
+        const int j = cols[i], f = ds.fmt[j];
+        const bool fits = (f == CYC_SPARSE || f == CYC_INDICATOR) && ds.col_len(j) <= 32 * kRunRounds;
+        const int* rows = ds.h_idx.data() + ds.col_ptr[j];
+        const int n = fits ? (int)ds.col_len(j) : 0;
+        bool joins = fits && i > start && i % kCh != 0 && i - start < kWarps;
+        for (int e = 0; joins && e < n; ++e) joins = seen[rows[e]] != id;
+        if (!joins) {
+            close(i);
+            ++id;
+        }
+        for (int e = 0; e < n; ++e) seen[rows[e]] = id;
+        if (!fits) {                             // a run by itself
+            close(i + 1);
+            ++id;
+        }
+    }
+    close((int)cols.size());
+    return r;
 }
 
 std::vector<int> ccd_rows(const Dataset& ds, int C) {

@@ -16,6 +16,7 @@ struct CcdArgs {
     int model, K, J, S, F, C;
     int threads;                  // per CTA, a multiple of 64 up to kCcdThreads
     int teams;                    // 2: the CTA's threads take the columns in two teams (lr, pr)
+    const unsigned char* runs;    // null, or by place in `cols`: columns of the run that starts there (ccd_runs; C 1, teams 1)
     int weights;                  // 0: all ones; 1: CV folds; 2: `w`
     int strict;                   // as the per-coordinate engine: a logistic row whose exb overflows is NaN,
                                   // and a row of weight zero that is NaN or infinite makes the sums NaN
@@ -63,6 +64,7 @@ struct CcdArgs {
 struct CcdShape {
     int C, threads, teams, slots;
     double cycle_us;
+    bool runs = false;            // take the columns in runs (ccd_runs)
 };
 CcdShape ccd_shape(const Dataset& ds, int F, int C = 0, bool varied = false);
 // cycles' worth of time that F fits take where `slots` run at a time: whole
@@ -72,6 +74,16 @@ inline double ccd_turns(int F, int slots, bool varied) {
     if (F <= slots) return 1.0;
     return varied ? (double)F / slots : (double)((F + slots - 1) / slots);
 }
+// Runs of at most 8 columns, next to one another in `cols`, that share no row: by
+// place, the length of the run that starts there (0 inside one).  `local`: the
+// predictors are in shared memory.  Also the modelled time of a cycle: a run by its
+// longest column, a column alone by its rounds, as measured on designs of 1k to
+// 900k rows (3 to 200 entries a column: 0.16 to 0.7 us a column).
+struct CcdRuns {
+    std::vector<unsigned char> len;
+    double cycle_us;
+};
+CcdRuns ccd_runs(const Dataset& ds, const std::vector<int>& cols, bool local);
 // row boundaries of C CTAs, at stratum starts for grouped models
 std::vector<int> ccd_rows(const Dataset& ds, int C);
 // the split of every column's entries over those boundaries

@@ -5,6 +5,7 @@
 #include <nvtx3/nvToolsExt.h>
 #include <cstdint>
 #include <cstdio>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -209,6 +210,7 @@ struct ColView {
 // ---------------------------------------------------------------------------
 // column batches of the batched solver (planned on the host, batch.cu)
 // ---------------------------------------------------------------------------
+struct CcdRuns;                  // ccd.cuh
 struct RunPlan {
     int C = 0, threads = 0;
     int cap = 0, dmax = 0, max_levels = 0;   // the batch shape it was planned with (short-column
@@ -260,6 +262,9 @@ struct Dataset {
     // stratum of every entry of d_idx (grouped models), built on first use
     bool have_entry_strata = false;
     DevBuf<int> d_entry_strat;
+
+    // runs of disjoint short columns (ccd_runs), per set of fixed columns
+    std::vector<std::pair<std::vector<int>, std::shared_ptr<const CcdRuns>>> disjoint_runs;
 
     // column batches of the batched solver, cached per cluster size and shape
     std::vector<RunPlan> run_plans;
