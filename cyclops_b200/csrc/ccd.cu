@@ -756,22 +756,18 @@ void launch_rows(CcdArgs a, const std::vector<int>& rpart, cudaStream_t stream) 
     const char* xs = std::getenv("CYC_BATCH_XB_SMEM");      // 0: global memory
     const bool fits = bytes <= kRowBytes && !(xs && std::atoi(xs) == 0);
     constexpr bool rows1 = MODEL == CYC_LR || MODEL == CYC_PR, two = sizeof(T) == 8 && rows1;
-    if constexpr (sizeof(T) == 8) {
-        if (fits) {
-            if constexpr (two) {
-                if (a.runs) return launch_one<T, MODEL, WM, true, 0>(a, bytes, stream);
-                if (a.teams == 2) return launch_one<T, MODEL, WM, true, 2>(a, bytes, stream);
-            }
-            return launch_one<T, MODEL, WM, true, 1>(a, bytes, stream);
+    auto with = [&](auto smem, size_t dyn) {
+        constexpr bool SM = decltype(smem)::value;
+        if constexpr (rows1) {
+            if (a.runs) return launch_one<T, MODEL, WM, SM, 0>(a, dyn, stream);
         }
-    }
-    if constexpr (rows1) {
-        if (a.runs) return launch_one<T, MODEL, WM, false, 0>(a, 0, stream);
-    }
-    if constexpr (two) {
-        if (a.teams == 2) return launch_one<T, MODEL, WM, false, 2>(a, 0, stream);
-    }
-    launch_one<T, MODEL, WM, false, 1>(a, 0, stream);
+        if constexpr (two) {
+            if (a.teams == 2) return launch_one<T, MODEL, WM, SM, 2>(a, dyn, stream);
+        }
+        launch_one<T, MODEL, WM, SM, 1>(a, dyn, stream);
+    };
+    if (fits) with(std::true_type{}, bytes);
+    else with(std::false_type{}, 0);
 }
 
 template <class T, int MODEL>
