@@ -385,7 +385,7 @@ def leg_poisson(api):
     out["persistent_fit"] = {
         "cycles": fit.iterations, "return_flag": fit.return_flag, "cycle_cap": cap, "seconds": wall,
         "kernel_ms": st["kernel_ms"], "seconds_per_cycle": st["kernel_ms"] / 1000.0 / max(1, fit.iterations),
-        "roofline": roofline_of(st["phase_bytes"][0], st["phase_ms"][0], "k_batch<double,PR,1> (one fit)")}
+        "roofline": roofline_of(st["phase_bytes"][0], st["phase_ms"][0], "k_ccd<double,PR> (one fit)")}
     api.fit_cyclops_model(ds, prior, api.create_control(max_iterations=1))
     f2 = api.fit_cyclops_model(ds, prior, api.create_control(max_iterations=2))
     st2 = api.last_run_stats()
@@ -435,7 +435,7 @@ def leg_cox(api, n_strata=0, whole_fit=True, columns=0):
                          "kernel_ms": st["kernel_ms"], "seconds_per_cycle": spc,
                          "update_entries": st["update_entries"],
                          "roofline": roofline_of(st["phase_bytes"][0], st["kernel_ms"],
-                                                 "cyc_fit cox kernels (numerator, gradient, update, risk-set rescans)")}
+                                                 "k_cox (one cluster) and the risk sets' set-up")}
     sub = min(500, data.J)
     sd = _first_columns(data, sub)
     lib, kind = cpu_ref()

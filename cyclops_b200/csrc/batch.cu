@@ -208,7 +208,7 @@ __device__ __forceinline__ void store_row(T* p, const T (&v)[N]) {
 // here: the registers they take make the rest of the persistent kernel spill.
 template <class T, int G>
 struct RowLayout {
-    static constexpr int FPT = (G % 4 != 0) ? G : 4;
+    static constexpr int FPT = 4;
     static constexpr int TPR = G / FPT;
     // row parts in flight per thread when rows arrive by cp.async
     static constexpr int D = 4;
