@@ -107,6 +107,7 @@ __global__ void k_add_logprior(int J, const double* __restrict__ beta, const int
 // CYC_FIT_ROUTE: "columns" or "cluster".
 bool long_columns(const Dataset& ds, const CcdShape& shape) {
     if (const char* e = std::getenv("CYC_FIT_ROUTE")) return std::strcmp(e, "columns") == 0;
+    if (std::getenv("CYC_BATCH_CLUSTER")) return false;      // the caller's cluster
     const bool grouped = model_grouped(ds.model);
     const bool local = (double)ds.K / shape.C * sizeof(double) <= 200 * 1024;      // predictors in shared memory
     const double deal = (double)shape.C * shape.threads / shape.teams;
